@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
     cnt = min(a.n_ngb[s], a.cap);
   }
   const int kmax = warp_max_i(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double gam = a.gamma, alpha = a.alpha, beta = a.beta;
   const double wi = pi.w, hh = 0.5 * wi;
   const double ih = hh > 0 ? 1.0 / hh : 0.0, ih2 = ih * ih, ih5 = ih2 * ih2 * ih;
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
   double prb_i = 0, cb_i = 0, bb_i = 0, omb_i = 0, psib_i = 0;
   for (int k = 0; k < kmax; k++) {
     if (k >= cnt) continue;
-    const int j = __ldg(lst + (size_t)k * kLeaf);
+    const int j = __ldg(lst + k);
     if (j == s) continue;
     const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j), fj = ld4(a.aux + j);
     const double4 abj = ld4(a.ab + j);
@@ -703,7 +703,6 @@ __global__ void k_adj_vsig(AdjArgs a) {
   const double vsb = a.asc[2];
   const int s = (int)a.asc[3];
   if (vsb == 0 || s < 0 || s >= a.n) return;
-  const int leaf = s / kLeaf, lane = s % kLeaf;
   const int cnt = min(a.n_ngb[s], a.cap);
   const double4 pi = a.pos[s], vi = a.vpup[s], hi4 = a.hyd[s];
   const double gam = a.gamma, beta = a.beta;
@@ -711,13 +710,13 @@ __global__ void k_adj_vsig(AdjArgs a) {
   int kbest = -1;
   double best = -1e300;
   for (int k = 0; k < cnt; k++) {
-    const int j = a.list[((size_t)leaf * a.cap + k) * kLeaf + lane];
+    const int j = a.list[(size_t)s * a.stride + k];
     const double vs = pair_vs(a, s, j, c_i, pi, vi);
     if (vs > best) { best = vs; kbest = k; }
   }
   if (kbest < 0) return;
   {
-    const int j = a.list[((size_t)leaf * a.cap + kbest) * kLeaf + lane];
+    const int j = a.list[(size_t)s * a.stride + kbest];
     const double4 pj = a.pos[j], vj = a.vpup[j];
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
@@ -826,14 +825,14 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
     cnt = min(a.n_ngb[s], a.cap);
   }
   const int kmax = warp_max_i(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
   const double i2w = w > 0 ? 2.0 / w : 0.0;
   // forward sums: from the kept step when it recorded them, else summed again
   double R = 0, O = 0, Qs = 0, S = 0, Dv = 0, Cx = 0, Cy = 0, Cz = 0;
   for (int k = 0; k < (a.dsum ? 0 : kmax); k++) {
     if (k >= cnt) continue;
-    const int j = __ldg(lst + (size_t)k * kLeaf);
+    const int j = __ldg(lst + k);
     const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j);
     const double mj = __ldg(&a.vel[j].w);
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
@@ -896,7 +895,7 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
   double xbx = 0, xby = 0, xbz = 0, vbx = 0, vby = 0, vbz = 0;
   for (int k = 0; k < kmax; k++) {
     if (k >= cnt) continue;
-    const int j = __ldg(lst + (size_t)k * kLeaf);
+    const int j = __ldg(lst + k);
     if (j == s) continue;
     const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j);
     const double mj = __ldg(&a.vel[j].w);
@@ -951,13 +950,13 @@ __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
     wbar = a.xb[s].w;
   }
   const int kmax = warp_max_i(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
   const double i2w = w > 0 ? 2.0 / w : 0.0;
   double Fw = 0;
   for (int k = 0; k < kmax; k++) {
     if (k >= cnt) continue;
-    const int j = __ldg(lst + (size_t)k * kLeaf);
+    const int j = __ldg(lst + k);
     const double4 pj = ld4(a.pos + j);
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     Fw -= k_digdh<double>(sqrt(dx * dx + dy * dy + dz * dz) * i2w);
@@ -968,7 +967,7 @@ __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
   if (__any_sync(0xffffffffu, lam != 0)) {
     for (int k = 0; k < kmax; k++) {
       if (k >= cnt || lam == 0) continue;
-      const int j = __ldg(lst + (size_t)k * kLeaf);
+      const int j = __ldg(lst + k);
       if (j == s) continue;
       const double4 pj = ld4(a.pos + j);
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;

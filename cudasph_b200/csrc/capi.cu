@@ -22,12 +22,10 @@ int morton_keys(int n, const double4 *pos, const double *x, const double *y, con
 int peano_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
                double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st);
 int tree_layout(int n, TreeView *t);
-int build_tree(const TreeView &t, const double4 *pos, float4 *lo, float4 *hi, cudaStream_t st);
+int build_tree(const TreeView &t, const double4 *pos, float4 *lo, float4 *hi, float4 *pf, cudaStream_t st);
 int launch_solve_range(const TreeView &t, double4 *pos, int *nevals, unsigned *flags, const sph_params &p,
-                       int *n_ngb, int *list, double *dcache, int cap, void *work, int leaf0, int leaf1,
-                       cudaStream_t st);
-size_t solve_work_bytes(int n, int nleaf);
-int launch_find_ngb(const TreeView &t, const double4 *pos, int *n_ngb, int *list, int cap, unsigned *flags,
+                       int *n_ngb, int *list, int cap, int stride, int leaf0, int leaf1, cudaStream_t st);
+int launch_find_ngb(const TreeView &t, double4 *pos, int *n_ngb, int *list, int cap, int stride, unsigned *flags,
                     int leaf0, int leaf1, cudaStream_t st);
 int launch_density(const HydroArgs &a, cudaStream_t st);
 int launch_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsigned *flags, cudaStream_t st);
@@ -87,11 +85,10 @@ struct sph_ctx {
   int cur = 0;
   double4 *old = nullptr;
   int *n_ngb = nullptr, *nevals = nullptr, *list = nullptr;
-  int list_cap = 0;  // per particle
-  double *dcache = nullptr;  // candidate squared distances of the h solve, layout of list
-  char *solve_work = nullptr;  // queue and saved lane states between the h solve's two kernels
+  int list_cap = 0;     // per particle
+  int list_stride = 0;  // entries between two particles' rows (whole 32-byte sectors)
   TreeView tree;
-  float4 *tlo = nullptr, *thi = nullptr;
+  float4 *tlo = nullptr, *thi = nullptr, *tpf = nullptr;
   void *tgws = nullptr;  // tree-gravity workspace (radix tree + node moments)
   uint64_t *keys = nullptr;
   uint32_t *vals = nullptr;
@@ -188,15 +185,11 @@ int alloc_lists(sph_ctx *c) {
   int cap = c->p.ngb_cap > 0 ? c->p.ngb_cap : (int)(4 * c->p.n_target) + 32;
   if (cap == c->list_cap && c->list) return SPH_OK;
   if (c->list) cudaFree(c->list);
-  if (c->dcache) cudaFree(c->dcache);
   c->list = nullptr;
-  c->dcache = nullptr;
   c->list_cap = cap;
-  size_t entries = (size_t)c->tree.count[0] * kLeaf * (size_t)cap;
+  c->list_stride = (cap + 7) / 8 * 8;
   c->lists_ok = false;
-  int rc = dalloc(&c->list, entries);
-  if (!rc) rc = dalloc(&c->dcache, entries);
-  return rc;
+  return dalloc(&c->list, (size_t)c->n * c->list_stride);
 }
 
 int check_params(const sph_params *p) {
@@ -240,7 +233,7 @@ FieldRef field_ref(sph_ctx *c, int field) {
 // this context's leaves: all of them, or its shard's contiguous range
 void shard_leaves(const sph_ctx *c, int &leaf0, int &leaf1) {
   long long lo, hi;
-  shard_range(c->tree.count[0], c->rank, c->world, lo, hi);
+  shard_range(c->tree.nleaf, c->rank, c->world, lo, hi);
   leaf0 = (int)lo;
   leaf1 = (int)hi;
 }
@@ -249,8 +242,9 @@ HydroArgs hydro_args(sph_ctx *c) {
   Fields &F = c->f[c->cur];
   HydroArgs a;
   a.n = c->n;
-  a.nleaf = c->tree.count[0];
+  a.nleaf = c->tree.nleaf;
   a.cap = c->list_cap;
+  a.stride = c->list_stride;
   a.pos = F.pos; a.vel = F.vel; a.hyd = F.hyd; a.dd = F.dd; a.dots = F.dots; a.vsig = F.vsig;
   a.n_ngb = c->n_ngb; a.list = c->list; a.ngb_acc = nullptr; a.aux = c->aux; a.dsum = nullptr;
   a.alpha = c->p.av_alpha; a.beta = c->p.av_beta; a.gamma = c->p.gamma;
@@ -298,9 +292,9 @@ extern "C" int cudasph_destroy(sph_ctx *c) {
     cudaFree(F.pos); cudaFree(F.vel); cudaFree(F.hyd); cudaFree(F.dd); cudaFree(F.dots); cudaFree(F.grav);
     cudaFree(F.vsig); cudaFree(F.id);
   }
-  cudaFree(c->old); cudaFree(c->n_ngb); cudaFree(c->nevals); cudaFree(c->list); cudaFree(c->dcache);
-  cudaFree(c->tlo); cudaFree(c->thi); cudaFree(c->tgws); cudaFree(c->keys); cudaFree(c->vals); cudaFree(c->sort_scratch);
-  cudaFree(c->bbox_part); cudaFree(c->box4); cudaFree(c->aux); cudaFree(c->solve_work); cudaFree(c->gsrc); cudaFree(c->gh2); cudaFree(c->mass_mixed); cudaFree(c->xbuf); cudaFree(c->flags);
+  cudaFree(c->old); cudaFree(c->n_ngb); cudaFree(c->nevals); cudaFree(c->list);
+  cudaFree(c->tlo); cudaFree(c->thi); cudaFree(c->tpf); cudaFree(c->tgws); cudaFree(c->keys); cudaFree(c->vals); cudaFree(c->sort_scratch);
+  cudaFree(c->bbox_part); cudaFree(c->box4); cudaFree(c->aux); cudaFree(c->gsrc); cudaFree(c->gh2); cudaFree(c->mass_mixed); cudaFree(c->xbuf); cudaFree(c->flags);
   cudaFree(c->sc); cudaFree(c->fin_part); cudaFree(c->flat); cudaFree(c->slot_of);
   cudaFree(c->pre_acc); cudaFree(c->dsum); cudaFree(c->xb); cudaFree(c->vb); cudaFree(c->ab); cudaFree(c->vpb); cudaFree(c->vpup);
   cudaFree(c->rhob); cudaFree(c->Pb); cudaFree(c->omb); cudaFree(c->psib); cudaFree(c->divb); cudaFree(c->curlb);
@@ -354,6 +348,7 @@ extern "C" int cudasph_create(const sph_params *params, int n, int device, sph_c
   TRY_ALLOC(dalloc(&c->nevals, n));
   TRY_ALLOC(dalloc(&c->tlo, nodes));
   TRY_ALLOC(dalloc(&c->thi, nodes));
+  TRY_ALLOC(dalloc(&c->tpf, n));
   TRY_ALLOC(dalloc((char **)&c->tgws, tree_gravity_workspace_bytes(n)));
   TRY_ALLOC(dalloc(&c->keys, n));
   TRY_ALLOC(dalloc(&c->vals, n));
@@ -361,7 +356,6 @@ extern "C" int cudasph_create(const sph_params *params, int n, int device, sph_c
   TRY_ALLOC(dalloc(&c->bbox_part, 148 * 2 * 6));
   TRY_ALLOC(dalloc(&c->box4, 4));
   TRY_ALLOC(dalloc(&c->aux, n));
-  TRY_ALLOC(dalloc(&c->solve_work, solve_work_bytes(n, c->tree.count[0])));
   TRY_ALLOC(dalloc(&c->gsrc, n));
   TRY_ALLOC(dalloc(&c->gh2, n));
   TRY_ALLOC(dalloc(&c->mass_mixed, 1));
@@ -554,7 +548,7 @@ extern "C" int cudasph_get_neighbours(sph_ctx *c, int *counts, int64_t *offsets,
   if (!c || !counts || !offsets) return SPH_ERR_ARG;
   if (!c->lists_ok) return SPH_ERR_STATE;
   SPH_CUDA_TRY(cudaSetDevice(c->device));
-  const int n = c->n, cap = c->list_cap, nleaf = c->tree.count[0];
+  const int n = c->n, cap = c->list_cap;
   std::vector<int> ids(n), cnt(n);
   SPH_CUDA_TRY(cudaMemcpyAsync(ids.data(), c->f[c->cur].id, sizeof(int) * n, cudaMemcpyDeviceToHost, c->st));
   SPH_CUDA_TRY(cudaMemcpyAsync(cnt.data(), c->n_ngb, sizeof(int) * n, cudaMemcpyDeviceToHost, c->st));
@@ -563,14 +557,13 @@ extern "C" int cudasph_get_neighbours(sph_ctx *c, int *counts, int64_t *offsets,
   offsets[0] = 0;
   for (int i = 0; i < n; i++) offsets[i + 1] = offsets[i] + counts[i];
   if (!list) return SPH_OK;
-  std::vector<int> lst((size_t)nleaf * kLeaf * cap);
+  std::vector<int> lst((size_t)n * c->list_stride);
   SPH_CUDA_TRY(cudaMemcpyAsync(lst.data(), c->list, sizeof(int) * lst.size(), cudaMemcpyDeviceToHost, c->st));
   SPH_CUDA_TRY(cudaStreamSynchronize(c->st));
   for (int s = 0; s < n; s++) {
-    const int leaf = s / kLeaf, lane = s % kLeaf;
     const int m = cnt[s] < cap ? cnt[s] : cap;
     int64_t o = offsets[ids[s]];
-    for (int k = 0; k < m; k++) list[o + k] = ids[lst[((size_t)leaf * cap + k) * kLeaf + lane]];
+    for (int k = 0; k < m; k++) list[o + k] = ids[lst[(size_t)s * c->list_stride + k]];
   }
   return SPH_OK;
 }
@@ -617,9 +610,10 @@ extern "C" int cudasph_build_tree(sph_ctx *c) {
     if (rc) return rc;
   }
   PhaseScope ps(c, SPH_PH_TREE);
-  LAUNCHED(build_tree(c->tree, c->f[c->cur].pos, c->tlo, c->thi, c->st));
+  LAUNCHED(build_tree(c->tree, c->f[c->cur].pos, c->tlo, c->thi, c->tpf, c->st));
   c->tree.lo = c->tlo;
   c->tree.hi = c->thi;
+  c->tree.pf = c->tpf;
   c->tree_ok = true;
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
@@ -635,8 +629,8 @@ extern "C" int cudasph_solve_range(sph_ctx *c) {
   PhaseScope ps(c, SPH_PH_SOLVE);
   int leaf0, leaf1;
   shard_leaves(c, leaf0, leaf1);
-  LAUNCHED(launch_solve_range(c->tree, c->f[c->cur].pos, c->nevals, c->flags, c->p, c->n_ngb, c->list, c->dcache,
-                              c->list_cap, c->solve_work, leaf0, leaf1, c->st));
+  LAUNCHED(launch_solve_range(c->tree, c->f[c->cur].pos, c->nevals, c->flags, c->p, c->n_ngb, c->list,
+                              c->list_cap, c->list_stride, leaf0, leaf1, c->st));
   // the solve writes the neighbour lists at the final ranges (find_ngb fused)
   c->lists_ok = true;
   c->density_ok = false;
@@ -655,7 +649,8 @@ extern "C" int cudasph_find_ngb(sph_ctx *c) {
   PhaseScope ps(c, SPH_PH_FIND);
   int leaf0, leaf1;
   shard_leaves(c, leaf0, leaf1);
-  LAUNCHED(launch_find_ngb(c->tree, c->f[c->cur].pos, c->n_ngb, c->list, c->list_cap, c->flags, leaf0, leaf1, c->st));
+  LAUNCHED(launch_find_ngb(c->tree, c->f[c->cur].pos, c->n_ngb, c->list, c->list_cap, c->list_stride, c->flags,
+                           leaf0, leaf1, c->st));
   c->lists_ok = true;
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
@@ -1031,8 +1026,9 @@ extern "C" int cudasph_adjoint(sph_ctx *c) {
   AdjArgs a;
   memset(&a, 0, sizeof(a));
   a.n = c->n;
-  a.nleaf = c->tree.count[0];
+  a.nleaf = c->tree.nleaf;
   a.cap = c->list_cap;
+  a.stride = c->list_stride;
   a.pos = F.pos; a.vel = F.vel; a.hyd = F.hyd; a.dd = F.dd; a.dots = F.dots; a.vsig = F.vsig;
   a.old = c->old; a.pre_acc = c->pre_acc; a.x0 = nullptr; a.vpup = c->vpup;
   a.n_ngb = c->n_ngb; a.list = c->list; a.sc = c->sc;
@@ -1138,8 +1134,9 @@ namespace sph {
 cudaStream_t ctx_stream(sph_ctx *c) { return c->st; }
 Fields &ctx_fields(sph_ctx *c) { return c->f[c->cur]; }
 int *ctx_n_ngb(sph_ctx *c) { return c->n_ngb; }
-int *ctx_list(sph_ctx *c, int *cap) {
+int *ctx_list(sph_ctx *c, int *cap, int *stride) {
   *cap = c->list_cap;
+  *stride = c->list_stride;
   return c->list;
 }
 const TreeView &ctx_tree(sph_ctx *c) { return c->tree; }

@@ -19,22 +19,25 @@
 
 namespace sph {
 
-constexpr int kLeaf = 32;        // particles per tree leaf = one warp
+constexpr int kLeaf = 32;        // particles per leaf: the unit of sharding and of the tree walk's groups
+constexpr int kCell = 8;         // particles per cell, the lowest level of the box tree
 constexpr int kFan = 32;         // children per internal node = one warp
-constexpr int kMaxLevels = 8;    // supports up to 32^8 leaves
-constexpr int kStack = 256;      // per-warp traversal stack (entries)
+constexpr int kMaxLevels = 8;    // supports up to 32^7 cells
 
-// Device-side view of the tree over Morton-ordered leaves.  Level 0 holds
-// the leaves, level top the single root.  Each box is stored as two float4
-// (lo.xyz, hi.xyz) rounded outward from the FP64 extrema, so that box tests
-// are conservative and the exact FP64 predicate decides membership.
+// Device-side view of the box tree over Morton-ordered particles.  Level 0
+// holds the cells of kCell consecutive particles, level top the single root.
+// Each box is stored as two float4 (lo.xyz, hi.xyz) rounded outward from the
+// FP64 extrema, so that box tests are conservative and the exact FP64
+// predicate decides membership.
 struct TreeView {
   int n;                       // particles
+  int nleaf;                   // leaves of kLeaf particles
   int levels;                  // number of levels (top = levels - 1)
   int count[kMaxLevels];       // nodes per level
   long long base[kMaxLevels];  // offset of each level in lo/hi
   const float4 *lo;
   const float4 *hi;
+  const float4 *pf;            // positions rounded to float
 };
 
 // All per-particle state arrays (one buffer set).
@@ -45,8 +48,9 @@ struct Fields {
 };
 
 // arguments of the density / hydro kernels (both precision forms)
+// (list: one row of `stride` entries per slot, the first min(n_ngb, cap) valid)
 struct HydroArgs {
-  int n, nleaf, cap;
+  int n, nleaf, cap, stride;
   int leaf0, leaf1;  // leaves [leaf0, leaf1) processed by this launch (a shard's range, or all)
   const double4 *pos, *vel;
   double4 *hyd, *dd, *dots;
@@ -62,7 +66,7 @@ struct HydroArgs {
 
 // arguments of the adjoint kernels (adjoint.cu)
 struct AdjArgs {
-  int n, nleaf, cap;
+  int n, nleaf, cap, stride;
   // forward state of the step (slot order)
   const double4 *pos;     // x1, w
   const double4 *vel;     // (v1), m

@@ -3,11 +3,11 @@
 // viscosity (dev_hydro_dots.cu:25-113, dev_art_visc.cu:8-32) and the j-side
 // pair force (add_ngb_acc, sph_accelerations.cpp:106-114).
 //
-// One warp per leaf, one lane per particle.  The neighbour list of lane l is
-// read from the leaf-sliced layout, so entry k of all 32 lanes is one
-// coalesced 128-byte load; neighbour records (double4 pos / vel / hydro /
-// dots_data) are gathered with 16-byte loads and mostly hit L1/L2 because
-// neighbours are Morton-close.  The j-side force of each pair is added to
+// S lanes per particle, 32 / S particles per warp.  The lanes of a
+// particle take consecutive entries of its list row: entries are ascending
+// slots, mostly runs of neighbouring slots, so the lanes' 32-byte records lie
+// in few 128-byte lines, and a warp waits only for the longest of 32 / S
+// lists.  The partial sums meet by shuffles at the end.  The j-side force of each pair is added to
 // the neighbour with an FP64 atomic (red.global.add.f64), which keeps the
 // pair force antisymmetric (momentum conserving) without a transposed list.
 //
@@ -103,18 +103,35 @@ __device__ __forceinline__ double kernel_dw(double u, double iu) {
 }
 
 
-__device__ __forceinline__ int leaf_max_count(int cnt) {
+// sum over the S lanes of a particle (every lane gets it)
+template <int S>
+__device__ __forceinline__ double sub_sum(double v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, o));
-  return cnt;
+  for (int o = S / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int S>
+__device__ __forceinline__ double sub_max(double v) {
+#pragma unroll
+  for (int o = S / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
 }
 
+// Lanes per particle.  Small sets take 16: with few warps in flight the loops
+// wait on one gather after another, and 16 lanes take a sixth of the rounds
+// (2,049 particles, density / hydro, us, 16, 8 and 4 lanes, and one lane per
+// particle: 10.5 / 22.5, 12.5 / 22.6, 16.4 / 26.6, 52 / 58).  Large sets are
+// bound by the FP64 pipe (density) and by L1 and the atomics (hydro), where
+// the shuffles at the end count (1,048,576 particles, density / hydro, ms, 2,
+// 4, 8, 16 lanes and one: 0.74 / 1.70, 0.77 / 1.61, 0.86 / 1.79, 1.08 / 2.22,
+// 0.84 / 1.78).
+constexpr int kSubSmall = 16, kSmallSet = 8192;
+constexpr int kSubDensity = 2, kSubHydro = 4;
+
+template <int S>
 __global__ void __launch_bounds__(128) k_density(HydroArgs a) {
-  const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (leaf >= a.leaf1) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
-  const bool valid = s < a.n;
+  const int s = a.leaf0 * kLeaf + (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
+  const bool valid = s < min(a.leaf1 * kLeaf, a.n);
   double4 pi = make_double4(0, 0, 0, 0), vi = make_double4(0, 0, 0, 0);
   int cnt = 0;
   if (valid) {
@@ -122,27 +139,26 @@ __global__ void __launch_bounds__(128) k_density(HydroArgs a) {
     vi = a.vel[s];
     cnt = min(a.n_ngb[s], a.cap);
   }
-  const int kmax = leaf_max_count(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
   const double i2w = 2.0 / w, hw = 0.5 * w;  // u = r (2 / range), 1 / u = (1 / r) (range / 2)
   double dens = 0, om = 0, ps = 0, sdig = 0, div = 0, cx = 0, cy = 0, cz = 0;
   // the neighbours' records are gathered one pair ahead of their use and
   // the list entries two ahead, so the loads overlap the pair arithmetic
-  int jn = cnt > 1 ? __ldg(lst + kLeaf) : 0;
+  int jn = sub + S < cnt ? __ldg(lst + sub + S) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn;
-  if (cnt > 0) {
-    const int j0 = __ldg(lst);
+  if (sub < cnt) {
+    const int j0 = __ldg(lst + sub);
     pn = ld4(a.pos + j0);
     vn = ld4(a.vel + j0);
   }
-  for (int k = 0; k < kmax; k++) {
-    if (k < cnt) {
+  for (int k = sub; k < cnt; k += S) {
+    {
       const double4 pj = pn, vj = vn;
-      if (k + 1 < cnt) {
+      if (k + S < cnt) {
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
-        if (k + 2 < cnt) jn = __ldg(lst + (size_t)(k + 2) * kLeaf);
+        if (k + 2 * S < cnt) jn = __ldg(lst + k + 2 * S);
       }
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
       double r, ir;
@@ -162,7 +178,10 @@ __global__ void __launch_bounds__(128) k_density(HydroArgs a) {
       cz += wt * (dx * dvy - dy * dvx);
     }
   }
-  if (!valid) return;
+  __syncwarp();
+  dens = sub_sum<S>(dens); om = sub_sum<S>(om); ps = sub_sum<S>(ps); sdig = sub_sum<S>(sdig);
+  div = sub_sum<S>(div); cx = sub_sum<S>(cx); cy = sub_sum<S>(cy); cz = sub_sum<S>(cz);
+  if (!valid || sub != 0) return;
   if (a.dsum) a.dsum[s] = make_double4(sdig, cx, cy, cz);
   double4 d = make_double4(0, 0, 0, 0);
   double rho = 0;
@@ -278,12 +297,10 @@ __device__ __forceinline__ void art_visc_pre(double ids, double drdv, const doub
 // 4 blocks per SM: the one-pair-ahead gathers need the registers (N = 1M:
 // 2.40 ms without them at 6 blocks per SM, 2.99 ms with them and spills at
 // 6, 1.89 ms with them at 4)
+template <int S>
 __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
-  const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (leaf >= a.leaf1) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
-  const bool valid = s < a.n;
+  const int s = a.leaf0 * kLeaf + (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
+  const bool valid = s < min(a.leaf1 * kLeaf, a.n);
   double4 pi = make_double4(0, 0, 0, 0), vi = make_double4(0, 0, 0, 1), hi4 = make_double4(0, 0, 0, 0),
           di = make_double4(0, 0, 0, 0), fi = make_double4(0, 0, 0, 0);
   int cnt = 0;
@@ -295,8 +312,7 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
     fi = a.aux[s];
     cnt = min(a.n_ngb[s], a.cap);
   }
-  const int kmax = leaf_max_count(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double hh = 0.5 * pi.w;
   const double prho2 = (hi4.x > 0) ? hi4.y / (hi4.x * hi4.x) : 0;
   const double h2 = hh * hh, h5 = h2 * h2 * hh;
@@ -309,23 +325,23 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
   double axi = 0, ayi = 0, azi = 0, udot = 0, vmax = 0;
   // the neighbours' records are gathered one pair ahead of their use and the
   // list entries two ahead (as in the density loop)
-  int jn = cnt > 1 ? __ldg(lst + kLeaf) : 0, jc = cnt > 0 ? __ldg(lst) : 0;
+  int jn = sub + S < cnt ? __ldg(lst + sub + S) : 0, jc = sub < cnt ? __ldg(lst + sub) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn, fn = pn;
-  if (cnt > 0) {
+  if (sub < cnt) {
     pn = ld4(a.pos + jc);
     vn = ld4(a.vel + jc);
     fn = ld4(a.aux + jc);
   }
-  for (int k = 0; k < kmax; k++) {
-    if (k < cnt) {
+  for (int k = sub; k < cnt; k += S) {
+    {
       const int j = jc;
       const double4 pj = pn, vj = vn, fj = fn;
-      if (k + 1 < cnt) {
+      if (k + S < cnt) {
         jc = jn;
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
         fn = ld4(a.aux + jn);
-        if (k + 2 < cnt) jn = __ldg(lst + (size_t)(k + 2) * kLeaf);
+        if (k + 2 * S < cnt) jn = __ldg(lst + k + 2 * S);
       }
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
       const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
@@ -344,7 +360,7 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
       ayi -= mj * acc * dy;
       azi -= mj * acc * dz;
       const double nacc = vi.w * acc;
-      if (a.ngb_acc) a.ngb_acc[(size_t)leaf * a.cap * kLeaf + (size_t)k * kLeaf + lane] = nacc;
+      if (a.ngb_acc) a.ngb_acc[(size_t)s * a.stride + k] = nacc;
       if (a.jside && j != s) {
         atomicAdd(&a.dots[j].x, nacc * dx);
         atomicAdd(&a.dots[j].y, nacc * dy);
@@ -354,7 +370,10 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
       udot += ud * drdv;
     }
   }
-  if (!valid) return;
+  __syncwarp();
+  axi = sub_sum<S>(axi); ayi = sub_sum<S>(ayi); azi = sub_sum<S>(azi); udot = sub_sum<S>(udot);
+  vmax = sub_max<S>(vmax);
+  if (!valid || sub != 0) return;
   atomicAdd(&a.dots[s].x, axi);
   atomicAdd(&a.dots[s].y, ayi);
   atomicAdd(&a.dots[s].z, azi);
@@ -364,7 +383,9 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
 
 int launch_density(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
-  k_density<<<((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, 0, st>>>(a);
+  const int n = (a.leaf1 - a.leaf0) * kLeaf;
+  if (n < kSmallSet) k_density<kSubSmall><<<(n * kSubSmall + 127) / 128, 128, 0, st>>>(a);
+  else k_density<kSubDensity><<<(n * kSubDensity + 127) / 128, 128, 0, st>>>(a);
   return 1;
 }
 int launch_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsigned *flags, cudaStream_t st) {
@@ -382,7 +403,9 @@ int launch_hydro(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
   // every particle's factors: a shard's pairs reach outside its own leaves
   int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);
-  k_hydro<<<((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, 0, st>>>(a);
+  const int n = (a.leaf1 - a.leaf0) * kLeaf;
+  if (n < kSmallSet) k_hydro<kSubSmall><<<(n * kSubSmall + 127) / 128, 128, 0, st>>>(a);
+  else k_hydro<kSubHydro><<<(n * kSubHydro + 127) / 128, 128, 0, st>>>(a);
   return launches + 1;
 }
 

@@ -58,12 +58,12 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
     cnt = min(a.n_ngb[s], a.cap);
   }
   const int kmax = leaf_max_count_m(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
   float iw_hi = 0.f, iw_lo = 0.f;  // 2 / range as a float-float pair
   if (w > 0) split_ff(2.0 / w, iw_hi, iw_lo);
   KSum dens, om, ps, sdig, div, cx, cy, cz;
-  int jn = cnt > 1 ? __ldg(lst + kLeaf) : 0;
+  int jn = cnt > 1 ? __ldg(lst + 1) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn;
   if (cnt > 0) {
     const int j0 = __ldg(lst);
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
       if (k + 1 < cnt) {
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
-        if (k + 2 < cnt) jn = __ldg(lst + (size_t)(k + 2) * kLeaf);
+        if (k + 2 < cnt) jn = __ldg(lst + k + 2);
       }
       const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
       const float u = mul_ff(sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx))), iw_hi, iw_lo);
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
     cnt = min(a.n_ngb[s], a.cap);
   }
   const int kmax = leaf_max_count_m(cnt);
-  const int *lst = a.list + (size_t)leaf * a.cap * kLeaf + lane;
+  const int *lst = a.list + (size_t)s * a.stride;
   const double hh = 0.5 * pi.w;
   float ih_hi = 0.f, ih_lo = 0.f;  // 1 / h as a float-float pair
   if (hh > 0) split_ff(1.0 / hh, ih_hi, ih_lo);
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
   float vmax = 0.f;
   for (int k = 0; k < kmax; k++) {
     if (k < cnt) {
-      const int j = __ldg(lst + (size_t)k * kLeaf);
+      const int j = __ldg(lst + k);
       const double4 pj = ld4(a.pos + j), vj = ld4(a.vel + j), fj = ld4(a.aux + j);
       const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
       const float dvx = (float)(vi.x - vj.x), dvy = (float)(vi.y - vj.y), dvz = (float)(vi.z - vj.z);

@@ -19,7 +19,7 @@ namespace sph {
 cudaStream_t ctx_stream(sph_ctx *c);
 Fields &ctx_fields(sph_ctx *c);
 int *ctx_n_ngb(sph_ctx *c);
-int *ctx_list(sph_ctx *c, int *cap);
+int *ctx_list(sph_ctx *c, int *cap, int *stride);
 const TreeView &ctx_tree(sph_ctx *c);
 void ctx_mark_positions(sph_ctx *c);
 int *ctx_slot_of(sph_ctx *c);
@@ -99,7 +99,7 @@ __global__ void k_legacy_hydro_in(int n, const float4 *__restrict__ hydro, const
 
 __global__ void k_legacy_sph_out(int n, const int *__restrict__ id, Fields F, const int *__restrict__ cnt,
                                  const int *__restrict__ list, const double *__restrict__ acc, int cap,
-                                 const int *__restrict__ offset, int *__restrict__ list_out,
+                                 int stride, const int *__restrict__ offset, int *__restrict__ list_out,
                                  float *__restrict__ acc_out, float4 *__restrict__ hydro, float4 *__restrict__ dd,
                                  float4 *__restrict__ dots, float4 *__restrict__ hydro2) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -111,11 +111,10 @@ __global__ void k_legacy_sph_out(int n, const int *__restrict__ id, Fields F, co
   dd[i] = make_float4((float)d.x, (float)d.y, (float)d.z, (float)d.w);
   dots[i] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
   hydro2[i].x = (float)F.vsig[s];
-  const int leaf = s / kLeaf, lane = s % kLeaf;
   const int m = min(cnt[s], cap);
   const int o = offset[i];
   for (int k = 0; k < m; k++) {
-    const size_t e = ((size_t)leaf * cap + k) * kLeaf + lane;
+    const size_t e = (size_t)s * stride + k;
     list_out[o + k] = id[list[e]];
     acc_out[o + k] = (float)acc[e];
   }
@@ -282,9 +281,9 @@ float host_sph_accelerations(int n_bodies, int ngb_tot, float av_alpha, float av
   cudaStream_t st = ctx_stream(c);
   Fields &F = ctx_fields(c);
   k_legacy_hydro_in<<<(n + 255) / 256, 256, 0, st>>>(n, (const float4 *)hydro_data, F.id, F);
-  int cap = 0;
-  int *list = ctx_list(c, &cap);
-  const size_t entries = (size_t)ctx_tree(c).count[0] * kLeaf * cap;
+  int cap = 0, stride = 0;
+  int *list = ctx_list(c, &cap, &stride);
+  const size_t entries = (size_t)n * stride;
   if (entries > g_acc_cap) {
     if (g_acc) cudaFree(g_acc);
     check(cudaMalloc((void **)&g_acc, sizeof(double) * entries), "cudaMalloc(ngb_acc)");
@@ -297,7 +296,7 @@ float host_sph_accelerations(int n_bodies, int ngb_tot, float av_alpha, float av
   a.ngb_acc = g_acc;
   a.jside = 0;  // the driver scatters the j-side itself (sph_accelerations.cpp:106-114)
   launch_hydro(a, st);
-  k_legacy_sph_out<<<(n + 255) / 256, 256, 0, st>>>(n, F.id, F, ctx_n_ngb(c), list, g_acc, cap, ngb_offset, ngb_list,
+  k_legacy_sph_out<<<(n + 255) / 256, 256, 0, st>>>(n, F.id, F, ctx_n_ngb(c), list, g_acc, cap, stride, ngb_offset, ngb_list,
                                                     ngb_acc, (float4 *)hydro_data, (float4 *)dots_data,
                                                     (float4 *)bodies_dots, (float4 *)hydro_data2);
   launch_invert(n, F.id, ctx_slot_of(c), st);

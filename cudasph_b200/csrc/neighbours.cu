@@ -1,248 +1,294 @@
 // neighbours.cu -- smoothing-length solve (dev_solve_range.cu:17-189) and
 // neighbour search (dev_find_ngb.cu:13-87) on the Morton tree.
 //
-// One warp owns one leaf (32 consecutive particles); lane l owns particle
-// 32*leaf + l.  The warp walks the tree together: at every internal node each
-// lane tests one child box, a ballot picks the children that overlap the
-// union of the lanes' search boxes, and the hits are pushed in reverse order
-// on a per-warp shared-memory stack, so leaves come out in ascending index
-// order.  A visited leaf's 32 positions are staged in shared memory and every
-// lane applies the exact FP64 predicate ds2 < range^2 to all of them.
+// One warp owns one target particle at a time.  It walks the tree for that
+// particle alone: at every internal node each lane tests one child box
+// against the target's ball, a ballot keeps the children hit, and the leaves
+// come out in ascending index order.  In a visited leaf lane k tests
+// candidate k in FP32 (a conservative test on float copies of the positions)
+// and the survivors are staged, in order, in the warp's shared memory; every
+// 32 staged candidates go through the exact FP64 predicate ds2 < range^2 at
+// once, one per lane, and the hits are appended to the particle's list row
+// in ascending slot order and evaluated one per lane.
 //
 // This translation unit is compiled without FMA contraction: the h solve and
 // the predicate then perform the same IEEE operations, in the same order
 // (ascending neighbour index), as an FP64 CPU evaluation of the reference's
 // loops, which makes the solved ranges and the neighbour sets reproducible
 // bit for bit against such an evaluation.
+//
+// Why a warp per particle and not a lane per particle (a warp per leaf of 32
+// targets, the earlier form): a leaf-warp lasts as long as its slowest lane's
+// iteration, and small sets have too few of them.  Solve phase, us, lane /
+// warp per particle: 2,049 particles 431 / 23, 16,384 540 / 85, 60,000 717 /
+// 233, 262,144 (an oscillating star, 1.4 evaluations per particle) 1907 /
+// 1103, 1,048,576 5348 / 3904; 130,001 particles from estimated ranges (3.7
+// evaluations, some ranges holding half the star) 69,400 / 3,450.  A steady
+// set with 1.00 evaluations per particle is the one that loses: 2,000,003
+// particles 5556 / 6020.  The kernel is bound by instruction issue (73 % of
+// the cycles at 262,144, about 2,700 instructions per particle; FP64 pipe 24
+// %, XU 18 %), so what helps is fewer instructions: cells of 8 particles
+// instead of leaves of 32 (5,400 -> 3,100 with shared walks), the group's
+// candidate pass (2,600), and occupancy.  Loading the next candidates ahead
+// of their test, or the next records ahead of their evaluation, cost 5 - 9 %
+// (registers).
 #include "common.cuh"
 #include "sph_math.cuh"
 
 namespace sph {
 
-constexpr int kWarpsPerBlock = 4;
+constexpr int kNgbWarps = 4;   // warps per block
+// queries reach a little past the range: the sliver test below needs it
+constexpr double kWiden = 1.0 + 1e-12;
+// ... and a group's candidates cover ranges up to this much larger, so that a
+// second evaluation, a per cent away, finds them at hand (3 % more candidates)
+constexpr double kSlack = 1.01;
+constexpr int kNgbBlocks = 9;  // resident blocks per SM (N = 1M: 8, 9, 10 and 12 of them 4.05, 3.90, 4.42, 4.60 ms)
 constexpr unsigned kFull = 0xffffffffu;
 
-struct LaneBox {
-  float lo[3], hi[3];
+constexpr int kQueue = 64;   // ring of cells awaiting their candidates' test (a power of two)
+constexpr int kGroup = 4;    // most targets of a warp
+constexpr int kCells = 256;  // cells a group's list holds (32 chunks of 4 cells fill one round of masks)
+constexpr int kRounds = kCells / 128;
+constexpr int kStage = 320;  // candidates of one target
+
+enum { kBr0 = 0, kBr1 = 1, kSolve = 2, kDone = 3 };
+
+// A particle's iteration state: the bracket / Newton / bisection steps of
+// dev_solve_range.cu:93-172 between evaluations.
+struct RangeIter {
+  double w, dx, f, x_left, f_try, rx, ry;
+  int phase, iter, keep, nev;
 };
 
+// shared memory of one warp
+template <int G>
 struct WarpSmem {
-  LaneBox lbox[kLeaf];  // the lanes' query boxes of the current walk
-  int stack[kStack];
-  double sx[kLeaf], sy[kLeaf], sz[kLeaf];
-  float4 sf[kLeaf];  // anchor-relative FP32 copies for the pre-filter
-  double tx[kLeaf], ty[kLeaf], tz[kLeaf];  // the warp's own particles (the targets)
-  // The speculative walk's per-target squared ranges and sliver bounds, and
-  // the boxes of the children of the node being visited: every lane reads
-  // them for the target or leaf at hand with one broadcast load, where a
-  // shuffle from the owning lane took two instructions per double (N = 1M:
-  // steady-state solve 3.83 -> 3.54 ms, the same ranges and lists).
-  double tr2[kLeaf], ts2[kLeaf];
-  float4 cbox[2 * kFan];  // lo of child k at [k], hi at [kFan + k]
+  alignas(16) double term[64];        // a batch's terms of the two sums, interleaved
+  unsigned mask[kMaxLevels];          // the walk: per level the children still to visit ...
+  int node[kMaxLevels];               // ... of this node
+  RangeIter it;                       // the target's iteration (lane 0 steps it)
+  int list[kCells];                   // cells that may meet a ball of the group, ascending
+  unsigned hits[G][kRounds][32];      // per target: candidates of each chunk of the list inside its ball
+  union {
+    unsigned short code[kStage];      // the target's candidates from the list: 8 * list index + particle
+    struct {
+      int stage[96];                  // or, found by a walk of its own: candidates awaiting the exact test
+      int cell[kQueue];               // and cells that meet the ball, both ascending
+    } own;
+  };
 };
 
-// Conservative FP32 pre-filter of the neighbour predicate.  Coordinates are
-// taken relative to a warp anchor (lane 0's particle) and rounded to FP32.
-// For a pair that is truly within range w of lane l, |x_j - anchor| <= B + w
-// where B bounds |x_l - anchor| over the warp, so the FP32 squared distance
-// differs from the exact one by less than w^2 (4.2e-7 (B + w)/w + 2.6e-7).
-// A candidate is rejected only when its FP32 squared distance exceeds
-// w^2 (1 + m) with m = 1e-6 (B + w)/w + 1e-6, i.e. when it is certainly
-// outside; everything else goes through the exact FP64 predicate, so the
-// neighbour sets are unchanged.  Lanes with m > 1e-2 skip the pre-filter.
-struct Prefilter {
-  double ax, ay, az;  // warp anchor
-  double B;           // sqrt(3) max |x_l - anchor| over the warp
-  float xf, yf, zf;   // this lane, anchor-relative
+// A query: everything within sqrt(r2) of the box [lo, hi] (a target's ball
+// when lo = hi).  Centres are rounded to float and the squared radius widened
+// to cover every rounding of the float tests (the rounding of the centre and
+// of a candidate's or box's coordinates, the subtractions, squares and sums:
+// under 4e-7 (|x| + |y| + |z|) absolute and 1e-6 relative), so a j with
+// |x_j - x| < r, and a box that holds one, always passes.  Whatever else
+// passes is decided by the exact predicate.
+struct Query {
+  float lo[3], hi[3], r2;
 };
 
-__device__ __forceinline__ Prefilter make_prefilter(bool on, double x, double y, double z) {
-  Prefilter f;
-  f.ax = __shfl_sync(0xffffffffu, x, 0);
-  f.ay = __shfl_sync(0xffffffffu, y, 0);
-  f.az = __shfl_sync(0xffffffffu, z, 0);
-  const double dx = x - f.ax, dy = y - f.ay, dz = z - f.az;
-  double b = on ? fmax(fabs(dx), fmax(fabs(dy), fabs(dz))) : 0.0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-  f.B = 1.7320508075688772 * b;
-  f.xf = (float)dx;
-  f.yf = (float)dy;
-  f.zf = (float)dz;
-  return f;
-}
-
-// the FP32 threshold for range w; negative = no pre-filter for this lane
-__device__ __forceinline__ float prefilter_threshold(const Prefilter &f, double w) {
-  if (!(w > 0)) return -1.f;
-  const double m = 1e-6 * (f.B + w) / w + 1e-6;
-  if (m > 1e-2) return -1.f;
-  return (float)(w * w * (1.0 + m));
-}
-
-__device__ __forceinline__ bool certainly_outside(const Prefilter &f, float thr, float4 q) {
-  const float dx = f.xf - q.x, dy = f.yf - q.y, dz = f.zf - q.z;
-  const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-  return thr >= 0.f && d2 > thr;
-}
-
-// Query box over the lanes that take part: [x - r, x + r] widened by a
-// relative 1e-15 of the magnitudes (covers the rounding of x - r) and
-// rounded outward to float.
-__device__ __forceinline__ void warp_query_box(bool on, double x, double y, double z, double r, float *ql, float *qh) {
-  double m0 = (fabs(x) + r) * 1e-15, m1 = (fabs(y) + r) * 1e-15, m2 = (fabs(z) + r) * 1e-15;
-  double l0 = on ? x - r - m0 : 1e308, l1 = on ? y - r - m1 : 1e308, l2 = on ? z - r - m2 : 1e308;
-  double h0 = on ? x + r + m0 : -1e308, h1 = on ? y + r + m1 : -1e308, h2 = on ? z + r + m2 : -1e308;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    l0 = fmin(l0, __shfl_xor_sync(kFull, l0, o));
-    l1 = fmin(l1, __shfl_xor_sync(kFull, l1, o));
-    l2 = fmin(l2, __shfl_xor_sync(kFull, l2, o));
-    h0 = fmax(h0, __shfl_xor_sync(kFull, h0, o));
-    h1 = fmax(h1, __shfl_xor_sync(kFull, h1, o));
-    h2 = fmax(h2, __shfl_xor_sync(kFull, h2, o));
-  }
-  ql[0] = __double2float_rd(l0); ql[1] = __double2float_rd(l1); ql[2] = __double2float_rd(l2);
-  qh[0] = __double2float_ru(h0); qh[1] = __double2float_ru(h1); qh[2] = __double2float_ru(h2);
-}
-
-// This lane's own query box [x - r, x + r], widened and rounded outward like
-// warp_query_box.  A leaf whose box misses it holds no j with d2 < r^2 for
-// this lane (both boxes contain everything they should), so the lane skips
-// the leaf's candidates, and the walk descends only into nodes whose box
-// meets the box of at least one active lane (not merely the union of the
-// lanes' boxes): the sets are unchanged, the work drops by more than half.
-__device__ __forceinline__ LaneBox lane_query_box(double x, double y, double z, double r) {
-  const double m0 = (fabs(x) + r) * 1e-15, m1 = (fabs(y) + r) * 1e-15, m2 = (fabs(z) + r) * 1e-15;
-  LaneBox b;
-  b.lo[0] = __double2float_rd(x - r - m0); b.lo[1] = __double2float_rd(y - r - m1); b.lo[2] = __double2float_rd(z - r - m2);
-  b.hi[0] = __double2float_ru(x + r + m0); b.hi[1] = __double2float_ru(y + r + m1); b.hi[2] = __double2float_ru(z + r + m2);
-  return b;
-}
-
-// This lane's query ball for the box test below: centre rounded to float
-// and the squared radius widened to cover every rounding of the float test
-// (the centre's rounding, the subtractions, squares and sums: under
-// 4e-7 (|x| + |y| + |z|) absolute and 1e-6 relative), so a leaf that holds a
-// j with |x_j - x| < r always passes.
-struct LaneBall {
-  float x, y, z, r2;
-};
-
-__device__ __forceinline__ LaneBall lane_ball(double x, double y, double z, double r) {
+__device__ __forceinline__ Query make_ball(double x, double y, double z, double r) {
   const double rr = r * (1.0 + 1e-6) + 4e-7 * (fabs(x) + fabs(y) + fabs(z));
-  LaneBall b;
-  b.x = (float)x; b.y = (float)y; b.z = (float)z;
-  b.r2 = __double2float_ru(rr * rr);
-  return b;
+  Query q;
+  q.lo[0] = q.hi[0] = (float)x;
+  q.lo[1] = q.hi[1] = (float)y;
+  q.lo[2] = q.hi[2] = (float)z;
+  q.r2 = __double2float_ru(rr * rr);
+  return q;
 }
 
-// does the box [bl, bh] come within the ball's radius of its centre?
-__device__ __forceinline__ bool lane_ball_hits(const LaneBall &q, const float *bl, const float *bh) {
-  const float dx = fmaxf(fmaxf(bl[0] - q.x, q.x - bh[0]), 0.f);
-  const float dy = fmaxf(fmaxf(bl[1] - q.y, q.y - bh[1]), 0.f);
-  const float dz = fmaxf(fmaxf(bl[2] - q.z, q.z - bh[2]), 0.f);
-  return dx * dx + dy * dy + dz * dz <= q.r2;
+__device__ __forceinline__ float dist2(float dx, float dy, float dz) { return fmaf(dz, dz, fmaf(dy, dy, dx * dx)); }
+
+__device__ __forceinline__ bool box_hit(const Query &q, const float4 &l, const float4 &h) {
+  return dist2(fmaxf(fmaxf(l.x - q.hi[0], q.lo[0] - h.x), 0.f), fmaxf(fmaxf(l.y - q.hi[1], q.lo[1] - h.y), 0.f),
+               fmaxf(fmaxf(l.z - q.hi[2], q.lo[2] - h.z), 0.f)) <= q.r2;
 }
 
-__device__ __forceinline__ bool lane_box_hits(const LaneBox &q, const float *bl, const float *bh) {
-  return (bl[0] <= q.hi[0]) & (bh[0] >= q.lo[0]) & (bl[1] <= q.hi[1]) & (bh[1] >= q.lo[1]) & (bl[2] <= q.hi[2]) &
-         (bh[2] >= q.lo[2]);
-}
+// The cells that meet a query, ascending, as masks over the 32 cells of a
+// node of level 1.  Warp-uniform.  The walk keeps one (node, children left)
+// pair per level in shared memory, so it needs no stack.
+struct Walk {
+  int level, node;   // the next node to expand, of level >= 2
+  unsigned parents;  // nodes of level 1 still to expand ...
+  int base;          // ... from this one on
+  bool more;
 
-// publish this lane's query box to the warp; returns the mask of active lanes
-__device__ __forceinline__ unsigned share_lane_boxes(WarpSmem &sm, const LaneBox &lb, bool on) {
+  template <class Smem>
+  __device__ __forceinline__ void start(const TreeView &t, Smem &sm) {
+    level = t.levels - 1;
+    node = 0;
+    base = 0;
+    parents = level == 1 ? 1u : 0u;
+    more = true;
+    __syncwarp();
+    if (lane_id() < kMaxLevels) sm.mask[lane_id()] = 0u;
+    __syncwarp();
+  }
+  // children of a node of level `lev` that meet the query
+  __device__ __forceinline__ unsigned expand(const TreeView &t, const Query &q, int lev, int nd) {
+    const int child = nd * kFan + (int)lane_id();
+    bool hit = false;
+    if (child < t.count[lev - 1]) {
+      const long long at = t.base[lev - 1] + child;
+      hit = box_hit(q, __ldg(t.lo + at), __ldg(t.hi + at));
+    }
+    return __ballot_sync(kFull, hit);
+  }
+  // the cells of one more node of level 1 (those from `first` on), while `more`
+  template <class Smem>
+  __device__ __forceinline__ unsigned next(const TreeView &t, Smem &sm, const Query &q, int &first) {
+    const int top = t.levels - 1;
+    if (top == 0) {  // a single cell
+      more = false;
+      first = 0;
+      return 1u;
+    }
+    if (parents == 0u) {  // down to the next nodes of level 1 (top >= 2)
+      for (;;) {
+        const unsigned c = expand(t, q, level, node);
+        const bool low = level == 2;
+        if (low) {
+          parents = c;
+          base = node * kFan;
+        } else if (lane_id() == 0) {
+          sm.node[level] = node;
+          sm.mask[level] = c;
+        }
+        __syncwarp();
+        // the next node above level 1: the lowest level with a child left
+        unsigned m = 0u;
+        int l = low ? 3 : level;
+        while (l <= top && (m = sm.mask[l]) == 0u) l++;
+        level = l - 1;
+        if (l <= top) {
+          node = sm.node[l] * kFan + __ffs(m) - 1;
+          __syncwarp();
+          if (lane_id() == 0) sm.mask[l] = m & (m - 1u);
+          __syncwarp();
+        }
+        if (low && parents != 0u) break;
+        if (l > top) {
+          more = false;
+          first = 0;
+          return 0u;
+        }
+      }
+    }
+    const int nd = base + __ffs(parents) - 1;
+    parents &= parents - 1u;
+    more = parents != 0u || level < top;
+    first = nd * kFan;
+    return expand(t, q, 1, nd);
+  }
+};
+
+// The group's cells into sm.list; their number, or -1 when they do not fit.
+template <class Smem>
+__device__ __forceinline__ int list_cells(const TreeView &t, Smem &sm, const Query &q) {
+  const int lane = (int)lane_id();
+  Walk walk;
+  walk.start(t, sm);
+  int n = 0;
+  while (walk.more) {
+    int first;
+    const unsigned c = walk.next(t, sm, q, first);
+    if (n + __popc(c) > kCells) return -1;
+    if ((c >> lane) & 1u) sm.list[n + __popc(c & ((1u << lane) - 1u))] = first + lane;
+    n += __popc(c);
+  }
   __syncwarp();
-  sm.lbox[lane_id()] = lb;
-  const unsigned m = __ballot_sync(kFull, on);
-  __syncwarp();
-  return m;
+  return n;
 }
 
-// Visit, in ascending order, every leaf whose box overlaps [ql, qh] (the
-// union of the lanes' query boxes) and the query box of at least one lane of
-// `onmask` (boxes in lbs).  All lanes call visit(leaf, lo, hi) together,
-// lo / hi = the leaf's box (float, rounded outward), read from cbox (2 kFan
-// float4 of the warp's shared memory, which visit must not write).  Returns
-// false on stack overflow.
-template <class Visit>
-__device__ bool walk_leaves(const TreeView &t, const float *ql, const float *qh, const LaneBox *lbs,
-                            unsigned onmask, int *stack, float4 *cbox, Visit &&visit) {
-  const unsigned lane = lane_id();
-  const int top = t.levels - 1;
-  if (top == 0) {
-    const float bl[3] = {-3e38f, -3e38f, -3e38f}, bh[3] = {3e38f, 3e38f, 3e38f};
-    visit(0, bl, bh);
+// Candidates of one target, ascending, up to 32 at a time (lane k holds
+// candidate k, -1 past the last): a superset of what its ball q holds.
+// Either the codes that the group's pass over its cell list left (total >=
+// 0), or a visit of the cells that meet the ball, taken from the group's list
+// (nlist >= 0, which must cover q) or from a walk of the tree: they queue up
+// until eight are at hand, then lanes 8c .. 8c + 7 load the particles of cell
+// c, four cells per load and two loads in flight.
+struct Source {
+  Walk walk;
+  int nlist, total, at, staged;
+  unsigned head, tail;
+
+  template <class Smem>
+  __device__ __forceinline__ void start(const TreeView &t, Smem &sm, int nlist_, int total_) {
+    nlist = nlist_;
+    total = total_;
+    at = staged = 0;
+    head = tail = 0;
+    if (total >= 0) return;
+    if (nlist < 0) walk.start(t, sm);
+    else walk.more = nlist > 0;
+  }
+  template <class Smem>
+  __device__ __forceinline__ bool next(const TreeView &t, Smem &sm, const Query &q, int &j) {
+    static_assert(kCell == 8, "four cells fill a warp");
+    const int lane = (int)lane_id();
+    if (total >= 0) {
+      if (at >= total) return false;
+      j = -1;
+      if (at + lane < total) {
+        const int code = sm.code[at + lane];
+        j = sm.list[code >> 3] * kCell + (code & 7);
+      }
+      at += 32;
+      return true;
+    }
+    const unsigned below = (1u << lane) - 1u;
+    while (staged < 32 && (walk.more || tail != head)) {
+      while (walk.more && tail - head < 8u) {
+        unsigned c;
+        int id;
+        if (nlist >= 0) {
+          bool hit = false;
+          id = at + lane < nlist ? sm.list[at + lane] : 0;
+          if (at + lane < nlist) hit = box_hit(q, __ldg(t.lo + id), __ldg(t.hi + id));
+          c = __ballot_sync(kFull, hit);
+          at += 32;
+          walk.more = at < nlist;
+        } else {
+          c = walk.next(t, sm, q, id);
+          id += lane;
+        }
+        if ((c >> lane) & 1u) sm.own.cell[(tail + (unsigned)__popc(c & below)) % kQueue] = id;
+        tail += (unsigned)__popc(c);
+      }
+      __syncwarp();
+      const unsigned take = min(tail - head, 8u);
+      const unsigned c0 = (unsigned)lane >> 3, c1 = 4u + c0;
+      int j0 = 0x7fffffff, j1 = 0x7fffffff;
+      if (c0 < take) j0 = sm.own.cell[(head + c0) % kQueue] * kCell + (lane & 7);
+      if (c1 < take) j1 = sm.own.cell[(head + c1) % kQueue] * kCell + (lane & 7);
+      float4 p0, p1;
+      if (j0 < t.n) p0 = __ldg(t.pf + j0);
+      if (j1 < t.n) p1 = __ldg(t.pf + j1);
+      head += take;
+      const bool in0 = j0 < t.n && dist2(p0.x - q.lo[0], p0.y - q.lo[1], p0.z - q.lo[2]) <= q.r2;
+      const bool in1 = j1 < t.n && dist2(p1.x - q.lo[0], p1.y - q.lo[1], p1.z - q.lo[2]) <= q.r2;
+      const unsigned m0 = __ballot_sync(kFull, in0), m1 = __ballot_sync(kFull, in1);
+      if (in0) sm.own.stage[staged + __popc(m0 & below)] = j0;
+      staged += __popc(m0);
+      if (in1) sm.own.stage[staged + __popc(m1 & below)] = j1;
+      staged += __popc(m1);
+      __syncwarp();
+    }
+    if (staged == 0) return false;
+    const int rest = max(staged - 32, 0);
+    j = lane < staged ? sm.own.stage[lane] : -1;
+    const int k0 = lane < rest ? sm.own.stage[32 + lane] : 0, k1 = 32 + lane < rest ? sm.own.stage[64 + lane] : 0;
+    __syncwarp();
+    if (lane < rest) sm.own.stage[lane] = k0;
+    if (32 + lane < rest) sm.own.stage[32 + lane] = k1;
+    __syncwarp();
+    staged = rest;
     return true;
   }
-  int sp = 1;
-  if (lane == 0) stack[0] = (top << 26);
-  __syncwarp();
-  while (sp > 0) {
-    --sp;
-    const int e = stack[sp];
-    __syncwarp();
-    const int level = e >> 26, node = e & ((1 << 26) - 1);
-    const int cl = level - 1;
-    const int child = node * kFan + (int)lane;
-    bool hit = false;
-    float4 l = make_float4(0.f, 0.f, 0.f, 0.f), h = l;
-    if (child < t.count[cl]) {
-      l = __ldg(&t.lo[t.base[cl] + child]);
-      h = __ldg(&t.hi[t.base[cl] + child]);
-      hit = (l.x <= qh[0]) & (h.x >= ql[0]) & (l.y <= qh[1]) & (h.y >= ql[1]) & (l.z <= qh[2]) & (h.z >= ql[2]);
-    }
-    if (hit) {  // ... and the box of some active lane
-      bool any = false;
-      unsigned mm = onmask;
-      while (mm && !any) {
-        const int L = __ffs(mm) - 1;
-        mm &= mm - 1;
-        const LaneBox q = lbs[L];
-        any = (l.x <= q.hi[0]) & (h.x >= q.lo[0]) & (l.y <= q.hi[1]) & (h.y >= q.lo[1]) & (l.z <= q.hi[2]) &
-              (h.z >= q.lo[2]);
-      }
-      hit = any;
-    }
-    unsigned m = __ballot_sync(kFull, hit);
-    if (cl == 0) {
-      if (m) {  // the leaves' boxes, for every lane at each visit
-        __syncwarp();
-        cbox[lane] = l;
-        cbox[kFan + lane] = h;
-        __syncwarp();
-      }
-      while (m) {
-        const int b = __ffs(m) - 1;
-        m &= m - 1;
-        const float4 lb4 = cbox[b], hb4 = cbox[kFan + b];
-        const float bl[3] = {lb4.x, lb4.y, lb4.z}, bh[3] = {hb4.x, hb4.y, hb4.z};
-        visit(node * kFan + b, bl, bh);
-      }
-      continue;
-    }
-    const int cnt = __popc(m);
-    if (sp + cnt > kStack) return false;
-    if (hit) stack[sp + cnt - 1 - __popc(m & ((1u << lane) - 1u))] = (cl << 26) | child;
-    sp += cnt;
-    __syncwarp();
-  }
-  return true;
-}
-
-__device__ __forceinline__ void stage_leaf(const double4 *__restrict__ pos, int n, int leaf, WarpSmem &sm,
-                                           const Prefilter &f) {
-  const int s = leaf * kLeaf + (int)lane_id();
-  __syncwarp();
-  if (s < n) {
-    const double4 p = ld4(pos + s);
-    sm.sx[lane_id()] = p.x;
-    sm.sy[lane_id()] = p.y;
-    sm.sz[lane_id()] = p.z;
-    sm.sf[lane_id()] = make_float4((float)(p.x - f.ax), (float)(p.y - f.ay), (float)(p.z - f.az), 0.f);
-  }
-  __syncwarp();
-}
+};
 
 struct SolveArgs {
   TreeView t;
@@ -251,38 +297,17 @@ struct SolveArgs {
   unsigned *flags;
   double n_target, rel_err, f_scale;
   int max_iter;
-  int *n_ngb;      // hard count at the final range
-  int *list;       // neighbour lists at the final range (layout of k_find_ngb)
-  double *dcache;  // squared distances of the cached candidates, layout of list
-  int cap;
-  int leaf0, leaf1;  // leaves processed by this launch
-  // the speculative first pass (k_solve_spec) hands the leaves it leaves
-  // unfinished to k_solve_range through a queue (null: no speculative pass)
-  int *queue;
-  int *queue_count;
-  struct SolveSave *save;  // per slot
-};
-
-enum { kBr0 = 0, kBr1 = 1, kSolve = 2, kDone = 3 };
-
-// radius of a candidate cache relative to the range that fills it: one
-// clamped Newton step of the bracket (f_scale = 10 %) stays inside it
-constexpr double kCacheMargin = 1.15;
-constexpr int kEvalBatch = 4;     // cache entries loaded ahead per evaluation step
-constexpr int kSpecBlocks = 8;    // resident blocks per SM of the speculative pass
-constexpr int kCompactBatch = 8;  // cache entries loaded ahead per compaction step
-
-// A lane's iteration state: the bracket / Newton / bisection steps of
-// dev_solve_range.cu:93-172 between evaluations.
-struct LaneIter {
-  double w, dx, f, x_left, f_try, rx, ry;
-  int phase, iter, keep, nev;
+  int ordered;  // batches whose terms are summed in list order, see eval_range
+  int *n_ngb;   // hard count at the final range
+  int *list;    // neighbour lists at the final range, one row of `stride` entries per slot
+  int cap, stride;
+  int s0, s1;   // slots processed by this launch
 };
 
 // One evaluation's epilogue (compute_ngb, dev_solve_range.cu:77-87) with the
 // smooth count sf and its derivative sum sg at it.w, and the step of the
-// lane's iteration to its next evaluation or the end.
-__device__ __forceinline__ void solve_advance(LaneIter &it, double sf, double sg, const SolveArgs &a) {
+// iteration to its next evaluation or the end.
+__device__ __forceinline__ void solve_advance(RangeIter &it, double sf, double sg, const SolveArgs &a) {
   const double rel = a.rel_err, fs = a.f_scale;
   it.nev++;
   it.f = sf - a.n_target;
@@ -348,534 +373,406 @@ __device__ __forceinline__ void solve_advance(LaneIter &it, double sf, double sg
   }
 }
 
-// a lane's state handed from the speculative pass to the resumed solve
-struct SolveSave {
-  double w, dx, f, x_left, f_try, rx, ry;
-  int phase, iter, keep, nev, cnt_list, bits;  // bits: 1 direct, 2 pending, 4 listed by the speculative pass
+
+// a / b rounded to nearest, y = 1 / b rounded to nearest: Markstein's method
+// (Computation of elementary functions on the IBM RISC System/6000, 1990).
+// The first correction brings q within an ulp, the second then rounds
+// correctly; b and the quotient are far from the ends of the exponent range.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  double q = __dmul_rn(a, y);
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// ig(u) and u d(ig)/du (k_ig and k_digdh of sph_math.cuh: the same operations
+// in the same order, each polynomial evaluated in one place so that the lanes
+// of a warp part as little as possible)
+__device__ __forceinline__ void count_terms(double u, double &ig, double &digdh) {
+  const double x = 4.0 * (1.0 - fabs(u - 1.0));
+  ig = 1.0;
+  if (x < 2) {
+    const double x3 = x * x * x;
+    if (x < 1) {
+      ig = x < 0 ? 0.0 : 4.0 * (div_by(x3, 3.0, 1.0 / 3.0) - 0.3 * x3 * x * x + 0.125 * x3 * x3);
+    } else {
+      ig = 4.0 * ((-1.0 / 60) + (2.0 / 3) * x3 - 0.75 * x3 * x + 0.3 * x3 * x * x -
+                  div_by(x3 * x3, 24.0, 1.0 / 24.0));
+    }
+  }
+  digdh = 0.0;
+  if (u > 0 && u < 2) {
+    const bool inner = u < 1;
+    const double v = 4.0 * (inner ? u : 2.0 - u);
+    if (v < 2) {
+      const double wv = v < 1 ? KC<double>::ipi * (1.0 - 1.5 * v * v + 0.75 * v * v * v)
+                              : KC<double>::ipi * 0.25 * (2.0 - v) * (2.0 - v) * (2.0 - v);
+      digdh = (inner ? 4.0 : -4.0) * u * (4.0 * KC<double>::pi * v * v * wv);
+    }
+  }
+}
+
+// one evaluation of a range
+struct Eval {
+  double sf, sg;   // smooth count and its derivative sum
+  double dmax;     // largest d2 inside the range
+  int count;       // particles inside the range
+  bool sliver;     // some candidate in [w^2, w^2 (1 + 2^-40))
+  bool many;       // given up: more than a.ordered batches
 };
 
-// Speculative first evaluation.  In steady state the previous step's range
-// (after the predictor) already passes the tolerance test for almost every
-// particle, so the first evaluation is also the last: the warp walks the
-// tree once at the ranges themselves, every hit (d2 < w^2) goes straight to
-// its lane's list (index only), and each lane evaluates f and f' over its
-// list in list order -- ascending index, the order of the walk and of the
-// CPU loop -- recomputing the FP64 d2 of each entry from the positions (the
-// same operations as the walk, so the same value).  No candidate cache is
-// written or read.  A lane done after this evaluation keeps the list when
-// its final range (w = (rx + ry) / 2, within a few ulp of the evaluated one)
-// leaves the set unchanged: every entry inside the final range (the largest
-// d2 checked), and, if the range grew, no candidate in the sliver just
-// outside the evaluated range (flagged during the walk).  Otherwise the
-// lane lists by a walk at its final range; lanes not done continue with the
-// candidate cache below.
-// This is its own kernel, with fewer registers (more resident warps) than
-// the candidate-cache solve; a leaf with a lane not done after it saves its
-// lanes' states and goes on a queue that k_solve_range then resumes.
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, kSpecBlocks) k_solve_spec(SolveArgs a) {
-  __shared__ WarpSmem smem[kWarpsPerBlock];
-  WarpSmem &sm = smem[threadIdx.x >> 5];
-  const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (leaf >= a.leaf1) return;
-  const int n = a.t.n;
-  const int s = leaf * kLeaf + (int)lane_id();
-  const bool valid = s < n;
-  double xi = 0, yi = 0, zi = 0, w0 = 0;
-  if (valid) {
-    const double4 p = a.pos[s];
-    xi = p.x; yi = p.y; zi = p.z; w0 = p.w;
-  }
-  const Prefilter pf = make_prefilter(valid && w0 > 0, xi, yi, zi);
-  sm.tx[lane_id()] = xi;
-  sm.ty[lane_id()] = yi;
-  sm.tz[lane_id()] = zi;
-  __syncwarp();
-  const size_t colbase = (size_t)leaf * a.cap * kLeaf;  // the warp's block of list / dcache
-  LaneIter it;
-  it.w = w0;
-  it.phase = (valid && w0 > 0) ? kBr0 : kDone;
-  it.dx = it.f = it.x_left = it.f_try = it.rx = it.ry = 0;
-  it.iter = it.keep = it.nev = 0;
-  double &w = it.w;
-  int &phase = it.phase, &nev = it.nev;
-  bool stack_ok = true;
-  const size_t col = (size_t)leaf * a.cap * kLeaf + lane_id();
-  int *lst = a.list + col;
-  const int cap = a.cap;
-  int cnt_list = 0;
-  bool direct = false;
-  bool pending = false;
-  auto advance = [&](double sf, double sg) { solve_advance(it, sf, sg, a); };
-  int spec_cnt = -1;  // >= 0: the speculative list is this lane's final list
-  if (__any_sync(kFull, phase != kDone)) {
-    const bool on = phase != kDone;
-    const double w_eval = w;
-    const double r2 = __dmul_rn(w, w);
-    const double r2hi = r2 * (1.0 + 0x1p-40);  // the sliver [w^2, r2hi)
-    const double rw = w * (1.0 + 1e-12);       // boxes and ball cover the sliver
-    float ql[3], qh[3];
-    warp_query_box(on, xi, yi, zi, rw, ql, qh);
-    const LaneBox lb = lane_query_box(xi, yi, zi, rw);
-    const LaneBall lball = lane_ball(xi, yi, zi, rw);
-    sm.tr2[lane_id()] = r2;  // published by the __syncwarp in share_lane_boxes
-    sm.ts2[lane_id()] = r2hi;
-    const unsigned onmask = share_lane_boxes(sm, lb, on);
-    int c = 0;
-    bool sliver = false;
-    stack_ok &= walk_leaves(a.t, ql, qh, sm.lbox, onmask, sm.stack, sm.cbox, [&](int lj, const float *bl, const float *bh) {
-      const int cntj = min(kLeaf, n - lj * kLeaf);
-      const unsigned tm = __ballot_sync(kFull, on && lane_box_hits(lb, bl, bh) && lane_ball_hits(lball, bl, bh));
-      if (!tm) return;
-      double xk = 1e300, yk = 1e300, zk = 1e300;  // past the last particle: never a neighbour
-      if ((int)lane_id() < cntj) {
-        const double4 p = ld4(a.pos + lj * kLeaf + (int)lane_id());
-        xk = p.x; yk = p.y; zk = p.z;
+// One walk at range w: writes the list row and, when `sums`, evaluates
+// f = sum ig and its derivative over it (dev_solve_range.cu:55-87).
+// The sums run in list order -- ascending index, the order of the CPU loop --
+// for bit-equal results: each lane computes the terms of its candidate and
+// even and odd lanes add up the two sums' terms one by one.  Beyond a.ordered
+// batches (about twice the neighbours aimed at) it gives up, unless `exact`:
+// the range is far too large and rough_sums is the cheaper way to see that.
+// nlist, total: see Source.
+template <bool SUMS, class Smem>
+__device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, const double4 &p, double w, int nlist,
+                                           int total, bool exact) {
+  const int lane = (int)lane_id();
+  const unsigned below = (1u << lane) - 1u;
+  const double r2 = __dmul_rn(w, w);
+  int *row = a.list + (size_t)s * a.stride;
+  Eval e;
+  e.count = 0;
+  e.sliver = false;
+  const double iw = 1.0 / w;
+  double acc = 0, dmax = -1.0;
+  int nb = 0, j;
+  const Query q = make_ball(p.x, p.y, p.z, w * kWiden);
+  Source src;
+  src.start(a.t, sm, nlist, total);
+  e.many = false;
+  while (src.next(a.t, sm, q, j)) {
+    if (SUMS && nb == a.ordered && !exact) {
+      e.many = true;
+      break;
+    }
+    double d2 = 1e300;
+    if (j >= 0) {
+      const double4 o = ld4(a.pos + j);
+      d2 = ds2_exact(p.x - o.x, p.y - o.y, p.z - o.z);
+    }
+    const bool hit = d2 < r2;
+    const unsigned hm = __ballot_sync(kFull, hit);
+    if (hit) {
+      const int idx = e.count + __popc(hm & below);
+      if (idx < a.cap) row[idx] = j;
+    }
+    e.count += __popc(hm);
+    if (SUMS) {
+      e.sliver |= !hit && d2 < r2 * (1.0 + 0x1p-40);
+      double tf = 0, tg = 0;
+      if (hit) {
+        count_terms(div_by(2 * sqrt(d2), w, iw), tf, tg);
+        dmax = fmax(dmax, d2);
       }
-      const int jk = lj * kLeaf + (int)lane_id();
-      const unsigned below = (1u << lane_id()) - 1u;
-      unsigned m = tm;
-      while (m) {  // two targets per round, as in the candidate-cache fill of k_solve_range
-        const int t0 = __ffs(m) - 1;
-        m &= m - 1u;
-        const int t1 = m ? __ffs(m) - 1 : t0;
-        const bool two = m != 0u;
-        m &= m - 1u;
-        const double r20 = sm.tr2[t0], r21 = sm.tr2[t1];
-        const double s20 = sm.ts2[t0], s21 = sm.ts2[t1];
-        const double d20 = ds2_exact(sm.tx[t0] - xk, sm.ty[t0] - yk, sm.tz[t0] - zk);
-        const double d21 = ds2_exact(sm.tx[t1] - xk, sm.ty[t1] - yk, sm.tz[t1] - zk);
-        const bool h0 = d20 < r20, h1 = two && d21 < r21;
-        const unsigned hm0 = __ballot_sync(kFull, h0), hm1 = __ballot_sync(kFull, h1);
-        const unsigned sm0 = __ballot_sync(kFull, !h0 && d20 < s20), sm1 = __ballot_sync(kFull, two && !h1 && d21 < s21);
-        const int b0 = __shfl_sync(kFull, c, t0), b1 = __shfl_sync(kFull, c, t1);
-        if (h0) {
-          const int idx = b0 + __popc(hm0 & below);
-          if (idx < cap) a.list[colbase + (size_t)idx * kLeaf + (size_t)t0] = jk;
-        }
-        if (h1) {
-          const int idx = b1 + __popc(hm1 & below);
-          if (idx < cap) a.list[colbase + (size_t)idx * kLeaf + (size_t)t1] = jk;
-        }
-        if ((int)lane_id() == t0) { c += __popc(hm0); sliver |= sm0 != 0u; }
-        if ((int)lane_id() == t1) { c += __popc(hm1); sliver |= sm1 != 0u; }  // t1 != t0 whenever hm1 | sm1 != 0
-      }
-    });
-    if (on && c <= cap) {
-      double sf = 0, sg = 0, dmax = -1.0;
-      for (int k0 = 0; k0 < c; k0 += kEvalBatch) {
-        int j[kEvalBatch];
-#pragma unroll
-        for (int q = 0; q < kEvalBatch; q++) j[q] = k0 + q < c ? lst[(size_t)(k0 + q) * kLeaf] : -1;
-        double4 pj[kEvalBatch];
-#pragma unroll
-        for (int q = 0; q < kEvalBatch; q++) pj[q] = j[q] >= 0 ? ld4(a.pos + j[q]) : make_double4(xi, yi, zi, 0);
-#pragma unroll
-        for (int q = 0; q < kEvalBatch; q++) {
-          if (j[q] >= 0) {
-            const double d2 = ds2_exact(xi - pj[q].x, yi - pj[q].y, zi - pj[q].z);
-            const double u = 2 * sqrt(d2) / w;
-            sf += k_ig<double>(u);
-            sg -= k_digdh<double>(u);
-            dmax = fmax(dmax, d2);
-          }
-        }
-      }
-      advance(sf, sg);
-      if (phase == kDone) {
-        const double wf2 = __dmul_rn(w, w);
-        const bool same = (w == w_eval) || (w < w_eval && dmax < wf2) || (w > w_eval && !sliver && wf2 < r2hi);
-        if (same) {
-          spec_cnt = c;
-          cnt_list = c;
-        } else {
-          direct = true;  // list by a walk at the final range
-          pending = true;
-        }
-      }
+      reinterpret_cast<double2 *>(sm.term)[lane] = make_double2(tf, -tg);
+      __syncwarp();
+      const double *term = sm.term + (lane & 1);
+#pragma unroll 8
+      for (int k = 0; k < 32; k++) acc += term[2 * k];
+      __syncwarp();
+      nb++;
     }
   }
-  if (!stack_ok && lane_id() == 0) raise_flag(a.flags, SPH_FLAG_STACK_OVERFLOW);
-  const bool more = phase != kDone || pending;
-  if (!__any_sync(kFull, more)) {
-    if (valid) {
-      a.pos[s].w = (w > 0) ? w : 0.0;
-      a.n_ngb[s] = cnt_list;
-      if (a.nevals) a.nevals[s] = nev;
+  if (SUMS) {
+    e.sf = __shfl_sync(kFull, acc, 0);
+    e.sg = __shfl_sync(kFull, acc, 1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(kFull, dmax, o));
+    e.dmax = dmax;
+    e.sliver = __any_sync(kFull, e.sliver);
+  }
+  return e;
+}
+
+// The two sums of a range far too large, in FP32 over every particle of the
+// cells that meet the ball: thousands of candidates, of which only the sign
+// and rough size of f and f' are wanted (clamped_for_sure).
+struct Rough {
+  double sf, sg;
+  double err;  // bound of either sum's error
+};
+
+template <class Smem>
+__device__ __forceinline__ Rough rough_sums(const SolveArgs &a, Smem &sm, const double4 &p, double w) {
+  const int lane = (int)lane_id();
+  const Query q = make_ball(p.x, p.y, p.z, w * kWiden);
+  const float i2w = (float)(2.0 / w);
+  Walk walk;
+  walk.start(a.t, sm);
+  double sf = 0, sg = 0, n = 0;
+  while (walk.more) {
+    int first;
+    const unsigned c = walk.next(a.t, sm, q, first);
+    float lf = 0.f, lg = 0.f;
+    for (int g = 0; g < 8; g++) {
+      if (((c >> (4 * g)) & 15u) == 0u) continue;  // four cells: 32 consecutive particles
+      const int j = (first + 4 * g) * kCell + lane;
+      if (j >= a.t.n) continue;
+      const float4 o = __ldg(a.t.pf + j);
+      const float u = sqrtf(dist2(o.x - q.lo[0], o.y - q.lo[1], o.z - q.lo[2])) * i2w;
+      lf += k_ig<float>(u);
+      lg -= k_digdh<float>(u);
     }
-    return;
+    sf += lf;
+    sg += lg;
+    n += 8 * __popc(c);
   }
-  if (valid) {
-    SolveSave v;
-    v.w = it.w; v.dx = it.dx; v.f = it.f; v.x_left = it.x_left; v.f_try = it.f_try; v.rx = it.rx; v.ry = it.ry;
-    v.phase = it.phase; v.iter = it.iter; v.keep = it.keep; v.nev = it.nev; v.cnt_list = cnt_list;
-    v.bits = (direct ? 1 : 0) | (pending ? 2 : 0) | (spec_cnt >= 0 ? 4 : 0);
-    a.save[s] = v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sf += __shfl_xor_sync(kFull, sf, o);
+    sg += __shfl_xor_sync(kFull, sg, o);
   }
-  if (lane_id() == 0) a.queue[atomicAdd(a.queue_count, 1)] = leaf;
+  // per term: u is off by at most 5e-7 (S / w + 2), S = |x| + |y| + |z|, from
+  // the rounded positions and the FP32 operations, and |ig'| < 4.3,
+  // |(u ig')'| < 90 on [0, 2]; about four times that is allowed for
+  const double per = 2e-4 * (fabs(p.x) + fabs(p.y) + fabs(p.z)) / w + 4e-4;
+  return {sf, sg, per * n + 1e-8 * a.n_target};
+}
+
+// Whether those sums take the iteration the same way as the exact ones: in
+// the bracket phase a step clamped to f_scale w depends on the signs of f and
+// f' only, so it is certain when both, and |f / f'| > f_scale w, hold by more
+// than the sums' error.
+__device__ __forceinline__ bool clamped_for_sure(const RangeIter &it, const Rough &r, const SolveArgs &a) {
+  const double f = fabs(r.sf - a.n_target), g = fabs(r.sg);
+  return (it.phase == kBr0 || it.phase == kBr1) && a.rel_err <= a.f_scale && f > r.err && g > r.err &&
+         f - r.err > a.f_scale * (g + r.err);
 }
 
 // dev_solve_range (dev_solve_range.cu:137-189): per particle, bracket the
 // root of f(w) = sum_j ig(2 r_ij / w) - N_target with clamped Newton steps
 // (dev_bracket_root :93-135), then safeguarded Newton / bisection until
-// |dx| < rel_err * w.  Each lane runs that iteration as a state machine.
-//
-// Candidate cache (find_ngb fused in): a lane whose range w is not covered
-// by its cache walks the tree once at radius 1.15 w and stores every j with
-// d2 < (1.15 w)^2 -- index in its column of the neighbour list, exact FP64
-// d2 in the same column of dcache -- in the walk's ascending order.  Every
-// evaluation of f (and of its derivative) then runs over the cached entries
-// with d2 < w^2 in that order, the same operations in the same order as a
-// walk at w, and the final list is the cache compacted in place to the final
-// range.  The lanes that need a walk in a round share it.  A lane whose
-// candidates exceed the list capacity falls back to walking at w for every
-// evaluation, writing its list as it goes (`direct`), with one list-only walk
-// when the final range differs from the last one evaluated (`pending`).
-// 6 blocks (24 warps) per SM: at N = 1M the capped form (80 registers, a
-// few spilled) took 12.1 ms per solve against 14.5 ms at 120 registers.
-// The candidate-cache solve of one leaf-warp, from the initial ranges or
-// (resume) from the states the speculative pass saved.
-__device__ __forceinline__ void solve_leaf(const SolveArgs &a, WarpSmem &sm, int leaf, bool resume) {
-  const int n = a.t.n;
-  const int s = leaf * kLeaf + (int)lane_id();
-  const bool valid = s < n;
-  double xi = 0, yi = 0, zi = 0, w0 = 0;
-  if (valid) {
-    const double4 p = a.pos[s];
-    xi = p.x; yi = p.y; zi = p.z; w0 = p.w;
-  }
-  const Prefilter pf = make_prefilter(valid && w0 > 0, xi, yi, zi);
-  sm.tx[lane_id()] = xi;
-  sm.ty[lane_id()] = yi;
-  sm.tz[lane_id()] = zi;
+// |dx| < rel_err * w.  Every evaluation is a walk at the range tested, which
+// writes the list at that range (find_ngb fused in).  In steady state the
+// previous step's range passes at once, so the first walk is the last: its
+// list is kept when the final range w = (rx + ry) / 2, a few ulp from the
+// evaluated one, leaves the set unchanged -- every entry inside the final
+// range (the largest d2 checked) and, if the range grew, no candidate in the
+// sliver just outside the evaluated range.  Otherwise one more walk lists at
+// the final range.
+template <class Smem>
+__device__ __forceinline__ void solve_particle(const SolveArgs &a, Smem &sm, int s, const double4 &p, int nlist,
+                                               int total, double w_list) {
+  RangeIter &it = sm.it;
   __syncwarp();
-  const size_t colbase = (size_t)leaf * a.cap * kLeaf;  // the warp's block of list / dcache
-  LaneIter it;
-  it.w = w0;
-  it.phase = (valid && w0 > 0) ? kBr0 : kDone;
-  it.dx = it.f = it.x_left = it.f_try = it.rx = it.ry = 0;
-  it.iter = it.keep = it.nev = 0;
-  double &w = it.w;
-  int &phase = it.phase, &nev = it.nev;
-  bool stack_ok = true;
-  const size_t col = (size_t)leaf * a.cap * kLeaf + lane_id();
-  int *lst = a.list + col;
-  const int cap = a.cap;
-  int cnt_list = 0;
-  bool direct = false;
-  bool pending = false;
-  auto advance = [&](double sf, double sg) { solve_advance(it, sf, sg, a); };
-  double &dx = it.dx, &f = it.f, &x_left = it.x_left, &f_try = it.f_try, &rx = it.rx, &ry = it.ry;
-  int &iter = it.iter, &keep = it.keep;
-  (void)dx; (void)f; (void)x_left; (void)f_try; (void)rx; (void)ry; (void)iter; (void)keep;
-  double *dc = a.dcache + col;
-  int ncache = 0;           // cached entries
-  double cache_r2 = -1.0;   // the cache holds every j with d2 < cache_r2
-  double w_list = -1.0;     // direct lanes: range of the list last written
-  int spec_cnt = -1;        // >= 0: the speculative pass listed this lane
-  if (resume && valid) {
-    const SolveSave v = a.save[s];
-    it.w = v.w; it.dx = v.dx; it.f = v.f; it.x_left = v.x_left; it.f_try = v.f_try; it.rx = v.rx; it.ry = v.ry;
-    it.phase = v.phase; it.iter = v.iter; it.keep = v.keep; it.nev = v.nev;
-    cnt_list = v.cnt_list;
-    direct = (v.bits & 1) != 0;
-    pending = (v.bits & 2) != 0;
-    spec_cnt = (v.bits & 4) ? v.cnt_list : -1;
+  if (lane_id() == 0) {
+    it.w = p.w;
+    it.phase = p.w > 0 ? kBr0 : kDone;
+    it.dx = it.f = it.x_left = it.f_try = it.rx = it.ry = 0;
+    it.iter = it.keep = it.nev = 0;
   }
-  while (true) {
-    const bool iterate = phase != kDone;
-    if (!__any_sync(kFull, iterate || pending)) break;
-    const double w2 = __dmul_rn(w, w);
-    const bool fill = iterate && !direct && !(w2 <= cache_r2);
-    const bool dwalk = (iterate && direct) || pending;
-    double sf = 0, sg = 0;
-    bool evaluated = false;
-    if (__any_sync(kFull, fill || dwalk)) {
-      const bool on = fill || dwalk;
-      const double r = fill ? w * kCacheMargin : w;
-      const double r2 = __dmul_rn(r, r);
-      float ql[3], qh[3];
-      warp_query_box(on, xi, yi, zi, r, ql, qh);
-      const float thr = prefilter_threshold(pf, r);
-      int c = 0;
-      const LaneBox lb = lane_query_box(xi, yi, zi, r);
-      const LaneBall lball = lane_ball(xi, yi, zi, r);
-      const unsigned onmask = share_lane_boxes(sm, lb, on);
-      const bool any_dwalk = __any_sync(kFull, dwalk);
-      stack_ok &= walk_leaves(a.t, ql, qh, sm.lbox, onmask, sm.stack, sm.cbox, [&](int lj, const float *bl, const float *bh) {
-        const int cntj = min(kLeaf, n - lj * kLeaf);
-        if (!any_dwalk) {
-          // Cache fills only: transposed.  Lane k holds candidate k of the
-          // leaf; for every lane t whose box meets the leaf, all 32 lanes
-          // apply t's exact predicate at once and a ballot appends the hits
-          // to t's column in ascending k -- the same entries, order and
-          // FP64 d2 as t testing the leaf itself, in |targets| rounds
-          // instead of 32 (a lane needs about half the leaves its warp
-          // visits).
-          const unsigned tm = __ballot_sync(kFull, on && lane_box_hits(lb, bl, bh) && lane_ball_hits(lball, bl, bh));
-          if (!tm) return;
-          double xk = 1e300, yk = 1e300, zk = 1e300;  // past the last particle: never a neighbour
-          if ((int)lane_id() < cntj) {
-            const double4 p = ld4(a.pos + lj * kLeaf + (int)lane_id());
-            xk = p.x; yk = p.y; zk = p.z;
-          }
-          const int jk = lj * kLeaf + (int)lane_id();
-          const unsigned below = (1u << lane_id()) - 1u;
-          unsigned m = tm;
-          while (m) {  // two targets per round: independent chains overlap
-            const int t0 = __ffs(m) - 1;
-            m &= m - 1u;
-            const int t1 = m ? __ffs(m) - 1 : t0;
-            const bool two = m != 0u;
-            m &= m - 1u;
-            const double r20 = __shfl_sync(kFull, r2, t0), r21 = __shfl_sync(kFull, r2, t1);
-            const double d20 = ds2_exact(sm.tx[t0] - xk, sm.ty[t0] - yk, sm.tz[t0] - zk);
-            const double d21 = ds2_exact(sm.tx[t1] - xk, sm.ty[t1] - yk, sm.tz[t1] - zk);
-            const bool h0 = d20 < r20, h1 = two && d21 < r21;
-            const unsigned hm0 = __ballot_sync(kFull, h0), hm1 = __ballot_sync(kFull, h1);
-            const int b0 = __shfl_sync(kFull, c, t0), b1 = __shfl_sync(kFull, c, t1);
-            if (h0) {
-              const int idx = b0 + __popc(hm0 & below);
-              if (idx < cap) {
-                const size_t off = colbase + (size_t)idx * kLeaf + (size_t)t0;
-                a.list[off] = jk;
-                a.dcache[off] = d20;
-              }
-            }
-            if (h1) {
-              const int idx = b1 + __popc(hm1 & below);
-              if (idx < cap) {
-                const size_t off = colbase + (size_t)idx * kLeaf + (size_t)t1;
-                a.list[off] = jk;
-                a.dcache[off] = d21;
-              }
-            }
-            if ((int)lane_id() == t0) c += __popc(hm0);
-            if ((int)lane_id() == t1) c += __popc(hm1);  // t1 != t0 whenever hm1 != 0
-          }
-          return;
-        }
-        stage_leaf(a.pos, n, lj, sm, pf);
-        if (on && lane_box_hits(lb, bl, bh)) {
-#pragma unroll 8
-          for (int k = 0; k < cntj; k++) {
-            if (certainly_outside(pf, thr, sm.sf[k])) continue;
-            const double d2 = ds2_exact(xi - sm.sx[k], yi - sm.sy[k], zi - sm.sz[k]);
-            if (d2 < r2) {
-              if (c < cap) {
-                lst[(size_t)c * kLeaf] = lj * kLeaf + k;
-                if (fill) dc[(size_t)c * kLeaf] = d2;
-              }
-              c++;
-              if (dwalk && iterate) {
-                const double u = 2 * sqrt(d2) / w;
-                sf += k_ig<double>(u);
-                sg -= k_digdh<double>(u);
-              }
-            }
-          }
-        }
-      });
-      if (fill) {
-        if (c <= cap) {
-          ncache = c;
-          cache_r2 = r2;
-        } else {
-          direct = true;  // evaluated by a walk at w from the next round on
-        }
-      }
-      if (dwalk) {
-        w_list = w;
-        cnt_list = c;
-        if (iterate) evaluated = true;
-        else pending = false;
-      }
+  __syncwarp();
+  int count = 0;
+  bool listed = true;  // the row holds the list of the final range
+  bool exact = false;
+  while (it.phase != kDone) {
+    const double w_eval = it.w;
+    if (w_eval > p.w * kSlack) total = -1;
+    const Eval e = eval_range<true>(a, sm, s, p, w_eval, w_eval <= w_list ? nlist : -1, total, exact);
+    if (e.many) {
+      const Rough r = rough_sums(a, sm, p, w_eval);
+      exact = !clamped_for_sure(it, r, a);
+      listed = false;
+      __syncwarp();
+      if (!exact && lane_id() == 0) solve_advance(it, r.sf, r.sg, a);
+      __syncwarp();
+      continue;
     }
-    if (iterate && !direct && w2 <= cache_r2) {
-      // the cache does not fit in L2 at large N: load a batch of entries
-      // before using any (the sums keep the entries' order)
-      for (int k0 = 0; k0 < ncache; k0 += kEvalBatch) {
-        double d2[kEvalBatch];
-#pragma unroll
-        for (int q = 0; q < kEvalBatch; q++) d2[q] = k0 + q < ncache ? dc[(size_t)(k0 + q) * kLeaf] : w2;
-#pragma unroll
-        for (int q = 0; q < kEvalBatch; q++) {
-          if (d2[q] < w2) {
-            const double u = 2 * sqrt(d2[q]) / w;
-            sf += k_ig<double>(u);
-            sg -= k_digdh<double>(u);
-          }
-        }
-      }
-      evaluated = true;
-    }
-    if (!evaluated) continue;
-    advance(sf, sg);
-    if (phase == kDone) {
-      if (direct) {
-        pending = w != w_list;
-      } else if (!(__dmul_rn(w, w) <= cache_r2)) {
-        direct = true;  // final range outside the cache: list by a walk
-        pending = true;
-      }
-    }
+    exact = false;
+    count = e.count;
+    __syncwarp();
+    if (lane_id() == 0) solve_advance(it, e.sf, e.sg, a);
+    __syncwarp();
+    const double w = it.w, wf2 = __dmul_rn(w, w);
+    listed = w == w_eval || (w < w_eval && e.dmax < wf2) ||
+             (w > w_eval && !e.sliver && wf2 < __dmul_rn(w_eval, w_eval) * (1.0 + 0x1p-40));
   }
-  if (valid && !direct && cache_r2 >= 0 && spec_cnt < 0) {
-    // the final list: the cached entries inside the final range, in order
-    const double w2 = __dmul_rn(w, w);
-    int c = 0;
-    // batches loaded before any store: a store goes to a slot c <= k below
-    // every slot a later batch reads
-    for (int k0 = 0; k0 < ncache; k0 += kCompactBatch) {
-      double d2[kCompactBatch];
-      int j[kCompactBatch];
-#pragma unroll
-      for (int q = 0; q < kCompactBatch; q++) {
-        const bool in = k0 + q < ncache;
-        d2[q] = in ? dc[(size_t)(k0 + q) * kLeaf] : w2;
-        j[q] = in ? lst[(size_t)(k0 + q) * kLeaf] : 0;
-      }
-#pragma unroll
-      for (int q = 0; q < kCompactBatch; q++) {
-        if (d2[q] < w2) {
-          lst[(size_t)c * kLeaf] = j[q];
-          c++;
-        }
-      }
-    }
-    cnt_list = c;
-  }
-  if (!stack_ok && lane_id() == 0) raise_flag(a.flags, SPH_FLAG_STACK_OVERFLOW);
-  if (cnt_list > cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
-  if (valid) {
+  const double w = it.w;
+  if (!listed)
+    count = eval_range<false>(a, sm, s, p, w, w <= w_list ? nlist : -1, w <= p.w * kSlack ? total : -1, false).count;
+  if (lane_id() == 0) {
+    if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
     a.pos[s].w = (w > 0) ? w : 0.0;
-    a.n_ngb[s] = cnt_list;
-    if (a.nevals) a.nevals[s] = nev;
+    a.n_ngb[s] = count;
+    if (a.nevals) a.nevals[s] = it.nev;
   }
 }
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 6) k_solve_range(SolveArgs a) {
-  __shared__ WarpSmem smem[kWarpsPerBlock];
-  WarpSmem &sm = smem[threadIdx.x >> 5];
-  const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (!a.queue) {
-    const int leaf = a.leaf0 + wid;
-    if (leaf < a.leaf1) solve_leaf(a, sm, leaf, false);
-    return;
-  }
-  // the leaves the speculative pass left, handed out to the resident warps
-  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-  const int count = *a.queue_count;
-  for (int q = wid; q < count; q += nw) {
-    solve_leaf(a, sm, a.queue[q], true);
+// The warp's targets first .. first + count - 1 and what they share: one walk
+// of the tree for the cells that may hold a neighbour of any of them at its
+// range (the targets are Morton neighbours, so these are little more than
+// each target's own), and one pass over those cells' particles that tests
+// every loaded candidate against all the targets, in FP32.
+template <int G>
+struct Group {
+  int first, count;
+  int nlist;      // cells in sm.list, -1: too many
+  double w_list;  // it covers ranges up to this
+
+  __device__ __forceinline__ void open(const SolveArgs &a, WarpSmem<G> &sm) {
+    const int lane = (int)lane_id();
+    first = a.s0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G;
+    count = min(G, a.s1 - first);
+    nlist = -1;
+    w_list = 0;
+    if (count <= 0) return;
+    double4 p = a.pos[first + min(lane % G, count - 1)];  // lanes past the last target repeat it
+    if (!(p.w > 0)) p.w = 0;
+    const Query mine = make_ball(p.x, p.y, p.z, p.w * kSlack * kWiden);
+    Query q = mine;
+    w_list = p.w;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        q.lo[d] = fminf(q.lo[d], __shfl_xor_sync(kFull, q.lo[d], o));
+        q.hi[d] = fmaxf(q.hi[d], __shfl_xor_sync(kFull, q.hi[d], o));
+      }
+      q.r2 = fmaxf(q.r2, __shfl_xor_sync(kFull, q.r2, o));
+      w_list = fmax(w_list, __shfl_xor_sync(kFull, w_list, o));
+    }
+    w_list *= kSlack;
+    nlist = list_cells(a.t, sm, q);
+    if (nlist <= 0) return;
+    float tx[G], ty[G], tz[G], tr[G];
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      tx[t] = __shfl_sync(kFull, mine.lo[0], t);
+      ty[t] = __shfl_sync(kFull, mine.lo[1], t);
+      tz[t] = __shfl_sync(kFull, mine.lo[2], t);
+      tr[t] = __shfl_sync(kFull, mine.r2, t);
+    }
+    for (int r = 0; r < kRounds && r * 128 < nlist; r++) {
+      unsigned m[G];
+#pragma unroll
+      for (int t = 0; t < G; t++) m[t] = 0u;
+      const int chunks = min(32, (nlist - r * 128 + 3) >> 2);
+      // lane's candidate of chunk c; past the last: infinitely far from every target
+      auto candidate = [&](int c) {
+        const int k = r * 128 + c * 4 + (lane >> 3);
+        const int j = k < nlist ? sm.list[k] * kCell + (lane & 7) : 0x7fffffff;
+        return j < a.t.n ? __ldg(a.t.pf + j) : make_float4(INFINITY, 0.f, 0.f, 0.f);
+      };
+      for (int c = 0; c < chunks; c++) {
+        const float4 o = candidate(c);
+#pragma unroll
+        for (int t = 0; t < G; t++) {
+          const unsigned b = __ballot_sync(kFull, dist2(o.x - tx[t], o.y - ty[t], o.z - tz[t]) <= tr[t]);
+          if (lane == c) m[t] = b;
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < G; t++) sm.hits[t][r][lane] = m[t];
+    }
     __syncwarp();
   }
-}
-
-struct FindArgs {
-  TreeView t;
-  const double4 *pos;
-  int *n_ngb;
-  int *list;       // [leaf][k][lane], cap entries per lane
-  int cap;
-  unsigned *flags;
-  int leaf0, leaf1;  // leaves processed by this launch
+  // target t's candidates as codes; their number, or -1 when they do not fit
+  __device__ __forceinline__ int stage(WarpSmem<G> &sm, int t) {
+    if (nlist < 0) return -1;
+    const int lane = (int)lane_id();
+    int total = 0;
+    __syncwarp();  // the previous target's codes are read
+    for (int r = 0; r < kRounds && r * 128 < nlist; r++) {
+      unsigned m = sm.hits[t][r][lane];
+      const int n = __popc(m);
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += v;
+      }
+      int at = total + incl - n;
+      total += __shfl_sync(kFull, incl, 31);
+      if (total > kStage) return -1;
+      const int base = (r * 32 + lane) * 32;
+      while (m) {
+        sm.code[at++] = (unsigned short)(base + __ffs(m) - 1);
+        m &= m - 1u;
+      }
+    }
+    __syncwarp();
+    return total;
+  }
 };
 
-// dev_find_ngb (dev_find_ngb.cu:13-87): every j with ds2 < range_i^2, in
-// ascending slot order, written to the leaf-sliced list (entry k of lane l of
-// leaf L at ((L * cap) + k) * 32 + l: the lanes of a warp read and write
-// their k-th neighbours in one 128-byte transaction).
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) k_find_ngb(FindArgs a) {
-  __shared__ WarpSmem smem[kWarpsPerBlock];
-  WarpSmem &sm = smem[threadIdx.x >> 5];
-  const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int n = a.t.n;
-  if (leaf >= a.leaf1) return;
-  const int s = leaf * kLeaf + (int)lane_id();
-  const bool valid = s < n;
-  double xi = 0, yi = 0, zi = 0, w = 0;
-  if (valid) {
-    const double4 p = a.pos[s];
-    xi = p.x; yi = p.y; zi = p.z; w = p.w;
-  }
-  const bool on = valid && w > 0;
-  float ql[3], qh[3];
-  warp_query_box(on, xi, yi, zi, w, ql, qh);
-  const double w2 = __dmul_rn(w, w);
-  const Prefilter pf = make_prefilter(on, xi, yi, zi);
-  const float thr = prefilter_threshold(pf, w);
-  int cnt = 0;
-  int *out = a.list + (size_t)leaf * a.cap * kLeaf + lane_id();
-  const int cap = a.cap;
-  bool ok = true;
-  if (__any_sync(kFull, on)) {
-    const LaneBox lb = lane_query_box(xi, yi, zi, w);
-    const unsigned onmask = share_lane_boxes(sm, lb, on);
-    ok = walk_leaves(a.t, ql, qh, sm.lbox, onmask, sm.stack, sm.cbox, [&](int lj, const float *bl, const float *bh) {
-      stage_leaf(a.pos, n, lj, sm, pf);
-      const int m = min(kLeaf, n - lj * kLeaf);
-      if (on && lane_box_hits(lb, bl, bh)) {
-#pragma unroll 8
-        for (int k = 0; k < m; k++) {
-          if (certainly_outside(pf, thr, sm.sf[k])) continue;
-          const double d2 = ds2_exact(xi - sm.sx[k], yi - sm.sy[k], zi - sm.sz[k]);
-          if (d2 < w2) {
-            if (cnt < cap) out[(size_t)cnt * kLeaf] = lj * kLeaf + k;
-            cnt++;
-          }
-        }
-      }
-    });
-  }
-  if (!ok && lane_id() == 0) raise_flag(a.flags, SPH_FLAG_STACK_OVERFLOW);
-  if (cnt > cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
-  if (valid) a.n_ngb[s] = cnt;
+template <int G>
+__global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(SolveArgs a) {
+  __shared__ WarpSmem<G> smem[kNgbWarps];
+  WarpSmem<G> &sm = smem[threadIdx.x >> 5];
+  Group<G> g;
+  g.open(a, sm);
+  for (int t = 0; t < g.count; t++)
+    solve_particle(a, sm, g.first + t, a.pos[g.first + t], g.nlist, g.stage(sm, t), g.w_list);
 }
 
-// scratch of the two-kernel solve: the queue count, the queue, the saved states
-size_t solve_work_bytes(int n, int nleaf) {
-  return 256 + ((size_t)nleaf * sizeof(int) + 255) / 256 * 256 + (size_t)n * sizeof(SolveSave);
+// dev_find_ngb (dev_find_ngb.cu:13-87): every j with ds2 < range_i^2, in
+// ascending slot order, at ranges set from outside.
+template <int G>
+__global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_find_ngb(SolveArgs a) {
+  __shared__ WarpSmem<G> smem[kNgbWarps];
+  WarpSmem<G> &sm = smem[threadIdx.x >> 5];
+  Group<G> g;
+  g.open(a, sm);
+  for (int t = 0; t < g.count; t++) {
+    const int s = g.first + t;
+    const double4 p = a.pos[s];
+    const int total = g.stage(sm, t);
+    int count = 0;
+    if (p.w > 0) count = eval_range<false>(a, sm, s, p, p.w, g.nlist, total, false).count;
+    if (lane_id() == 0) {
+      if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
+      a.n_ngb[s] = count;
+    }
+  }
+}
+
+template <int G>
+static void launch_group(const SolveArgs &a, bool solve, cudaStream_t st) {
+  const int warps = (a.s1 - a.s0 + G - 1) / G, blocks = (warps + kNgbWarps - 1) / kNgbWarps;
+  if (solve) k_solve_range<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
+  else k_find_ngb<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
+}
+
+// Four targets to a warp share the walk once that leaves enough warps: the
+// GPU holds 148 * 9 * 4 of them, and the launch should be four times that
+// with four targets each.  Below, one target to a warp (solve, us, by targets
+// to a warp 1 / 2 / 4 / 8: 16,384 particles 93 / 129 / 170 / 306; 60,000
+// 256 / 260 / 270 / 392; 262,144 1358 / 1187 / 1128 / 1236; 1,048,576 5417 /
+// 4442 / 4014 / 4055).
+constexpr int kShareFrom = 148 * kNgbBlocks * kNgbWarps * 16;
+
+static void launch_ngb(const SolveArgs &a, bool solve, cudaStream_t st) {
+  if (a.s1 - a.s0 >= kShareFrom) launch_group<kGroup>(a, solve, st);
+  else launch_group<1>(a, solve, st);
 }
 
 // leaves [leaf0, leaf1) (a shard's range, or 0 and the leaf count)
 int launch_solve_range(const TreeView &t, double4 *pos, int *nevals, unsigned *flags, const sph_params &p,
-                       int *n_ngb, int *list, double *dcache, int cap, void *work, int leaf0, int leaf1,
-                       cudaStream_t st) {
+                       int *n_ngb, int *list, int cap, int stride, int leaf0, int leaf1, cudaStream_t st) {
   SolveArgs a;
   a.t = t; a.pos = pos; a.nevals = nevals; a.flags = flags;
-  a.n_ngb = n_ngb; a.list = list; a.dcache = dcache; a.cap = cap;
+  a.n_ngb = n_ngb; a.list = list; a.cap = cap; a.stride = stride;
   a.n_target = p.n_target; a.rel_err = p.rel_err; a.f_scale = p.f_scale; a.max_iter = p.max_iter;
-  a.leaf0 = leaf0; a.leaf1 = leaf1;
-  a.queue = nullptr; a.queue_count = nullptr; a.save = nullptr;
-  const int warps = leaf1 - leaf0;
-  if (warps <= 0) return 0;
-  const int blocks = (warps + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  // the speculative first evaluation pays when the previous range is likely
-  // to pass the tolerance test already (not with a tight tolerance)
-  if (p.rel_err < 1e-8 || !work) {
-    k_solve_range<<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
-    return 1;
-  }
-  char *w = (char *)work;
-  a.queue_count = (int *)w;
-  a.queue = (int *)(w + 256);
-  a.save = (SolveSave *)(w + 256 + ((size_t)t.count[0] * sizeof(int) + 255) / 256 * 256);
-  cudaMemsetAsync(a.queue_count, 0, sizeof(int), st);
-  k_solve_spec<<<blocks, kWarpsPerBlock * 32, 0, st>>>(a);
-  // the resumed leaves (about a tenth in steady state) on the resident warps
-  const int resident = 148 * 6;
-  k_solve_range<<<blocks < resident ? blocks : resident, kWarpsPerBlock * 32, 0, st>>>(a);
-  return 2;
+  a.ordered = 4 + (int)fmin(p.n_target / 16.0, 1e6);
+  a.s0 = leaf0 * kLeaf; a.s1 = min(leaf1 * kLeaf, t.n);
+  if (a.s1 <= a.s0) return 0;
+  launch_ngb(a, true, st);
+  return 1;
 }
 
-int launch_find_ngb(const TreeView &t, const double4 *pos, int *n_ngb, int *list, int cap, unsigned *flags,
+int launch_find_ngb(const TreeView &t, double4 *pos, int *n_ngb, int *list, int cap, int stride, unsigned *flags,
                     int leaf0, int leaf1, cudaStream_t st) {
-  FindArgs a;
-  a.t = t; a.pos = pos; a.n_ngb = n_ngb; a.list = list; a.cap = cap; a.flags = flags;
-  a.leaf0 = leaf0; a.leaf1 = leaf1;
-  const int warps = leaf1 - leaf0;
-  if (warps <= 0) return 0;
-  k_find_ngb<<<(warps + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, st>>>(a);
+  SolveArgs a = {};
+  a.t = t; a.pos = pos; a.flags = flags;
+  a.n_ngb = n_ngb; a.list = list; a.cap = cap; a.stride = stride;
+  a.s0 = leaf0 * kLeaf; a.s1 = min(leaf1 * kLeaf, t.n);
+  if (a.s1 <= a.s0) return 0;
+  launch_ngb(a, false, st);
   return 1;
 }
 

@@ -236,7 +236,7 @@ __global__ void k_tree_moments(int n, const double4 *__restrict__ src, TgWork w)
 
 // -------------------------------- the walk -----------------------------------
 struct TreeGravArgs {
-  TreeView t;          // the SPH tree: its leaves are the groups
+  TreeView t;          // its leaves of kLeaf particles are the groups
   TgWork w;            // the gravity tree
   const double4 *src;  // {x, y, z, m} per particle, tree order
   const uint64_t *keys;  // the sorted keys of that order
@@ -607,7 +607,7 @@ int launch_tree_gravity(const TreeView &t, const uint64_t *keys, const double4 *
   }
   if (world > 1) cudaMemsetAsync(out, 0, sizeof(double4) * n, st);
   long long l0, l1;
-  shard_range(t.count[0], rank, world, l0, l1);
+  shard_range(t.nleaf, rank, world, l0, l1);
   if (l1 <= l0) return launches;
   TreeGravArgs a;
   a.t = t; a.w = w; a.src = src; a.keys = keys; a.out = out; a.flags = flags;
