@@ -83,6 +83,35 @@ __device__ __noinline__ void spline_near(R dx, R dy, R dz, R r2, R mj, R hi2, R 
   az = fma(dz, g, az);
 }
 
+// ------------------------------- slices --------------------------------------
+// A launch with too few blocks for the GPU cuts each block's sources into
+// `slices` parts, one block each (grav_slices below).  Slice q of [lo, hi) is
+// a whole number of UNIT-source batches, the sources whose FP32 terms the
+// mixed kernels add up before they fold into FP64: the sums then do not
+// depend on the slices but by the order of the FP64 additions.  The parts
+// meet by atomics in an output cleared beforehand.
+template <int UNIT>
+__device__ __forceinline__ void source_slice(int &lo, int &hi, unsigned q, int slices) {
+  if (slices == 1) return;
+  const int nb = (hi - lo + UNIT - 1) / UNIT;
+  const int b = nb * (int)q / slices, e = nb * ((int)q + 1) / slices;
+  hi = min(hi, lo + e * UNIT);
+  lo += b * UNIT;
+}
+
+__device__ __forceinline__ void add_sums(double4 *out, double x, double y, double z, double w) {
+  double *o = reinterpret_cast<double *>(out);
+  atomicAdd(o, x);
+  atomicAdd(o + 1, y);
+  atomicAdd(o + 2, z);
+  atomicAdd(o + 3, w);
+}
+
+__device__ __forceinline__ void store_sums(double4 *out, double x, double y, double z, double w, int slices) {
+  if (slices == 1) *out = make_double4(x, y, z, w);
+  else add_sums(out, x, y, z, w);
+}
+
 // -------------------------------- FP64 --------------------------------------
 // One-sided form: every i of the block against the sources [jlo, jhi); with
 // tile > 0 the range is the tile of `tile` particles that holds the block
@@ -90,13 +119,14 @@ __device__ __noinline__ void spline_near(R dx, R dy, R dz, R r2, R mj, R hi2, R 
 template <int SOFT, int R>
 __global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *__restrict__ src,
                                                         const double *__restrict__ h2src, double4 *__restrict__ out,
-                                                        double eps2, double G, int tile, int block0) {
+                                                        double eps2, double G, int tile, int block0, int slices) {
   __shared__ double4 sj[kGThreads];
   __shared__ double sh[SOFT == SPH_SOFT_SPLINE ? kGThreads : 1];
   const int t = threadIdx.x;
-  const int i0 = (blockIdx.x + block0) * kGThreads * R;
-  const int jlo = tile > 0 ? (i0 / tile) * tile : 0;
-  const int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  const int i0 = (blockIdx.x / slices + block0) * kGThreads * R;
+  int jlo = tile > 0 ? (i0 / tile) * tile : 0;
+  int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  source_slice<32>(jlo, jhi, blockIdx.x % slices, slices);
   double xi[R], yi[R], zi[R], hi2[R], ax[R], ay[R], az[R], pot[R];
 #pragma unroll
   for (int r = 0; r < R; r++) {
@@ -160,7 +190,7 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *__
 #pragma unroll
   for (int r = 0; r < R; r++) {
     const int i = i0 + r * kGThreads + t;
-    if (i < n) out[i] = make_double4(G * ax[r], G * ay[r], G * az[r], G * pot[r]);
+    if (i < n) store_sums(out + i, G * ax[r], G * ay[r], G * az[r], G * pot[r], slices);
   }
 }
 
@@ -177,11 +207,13 @@ __device__ __forceinline__ void kahan_add(float &hi, float &lo, float v) {
 template <int SOFT, int R>
 __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *__restrict__ src,
                                                         const double *__restrict__ h2src, double4 *__restrict__ out,
-                                                        float eps2, double G, int block0) {
+                                                        float eps2, double G, int block0, int slices) {
   __shared__ float4 sj[kGThreads];
   __shared__ float sh[SOFT == SPH_SOFT_SPLINE ? kGThreads : 1];
   const int t = threadIdx.x;
-  const int i0 = (blockIdx.x + block0) * kGThreads * R;
+  const int i0 = (blockIdx.x / slices + block0) * kGThreads * R;
+  int jlo = 0, jhi = n;
+  source_slice<kGThreads>(jlo, jhi, blockIdx.x % slices, slices);
   const double4 anc = src[min(i0, n - 1)];
   float xi[R], yi[R], zi[R], hi2[R];
   float ahi[R][4], alo[R][4];
@@ -196,16 +228,16 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *__
 #pragma unroll
     for (int c = 0; c < 4; c++) ahi[r][c] = alo[r][c] = 0.f;
   }
-  for (int j0 = 0; j0 < n; j0 += kGThreads) {
+  for (int j0 = jlo; j0 < jhi; j0 += kGThreads) {
     const int j = j0 + t;
     __syncthreads();
-    if (j < n) {
+    if (j < jhi) {
       const double4 q = src[j];
       sj[t] = make_float4((float)(q.x - anc.x), (float)(q.y - anc.y), (float)(q.z - anc.z), (float)q.w);
       if (SOFT == SPH_SOFT_SPLINE) sh[t] = (float)h2src[j];
     }
     __syncthreads();
-    const int m = min(kGThreads, n - j0);
+    const int m = min(kGThreads, jhi - j0);
     float px[R], py[R], pz[R], pp[R];
 #pragma unroll
     for (int r = 0; r < R; r++) px[r] = py[r] = pz[r] = pp[r] = 0.f;
@@ -280,8 +312,8 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *__
   for (int r = 0; r < R; r++) {
     const int i = i0 + r * kGThreads + t;
     if (i < n)
-      out[i] = make_double4(G * ((double)ahi[r][0] + (double)alo[r][0]), G * ((double)ahi[r][1] + (double)alo[r][1]),
-                            G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]));
+      store_sums(out + i, G * ((double)ahi[r][0] + (double)alo[r][0]), G * ((double)ahi[r][1] + (double)alo[r][1]),
+                 G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]), slices);
   }
 }
 
@@ -302,12 +334,13 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *__
 template <int RP>  // i-particle pairs per thread
 __global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const double4 *__restrict__ src,
                                                                   double4 *__restrict__ out, float eps2, double G,
-                                                                  int tile, int block0) {
+                                                                  int tile, int block0, int slices) {
   __shared__ ulonglong2 sj[kGThreads][2];
   const int t = threadIdx.x;
-  const int i0 = (blockIdx.x + block0) * kGThreads * 2 * RP;
-  const int jlo = tile > 0 ? (i0 / tile) * tile : 0;
-  const int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  const int i0 = (blockIdx.x / slices + block0) * kGThreads * 2 * RP;
+  int jlo = tile > 0 ? (i0 / tile) * tile : 0;
+  int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  source_slice<kGThreads>(jlo, jhi, blockIdx.x % slices, slices);
   const double4 anc = src[min(i0, n - 1)];
   f32x2 xi[RP], yi[RP], zi[RP];
   float ahi[2 * RP][4], alo[2 * RP][4];
@@ -382,8 +415,8 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const d
   for (int r = 0; r < 2 * RP; r++) {
     const int i = i0 + r * kGThreads + t;
     if (i < n)
-      out[i] = make_double4(G * ((double)ahi[r][0] + (double)alo[r][0]), G * ((double)ahi[r][1] + (double)alo[r][1]),
-                            G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]));
+      store_sums(out + i, G * ((double)ahi[r][0] + (double)alo[r][0]), G * ((double)ahi[r][1] + (double)alo[r][1]),
+                 G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]), slices);
   }
 }
 
@@ -438,10 +471,13 @@ template <bool UNI>
 __device__ __forceinline__ void sym_plummer_item(long long item, int n, int nt, const double4 *__restrict__ src,
                                                  double4 *__restrict__ out, float eps2, double G,
                                                  float (&red)[2][kSymWarps][4][32],
-                                                 double (&iacc)[2 * kSymRP * 4][kSymWarps * 32]) {
+                                                 double (&iacc)[2 * kSymRP * 4][kSymWarps * 32], unsigned slice,
+                                                 int slices) {
   int b, t_lo, t_hi;
   sym_item(item, nt, b, t_lo, t_hi);
-  const int j_lo = t_lo * kSymTile, j_hi = min(t_hi * kSymTile, n);
+  int j_lo = t_lo * kSymTile, j_hi = min(t_hi * kSymTile, n);
+  source_slice<32>(j_lo, j_hi, slice, slices);
+  if (j_lo >= j_hi) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nxt = (l + 1) & 31;
   const int i0 = b * kSymTile;
   const double4 anc = src[i0];
@@ -566,18 +602,19 @@ __device__ __forceinline__ void sym_plummer_item(long long item, int n, int nt, 
 }
 
 // mass_mixed: device word, 0 when all masses are equal (nullptr: general form);
-// block b runs work item item0 + b
+// block b runs slice b % slices of work item item0 + b / slices
 __global__ void __launch_bounds__(kSymWarps * 32, 4) k_grav_sym_plummer(int n, int nt, const double4 *__restrict__ src,
                                                                          double4 *__restrict__ out, float eps2,
                                                                          double G, const int *__restrict__ mass_mixed,
-                                                                         long long item0) {
+                                                                         long long item0, int slices) {
   __shared__ float red[2][kSymWarps][4][32];
   __shared__ double iacc[2 * kSymRP * 4][kSymWarps * 32];  // [i-slot * 4 + component][thread]
-  const long long item = item0 + blockIdx.x;
+  const long long item = item0 + blockIdx.x / slices;
+  const unsigned slice = blockIdx.x % slices;
   if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
-    sym_plummer_item<true>(item, n, nt, src, out, eps2, G, red, iacc);
+    sym_plummer_item<true>(item, n, nt, src, out, eps2, G, red, iacc, slice, slices);
   else
-    sym_plummer_item<false>(item, n, nt, src, out, eps2, G, red, iacc);
+    sym_plummer_item<false>(item, n, nt, src, out, eps2, G, red, iacc, slice, slices);
 }
 
 // ------------------- FP64, symmetric pair form ------------------------------
@@ -598,13 +635,58 @@ constexpr int kSym64Warps = 2;
 constexpr int kSym64R = 8;
 static_assert(2 * kSym64Warps * 32 * kSym64R == kSymTile, "the FP64 form shares the tile layout");
 
-template <bool UNI>
+// Spline softening (SOFT), each pair once as well (one-sided before: 60,000
+// particles with 24 neighbours 21.2 -> 4.3 ms, 5,000 2.03 -> 0.28): a pair farther apart than both ranges is Newtonian,
+// the rest -- about the neighbour count per particle -- follow the polynomials
+// of sph_grav_kernel.cu:40-106, whose acceleration factor is the same for both
+// sides and whose potential uses each side's own range.  "Far" is decided on
+// the high words of the FP64 squares (one integer compare, off the FP64
+// pipe; equal high words count as near), near pairs drop out of the main
+// sums by a squared distance of 1e300 and are added by sym_near when any lane
+// of the warp has one.  FP64 pipe bound like the Plummer form; the diagonal
+// tiles, where two of three warps hold a near pair, stay one-sided.
+struct NearPair {
+  double g;       // acceleration factor without the masses
+  double pi, pj;  // potentials at i and at j without the masses
+};
+
+__device__ __noinline__ NearPair spline_pair(double r2, double hi2, double hj2) {
+  const double inv = r2 > 0 ? rsqrt_f64(r2) : 0.0;
+  const double far = 0.5 * inv * inv * inv;
+  NearPair v;
+  v.g = far;
+  v.pi = -inv;
+  if (r2 < hi2) {
+    const double u2 = r2 / hi2, h = sqrt(hi2);
+    double ga;
+    spline_poly<double>(sqrt(u2), u2, ga, v.pi);
+    v.g = 0.5 * ga / (hi2 * h);
+    v.pi /= h;
+  }
+  double gj = far;
+  v.pj = -inv;
+  if (r2 < hj2) {
+    const double u2 = r2 / hj2, h = sqrt(hj2);
+    double ga;
+    spline_poly<double>(sqrt(u2), u2, ga, v.pj);
+    gj = 0.5 * ga / (hj2 * h);
+    v.pj /= h;
+  }
+  v.g += gj;
+  return v;
+}
+
+template <bool UNI, int SOFT>
 __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, const double4 *__restrict__ src,
-                                             double4 *__restrict__ out, double eps2, double G,
-                                             double (&red)[2][kSym64Warps][4][32], int half) {
+                                             const double *__restrict__ h2src, double4 *__restrict__ out, double eps2,
+                                             double G, double (&red)[2][kSym64Warps][4][32], int half, unsigned slice,
+                                             int slices) {
+  constexpr bool SPL = SOFT == SPH_SOFT_SPLINE;
   int b, t_lo, t_hi;
   sym_item(item, nt, b, t_lo, t_hi);
-  const int j_lo = t_lo * kSymTile, j_hi = min(t_hi * kSymTile, n);
+  int j_lo = t_lo * kSymTile, j_hi = min(t_hi * kSymTile, n);
+  source_slice<32>(j_lo, j_hi, slice, slices);
+  if (j_lo >= j_hi) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nxt = (l + 1) & 31;
   const int ib = b * kSymTile + half * (kSymTile / 2) + w * 32 * kSym64R + l;
   const double4 far = src[b * kSymTile];  // position given to padding i-slots
@@ -612,28 +694,36 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
 
   double xi[kSym64R], yi[kSym64R], zi[kSym64R], nmi[kSym64R];
   double ax[kSym64R], ay[kSym64R], az[kSym64R], ap[kSym64R];
+  int hi[kSym64R];  // SPL: high words of the squared ranges
 #pragma unroll
   for (int r = 0; r < kSym64R; r++) {
     const int i = ib + r * 32;  // i-tiles of work items are full tiles (b < nt - 1)
     const double4 q = i < n ? src[i] : make_double4(far.x, far.y, far.z, 0.0);
     xi[r] = q.x; yi[r] = q.y; zi[r] = q.z; nmi[r] = -q.w;
+    hi[r] = SPL && i < n ? __double2hiint(h2src[i]) : 0;
     ax[r] = ay[r] = az[r] = ap[r] = 0.0;
   }
   int k = 0;
   for (int jb = j_lo; jb < j_hi; jb += 32, k ^= 1) {
     // padding source: massless at a real position of the i-tile (s^2 >= eps^2 > 0);
-    // UNI: 1e150 away (d / s^3 underflows to 0; mj is unused)
+    // UNI and SPL: 1e150 away (d / s^3 underflows to 0; mj is unused or 0)
     const bool real = jb + l < j_hi;
-    const double4 q = real ? src[jb + l] : (UNI ? make_double4(1e150, 1e150, 1e150, 0.0)
-                                                : make_double4(far.x, far.y, far.z, 0.0));
+    const double4 q = real ? src[jb + l] : (UNI || SPL ? make_double4(1e150, 1e150, 1e150, 0.0)
+                                                       : make_double4(far.x, far.y, far.z, 0.0));
     double xj = q.x, yj = q.y, zj = q.z, mj = UNI ? (real ? 1.0 : 0.0) : q.w;
+    int hj = SPL && real ? __double2hiint(h2src[jb + l]) : 0;
     double bx = 0.0, by = 0.0, bz = 0.0, bp = 0.0;
 #pragma unroll 1
     for (int s = 0; s < 32; s++) {
+      unsigned near = 0u;  // SPL: bit r set where pair r is within a range
 #pragma unroll
       for (int r = 0; r < kSym64R; r++) {
         const double dx = xj - xi[r], dy = yj - yi[r], dz = zj - zi[r];
-        const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
+        double r2 = SPL ? fma(dz, dz, fma(dy, dy, dx * dx)) : fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
+        if (SPL && __double2hiint(r2) <= max(hi[r], hj)) {
+          near |= 1u << r;
+          r2 = 1e300;
+        }
         const double inv = rsqrt_f64(r2);
         const double inv3 = inv * inv * inv;
         if (UNI) {
@@ -657,10 +747,31 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
           bp = fma(nmi[r], inv, bp);
         }
       }
+      if (SPL && __any_sync(0xffffffffu, near != 0u)) {
+        const int j = jb + ((l + s) & 31);  // the source at this lane now (near: a real one)
+#pragma unroll
+        for (int r = 0; r < kSym64R; r++) {
+          if ((near >> r) & 1u) {
+            const double dx = xj - xi[r], dy = yj - yi[r], dz = zj - zi[r];
+            const NearPair v = spline_pair(fma(dz, dz, fma(dy, dy, dx * dx)), h2src[ib + r * 32], h2src[j]);
+            const double gi = UNI ? v.g : mj * v.g, gj = UNI ? v.g : nmi[r] * v.g;
+            ax[r] = fma(dx, gi, ax[r]);
+            ay[r] = fma(dy, gi, ay[r]);
+            az[r] = fma(dz, gi, az[r]);
+            ap[r] += UNI ? v.pi : mj * v.pi;
+            bx = fma(dx, gj, bx);
+            by = fma(dy, gj, by);
+            bz = fma(dz, gj, bz);
+            bp -= UNI ? v.pj : nmi[r] * v.pj;
+          }
+        }
+        __syncwarp();
+      }
       xj = __shfl_sync(0xffffffffu, xj, nxt);
       yj = __shfl_sync(0xffffffffu, yj, nxt);
       zj = __shfl_sync(0xffffffffu, zj, nxt);
       if (!UNI) mj = __shfl_sync(0xffffffffu, mj, nxt);
+      if (SPL) hj = __shfl_sync(0xffffffffu, hj, nxt);
       bx = __shfl_sync(0xffffffffu, bx, nxt);
       by = __shfl_sync(0xffffffffu, by, nxt);
       bz = __shfl_sync(0xffffffffu, bz, nxt);
@@ -682,25 +793,25 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
 #pragma unroll
   for (int r = 0; r < kSym64R; r++) {
     const int i = ib + r * 32;
-    if (i < n) {
-      double *o = reinterpret_cast<double *>(out + i);
-      atomicAdd(o + 0, G * mi_scale * ax[r]);
-      atomicAdd(o + 1, G * mi_scale * ay[r]);
-      atomicAdd(o + 2, G * mi_scale * az[r]);
-      atomicAdd(o + 3, G * mi_scale * ap[r]);
-    }
+    if (i < n) add_sums(out + i, G * mi_scale * ax[r], G * mi_scale * ay[r], G * mi_scale * az[r], G * mi_scale * ap[r]);
   }
 }
 
+// block b runs slice b / 2 % slices of work item item0 + b / 2 / slices, on
+// one half of its i-tile (b & 1)
+template <int SOFT>
 __global__ void __launch_bounds__(kSym64Warps * 32) k_grav_sym_f64(int n, int nt, const double4 *__restrict__ src,
+                                                                  const double *__restrict__ h2src,
                                                                   double4 *__restrict__ out, double eps2, double G,
-                                                                  const int *__restrict__ mass_mixed, long long item0) {
+                                                                  const int *__restrict__ mass_mixed, long long item0,
+                                                                  int slices) {
   __shared__ double red[2][kSym64Warps][4][32];
-  const long long item = item0 + (blockIdx.x >> 1);  // two blocks per item, one per half of the i-tile
+  const unsigned q = blockIdx.x >> 1;
+  const long long item = item0 + q / slices;
   if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
-    sym_f64_item<true>(item, n, nt, src, out, eps2, G, red, blockIdx.x & 1);
+    sym_f64_item<true, SOFT>(item, n, nt, src, h2src, out, eps2, G, red, blockIdx.x & 1, q % slices, slices);
   else
-    sym_f64_item<false>(item, n, nt, src, out, eps2, G, red, blockIdx.x & 1);
+    sym_f64_item<false, SOFT>(item, n, nt, src, h2src, out, eps2, G, red, blockIdx.x & 1, q % slices, slices);
 }
 
 // blocks [lo, hi) of a one-sided or symmetric launch (nothing when empty)
@@ -745,62 +856,86 @@ static GravPlan grav_plan(int n, int soft_mode, int precision, int rank, int wor
   return g;
 }
 
+// Slices of each block's sources (source_slice), a power of two: while the
+// launch has fewer blocks than `want` and a slice keeps `least` sources.
+// Uncut, a small set leaves most of the GPU idle (16,384 particles have 120
+// tile pairs for 592 resident blocks) and a launch of one to a few rounds of
+// blocks ends on a nearly empty one.  Gravity phase, us, uncut / cut: FP64
+// 1,000 particles 107 / 21, 2,049 331 / 33, 6,000 334 / 69, 16,384 348 / 245,
+// 100,003 8402 / 6875; mixed 6,000 239 / 56, 16,384 244 / 150, 30,000 417 /
+// 335, 65,536 1485 / 1331, 100,003 4303 / 2992, 262,144 19,980 / 19,360 (four
+// rounds instead of sixteen: 100,003 3193, 262,144 19,967).  From about
+// 400,000 particles on nothing is cut.
+static int grav_slices(long long blocks, int sources, long long want, int least) {
+  int s = 1;
+  while (blocks * s < want && sources / (2 * s) >= least) s *= 2;
+  return s;
+}
+
 // src = {x, y, z, m} per particle; h2src = range^2 (spline mode only).
 // Shard `rank` of `world` (world > 1) computes its contiguous share of the
 // one-sided blocks (diagonal tiles, or all pairs for small n / spline
 // softening) and of the symmetric work items into `out`, which it zeroes
 // first: the element-wise sum of the shards' outputs is the whole sum.
+// FP64 spline softening on one rank takes the symmetric tiles as well.
 int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out, int soft_mode, double eps, double G,
                    int precision, const int *mass_mixed, int rank, int world, cudaStream_t st) {
   if (n <= 0) return 0;
-  if (world > 1) cudaMemsetAsync(out, 0, sizeof(double4) * n, st);
   const double eps2 = eps * eps;
-  const GravPlan g = grav_plan(n, soft_mode, precision, rank, world);
+  GravPlan g = grav_plan(n, soft_mode, precision, rank, world);
   const int nt = g.nt;
+  if (soft_mode == SPH_SOFT_SPLINE && precision == SPH_PREC_FP64 && world == 1 && nt >= 2) {
+    g.tile = kSymTile;
+    g.items = Span{0, sym_items(nt)};
+  }
   const Span &blocks = g.blocks, &items = g.items;
+  // one-sided blocks: four to an SM; symmetric blocks run four to an SM
+  // (registers): sixteen rounds of them while a slice keeps 256 sources, two
+  // rounds while it keeps 32
+  const int sources = g.tile > 0 ? g.tile : n;
+  const int sb = blocks.empty() ? 1 : grav_slices(blocks.hi - blocks.lo, sources, 148 * 4,
+                                                  precision == SPH_PREC_FP64 ? 32 : kGThreads);
+  int si = 1;
+  if (!items.empty()) {
+    const long long per = (items.hi - items.lo) * (precision == SPH_PREC_FP64 ? 2 : 1);
+    si = grav_slices(per, g.chunk * kSymTile, 592 * 16, 256);
+    si *= grav_slices(per * si, g.chunk * kSymTile / si, 592 * 2, 32);
+  }
+  if (world > 1 || sb > 1) cudaMemsetAsync(out, 0, sizeof(double4) * n, st);
   int launches = 0;
   if (precision == SPH_PREC_FP64) {
     constexpr int R = 2;
     static_assert(kSymTile % (kGThreads * R) == 0, "diagonal tiles must hold whole blocks");
-    if (soft_mode == SPH_SOFT_PLUMMER) {
-      // diagonal tiles one-sided (all pairs when there is a single tile), then the items above them
-      if (!blocks.empty()) {
-        k_grav_f64<SPH_SOFT_PLUMMER, R><<<blocks.grid(), kGThreads, 0, st>>>(n, src, h2src, out, eps2, G, g.tile,
-                                                                            (int)blocks.lo);
-        launches++;
-      }
-      if (!items.empty()) {
-        k_grav_sym_f64<<<items.grid() * 2, kSym64Warps * 32, 0, st>>>(n, nt, src, out, eps2, G, mass_mixed, items.lo);
-        launches++;
-      }
-    } else if (!blocks.empty()) {
-      k_grav_f64<SPH_SOFT_SPLINE, R><<<blocks.grid(), kGThreads, 0, st>>>(n, src, h2src, out, eps2, G, 0,
-                                                                         (int)blocks.lo);
+    // diagonal tiles one-sided (all pairs when there is a single tile), then the items above them
+    const bool plummer = soft_mode == SPH_SOFT_PLUMMER;
+    if (!blocks.empty()) {
+      (plummer ? k_grav_f64<SPH_SOFT_PLUMMER, R> : k_grav_f64<SPH_SOFT_SPLINE, R>)
+          <<<blocks.grid() * sb, kGThreads, 0, st>>>(n, src, h2src, out, eps2, G, g.tile, (int)blocks.lo, sb);
       launches++;
     }
-  } else {
-    if (soft_mode == SPH_SOFT_PLUMMER) {
-      constexpr int RP = 1;
-      static_assert(kSymTile % (kGThreads * 2 * RP) == 0, "diagonal tiles must hold whole blocks");
-      // diagonal tiles store, the symmetric items add on top
-      if (!blocks.empty()) {
-        k_grav_f32x2_plummer<RP><<<blocks.grid(), kGThreads, 0, st>>>(n, src, out, (float)eps2, G, g.tile,
-                                                                     (int)blocks.lo);
-        launches++;
-      }
-      if (!items.empty()) {
-        k_grav_sym_plummer<<<items.grid(), kSymWarps * 32, 0, st>>>(n, nt, src, out, (float)eps2, G, mass_mixed,
-                                                                    items.lo);
-        launches++;
-      }
-    } else {
-      constexpr int R = 4;
-      if (!blocks.empty()) {
-        k_grav_f32<SPH_SOFT_SPLINE, R><<<blocks.grid(), kGThreads, 0, st>>>(n, src, h2src, out, (float)eps2, G,
-                                                                           (int)blocks.lo);
-        launches++;
-      }
+    if (!items.empty()) {
+      (plummer ? k_grav_sym_f64<SPH_SOFT_PLUMMER> : k_grav_sym_f64<SPH_SOFT_SPLINE>)
+          <<<items.grid() * 2 * si, kSym64Warps * 32, 0, st>>>(n, nt, src, h2src, out, eps2, G, mass_mixed, items.lo,
+                                                               si);
+      launches++;
     }
+  } else if (soft_mode == SPH_SOFT_PLUMMER) {
+    constexpr int RP = 1;
+    static_assert(kSymTile % (kGThreads * 2 * RP) == 0, "diagonal tiles must hold whole blocks");
+    if (!blocks.empty()) {
+      k_grav_f32x2_plummer<RP><<<blocks.grid() * sb, kGThreads, 0, st>>>(n, src, out, (float)eps2, G, g.tile,
+                                                                        (int)blocks.lo, sb);
+      launches++;
+    }
+    if (!items.empty()) {
+      k_grav_sym_plummer<<<items.grid() * si, kSymWarps * 32, 0, st>>>(n, nt, src, out, (float)eps2, G, mass_mixed,
+                                                                       items.lo, si);
+      launches++;
+    }
+  } else if (!blocks.empty()) {
+    k_grav_f32<SPH_SOFT_SPLINE, 4><<<blocks.grid() * sb, kGThreads, 0, st>>>(n, src, h2src, out, (float)eps2, G,
+                                                                            (int)blocks.lo, sb);
+    launches++;
   }
   return launches;
 }

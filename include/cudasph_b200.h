@@ -308,7 +308,9 @@ int cudasph_radix_sort_u64_noalloc(int n, uint64_t *keys, uint32_t *vals, void *
  * per one-sided block, [2..3] = the shard's one-sided blocks [lo, hi) (each
  * block's particles against the sources of their own tile, or against all
  * sources when the tile is 0), [4..5] = its symmetric work items [lo, hi),
- * [6] = tiles, [7] = tiles per item.  No counterpart in the reference (one
+ * [6] = tiles, [7] = tiles per item.  A single FP64 rank with spline softening
+ * runs the symmetric items of the tiles too, which this plan of the shards'
+ * work does not list.  No counterpart in the reference (one
  * GPU, CUDA_gravity.cpp:3-71). */
 int cudasph_gravity_plan(int n, int precision, int soft_mode, int rank, int world, long long *out8);
 /* symmetric work item -> i-tile `row` and j-tiles [t_lo, t_hi) above it;
