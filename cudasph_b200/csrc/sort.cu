@@ -5,18 +5,14 @@
 // Keys: positions quantised to 21 bits per dimension in the bounding cube
 // (scale = 2^21 / max extent, like domain_fac of sort_bodies.cpp:135), bits
 // interleaved x-y-z from the top.  The sort is an 8-bit-digit LSD radix sort
-// (8 passes over 64-bit keys): per pass a per-block digit histogram, one
-// exclusive scan over [digit][block], and a stable scatter in which each
-// warp ranks equal digits with __match_any_sync.  Ties keep their input
-// order, so with values = slot indices the permutation equals a stable sort.
+// (8 passes over 64-bit keys), one launch per pass, described below.  Ties
+// keep their input order, so with values = slot indices the permutation
+// equals a stable sort.
 #include <cstdio>
 
 #include "common.cuh"
 
 namespace sph {
-
-constexpr int kRadixThreads = 256;
-constexpr int kRadixChunk = 4096;  // keys per block per pass
 
 __global__ void k_bbox_partial(int n, const double4 *__restrict__ pos, const double *__restrict__ x,
                                const double *__restrict__ y, const double *__restrict__ z, double *__restrict__ part) {
@@ -52,12 +48,36 @@ __global__ void k_bbox_partial(int n, const double4 *__restrict__ pos, const dou
   }
 }
 
+// the bounding box from the block partials (at most one per thread), by one
+// block (thread 0 alone walked them before: 85 us for 296 partials, now 4)
+constexpr int kBoxBlocks = 148 * 2, kBoxThreads = 320;
+__device__ __forceinline__ void fold_box(int nb, const double *__restrict__ part, double *lo, double *hi) {
+  __shared__ double s[kBoxThreads / 32][6];
+  const int t = threadIdx.x;
+  for (int d = 0; d < 3; d++) {
+    lo[d] = t < nb ? part[t * 6 + d] : 1e308;
+    hi[d] = t < nb ? part[t * 6 + 3 + d] : -1e308;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+  if (lane_id() == 0)
+    for (int d = 0; d < 3; d++) { s[t >> 5][d] = lo[d]; s[t >> 5][3 + d] = hi[d]; }
+  __syncthreads();
+  for (int w = 0; w < kBoxThreads / 32; w++)
+    for (int d = 0; d < 3; d++) { lo[d] = fmin(lo[d], s[w][d]); hi[d] = fmax(hi[d], s[w][3 + d]); }
+}
+
 // box4 = {lo.x, lo.y, lo.z, scale}; scale = 2^21 / max extent (0 if degenerate)
-__global__ void k_bbox_final(int nb, const double *__restrict__ part, double *__restrict__ box4) {
+__global__ void __launch_bounds__(kBoxThreads) k_bbox_final(int nb, const double *__restrict__ part,
+                                                            double *__restrict__ box4) {
+  double lo[3], hi[3];
+  fold_box(nb, part, lo, hi);
   if (threadIdx.x != 0) return;
-  double lo[3] = {1e308, 1e308, 1e308}, hi[3] = {-1e308, -1e308, -1e308};
-  for (int b = 0; b < nb; b++)
-    for (int d = 0; d < 3; d++) { lo[d] = fmin(lo[d], part[b * 6 + d]); hi[d] = fmax(hi[d], part[b * 6 + 3 + d]); }
   double size = hi[0] - lo[0];
   if (hi[1] - lo[1] > size) size = hi[1] - lo[1];
   if (hi[2] - lo[2] > size) size = hi[2] - lo[2];
@@ -98,135 +118,305 @@ __global__ void k_morton(int n, const double4 *__restrict__ pos, const double *_
   if (vals) vals[i] = (uint32_t)i;
 }
 
-// per-block digit histogram, stored digit-major: hist[d * nb + block]
-__global__ void __launch_bounds__(kRadixThreads) k_radix_hist(int n, const uint64_t *__restrict__ keys, int shift,
-                                                              unsigned *__restrict__ hist) {
+// ---------------------------------------------------------------------------
+// The radix sort.  The keys are cut into tiles of 2,048 or 4,096; a pass needs, for
+// every tile, the number of its keys of each digit.  Those counts come from
+// the pass before: when a key is written to its place, the place's tile and
+// the key's next digit are known, and one count is added (a warp's equal ones
+// together).  So a pass is one launch: each block adds up the counts of the
+// tiles before its own and of all smaller digits, ranks its keys, sorts them
+// by digit in shared memory and writes runs of equal digits.  Only the first
+// pass needs a launch of its own for its counts.
+//
+// Three count tables rotate: a pass reads one, adds to the next and clears
+// its row of the third, which is the next one's to add to.
+//
+// Before, a pass was a histogram, a scan in one block and a scatter with four
+// block barriers per 256 keys: 25 - 45 us a pass at every size.  Whole
+// sort, us, before / now: 2,049 keys 134 / 34, 16,384 184 / 73, 262,144 207 /
+// 104, 1,048,576 353 / 183, 2,000,003 656 / 340.
+// ---------------------------------------------------------------------------
+constexpr int kRadixItems = 8;  // keys per thread
+constexpr int kTileSmall = 256 * kRadixItems, kTileLarge = 512 * kRadixItems;
+// up to so many tiles every block reads the whole table of counts (1 KB a
+// tile) itself; beyond, a launch before each pass adds them up
+constexpr int kDirectTiles = 256;
+
+template <int T>  // threads of a block
+struct RadixSmem {
+  union {
+    uint64_t key[T * kRadixItems];
+    uint32_t val[T * kRadixItems];
+    unsigned fold[2][T / 64][256];
+  };
+  unsigned short count[T / 32][256];
+  unsigned start[256];  // first place of each digit in the sorted tile
+  unsigned dest[256];   // global place of a digit's first key of this tile, less its place in the sorted tile
+  unsigned warp_sum[8];
+};
+static_assert(sizeof(RadixSmem<512>) <= 48 * 1024, "static shared memory");
+
+// exclusive sum over the 256 values of threads 0 .. 255 (all threads call)
+template <int T>
+__device__ __forceinline__ unsigned scan256(RadixSmem<T> &sm, unsigned v) {
+  const int t = threadIdx.x, l = t & 31;
+  unsigned inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (l >= o) inc += u;
+  }
+  __syncthreads();
+  if (t < 256 && l == 31) sm.warp_sum[t >> 5] = inc;
+  __syncthreads();
+  unsigned before = 0;
+  for (int w = 0; w < 8; w++)
+    if (w < (t >> 5)) before += sm.warp_sum[w];
+  return before + inc - v;
+}
+
+// Places of the thread's keys in the tile sorted by digit (stable: a warp
+// holds consecutive keys, item by item), and sm.start.  Past the tile's last
+// key the caller passes all ones: those take the last places.
+template <int T>
+__device__ __forceinline__ void rank_tile(RadixSmem<T> &sm, const uint64_t (&k)[kRadixItems], int shift,
+                                          unsigned (&place)[kRadixItems]) {
+  const int t = threadIdx.x, w = t >> 5, l = t & 31;
+  const unsigned lt = (1u << l) - 1u;
+  for (int d = l; d < 256; d += 32) sm.count[w][d] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const unsigned d = (unsigned)(k[i] >> shift) & 255u;
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+      const bool bit = (d >> b) & 1u;
+      const unsigned m = __ballot_sync(0xffffffffu, bit);
+      peers &= bit ? m : ~m;
+    }
+    const unsigned before = sm.count[w][d];
+    place[i] = before + __popc(peers & lt);
+    __syncwarp();
+    if ((peers & lt) == 0u) sm.count[w][d] = (unsigned short)(before + __popc(peers));
+    __syncwarp();
+  }
+  __syncthreads();
+  unsigned total = 0;
+  if (t < 256)
+    for (int v = 0; v < T / 32; v++) {
+      const unsigned c = sm.count[v][t];
+      sm.count[v][t] = (unsigned short)total;
+      total += c;
+    }
+  const unsigned first = scan256(sm, total);
+  if (t < 256) sm.start[t] = first;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const unsigned d = (unsigned)(k[i] >> shift) & 255u;
+    place[i] += sm.start[d] + sm.count[w][d];
+  }
+}
+
+// counts of the first digit, and the second table cleared
+template <int T>
+__global__ void __launch_bounds__(T) k_radix_count(int n, const uint64_t *__restrict__ keys,
+                                                               unsigned *__restrict__ table,
+                                                               unsigned *__restrict__ next) {
   __shared__ unsigned h[256];
-  h[threadIdx.x] = 0;
+  const int t = threadIdx.x;
+  if (t < 256) h[t] = 0;
   __syncthreads();
-  int beg = blockIdx.x * kRadixChunk, end = min(n, beg + kRadixChunk);
-  for (int i = beg + threadIdx.x; i < end; i += kRadixThreads) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
+  const int beg = blockIdx.x * T * kRadixItems, end = min(n, beg + T * kRadixItems);
+  for (int i = beg + t; i < end; i += T) atomicAdd(&h[keys[i] & 255u], 1u);
   __syncthreads();
-  hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
-}
-
-// exclusive scan of m entries in one block of 1024 threads: warp w owns the
-// contiguous segment [w * seg, (w + 1) * seg) and walks it in coalesced
-// 32-entry chunks (warp shuffle scan per chunk); a first pass sums the
-// segments, a block scan of the 32 segment sums gives each warp its offset,
-// a second pass writes the prefixes.
-__global__ void __launch_bounds__(1024) k_radix_scan(int m, unsigned *__restrict__ hist) {
-  __shared__ unsigned seg_sum[32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int seg = (m + 31) / 32;
-  const int beg = w * seg, end = min(m, beg + seg);
-  unsigned tot = 0;
-  for (int i = beg + l; i < end; i += 32) tot += hist[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if (l == 0) seg_sum[w] = tot;
-  __syncthreads();
-  if (w == 0) {
-    const unsigned v = seg_sum[l];
-    unsigned inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (l >= o) inc += t;
-    }
-    seg_sum[l] = inc - v;  // exclusive
-  }
-  __syncthreads();
-  unsigned run = seg_sum[w];
-  for (int c = beg; c < end; c += 32) {
-    const int i = c + l;
-    const unsigned v = i < end ? hist[i] : 0u;
-    unsigned inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (l >= o) inc += t;
-    }
-    if (i < end) hist[i] = run + inc - v;
-    run += __shfl_sync(0xffffffffu, inc, 31);
+  if (t < 256) {
+    table[blockIdx.x * 256 + t] = h[t];
+    next[blockIdx.x * 256 + t] = 0u;
   }
 }
 
-__global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(int n, const uint64_t *__restrict__ kin,
-                                                                 const uint32_t *__restrict__ vin,
-                                                                 uint64_t *__restrict__ kout,
-                                                                 uint32_t *__restrict__ vout, int shift,
-                                                                 const unsigned *__restrict__ hist) {
-  __shared__ unsigned s_base[256];
-  __shared__ unsigned s_cnt[kRadixThreads / 32][256];
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  s_base[t] = hist[t * gridDim.x + blockIdx.x];
-#pragma unroll
-  for (int w = 0; w < kRadixThreads / 32; w++) s_cnt[w][t] = 0;
+// many tiles: each tile's counts replaced by those of the tiles before it,
+// and the digits' totals; 32 digits per block, 32 runs of tiles per digit
+__global__ void __launch_bounds__(1024) k_radix_prefix(int tiles, unsigned *__restrict__ table,
+                                                       unsigned *__restrict__ total) {
+  __shared__ unsigned run[32][33];
+  const int d = threadIdx.x & 31, r = threadIdx.x >> 5, digit = blockIdx.x * 32 + d;
+  const int b = (int)((long long)tiles * r / 32), e = (int)((long long)tiles * (r + 1) / 32);
+  unsigned s = 0;
+  for (int i = b; i < e; i++) s += table[(size_t)i * 256 + digit];
+  run[r][d] = s;
   __syncthreads();
-  const int beg = blockIdx.x * kRadixChunk, end = min(n, beg + kRadixChunk);
-  const unsigned lt = (1u << lane) - 1u;
-  for (int base = beg; base < end; base += kRadixThreads) {
-    int i = base + t;
-    bool valid = i < end;
-    uint64_t k = valid ? kin[i] : 0;
-    uint32_t v = valid ? vin[i] : 0;
-    unsigned d = valid ? (unsigned)((k >> shift) & 255u) : 256u;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    unsigned rank = __popc(peers & lt);
-    if (valid && rank == 0) s_cnt[warp][d] = __popc(peers);
+  unsigned before = 0, all = 0;
+  for (int q = 0; q < 32; q++) {
+    if (q == r) before = all;
+    all += run[q][d];
+  }
+  for (int i = b; i < e; i++) {
+    const unsigned c = table[(size_t)i * 256 + digit];
+    table[(size_t)i * 256 + digit] = before;
+    before += c;
+  }
+  if (r == 0) total[digit] = all;
+}
+
+// One pass.  total: null when the block adds the counts up itself.  next,
+// clear: null in the last pass.
+template <int T>
+__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_radix_pass(int n, int tiles, const uint64_t *__restrict__ kin,
+                                                              const uint32_t *__restrict__ vin,
+                                                              uint64_t *__restrict__ kout,
+                                                              uint32_t *__restrict__ vout, int shift,
+                                                              const unsigned *__restrict__ table,
+                                                              const unsigned *__restrict__ total,
+                                                              unsigned *__restrict__ next,
+                                                              unsigned *__restrict__ clear) {
+  constexpr int kTile = T * kRadixItems;
+  __shared__ RadixSmem<T> sm;
+  const int t = threadIdx.x, w = t >> 5, l = t & 31, tile = blockIdx.x;
+  const int beg = tile * kTile, held = min(n - beg, kTile);
+  uint64_t k[kRadixItems];
+  uint32_t v[kRadixItems];
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const int at = w * (32 * kRadixItems) + i * 32 + l;
+    k[i] = at < held ? kin[beg + at] : ~0ull;
+    v[i] = at < held ? vin[beg + at] : 0u;
+  }
+  // digit t: keys of it in earlier tiles, and in all
+  unsigned before = 0, all = 0;
+  if (total) {
+    if (t < 256) {
+      before = table[(size_t)tile * 256 + t];
+      all = total[t];
+    }
+  } else {
+    const int g = t >> 6, q = t & 63;  // row group, four digits
+    uint4 b4 = make_uint4(0, 0, 0, 0), a4 = b4;
+    for (int r = g; r < tiles; r += T / 64) {
+      const uint4 c = *reinterpret_cast<const uint4 *>(table + (size_t)r * 256 + q * 4);
+      a4.x += c.x; a4.y += c.y; a4.z += c.z; a4.w += c.w;
+      if (r < tile) { b4.x += c.x; b4.y += c.y; b4.z += c.z; b4.w += c.w; }
+    }
+    *reinterpret_cast<uint4 *>(&sm.fold[0][g][q * 4]) = b4;
+    *reinterpret_cast<uint4 *>(&sm.fold[1][g][q * 4]) = a4;
     __syncthreads();
-    {  // thread t owns digit t: exclusive prefix across warps
-      unsigned run = s_base[t];
-#pragma unroll
-      for (int w = 0; w < kRadixThreads / 32; w++) {
-        unsigned c = s_cnt[w][t];
-        s_cnt[w][t] = run;
-        run += c;
+    if (t < 256)
+      for (int r = 0; r < T / 64; r++) {
+        before += sm.fold[0][r][t];
+        all += sm.fold[1][r][t];
       }
-      s_base[t] = run;
-    }
-    __syncthreads();
-    if (valid) {
-      unsigned o = s_cnt[warp][d] + rank;
-      kout[o] = k;
-      vout[o] = v;
-    }
-    __syncthreads();
+  }
+  before += scan256(sm, all);
+  unsigned place[kRadixItems];
+  rank_tile(sm, k, shift, place);
+  if (t < 256) {
+    sm.dest[t] = before - sm.start[t];
+    if (clear) clear[(size_t)tile * 256 + t] = 0u;
+  }
 #pragma unroll
-    for (int w = 0; w < kRadixThreads / 32; w++) s_cnt[w][t] = 0;
-    __syncthreads();
+  for (int i = 0; i < kRadixItems; i++) sm.key[place[i]] = k[i];
+  __syncthreads();
+  unsigned to[kRadixItems];
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const int at = i * T + t;
+    const uint64_t key = sm.key[at];
+    to[i] = sm.dest[(unsigned)(key >> shift) & 255u] + (unsigned)at;
+    if (at < held) kout[to[i]] = key;
+    if (next) {
+      const unsigned slot = at < held ? to[i] / kTile * 256u + ((unsigned)(key >> (shift + 8)) & 255u) : 0xffffffffu;
+      const unsigned peers = __match_any_sync(0xffffffffu, slot);
+      if (at < held && (peers & ((1u << l) - 1u)) == 0u) atomicAdd(next + slot, (unsigned)__popc(peers));
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) sm.val[place[i]] = v[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const int at = i * T + t;
+    if (at < held) vout[to[i]] = sm.val[at];
   }
 }
 
-size_t radix_scratch_bytes(int n) {
-  size_t nb = (size_t)(n + kRadixChunk - 1) / kRadixChunk;
-  if (nb == 0) nb = 1;
-  size_t b = 0;
-  b += ((size_t)n * 8 + 255) / 256 * 256;    // keys ping-pong
-  b += ((size_t)n * 4 + 255) / 256 * 256;    // vals ping-pong
-  b += (256 * nb * 4 + 255) / 256 * 256;     // histograms
-  return b;
+// a single tile: all passes in one launch, in place
+__global__ void __launch_bounds__(512) k_radix_tile(int n, uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+  __shared__ RadixSmem<512> sm;
+  const int t = threadIdx.x, w = t >> 5, l = t & 31;
+  uint64_t k[kRadixItems];
+  uint32_t v[kRadixItems];
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const int at = w * (32 * kRadixItems) + i * 32 + l;
+    k[i] = at < n ? keys[at] : ~0ull;  // stable: these stay last among equals
+    v[i] = at < n ? vals[at] : 0u;
+  }
+#pragma unroll 1
+  for (int shift = 0; shift < 64; shift += 8) {
+    unsigned place[kRadixItems];
+    rank_tile(sm, k, shift, place);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) sm.key[place[i]] = k[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) k[i] = sm.key[w * (32 * kRadixItems) + i * 32 + l];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) sm.val[place[i]] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRadixItems; i++) v[i] = sm.val[w * (32 * kRadixItems) + i * 32 + l];
+  }
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const int at = w * (32 * kRadixItems) + i * 32 + l;
+    if (at < n) {
+      keys[at] = k[i];
+      vals[at] = v[i];
+    }
+  }
 }
 
-// Stable sort of (keys, vals); result in keys/vals.  Returns launches.
-int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStream_t st) {
-  if (n <= 1) return 0;
-  int nb = (n + kRadixChunk - 1) / kRadixChunk;
-  char *p = (char *)scratch;
+constexpr size_t round256(size_t b) { return (b + 255) / 256 * 256; }
+
+// ping-pong keys and values, three tables of counts, the digits' totals
+constexpr size_t radix_bytes(size_t n) {
+  return round256(n * 8) + round256(n * 4) + 3 * 1024 * ((n + kTileSmall - 1) / kTileSmall) + 1024 + 16;
+}
+size_t radix_scratch_bytes(int n) { return radix_bytes((size_t)n); }
+
+template <int T>
+static int radix_passes(int n, uint64_t *keys, uint32_t *vals, char *p, cudaStream_t st) {
+  const int tiles = (n + T * kRadixItems - 1) / (T * kRadixItems);
   uint64_t *k2 = (uint64_t *)p;
-  p += ((size_t)n * 8 + 255) / 256 * 256;
+  p += round256((size_t)n * 8);
   uint32_t *v2 = (uint32_t *)p;
-  p += ((size_t)n * 4 + 255) / 256 * 256;
-  unsigned *hist = (unsigned *)p;
+  p += round256((size_t)n * 4);
+  unsigned *table[3];
+  for (int i = 0; i < 3; i++) {
+    table[i] = (unsigned *)p;
+    p += 1024 * (size_t)tiles;
+  }
+  unsigned *total = tiles > kDirectTiles ? (unsigned *)p : nullptr;
   uint64_t *ka = keys, *kb = k2;
   uint32_t *va = vals, *vb = v2;
-  int launches = 0;
-  for (int shift = 0; shift < 64; shift += 8) {
-    k_radix_hist<<<nb, kRadixThreads, 0, st>>>(n, ka, shift, hist);
-    k_radix_scan<<<1, 1024, 0, st>>>(256 * nb, hist);
-    k_radix_scatter<<<nb, kRadixThreads, 0, st>>>(n, ka, va, kb, vb, shift, hist);
-    launches += 3;
+  k_radix_count<T><<<tiles, T, 0, st>>>(n, ka, table[0], table[1]);
+  int launches = 1;
+  for (int pass = 0; pass < 8; pass++) {
+    unsigned *now = table[pass % 3];
+    const bool last = pass == 7;
+    if (total) {
+      k_radix_prefix<<<8, 1024, 0, st>>>(tiles, now, total);
+      launches++;
+    }
+    k_radix_pass<T><<<tiles, T, 0, st>>>(n, tiles, ka, va, kb, vb, pass * 8, now, total,
+                                         last ? nullptr : table[(pass + 1) % 3],
+                                         last ? nullptr : table[(pass + 2) % 3]);
+    launches++;
     uint64_t *tk = ka; ka = kb; kb = tk;
     uint32_t *tv = va; va = vb; vb = tv;
   }
@@ -234,14 +424,30 @@ int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStr
   return launches;
 }
 
+// Stable sort of (keys, vals); result in keys/vals.  Returns launches.
+// Up to one large tile a single block does it all.  Small tiles while the
+// direct sum of the counts reaches (16,384 keys: small / large 73 / 101 us;
+// 262,144 104 / 116); then large ones, which halve the counts to add up
+// (1,048,576: 214 / 183).
+int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStream_t st) {
+  if (n <= 1) return 0;
+  if (n <= kTileLarge) {
+    k_radix_tile<<<1, 512, 0, st>>>(n, keys, vals);
+    return 1;
+  }
+  char *p = (char *)(((uintptr_t)scratch + 15) / 16 * 16);  // the tables are read 16 bytes at a time
+  return n <= kDirectTiles * kTileSmall ? radix_passes<256>(n, keys, vals, p, st)
+                                        : radix_passes<512>(n, keys, vals, p, st);
+}
+
 // bounding box + Morton keys of positions (double4 records or separate x/y/z)
 int morton_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
                 double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st) {
-  int nb = 148 * 2;
+  int nb = kBoxBlocks;
   if (nb * 256 > n) nb = (n + 255) / 256;
   if (nb < 1) nb = 1;
   k_bbox_partial<<<nb, 256, 0, st>>>(n, pos, x, y, z, part);
-  k_bbox_final<<<1, 32, 0, st>>>(nb, part, box4);
+  k_bbox_final<<<1, kBoxThreads, 0, st>>>(nb, part, box4);
   k_morton<<<(n + 255) / 256, 256, 0, st>>>(n, pos, x, y, z, box4, keys, vals);
   return 3;
 }
@@ -380,11 +586,11 @@ constexpr int kPhBits = 18;  // BITS_PER_DIMENSION, sort_bodies.cpp:3
 // float-rounded positions is the rounded double box): box4 = {lo.x, lo.y,
 // lo.z, domain_fac}, domain_fac = float(1.0 / size * 2^18) with size the
 // largest float extent; 0 for a degenerate box (all keys 0)
-__global__ void k_peano_box_final(int nb, const double *__restrict__ part, double *__restrict__ box4) {
+__global__ void __launch_bounds__(kBoxThreads) k_peano_box_final(int nb, const double *__restrict__ part,
+                                                                 double *__restrict__ box4) {
+  double lo[3], hi[3];
+  fold_box(nb, part, lo, hi);
   if (threadIdx.x != 0) return;
-  double lo[3] = {1e308, 1e308, 1e308}, hi[3] = {-1e308, -1e308, -1e308};
-  for (int b = 0; b < nb; b++)
-    for (int d = 0; d < 3; d++) { lo[d] = fmin(lo[d], part[b * 6 + d]); hi[d] = fmax(hi[d], part[b * 6 + 3 + d]); }
   float lf[3], ext[3];
   for (int d = 0; d < 3; d++) {
     lf[d] = __double2float_rn(lo[d]);
@@ -423,27 +629,24 @@ __global__ void k_peano_pos(int n, const double4 *__restrict__ pos, const double
 // bounding box + Peano-Hilbert keys of positions (double4 records or x/y/z)
 int peano_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
                double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st) {
-  int nb = 148 * 2;
+  int nb = kBoxBlocks;
   if (nb * 256 > n) nb = (n + 255) / 256;
   if (nb < 1) nb = 1;
   k_bbox_partial<<<nb, 256, 0, st>>>(n, pos, x, y, z, part);
-  k_peano_box_final<<<1, 32, 0, st>>>(nb, part, box4);
+  k_peano_box_final<<<1, kBoxThreads, 0, st>>>(nb, part, box4);
   k_peano_pos<<<(n + 255) / 256, 256, 0, st>>>(n, pos, x, y, z, box4, keys, vals);
   return 3;
 }
 
 // ---------------------------------------------------------------------------
 // Allocation-free variant of the radix sort.  Its scratch (ping-pong key and
-// value buffers plus the per-block digit histograms) is a file-scope device
+// value buffers plus the tiles' digit counts) is a file-scope device
 // array sized for kNoAllocMaxKeys keys; every GPU that loads this library
 // holds those bytes until the process exits.
 // ---------------------------------------------------------------------------
 constexpr int kNoAllocMaxKeys = CUDASPH_SORT_NOALLOC_MAX_KEYS;
 static_assert(kNoAllocMaxKeys == (1 << 18), "header and library disagree");
-constexpr size_t round256(size_t b) { return (b + 255) / 256 * 256; }
-constexpr size_t kNoAllocScratchBytes =
-    round256((size_t)kNoAllocMaxKeys * 8) + round256((size_t)kNoAllocMaxKeys * 4) +
-    round256(256 * (((size_t)kNoAllocMaxKeys + kRadixChunk - 1) / kRadixChunk) * 4);
+constexpr size_t kNoAllocScratchBytes = radix_bytes(kNoAllocMaxKeys);
 
 static __device__ __align__(256) unsigned char g_noalloc_sort_scratch[kNoAllocScratchBytes];
 
@@ -539,8 +742,8 @@ extern "C" int cudasph_radix_sort_u64_noalloc(int n, uint64_t *keys, uint32_t *v
   void *scratch = nullptr;
   int rc = noalloc_scratch(&scratch);
   if (rc) return rc;
-  // nothing in the scratch has to start at zero: every pass rewrites all
-  // histogram entries and every key/value slot it later reads
+  // nothing in the scratch has to start at zero: the counts are cleared and
+  // every key/value slot is written before it is read
   sph::radix_sort_u64(n, keys, vals, scratch, (cudaStream_t)stream);
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;

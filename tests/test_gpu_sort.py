@@ -1,0 +1,36 @@
+"""The radix sort at the edges of its tiles and of its three forms (one block;
+small tiles; large tiles with the counts added up by the passes or by a launch
+of their own): keys and permutation equal to a stable CPU sort, bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 2, 31, 255, 2047, 2048, 4095, 4096, 4097, 6144, 524287, 524288, 524289, 1048576, 1048577, 1300001]
+
+
+def _keys(n, kind):
+    rs = np.random.default_rng(n)
+    k = rs.integers(0, 1 << 63, n, dtype=np.uint64) * np.uint64(2) + rs.integers(0, 2, n, dtype=np.uint64)
+    if kind == "ties":
+        k &= np.uint64(0x8001000300000701)
+    if kind == "ones":  # the value that pads a part-filled tile
+        k[::3] = np.uint64(0xFFFFFFFFFFFFFFFF)
+    return k
+
+
+@pytest.mark.parametrize("kind", ["random", "ties", "ones"])
+@pytest.mark.parametrize("n", SIZES)
+def test_radix_sort_is_the_stable_order(n, kind):
+    import torch
+    from cudasph_b200._capi import check, lib
+    k = _keys(n, kind)
+    order = np.argsort(k, kind="stable")
+    dk = torch.from_numpy(k.view(np.int64).copy()).cuda()
+    dv = torch.arange(n, dtype=torch.int32, device="cuda")
+    # a scratch buffer aligned to 8 bytes only, filled with rubbish
+    scratch = torch.full((lib().cudasph_sort_scratch_bytes(n) // 8 + 2,), -1, dtype=torch.int64, device="cuda")[1:]
+    s = torch.cuda.current_stream().cuda_stream
+    check(lib().cudasph_radix_sort_u64(n, dk.data_ptr(), dv.data_ptr(), scratch.data_ptr(), s))
+    assert np.array_equal(dk.cpu().numpy().view(np.uint64), k[order])
+    assert np.array_equal(dv.cpu().numpy(), order)
