@@ -20,15 +20,16 @@
 // Why a warp per particle and not a lane per particle (a warp per leaf of 32
 // targets, the earlier form): a leaf-warp lasts as long as its slowest lane's
 // iteration, and small sets have too few of them.  Solve phase, us, lane /
-// warp per particle: 2,049 particles 431 / 23, 16,384 540 / 85, 60,000 717 /
-// 233, 262,144 (an oscillating star, 1.4 evaluations per particle) 1907 /
-// 1103, 1,048,576 5348 / 3904; 130,001 particles from estimated ranges (3.7
-// evaluations, some ranges holding half the star) 69,400 / 3,450.  A steady
-// set with 1.00 evaluations per particle is the one that loses: 2,000,003
-// particles 5556 / 6020.  The kernel is bound by instruction issue (73 % of
-// the cycles at 262,144, about 2,700 instructions per particle; FP64 pipe 24
-// %, XU 18 %), so what helps is fewer instructions: cells of 8 particles
-// instead of leaves of 32 (5,400 -> 3,100 with shared walks), the group's
+// warp per particle: 2,049 particles 433 / 31, 16,384 535 / 88, 60,000 709 /
+// 266, 262,144 (an oscillating star, 1.4 evaluations per particle) 1833 /
+// 1151, 1,048,576 4283 / 3769; from estimated ranges (3.7 evaluations, some
+// ranges holding half the star) 130,001 particles 69,300 / 3,760, 1,000,000
+// 61,000 / 13,200.  A uniform steady set with 1.00 evaluations per particle
+// is the one that loses: 2,000,003 particles 5485 / 6111 (from estimates
+// 21,300 / 22,200).  The kernel is bound by instruction issue (73 % of the
+// cycles at 262,144, about 2,700 instructions per particle; FP64 pipe 24 %,
+// XU 18 %), so what helps is fewer instructions: cells of 8 particles instead
+// of leaves of 32 with walks shared by a group (5,400 -> 3,100), the group's
 // candidate pass (2,600), and occupancy.  Loading the next candidates ahead
 // of their test, or the next records ahead of their evaluation, cost 5 - 9 %
 // (registers).
@@ -40,10 +41,12 @@ namespace sph {
 constexpr int kNgbWarps = 4;   // warps per block
 // queries reach a little past the range: the sliver test below needs it
 constexpr double kWiden = 1.0 + 1e-12;
-// ... and a group's candidates cover ranges up to this much larger, so that a
-// second evaluation, a per cent away, finds them at hand (3 % more candidates)
-constexpr double kSlack = 1.01;
+// ... and a group's candidates cover ranges up to this much larger: a second
+// evaluation, a per cent away in a running simulation, finds them at hand (3 %
+// more candidates), and particles that need more rounds move by up to 10 %
+constexpr double kSlack = 1.01, kSlackMore = 1.13;
 constexpr int kNgbBlocks = 9;  // resident blocks per SM (N = 1M: 8, 9, 10 and 12 of them 4.05, 3.90, 4.42, 4.60 ms)
+constexpr int kMoreBlocks = 6;  // of the later rounds (2,000,003 particles from estimates: 6 / 8 / 9 of them 21.6, 22.5, 22.7 ms)
 constexpr unsigned kFull = 0xffffffffu;
 
 constexpr int kQueue = 64;   // ring of cells awaiting their candidates' test (a power of two)
@@ -68,6 +71,8 @@ struct WarpSmem {
   unsigned mask[kMaxLevels];          // the walk: per level the children still to visit ...
   int node[kMaxLevels];               // ... of this node
   RangeIter it;                       // the target's iteration (lane 0 steps it)
+  double w_list, bound;               // ranges up to which the list, and the target's candidates, reach
+  int nlist;                          // cells in the list, -1: too many
   int list[kCells];                   // cells that may meet a ball of the group, ascending
   unsigned hits[G][kRounds][32];      // per target: candidates of each chunk of the list inside its ball
   union {
@@ -302,7 +307,21 @@ struct SolveArgs {
   int *list;    // neighbour lists at the final range, one row of `stride` entries per slot
   int cap, stride;
   int s0, s1;   // slots processed by this launch
+  // groups with targets left after the first round: {first slot, mask of the
+  // targets}, their number, and the targets' states by slot
+  int2 *queue;
+  int *queued;
+  RangeIter *save;
 };
+
+__device__ __forceinline__ RangeIter start_iter(double w) {
+  RangeIter it;
+  it.w = w;
+  it.phase = w > 0 ? kBr0 : kDone;
+  it.dx = it.f = it.x_left = it.f_try = it.rx = it.ry = 0;
+  it.iter = it.keep = it.nev = 0;
+  return it;
+}
 
 // One evaluation's epilogue (compute_ngb, dev_solve_range.cu:77-87) with the
 // smooth count sf and its derivative sum sg at it.w, and the step of the
@@ -495,6 +514,7 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
 struct Rough {
   double sf, sg;
   double err;  // bound of either sum's error
+  double n;    // particles of the cells
 };
 
 template <class Smem>
@@ -531,7 +551,7 @@ __device__ __forceinline__ Rough rough_sums(const SolveArgs &a, Smem &sm, const 
   // the rounded positions and the FP32 operations, and |ig'| < 4.3,
   // |(u ig')'| < 90 on [0, 2]; about four times that is allowed for
   const double per = 2e-4 * (fabs(p.x) + fabs(p.y) + fabs(p.z)) / w + 4e-4;
-  return {sf, sg, per * n + 1e-8 * a.n_target};
+  return {sf, sg, per * n + 1e-8 * a.n_target, n};
 }
 
 // Whether those sums take the iteration the same way as the exact ones: in
@@ -547,41 +567,51 @@ __device__ __forceinline__ bool clamped_for_sure(const RangeIter &it, const Roug
 // dev_solve_range (dev_solve_range.cu:137-189): per particle, bracket the
 // root of f(w) = sum_j ig(2 r_ij / w) - N_target with clamped Newton steps
 // (dev_bracket_root :93-135), then safeguarded Newton / bisection until
-// |dx| < rel_err * w.  Every evaluation is a walk at the range tested, which
-// writes the list at that range (find_ngb fused in).  In steady state the
-// previous step's range passes at once, so the first walk is the last: its
-// list is kept when the final range w = (rx + ry) / 2, a few ulp from the
-// evaluated one, leaves the set unchanged -- every entry inside the final
-// range (the largest d2 checked) and, if the range grew, no candidate in the
-// sliver just outside the evaluated range.  Otherwise one more walk lists at
-// the final range.
-template <class Smem>
-__device__ __forceinline__ void solve_particle(const SolveArgs &a, Smem &sm, int s, const double4 &p, int nlist,
-                                               int total, double w_list) {
+// |dx| < rel_err * w.  Every evaluation writes the list at the range it tests
+// (find_ngb fused in).  In steady state the previous step's range passes at
+// once, so the first evaluation is the last: its list is kept when the final
+// range w = (rx + ry) / 2, a few ulp from the evaluated one, leaves the set
+// unchanged -- every entry inside the final range (the largest d2 checked)
+// and, if the range grew, no candidate in the sliver just outside the
+// evaluated range.  Otherwise the list is written once more at the final
+// range.
+//
+// The targets of a group go through their iterations in rounds: the cells and
+// candidates are gathered once for all of them, with some slack, each target
+// is evaluated as long as its ranges stay inside, and those that leave it
+// share the next round (a walk of its own per evaluation took 40 ms instead
+// of 22 for 2,000,003 particles from estimated ranges).
+// One round for target t: evaluations as long as the group's candidates reach
+// (sm.bound, sm.w_list).  True when done.
+// FIRST: the round that is the last one for nearly every particle of a running
+// simulation; a range that is far too large is left to the next.
+template <bool FIRST, class Smem>
+__device__ __forceinline__ bool solve_round(const SolveArgs &a, Smem &sm, int s, int total) {
+  const double4 p = a.pos[s];
   RangeIter &it = sm.it;
-  __syncwarp();
-  if (lane_id() == 0) {
-    it.w = p.w;
-    it.phase = p.w > 0 ? kBr0 : kDone;
-    it.dx = it.f = it.x_left = it.f_try = it.rx = it.ry = 0;
-    it.iter = it.keep = it.nev = 0;
-  }
-  __syncwarp();
   int count = 0;
-  bool listed = true;  // the row holds the list of the final range
+  bool listed = !(it.w > 0);  // the row holds the list of the final range
   bool exact = false;
   while (it.phase != kDone) {
     const double w_eval = it.w;
-    if (w_eval > p.w * kSlack) total = -1;
-    const Eval e = eval_range<true>(a, sm, s, p, w_eval, w_eval <= w_list ? nlist : -1, total, exact);
-    if (e.many) {
-      const Rough r = rough_sums(a, sm, p, w_eval);
+    if (w_eval > sm.bound) return false;
+    const Eval e = eval_range<true>(a, sm, s, p, w_eval, w_eval <= sm.w_list ? sm.nlist : -1, total, exact);
+    if (FIRST && e.many) return false;
+    if (!FIRST && e.many) {
+      Rough r = rough_sums(a, sm, p, w_eval);
       exact = !clamped_for_sure(it, r, a);
+      if (exact) continue;  // once more, all of it
+      for (;;) {
+        __syncwarp();
+        if (lane_id() == 0) solve_advance(it, r.sf, r.sg, a);
+        __syncwarp();
+        if (it.phase == kDone || r.n < 32.0 * a.ordered) break;
+        r = rough_sums(a, sm, p, it.w);
+        if (!clamped_for_sure(it, r, a)) break;
+      }
+      if (it.phase != kDone) return false;
       listed = false;
-      __syncwarp();
-      if (!exact && lane_id() == 0) solve_advance(it, r.sf, r.sg, a);
-      __syncwarp();
-      continue;
+      break;
     }
     exact = false;
     count = e.count;
@@ -591,16 +621,18 @@ __device__ __forceinline__ void solve_particle(const SolveArgs &a, Smem &sm, int
     const double w = it.w, wf2 = __dmul_rn(w, w);
     listed = w == w_eval || (w < w_eval && e.dmax < wf2) ||
              (w > w_eval && !e.sliver && wf2 < __dmul_rn(w_eval, w_eval) * (1.0 + 0x1p-40));
+    if (sm.nlist < 0 && it.phase != kDone) return false;  // a smaller range may find a list
   }
   const double w = it.w;
   if (!listed)
-    count = eval_range<false>(a, sm, s, p, w, w <= w_list ? nlist : -1, w <= p.w * kSlack ? total : -1, false).count;
+    count = eval_range<false>(a, sm, s, p, w, w <= sm.w_list ? sm.nlist : -1, w <= sm.bound ? total : -1, false).count;
   if (lane_id() == 0) {
     if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
     a.pos[s].w = (w > 0) ? w : 0.0;
     a.n_ngb[s] = count;
     if (a.nevals) a.nevals[s] = it.nev;
   }
+  return true;
 }
 
 // The warp's targets first .. first + count - 1 and what they share: one walk
@@ -611,21 +643,21 @@ __device__ __forceinline__ void solve_particle(const SolveArgs &a, Smem &sm, int
 template <int G>
 struct Group {
   int first, count;
-  int nlist;      // cells in sm.list, -1: too many
-  double w_list;  // it covers ranges up to this
 
-  __device__ __forceinline__ void open(const SolveArgs &a, WarpSmem<G> &sm) {
-    const int lane = (int)lane_id();
-    first = a.s0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G;
-    count = min(G, a.s1 - first);
-    nlist = -1;
-    w_list = 0;
-    if (count <= 0) return;
-    double4 p = a.pos[first + min(lane % G, count - 1)];  // lanes past the last target repeat it
+  // for the targets of the mask `todo`, at their ranges or (SAVED) their
+  // saved iterations'
+  template <bool SAVED>
+  __device__ __forceinline__ void open(const SolveArgs &a, WarpSmem<G> &sm, unsigned todo, double slack) {
+    const int lane = (int)lane_id(), t0 = lane % G;
+    // lanes whose target has no part in this repeat the first that has
+    const int tt = (todo >> t0) & 1u ? t0 : __ffs(todo) - 1;
+    double4 p = a.pos[first + tt];
+    if (SAVED) p.w = a.save[first + tt].w;
     if (!(p.w > 0)) p.w = 0;
-    const Query mine = make_ball(p.x, p.y, p.z, p.w * kSlack * kWiden);
+    Query mine = make_ball(p.x, p.y, p.z, p.w * slack * kWiden);
     Query q = mine;
-    w_list = p.w;
+    double w_list = p.w * slack;
+    if (tt != t0) mine.r2 = -1.f;
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
 #pragma unroll
@@ -636,8 +668,12 @@ struct Group {
       q.r2 = fmaxf(q.r2, __shfl_xor_sync(kFull, q.r2, o));
       w_list = fmax(w_list, __shfl_xor_sync(kFull, w_list, o));
     }
-    w_list *= kSlack;
-    nlist = list_cells(a.t, sm, q);
+    const int nlist = list_cells(a.t, sm, q);
+    if (lane == 0) {
+      sm.w_list = w_list;
+      sm.nlist = nlist;
+    }
+    __syncwarp();
     if (nlist <= 0) return;
     float tx[G], ty[G], tz[G], tr[G];
 #pragma unroll
@@ -671,12 +707,18 @@ struct Group {
     }
     __syncwarp();
   }
-  // target t's candidates as codes; their number, or -1 when they do not fit
-  __device__ __forceinline__ int stage(WarpSmem<G> &sm, int t) {
-    if (nlist < 0) return -1;
-    const int lane = (int)lane_id();
+  // target t, at iteration `it` (lane 0's): its candidates as codes; their
+  // number, or -1 when they do not fit
+  __device__ __forceinline__ int stage(WarpSmem<G> &sm, int t, const RangeIter &it, double slack) {
+    const int lane = (int)lane_id(), nlist = sm.nlist;
     int total = 0;
     __syncwarp();  // the previous target's codes are read
+    if (lane == 0) {
+      sm.it = it;
+      sm.bound = it.w * slack;
+    }
+    __syncwarp();
+    if (nlist < 0) return -1;
     for (int r = 0; r < kRounds && r * 128 < nlist; r++) {
       unsigned m = sm.hits[t][r][lane];
       const int n = __popc(m);
@@ -700,30 +742,75 @@ struct Group {
   }
 };
 
+// The first round.  A group with a target left goes on a queue for
+// k_solve_more, its targets' states by their slots: in one kernel the later
+// rounds' code would cost the first one registers and with them resident
+// warps (steady solve of 2,000,003 particles 6.9 ms instead of 6.1).
 template <int G>
-__global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(SolveArgs a) {
+__global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(const __grid_constant__ SolveArgs a) {
   __shared__ WarpSmem<G> smem[kNgbWarps];
   WarpSmem<G> &sm = smem[threadIdx.x >> 5];
   Group<G> g;
-  g.open(a, sm);
-  for (int t = 0; t < g.count; t++)
-    solve_particle(a, sm, g.first + t, a.pos[g.first + t], g.nlist, g.stage(sm, t), g.w_list);
+  g.first = a.s0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G;
+  g.count = min(G, a.s1 - g.first);
+  if (g.count <= 0) return;
+  g.template open<false>(a, sm, (1u << g.count) - 1u, kSlack);
+  unsigned todo = 0u;
+  for (int t = 0; t < g.count; t++) {
+    const int s = g.first + t;
+    const int total = g.stage(sm, t, start_iter(a.pos[s].w), kSlack);
+    if (!solve_round<true>(a, sm, s, total)) {
+      todo |= 1u << t;
+      if (lane_id() == 0) a.save[s] = sm.it;
+    }
+  }
+  if (todo != 0u && lane_id() == 0) a.queue[atomicAdd(a.queued, 1)] = make_int2(g.first, (int)todo);
+}
+
+// The rounds after it, until every target is done.
+template <int G>
+__global__ void __launch_bounds__(kNgbWarps * 32, kMoreBlocks) k_solve_more(const __grid_constant__ SolveArgs a) {
+  __shared__ WarpSmem<G> smem[kNgbWarps];
+  WarpSmem<G> &sm = smem[threadIdx.x >> 5];
+  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+  const int queued = *a.queued;
+  for (int q = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < queued; q += warps) {
+    const int2 entry = a.queue[q];
+    Group<G> g;
+    g.first = entry.x;
+    g.count = min(G, a.s1 - g.first);
+    unsigned todo = (unsigned)entry.y;
+    while (todo != 0u) {
+      g.template open<true>(a, sm, todo, kSlackMore);
+      for (unsigned m = todo; m != 0u; m &= m - 1u) {
+        const int t = __ffs(m) - 1;
+        const int s = g.first + t;
+        const int total = g.stage(sm, t, a.save[s], kSlackMore);
+        if (solve_round<false>(a, sm, s, total)) todo &= ~(1u << t);
+        else if (lane_id() == 0) a.save[s] = sm.it;
+      }
+      __syncwarp();  // the saved ranges are read by other lanes
+    }
+  }
 }
 
 // dev_find_ngb (dev_find_ngb.cu:13-87): every j with ds2 < range_i^2, in
 // ascending slot order, at ranges set from outside.
 template <int G>
-__global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_find_ngb(SolveArgs a) {
+__global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_find_ngb(const __grid_constant__ SolveArgs a) {
   __shared__ WarpSmem<G> smem[kNgbWarps];
   WarpSmem<G> &sm = smem[threadIdx.x >> 5];
   Group<G> g;
-  g.open(a, sm);
+  g.first = a.s0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G;
+  g.count = min(G, a.s1 - g.first);
+  if (g.count <= 0) return;
+  g.template open<false>(a, sm, (1u << g.count) - 1u, 1.0);
   for (int t = 0; t < g.count; t++) {
     const int s = g.first + t;
     const double4 p = a.pos[s];
-    const int total = g.stage(sm, t);
+    const int total = g.stage(sm, t, start_iter(p.w), 1.0);
     int count = 0;
-    if (p.w > 0) count = eval_range<false>(a, sm, s, p, p.w, g.nlist, total, false).count;
+    if (p.w > 0) count = eval_range<false>(a, sm, s, p, p.w, sm.nlist, total, false).count;
     if (lane_id() == 0) {
       if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
       a.n_ngb[s] = count;
@@ -734,8 +821,13 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_find_ngb(SolveAr
 template <int G>
 static void launch_group(const SolveArgs &a, bool solve, cudaStream_t st) {
   const int warps = (a.s1 - a.s0 + G - 1) / G, blocks = (warps + kNgbWarps - 1) / kNgbWarps;
-  if (solve) k_solve_range<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
-  else k_find_ngb<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
+  if (!solve) {
+    k_find_ngb<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
+    return;
+  }
+  cudaMemsetAsync(a.queued, 0, sizeof(int), st);
+  k_solve_range<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
+  k_solve_more<G><<<blocks < 148 * kMoreBlocks ? blocks : 148 * kMoreBlocks, kNgbWarps * 32, 0, st>>>(a);
 }
 
 // Four targets to a warp share the walk once that leaves enough warps: the
@@ -751,9 +843,15 @@ static void launch_ngb(const SolveArgs &a, bool solve, cudaStream_t st) {
   else launch_group<1>(a, solve, st);
 }
 
+// scratch of the solve: the queue's length, the queue, the saved states
+size_t solve_work_bytes(int n) {
+  return 256 + ((size_t)n * sizeof(int2) + 255) / 256 * 256 + (size_t)n * sizeof(RangeIter);
+}
+
 // leaves [leaf0, leaf1) (a shard's range, or 0 and the leaf count)
 int launch_solve_range(const TreeView &t, double4 *pos, int *nevals, unsigned *flags, const sph_params &p,
-                       int *n_ngb, int *list, int cap, int stride, int leaf0, int leaf1, cudaStream_t st) {
+                       int *n_ngb, int *list, int cap, int stride, void *work, int leaf0, int leaf1,
+                       cudaStream_t st) {
   SolveArgs a;
   a.t = t; a.pos = pos; a.nevals = nevals; a.flags = flags;
   a.n_ngb = n_ngb; a.list = list; a.cap = cap; a.stride = stride;
@@ -761,8 +859,11 @@ int launch_solve_range(const TreeView &t, double4 *pos, int *nevals, unsigned *f
   a.ordered = 4 + (int)fmin(p.n_target / 16.0, 1e6);
   a.s0 = leaf0 * kLeaf; a.s1 = min(leaf1 * kLeaf, t.n);
   if (a.s1 <= a.s0) return 0;
+  a.queued = (int *)work;
+  a.queue = (int2 *)((char *)work + 256);
+  a.save = (RangeIter *)((char *)work + 256 + ((size_t)t.n * sizeof(int2) + 255) / 256 * 256);
   launch_ngb(a, true, st);
-  return 1;
+  return 2;
 }
 
 int launch_find_ngb(const TreeView &t, double4 *pos, int *n_ngb, int *list, int cap, int stride, unsigned *flags,
