@@ -22,32 +22,48 @@
 
 #include "common.cuh"
 #include "pairmath.cuh"
-#include "sph_math.cuh"
+#include "sphpair.cuh"
 
 namespace sph {
 
 // ---------------------------------------------------------------------------
 // derivatives of the kernel functions, d/du
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double kd_dw(double u) {
-  const double ipi = 0.318309886183791;
+// (iu = 1 / u)
+__device__ __forceinline__ double kd_dw(double u, double iu) {
+  constexpr double ipi = KC<double>::ipi;
   if (u < 1) return 2.25 * ipi;
-  if (u < 2) return 0.75 * ipi * (4 - u * u) / (u * u);
+  if (u < 2) return 0.75 * ipi * (4 * iu * iu - 1);
   return 0;
 }
-__device__ __forceinline__ double kd_dig(double u) {
-  const double c = 256.0 * 3.141592653589793;
-  if (u <= 0) return 0;
-  if (u < 1) return c * (k_w<double>(4 * u) + 16 * u * u * k_dw<double>(4 * u));
-  if (u < 2) {
-    const double s = 2 - u;
-    return c * (2 * s * k_w<double>(4 * s) / u + 16 * s * s * s * k_dw<double>(4 * s) / u +
-                s * s * k_w<double>(4 * s) / (u * u));
+// k_dig = (1/u) d(ig)/du and its derivative, from W(x) and x dW/dx at x = 4u
+// (u < 1) or x = 4 (2 - u)
+__device__ __forceinline__ void kd_dig(double u, double iu, double &dig, double &ddig) {
+  constexpr double ipi = KC<double>::ipi, c = 256.0 * KC<double>::pi;
+  dig = ddig = 0;
+  if (!(u > 0) || !(u < 2)) return;
+  const double s = u < 1 ? u : 2 - u, x = 4 * s;
+  if (!(x < 2)) return;
+  double w, xdw;
+  if (x < 1) {
+    const double x2 = x * x;
+    w = ipi * (1 - 1.5 * x2 + 0.75 * x2 * x);
+    xdw = ipi * x2 * (-3 + 2.25 * x);
+  } else {
+    const double t = 2 - x;
+    w = 0.25 * ipi * t * t * t;
+    xdw = -0.75 * ipi * x * t * t;
   }
-  return 0;
+  if (u < 1) {
+    dig = c * u * w;
+    ddig = c * (w + xdw);
+  } else {
+    dig = -c * s * s * w * iu;
+    ddig = c * s * iu * (2 * w + xdw + s * w * iu);
+  }
 }
 __device__ __forceinline__ double kd_dwdh(double u) {
-  const double ipi = 0.318309886183791;
+  constexpr double ipi = KC<double>::ipi;
   if (u < 1) return ipi * (15 * u - 13.5 * u * u);
   if (u < 2) return ipi * (12 - 15 * u + 4.5 * u * u);
   return 0;
@@ -57,18 +73,11 @@ __device__ __forceinline__ double kd_dphidh(double u) {
   if (u < 2) return -8 * u + 12 * u * u - 6 * u * u * u + u * u * u * u;
   return 0;
 }
-__device__ __forceinline__ double kd_digdh(double u) { return 2 * u * k_dig<double>(u) + u * u * kd_dig(u); }
 
 // AdjArgs: see common.cuh
 
 
 constexpr int kAT = 256;  // threads of the per-particle kernels
-
-__device__ __forceinline__ int warp_max_i(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 
 __device__ __forceinline__ void atomic_add3(double4 *p, double x, double y, double z) {
   atomicAdd(&p->x, x);
@@ -148,17 +157,45 @@ __global__ void __launch_bounds__(kAT) k_adj_argmin(AdjArgs a) {
 }
 
 // -- 4. fold: dtbar, the arg-min particle, the timestep adjoint --------------
-__global__ void k_adj_timestep(AdjArgs a, int nb_kick, int nb_min) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// (one block; one thread walked the partials before: 28 us at 65,536 particles)
+constexpr int kFold = 512;
+
+// sum of part[0 .. nb) over a block of kFold threads, in a fixed order
+__device__ __forceinline__ double fold_sum(int nb, const double *part) {
+  __shared__ double ws[kFold / 32];
   double f = 0;
-  for (int b = 0; b < nb_kick; b++) f += a.part[b];
+  for (int b = threadIdx.x; b < nb; b += kFold) f += part[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+  if (lane_id() == 0) ws[threadIdx.x >> 5] = f;
+  __syncthreads();
+  double t = 0;
+  for (int k = 0; k < kFold / 32; k++) t += ws[k];
+  return t;
+}
+
+__global__ void __launch_bounds__(kFold) k_adj_timestep(AdjArgs a, int nb_kick, int nb_min) {
+  const double f = fold_sum(nb_kick, a.part);
   double t = 1e300;
   int idx = 0;
-  for (int b = 0; b < nb_min; b++) {
+  for (int b = threadIdx.x; b < nb_min; b += kFold) {
     const double tb = a.part[nb_kick + 2 * b];
     const int ib = (int)a.part[nb_kick + 2 * b + 1];
     if (tb < t || (tb == t && ib < idx)) { t = tb; idx = ib; }
   }
+  __shared__ double st[kFold / 32];
+  __shared__ int si[kFold / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double t2 = __shfl_xor_sync(0xffffffffu, t, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, idx, o);
+    if (t2 < t || (t2 == t && i2 < idx)) { t = t2; idx = i2; }
+  }
+  if (lane_id() == 0) { st[threadIdx.x >> 5] = t; si[threadIdx.x >> 5] = idx; }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int k = 1; k < kFold / 32; k++)
+    if (st[k] < t || (st[k] == t && si[k] < idx)) { t = st[k]; idx = si[k]; }
   const double dtb1 = a.asc[0] + 0.5 * f;
   a.asc[1] = 0.5 * f;  // dtbar0 so far (predictor terms follow)
   a.asc[3] = (double)idx;
@@ -194,15 +231,16 @@ constexpr int kGA = 128;
 
 __global__ void __launch_bounds__(kGA) k_adj_grav_f64(int n, const double4 *__restrict__ src,
                                                       const double4 *__restrict__ ab, double4 *__restrict__ xb,
-                                                      double eps2, double G, int tile) {
+                                                      double eps2, double G, int tile, int slices) {
   __shared__ double4 sp[kGA];
   __shared__ double4 sg[kGA];
   const int t = threadIdx.x;
-  const int i = blockIdx.x * kGA + t;
+  const int i0 = blockIdx.x / slices * kGA;
+  const int i = i0 + t;
   const int ii = min(i, n - 1);
-  const int i0 = blockIdx.x * kGA;
-  const int jlo = tile > 0 ? (i0 / tile) * tile : 0;
-  const int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  int jlo = tile > 0 ? (i0 / tile) * tile : 0;
+  int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  source_slice<kGA>(jlo, jhi, blockIdx.x % slices, slices);
   const double4 pi = src[ii];
   const double4 gi4 = ab[ii];
   const double mi = pi.w, gix = gi4.x, giy = gi4.y, giz = gi4.z;
@@ -236,9 +274,7 @@ __global__ void __launch_bounds__(kGA) k_adj_grav_f64(int n, const double4 *__re
     }
   }
   if (i < n) {
-    double4 x = xb[i];
-    x.x += G * rx; x.y += G * ry; x.z += G * rz;
-    xb[i] = x;
+    atomic_add3(xb + i, G * rx, G * ry, G * rz);
   }
 }
 
@@ -246,15 +282,16 @@ __global__ void __launch_bounds__(kGA) k_adj_grav_f64(int n, const double4 *__re
 // anchor, FP64 per-tile accumulation
 __global__ void __launch_bounds__(kGA) k_adj_grav_f32(int n, const double4 *__restrict__ src,
                                                       const double4 *__restrict__ ab, double4 *__restrict__ xb,
-                                                      float eps2, double G, int tile) {
+                                                      float eps2, double G, int tile, int slices) {
   __shared__ float4 sp[kGA];
   __shared__ float4 sg[kGA];
   const int t = threadIdx.x;
-  const int i = blockIdx.x * kGA + t;
+  const int i0 = blockIdx.x / slices * kGA;
+  const int i = i0 + t;
   const int ii = min(i, n - 1);
-  const int i0 = blockIdx.x * kGA;
-  const int jlo = tile > 0 ? (i0 / tile) * tile : 0;
-  const int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  int jlo = tile > 0 ? (i0 / tile) * tile : 0;
+  int jhi = tile > 0 ? min(jlo + tile, n) : n;
+  source_slice<kGA>(jlo, jhi, blockIdx.x % slices, slices);
   const double4 anc = src[min(i0, n - 1)];
   const double4 pi = src[ii];
   const double4 gi4 = ab[ii];
@@ -292,9 +329,7 @@ __global__ void __launch_bounds__(kGA) k_adj_grav_f32(int n, const double4 *__re
     rx += px; ry += py; rz += pz;
   }
   if (i < n) {
-    double4 x = xb[i];
-    x.x += G * rx; x.y += G * ry; x.z += G * rz;
-    xb[i] = x;
+    atomic_add3(xb + i, G * rx, G * ry, G * rz);
   }
 }
 
@@ -318,10 +353,13 @@ template <bool UNI>
 __device__ __forceinline__ void adj_sym_f32_item(long long item, int n, int nt, const double4 *__restrict__ src,
                                                  const double4 *__restrict__ ab, double4 *__restrict__ xb,
                                                  float eps2, double G, float (&red)[2][kAdjWarps][3][32],
-                                                 double (&iacc)[2 * kAdjRP * 3][kAdjWarps * 32]) {
+                                                 double (&iacc)[2 * kAdjRP * 3][kAdjWarps * 32], unsigned slice,
+                                                 int slices) {
   int b, t_lo, t_hi;
   sym_item(item, nt, b, t_lo, t_hi);
-  const int j_lo = t_lo * kAdjTile, j_hi = min(t_hi * kAdjTile, n);
+  int j_lo = t_lo * kAdjTile, j_hi = min(t_hi * kAdjTile, n);
+  source_slice<32>(j_lo, j_hi, slice, slices);
+  if (j_lo >= j_hi) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nxt = (l + 1) & 31;
   const int i0 = b * kAdjTile;
   const double4 anc = src[i0];
@@ -443,13 +481,13 @@ __device__ __forceinline__ void adj_sym_f32_item(long long item, int n, int nt, 
 __global__ void __launch_bounds__(kAdjWarps * 32) k_adj_grav_sym_f32(int n, int nt, const double4 *__restrict__ src,
                                                                     const double4 *__restrict__ ab,
                                                                     double4 *__restrict__ xb, float eps2, double G,
-                                                                    const int *__restrict__ mass_mixed) {
+                                                                    const int *__restrict__ mass_mixed, int slices) {
   __shared__ float red[2][kAdjWarps][3][32];
   __shared__ double iacc[2 * kAdjRP * 3][kAdjWarps * 32];  // [i-slot * 3 + component][thread]
   if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
-    adj_sym_f32_item<true>(blockIdx.x, n, nt, src, ab, xb, eps2, G, red, iacc);
+    adj_sym_f32_item<true>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, iacc, blockIdx.x % slices, slices);
   else
-    adj_sym_f32_item<false>(blockIdx.x, n, nt, src, ab, xb, eps2, G, red, iacc);
+    adj_sym_f32_item<false>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, iacc, blockIdx.x % slices, slices);
 }
 
 // Symmetric FP64 form: absolute coordinates, kAdj64R i-particles per lane
@@ -462,10 +500,13 @@ static_assert(kAdj64Warps * 32 * kAdj64R == kAdjTile, "the FP64 form shares the 
 template <bool UNI>
 __device__ __forceinline__ void adj_sym_f64_item(long long item, int n, int nt, const double4 *__restrict__ src,
                                                  const double4 *__restrict__ ab, double4 *__restrict__ xb,
-                                                 double eps2, double G, double (&red)[2][kAdj64Warps][3][32]) {
+                                                 double eps2, double G, double (&red)[2][kAdj64Warps][3][32], unsigned slice,
+                                                 int slices) {
   int b, t_lo, t_hi;
   sym_item(item, nt, b, t_lo, t_hi);
-  const int j_lo = t_lo * kAdjTile, j_hi = min(t_hi * kAdjTile, n);
+  int j_lo = t_lo * kAdjTile, j_hi = min(t_hi * kAdjTile, n);
+  source_slice<32>(j_lo, j_hi, slice, slices);
+  if (j_lo >= j_hi) return;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nxt = (l + 1) & 31;
   const int ib = b * kAdjTile + w * 32 * kAdj64R + l;
   const double4 far = src[b * kAdjTile];  // position given to padding slots
@@ -544,15 +585,15 @@ __device__ __forceinline__ void adj_sym_f64_item(long long item, int n, int nt, 
 __global__ void __launch_bounds__(kAdj64Warps * 32) k_adj_grav_sym_f64(int n, int nt, const double4 *__restrict__ src,
                                                                       const double4 *__restrict__ ab,
                                                                       double4 *__restrict__ xb, double eps2, double G,
-                                                                      const int *__restrict__ mass_mixed) {
+                                                                      const int *__restrict__ mass_mixed, int slices) {
   __shared__ double red[2][kAdj64Warps][3][32];
   if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
-    adj_sym_f64_item<true>(blockIdx.x, n, nt, src, ab, xb, eps2, G, red);
+    adj_sym_f64_item<true>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, blockIdx.x % slices, slices);
   else
-    adj_sym_f64_item<false>(blockIdx.x, n, nt, src, ab, xb, eps2, G, red);
+    adj_sym_f64_item<false>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, blockIdx.x % slices, slices);
 }
 
-// -- 6. hydro VJP (warp per leaf, lane per particle, lists of find_ngb) ------
+// -- 6. hydro VJP (S lanes per particle, lists of find_ngb) --------------------
 // Per pair the forward computes (dev_hydro_dots.cu:25-84 with the j-side):
 //   a_i -= m_j acc d,  a_j += m_i acc d,  du_i += ud * drdv
 // with d = x_i - x_j, ds = |d|, u = ds / h_i, h_i = w_i / 2,
@@ -562,11 +603,16 @@ __global__ void __launch_bounds__(kAdj64Warps * 32) k_adj_grav_sym_f64(int n, in
 // where pr = P / rho^2, c = sqrt(gamma P / rho), b = Balsara factor.  The
 // reverse sweep leaves xbar, vpbar, wbar_i and the adjoints of the
 // per-particle pr, c, b, om, psi (folded into rho, P, div, curl, w later).
+//
+// These loops are bound by the FP64 atomics of the neighbour's side and the
+// gathers.  As in the forward loops S lanes share a particle and no pair
+// divides; positions and masses come as one record, the gravity sources.
+// N = 65,536, us, one lane per particle with divisions / now: hydro 644 / 221,
+// density 468 / 208, h solve 310 / 80 (which also takes its sum from the kept
+// density loop and skips the flat middle of ig).
+template <int S>
 __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
-  const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (leaf >= a.nleaf) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
+  const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < a.n;
   double4 pi = make_double4(0, 0, 0, 1), vi = make_double4(0, 0, 0, 0), hi4 = make_double4(1, 0, 0, 0),
           di = make_double4(0, 0, 0, 0), abi = make_double4(0, 0, 0, 0);
@@ -578,10 +624,9 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
     hi4 = a.hyd[s];
     di = a.dd[s];
     abi = a.ab[s];
-    mi = a.vel[s].w;
+    mi = a.src[s].w;
     cnt = min(a.n_ngb[s], a.cap);
   }
-  const int kmax = warp_max_i(cnt);
   const int *lst = a.list + (size_t)s * a.stride;
   const double gam = a.gamma, alpha = a.alpha, beta = a.beta;
   const double wi = pi.w, hh = 0.5 * wi;
@@ -594,30 +639,33 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
   // i-side accumulators
   double xbx = 0, xby = 0, xbz = 0, vbx = 0, vby = 0, vbz = 0, ihb = 0;
   double prb_i = 0, cb_i = 0, bb_i = 0, omb_i = 0, psib_i = 0;
-  for (int k = 0; k < kmax; k++) {
-    if (k >= cnt) continue;
+  for (int k = sub; k < cnt; k += S) {
     const int j = __ldg(lst + k);
     if (j == s) continue;
-    const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j), fj = ld4(a.aux + j);
+    const double4 pj = ld4(a.src + j), vj = ld4(a.vpup + j), fj = ld4(a.aux + j);
     const double4 abj = ld4(a.ab + j);
-    const double mj = __ldg(&a.vel[j].w);
+    const double mj = pj.w;
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
-    const double ds = sqrt(dx * dx + dy * dy + dz * dz);
-    const double ids = ds > 0 ? 1.0 / ds : 0.0, imj = 1.0 / mj;
+    double ds, ids;
+    dist_and_inverse(dx * dx + dy * dy + dz * dz, ds, ids);
+    const double imj = fj.w;
     const double drdv = dx * dvx + dy * dvy + dz * dvz;
-    const double u = ds * ih;
+    const double u = ds * ih, iu = ids * hh;
     const double pr_j = fj.y, c_j = fj.x, b_j = fj.z;  // the neighbour's factors (k_hydro_prep)
     // forward
     const bool neg = drdv < 0;
-    const double S = c_i + c_j, B = b_i + b_j, Q = pr_i + pr_j;
-    double mu0 = 0, mu = 0, visc = 0;
+    const double B = b_i + b_j, Q = pr_i + pr_j;
+    double mu0 = 0, mu = 0, visc = 0, iS = 0;
     if (neg) {
-      mu0 = drdv * ids / S;
+      iS = 1.0 / (c_i + c_j);
+      mu0 = drdv * ids * iS;
       mu = mu0 * B;
       visc = Q * (-alpha * mu + beta * mu * mu);
     }
-    const double dwu = k_dw<double>(u), digu = k_dig<double>(u);
+    const double dwu = kernel_dw(u, iu);
+    double digu, ddigu;
+    kd_dig(u, iu, digu, ddigu);
     const double A1 = pr_i + 0.5 * visc;
     const double K2 = pr_i * om_i + 0.5 * psi_i;
     const double acc = A1 * dwu * ih5 - K2 * imj * digu * ih2;
@@ -649,9 +697,9 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
       const double mu0b = mub * B;
       const double Bb = mub * mu0;
       bb_i += Bb;
-      const double Sb = -mu0b * mu0 / S;
+      const double Sb = -mu0b * mu0 * iS;
       cb_i += Sb;
-      drdvb += mu0b * ids / S;
+      drdvb += mu0b * ids * iS;
       const double dsb_v = -mu0b * mu0 * ids;
       atomicAdd(&a.prb[j], prjb);
       atomicAdd(&a.bb[j], Bb);
@@ -659,7 +707,7 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
       dxb += dsb_v * dx * ids; dyb += dsb_v * dy * ids; dzb += dsb_v * dz * ids;
     }
     // u = ds * ih
-    const double ub = dwub * kd_dw(u) + digub * kd_dig(u);
+    const double ub = dwub * kd_dw(u, iu) + digub * ddigu;
     ihb += ub * ds;
     const double dsb = ub * ih;
     dxb += dsb * dx * ids; dyb += dsb * dy * ids; dzb += dsb * dz * ids;  // ids = 0 where ds = 0
@@ -671,7 +719,12 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
     atomic_add3(&a.xb[j], -dxb, -dyb, -dzb);
     atomic_add3(&a.vpb[j], -dvxb, -dvyb, -dvzb);
   }
-  if (!valid) return;
+  __syncwarp();
+  xbx = sub_sum<S>(xbx); xby = sub_sum<S>(xby); xbz = sub_sum<S>(xbz);
+  vbx = sub_sum<S>(vbx); vby = sub_sum<S>(vby); vbz = sub_sum<S>(vbz);
+  ihb = sub_sum<S>(ihb); prb_i = sub_sum<S>(prb_i); cb_i = sub_sum<S>(cb_i); bb_i = sub_sum<S>(bb_i);
+  omb_i = sub_sum<S>(omb_i); psib_i = sub_sum<S>(psib_i);
+  if (!valid || sub != 0) return;
   atomic_add3(&a.xb[s], xbx, xby, xbz);
   atomic_add3(&a.vpb[s], vbx, vby, vbz);
   // ih = 2 / w  ->  wbar += ihb * (-2 / w^2) = -ihb ih^2 / 2
@@ -698,8 +751,8 @@ __device__ __forceinline__ double pair_vs(const AdjArgs &a, int s, int j, double
   return vs;
 }
 
+// one warp, its lanes over the list (one thread: 71 us)
 __global__ void k_adj_vsig(AdjArgs a) {
-  if (threadIdx.x != 0) return;
   const double vsb = a.asc[2];
   const int s = (int)a.asc[3];
   if (vsb == 0 || s < 0 || s >= a.n) return;
@@ -707,14 +760,19 @@ __global__ void k_adj_vsig(AdjArgs a) {
   const double4 pi = a.pos[s], vi = a.vpup[s], hi4 = a.hyd[s];
   const double gam = a.gamma, beta = a.beta;
   const double c_i = sqrt(gam * hi4.y / hi4.x);
-  int kbest = -1;
+  int kbest = 0x7fffffff;
   double best = -1e300;
-  for (int k = 0; k < cnt; k++) {
-    const int j = a.list[(size_t)s * a.stride + k];
-    const double vs = pair_vs(a, s, j, c_i, pi, vi);
+  for (int k = (int)lane_id(); k < cnt; k += 32) {
+    const double vs = pair_vs(a, s, a.list[(size_t)s * a.stride + k], c_i, pi, vi);
     if (vs > best) { best = vs; kbest = k; }
   }
-  if (kbest < 0) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double v2 = __shfl_xor_sync(0xffffffffu, best, o);
+    const int k2 = __shfl_xor_sync(0xffffffffu, kbest, o);
+    if (v2 > best || (v2 == best && k2 < kbest)) { best = v2; kbest = k2; }
+  }
+  if (threadIdx.x != 0 || kbest == 0x7fffffff) return;
   {
     const int j = a.list[(size_t)s * a.stride + kbest];
     const double4 pj = a.pos[j], vj = a.vpup[j];
@@ -806,16 +864,14 @@ __global__ void k_adj_particle(AdjArgs a) {
   a.xb[i].w += wb;
 }
 
-// -- 9. density VJP (warp per leaf): epilogue reverse, then pairs ------------
+// -- 9. density VJP (S lanes per particle): epilogue reverse, then pairs ------
 // Forward (dev_density_loop.cu:29-86, with m_j in the divergence weight):
 //   R = sum m_j W(u), O = sum m_j dwdh(u), Q = sum m_j dphidh(u), S = -sum digdh(u),
 //   Dv = sum m_j dw(u) (d.dv), Cv = sum m_j dw(u) (d x dv),  u = 2 ds / w
 //   rho = R/h^3, om = O/(h^3 S), psi = Q/(h S), div = Dv/(rho h^5), curl = |Cv|/(rho h^5)
+template <int S>
 __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
-  const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (leaf >= a.nleaf) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
+  const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < a.n;
   double4 pi = make_double4(0, 0, 0, 1), vi = make_double4(0, 0, 0, 0);
   int cnt = 0;
@@ -824,14 +880,12 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
     vi = a.vpup[s];
     cnt = min(a.n_ngb[s], a.cap);
   }
-  const int kmax = warp_max_i(cnt);
   const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
-  const double i2w = w > 0 ? 2.0 / w : 0.0;
+  const double i2w = w > 0 ? 2.0 / w : 0.0, hw = 0.5 * w, iw = 0.5 * i2w;
   // forward sums: from the kept step when it recorded them, else summed again
-  double R = 0, O = 0, Qs = 0, S = 0, Dv = 0, Cx = 0, Cy = 0, Cz = 0;
-  for (int k = 0; k < (a.dsum ? 0 : kmax); k++) {
-    if (k >= cnt) continue;
+  double R = 0, O = 0, Qs = 0, Sg = 0, Dv = 0, Cx = 0, Cy = 0, Cz = 0;
+  for (int k = a.dsum ? cnt : sub; k < cnt; k += S) {
     const int j = __ldg(lst + k);
     const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j);
     const double mj = __ldg(&a.vel[j].w);
@@ -841,21 +895,26 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
     R += mj * k_w<double>(u);
     O += mj * k_dwdh<double>(u);
     Qs += mj * k_dphidh<double>(u);
-    S -= k_digdh<double>(u);
+    Sg -= k_digdh<double>(u);
     const double wt = mj * k_dw<double>(u);
     Dv += wt * (dx * dvx + dy * dvy + dz * dvz);
     Cx += wt * (dy * dvz - dz * dvy);
     Cy += wt * (dz * dvx - dx * dvz);
     Cz += wt * (dx * dvy - dy * dvx);
   }
-  // epilogue reverse
+  if (!a.dsum) {
+    __syncwarp();
+    R = sub_sum<S>(R); O = sub_sum<S>(O); Qs = sub_sum<S>(Qs); Sg = sub_sum<S>(Sg); Dv = sub_sum<S>(Dv);
+    Cx = sub_sum<S>(Cx); Cy = sub_sum<S>(Cy); Cz = sub_sum<S>(Cz);
+  }
+  // epilogue reverse (every lane of the particle; wb on the first)
   double Rb = 0, Ob = 0, Qb = 0, Sb = 0, Dvb = 0, Cxb = 0, Cyb = 0, Czb = 0, wb = 0;
   if (valid && w > 0 && cnt > 0) {
     const double h = 0.5 * w, h3 = h * h * h, h5 = h3 * h * h;
     double rho, div, om_k = 0, ps_k = 0;
     if (a.dsum) {  // the forward outputs and the sums they do not determine (S and the curl vector)
       const double4 sm4 = a.dsum[s], d4 = a.dd[s];
-      S = sm4.x; Cx = sm4.y; Cy = sm4.z; Cz = sm4.w;
+      Sg = sm4.x; Cx = sm4.y; Cy = sm4.z; Cz = sm4.w;
       rho = a.hyd[s].x;
       div = d4.x;
       om_k = d4.z;
@@ -877,38 +936,40 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
     }
     rhob -= curlb * curl / rho;
     hb -= 5.0 * curlb * curl / h;
-    if (S != 0) {
-      const double om = a.dsum ? om_k : O / (h3 * S), ps = a.dsum ? ps_k : Qs / (h * S);
+    if (Sg != 0) {
+      const double om = a.dsum ? om_k : O / (h3 * Sg), ps = a.dsum ? ps_k : Qs / (h * Sg);
       const double omb = a.omb[s], psb = a.psib[s];
-      Ob = omb / (h3 * S);
-      Sb -= omb * om / S;
+      Ob = omb / (h3 * Sg);
+      Sb -= omb * om / Sg;
       hb -= 3.0 * omb * om / h;
-      Qb = psb / (h * S);
-      Sb -= psb * ps / S;
+      Qb = psb / (h * Sg);
+      Sb -= psb * ps / Sg;
       hb -= psb * ps / h;
     }
     Rb = rhob / h3;
     hb -= 3.0 * rhob * rho / h;
-    wb = 0.5 * hb;
+    wb = sub == 0 ? 0.5 * hb : 0.0;
   }
   // pairs
   double xbx = 0, xby = 0, xbz = 0, vbx = 0, vby = 0, vbz = 0;
-  for (int k = 0; k < kmax; k++) {
-    if (k >= cnt) continue;
+  for (int k = sub; k < cnt; k += S) {
     const int j = __ldg(lst + k);
     if (j == s) continue;
-    const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j);
-    const double mj = __ldg(&a.vel[j].w);
+    const double4 pj = ld4(a.src + j), vj = ld4(a.vpup + j);
+    const double mj = pj.w;
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
-    const double ds = sqrt(dx * dx + dy * dy + dz * dz);
-    const double u = ds * i2w;
-    const double dwu = k_dw<double>(u);
+    double ds, ids;
+    dist_and_inverse(dx * dx + dy * dy + dz * dz, ds, ids);
+    const double u = ds * i2w, iu = ids * hw;
+    const double dwu = kernel_dw(u, iu);
+    double dig, ddig;
+    kd_dig(u, iu, dig, ddig);
     const double drdv = dx * dvx + dy * dvy + dz * dvz;
     const double crx = dy * dvz - dz * dvy, cry = dz * dvx - dx * dvz, crz = dx * dvy - dy * dvx;
     const double cdot = Cxb * crx + Cyb * cry + Czb * crz;
-    const double ub = mj * (Rb * u * dwu + Ob * kd_dwdh(u) + Qb * kd_dphidh(u)) - Sb * kd_digdh(u) +
-                      mj * kd_dw(u) * (Dvb * drdv + cdot);
+    const double ub = mj * (Rb * u * dwu + Ob * kd_dwdh(u) + Qb * kd_dphidh(u)) - Sb * u * (2 * dig + u * ddig) +
+                      mj * kd_dw(u, iu) * (Dvb * drdv + cdot);
     const double wt = mj * dwu;
     // d/d(d) of Dvb (d.dv) + Cb.(d x dv) = Dvb dv + dv x Cb ; d/d(dv) = Dvb d + Cb x d
     double dxb = wt * (Dvb * dvx + (dvy * Czb - dvz * Cyb));
@@ -917,17 +978,19 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
     const double dvxb = wt * (Dvb * dx + (Cyb * dz - Czb * dy));
     const double dvyb = wt * (Dvb * dy + (Czb * dx - Cxb * dz));
     const double dvzb = wt * (Dvb * dz + (Cxb * dy - Cyb * dx));
-    if (ds > 0) {
-      const double g = ub * i2w / ds;
-      dxb += g * dx; dyb += g * dy; dzb += g * dz;
-    }
-    wb -= ub * u / w;
+    const double g = ub * i2w * ids;  // ids = 0 where ds = 0
+    dxb += g * dx; dyb += g * dy; dzb += g * dz;
+    wb -= ub * u * iw;
     xbx += dxb; xby += dyb; xbz += dzb;
     vbx += dvxb; vby += dvyb; vbz += dvzb;
     atomic_add3(&a.xb[j], -dxb, -dyb, -dzb);
     atomic_add3(&a.vpb[j], -dvxb, -dvyb, -dvzb);
   }
-  if (!valid) return;
+  __syncwarp();
+  xbx = sub_sum<S>(xbx); xby = sub_sum<S>(xby); xbz = sub_sum<S>(xbz);
+  vbx = sub_sum<S>(vbx); vby = sub_sum<S>(vby); vbz = sub_sum<S>(vbz);
+  wb = sub_sum<S>(wb);
+  if (!valid || sub != 0) return;
   atomic_add3(&a.xb[s], xbx, xby, xbz);
   atomic_add3(&a.vpb[s], vbx, vby, vbz);
   atomicAdd(&a.xb[s].w, wb);
@@ -935,11 +998,10 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
 
 // -- 10. h-solve implicit derivative: xbar -= lambda_i dF_i/dx, lambda_i = wbar_i / F_w,i
 // F_i = sum_j ig(2 ds/w_i) - N;  F_w = -(1/w) sum digdh(u);  dF_i/dx_i = sum_j 4 dig(u)/w^2 d_ij
+// The sum of F_w is the kept density loop's {S}, or is taken again.
+template <int S>
 __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
-  const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (leaf >= a.nleaf) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
+  const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < a.n;
   double4 pi = make_double4(0, 0, 0, 1);
   int cnt = 0;
@@ -949,35 +1011,42 @@ __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
     cnt = min(a.n_ngb[s], a.cap);
     wbar = a.xb[s].w;
   }
-  const int kmax = warp_max_i(cnt);
   const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
-  const double i2w = w > 0 ? 2.0 / w : 0.0;
+  const double i2w = w > 0 ? 2.0 / w : 0.0, hw = 0.5 * w;
   double Fw = 0;
-  for (int k = 0; k < kmax; k++) {
-    if (k >= cnt) continue;
-    const int j = __ldg(lst + k);
-    const double4 pj = ld4(a.pos + j);
-    const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-    Fw -= k_digdh<double>(sqrt(dx * dx + dy * dy + dz * dz) * i2w);
+  if (a.dsum) {
+    if (valid) Fw = a.dsum[s].x;
+  } else {
+    for (int k = sub; k < cnt; k += S) {
+      const double4 pj = ld4(a.src + __ldg(lst + k));
+      const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      Fw -= k_digdh<double>(sqrt(dx * dx + dy * dy + dz * dz) * i2w);
+    }
+    __syncwarp();
+    Fw = sub_sum<S>(Fw);
   }
   Fw = w > 0 ? Fw / w : 0.0;
   const double lam = (valid && Fw != 0 && wbar != 0) ? wbar / Fw : 0.0;
   double xbx = 0, xby = 0, xbz = 0;
-  if (__any_sync(0xffffffffu, lam != 0)) {
-    for (int k = 0; k < kmax; k++) {
-      if (k >= cnt || lam == 0) continue;
+  if (lam != 0) {
+    const double f = -lam * i2w * i2w;  // -4 lambda / w^2
+    for (int k = sub; k < cnt; k += S) {
       const int j = __ldg(lst + k);
       if (j == s) continue;
-      const double4 pj = ld4(a.pos + j);
+      const double4 pj = ld4(a.src + j);
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-      const double u = sqrt(dx * dx + dy * dy + dz * dz) * i2w;
-      const double c = -lam * 4.0 * k_dig<double>(u) / (w * w);
+      double ds, ids;
+      dist_and_inverse(dx * dx + dy * dy + dz * dz, ds, ids);
+      const double c = f * ig_dig(ds * i2w, ids * hw);
+      if (c == 0) continue;  // most of the ball: ig is flat between u = 1/2 and 3/2
       xbx += c * dx; xby += c * dy; xbz += c * dz;
       atomic_add3(&a.xb[j], -c * dx, -c * dy, -c * dz);
     }
   }
-  if (!valid) return;
+  __syncwarp();
+  xbx = sub_sum<S>(xbx); xby = sub_sum<S>(xby); xbz = sub_sum<S>(xbz);
+  if (!valid || sub != 0) return;
   atomic_add3(&a.xb[s], xbx, xby, xbz);
 }
 
@@ -1010,11 +1079,9 @@ __global__ void __launch_bounds__(kAT) k_adj_predict(AdjArgs a) {
   }
 }
 
-__global__ void k_adj_predict_final(AdjArgs a, int nb) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double t = 0;
-  for (int b = 0; b < nb; b++) t += a.part[b];
-  a.asc[1] += t;
+__global__ void __launch_bounds__(kFold) k_adj_predict_final(AdjArgs a, int nb) {
+  const double t = fold_sum(nb, a.part);
+  if (threadIdx.x == 0) a.asc[1] += t;
 }
 
 // block partials: nb (kick sum) + 2 nb (arg-min value, index), reused by the predictor sum
@@ -1027,44 +1094,55 @@ int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const doubl
 int launch_adjoint(AdjArgs a, const double4 *src, const int *mass_mixed, double eps, double G, int precision,
                    cudaStream_t st) {
   const int n = a.n;
+  a.src = src;
   const int nb = (n + kAT - 1) / kAT;
-  const int warps_blocks = (a.nleaf * 32 + 127) / 128;
+  // lanes per particle as in the forward loops
+  constexpr int kSmall = 16, kLarge = 4, kSmallSet = 8192;
+  const bool small = n < kSmallSet;
+  const int list_blocks = (int)(((long long)n * (small ? kSmall : kLarge) + 127) / 128);
   int launches = 0;
   k_adj_init<<<nb, kAT, 0, st>>>(a); launches++;
   k_adj_kick<<<nb, kAT, 0, st>>>(a); launches++;
   AdjArgs b = a;
   b.part = a.part + nb;
   k_adj_argmin<<<nb, kAT, 0, st>>>(b); launches++;
-  k_adj_timestep<<<1, 32, 0, st>>>(a, nb, nb); launches++;
+  k_adj_timestep<<<1, kFold, 0, st>>>(a, nb, nb); launches++;
   {
-    // diagonal tiles one-sided (plain read-modify-write of xbar), then the
+    // diagonal tiles one-sided, then the
     // pairs above them once each (atomics on top)
     static_assert(kAdjTile % kGA == 0, "diagonal tiles must hold whole blocks");
     const int nt = (n + kAdjTile - 1) / kAdjTile;
     const int tile = nt < 2 ? 0 : kAdjTile;
-    if (precision == SPH_PREC_FP64)
-      k_adj_grav_f64<<<(n + kGA - 1) / kGA, kGA, 0, st>>>(n, src, a.ab, a.xb, eps * eps, G, tile);
-    else
-      k_adj_grav_f32<<<(n + kGA - 1) / kGA, kGA, 0, st>>>(n, src, a.ab, a.xb, (float)(eps * eps), G, tile);
+    const bool fp64 = precision == SPH_PREC_FP64;
+    // cut into source slices as the forward sums are (grav_slices): the whole
+    // reverse sweep of 2,000 particles 1050 -> 133 us, 20,011 1358 -> 526; two
+    // FP64 or three mixed symmetric blocks run on an SM
+    const int blocks = (n + kGA - 1) / kGA, sb = grav_slices(blocks, tile ? tile : n, 148 * 4, kGA);
+    if (fp64) k_adj_grav_f64<<<blocks * sb, kGA, 0, st>>>(n, src, a.ab, a.xb, eps * eps, G, tile, sb);
+    else k_adj_grav_f32<<<blocks * sb, kGA, 0, st>>>(n, src, a.ab, a.xb, (float)(eps * eps), G, tile, sb);
     launches++;
     if (nt >= 2) {
-      if (precision == SPH_PREC_FP64)
-        k_adj_grav_sym_f64<<<(unsigned)sym_items(nt), kAdj64Warps * 32, 0, st>>>(n, nt, src, a.ab, a.xb, eps * eps, G,
-                                                                                  mass_mixed);
+      const long long items = sym_items(nt), resident = 148 * (fp64 ? 2 : 3);
+      const int per = sym_chunk(nt) * kAdjTile;
+      int si = grav_slices(items, per, resident * 16, 256);
+      si *= grav_slices(items * si, per / si, resident * 2, 32);
+      if (fp64)
+        k_adj_grav_sym_f64<<<(unsigned)(items * si), kAdj64Warps * 32, 0, st>>>(n, nt, src, a.ab, a.xb, eps * eps, G,
+                                                                                mass_mixed, si);
       else
-        k_adj_grav_sym_f32<<<(unsigned)sym_items(nt), kAdjWarps * 32, 0, st>>>(n, nt, src, a.ab, a.xb,
-                                                                            (float)(eps * eps), G, mass_mixed);
+        k_adj_grav_sym_f32<<<(unsigned)(items * si), kAdjWarps * 32, 0, st>>>(n, nt, src, a.ab, a.xb,
+                                                                              (float)(eps * eps), G, mass_mixed, si);
       launches++;
     }
   }
   launches += launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);  // the neighbours' factors
-  k_adj_hydro<<<warps_blocks, 128, 0, st>>>(a); launches++;
+  (small ? k_adj_hydro<kSmall> : k_adj_hydro<kLarge>)<<<list_blocks, 128, 0, st>>>(a); launches++;
   k_adj_vsig<<<1, 32, 0, st>>>(a); launches++;
   k_adj_particle<<<nb, kAT, 0, st>>>(a); launches++;
-  k_adj_density<<<warps_blocks, 128, 0, st>>>(a); launches++;
-  k_adj_hsolve<<<warps_blocks, 128, 0, st>>>(a); launches++;
+  (small ? k_adj_density<kSmall> : k_adj_density<kLarge>)<<<list_blocks, 128, 0, st>>>(a); launches++;
+  (small ? k_adj_hsolve<kSmall> : k_adj_hsolve<kLarge>)<<<list_blocks, 128, 0, st>>>(a); launches++;
   k_adj_predict<<<nb, kAT, 0, st>>>(a); launches++;
-  k_adj_predict_final<<<1, 32, 0, st>>>(a, nb); launches++;
+  k_adj_predict_final<<<1, kFold, 0, st>>>(a, nb); launches++;
   return launches;
 }
 

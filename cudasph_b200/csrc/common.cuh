@@ -77,6 +77,7 @@ struct AdjArgs {
   const double4 *old;     // v0, u0
   const double4 *pre_acc; // a0, du0
   const double4 *x0;      // x0 (pre-predict positions)
+  const double4 *src;     // x1, m
   double4 *vpup;          // vp, up (recomputed)
   const int *n_ngb, *list;
   const double *sc;       // forward scalars: [0] dt0  [1] dt1
@@ -177,6 +178,37 @@ __host__ __device__ __forceinline__ void sym_item(long long item, int nt, int &b
 
 // number of work items for nt tiles
 __host__ __device__ __forceinline__ long long sym_items(int nt) { return nt >= 2 ? sym_S(nt - 1, sym_chunk(nt)) : 0; }
+
+// A launch with too few blocks for the GPU cuts each block's sources into
+// `slices` parts, one block each (grav_slices below).  Slice q of [lo, hi) is
+// a whole number of UNIT-source batches, the sources whose FP32 terms the
+// mixed kernels add up before they fold into FP64: the sums then do not
+// depend on the slices but by the order of the FP64 additions.  The parts
+// meet by atomics in an output cleared beforehand.
+template <int UNIT>
+__device__ __forceinline__ void source_slice(int &lo, int &hi, unsigned q, int slices) {
+  if (slices == 1) return;
+  const int nb = (hi - lo + UNIT - 1) / UNIT;
+  const int b = nb * (int)q / slices, e = nb * ((int)q + 1) / slices;
+  hi = min(hi, lo + e * UNIT);
+  lo += b * UNIT;
+}
+
+// Slices of each block's sources (source_slice), a power of two: while the
+// launch has fewer blocks than `want` and a slice keeps `least` sources.
+// Uncut, a small set leaves most of the GPU idle (16,384 particles have 120
+// tile pairs for 592 resident blocks) and a launch of one to a few rounds of
+// blocks ends on a nearly empty one.  Gravity phase, us, uncut / cut: FP64
+// 1,000 particles 107 / 21, 2,049 331 / 33, 6,000 334 / 69, 16,384 348 / 245,
+// 100,003 8402 / 6875; mixed 6,000 239 / 56, 16,384 244 / 150, 30,000 417 /
+// 335, 65,536 1485 / 1331, 100,003 4303 / 2992, 262,144 19,980 / 19,360 (four
+// rounds instead of sixteen: 100,003 3193, 262,144 19,967).  From about
+// 400,000 particles on nothing is cut.
+inline int grav_slices(long long blocks, int sources, long long want, int least) {
+  int s = 1;
+  while (blocks * s < want && sources / (2 * s) >= least) s *= 2;
+  return s;
+}
 
 // Contiguous balanced split of [0, count) over `world` shards: shard `rank`
 // owns [count * rank / world, count * (rank + 1) / world).
