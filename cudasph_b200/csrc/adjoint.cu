@@ -87,6 +87,7 @@ __device__ __forceinline__ void atomic_add3(double4 *p, double x, double y, doub
 
 // -- 1. vp, up of the forward predictor; clear the internal adjoints ---------
 __global__ void k_adj_init(AdjArgs a) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   const double dth = 0.5 * a.sc[0];
@@ -101,6 +102,7 @@ __global__ void k_adj_init(AdjArgs a) {
 
 // -- 2. kick adjoint + the reduction sum(vbar.a1 + ubar du1) -----------------
 __global__ void __launch_bounds__(kAT) k_adj_kick(AdjArgs a) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double s = 0;
   if (i < a.n) {
@@ -132,6 +134,7 @@ __device__ __forceinline__ double tau_of(double w, double vs, double up, double 
 
 // -- 3. arg-min of tau over particles (block partials) -----------------------
 __global__ void __launch_bounds__(kAT) k_adj_argmin(AdjArgs a) {
+  grid_enter();
   double t = 1e300;
   int idx = 0x7fffffff;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
@@ -175,6 +178,7 @@ __device__ __forceinline__ double fold_sum(int nb, const double *part) {
 }
 
 __global__ void __launch_bounds__(kFold) k_adj_timestep(AdjArgs a, int nb_kick, int nb_min) {
+  grid_enter();
   const double f = fold_sum(nb_kick, a.part);
   double t = 1e300;
   int idx = 0;
@@ -229,9 +233,9 @@ __global__ void __launch_bounds__(kFold) k_adj_timestep(AdjArgs a, int nb_kick, 
 // diagonal tiles (tile > 0) or all pairs of a small system (tile = 0).
 constexpr int kGA = 128;
 
-__global__ void __launch_bounds__(kGA) k_adj_grav_f64(int n, const double4 *__restrict__ src,
-                                                      const double4 *__restrict__ ab, double4 *__restrict__ xb,
+__global__ void __launch_bounds__(kGA) k_adj_grav_f64(int n, const double4 *src, const double4 *ab, double4 *xb,
                                                       double eps2, double G, int tile, int slices) {
+  grid_enter();
   __shared__ double4 sp[kGA];
   __shared__ double4 sg[kGA];
   const int t = threadIdx.x;
@@ -280,9 +284,9 @@ __global__ void __launch_bounds__(kGA) k_adj_grav_f64(int n, const double4 *__re
 
 // mixed form of the gravity VJP: FP32 pair terms relative to the block's FP64
 // anchor, FP64 per-tile accumulation
-__global__ void __launch_bounds__(kGA) k_adj_grav_f32(int n, const double4 *__restrict__ src,
-                                                      const double4 *__restrict__ ab, double4 *__restrict__ xb,
+__global__ void __launch_bounds__(kGA) k_adj_grav_f32(int n, const double4 *src, const double4 *ab, double4 *xb,
                                                       float eps2, double G, int tile, int slices) {
+  grid_enter();
   __shared__ float4 sp[kGA];
   __shared__ float4 sg[kGA];
   const int t = threadIdx.x;
@@ -478,13 +482,13 @@ __device__ __forceinline__ void adj_sym_f32_item(long long item, int n, int nt, 
 }
 
 // mass_mixed: the forward step's device word, 0 when all masses are equal
-__global__ void __launch_bounds__(kAdjWarps * 32) k_adj_grav_sym_f32(int n, int nt, const double4 *__restrict__ src,
-                                                                    const double4 *__restrict__ ab,
-                                                                    double4 *__restrict__ xb, float eps2, double G,
-                                                                    const int *__restrict__ mass_mixed, int slices) {
+__global__ void __launch_bounds__(kAdjWarps * 32) k_adj_grav_sym_f32(int n, int nt, const double4 *src,
+                                                                     const double4 *ab, double4 *xb, float eps2,
+                                                                     double G, const int *mass_mixed, int slices) {
+  grid_enter();
   __shared__ float red[2][kAdjWarps][3][32];
   __shared__ double iacc[2 * kAdjRP * 3][kAdjWarps * 32];  // [i-slot * 3 + component][thread]
-  if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
+  if (mass_mixed != nullptr && ldg(mass_mixed) == 0)
     adj_sym_f32_item<true>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, iacc, blockIdx.x % slices, slices);
   else
     adj_sym_f32_item<false>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, iacc, blockIdx.x % slices, slices);
@@ -582,12 +586,12 @@ __device__ __forceinline__ void adj_sym_f64_item(long long item, int n, int nt, 
   }
 }
 
-__global__ void __launch_bounds__(kAdj64Warps * 32) k_adj_grav_sym_f64(int n, int nt, const double4 *__restrict__ src,
-                                                                      const double4 *__restrict__ ab,
-                                                                      double4 *__restrict__ xb, double eps2, double G,
-                                                                      const int *__restrict__ mass_mixed, int slices) {
+__global__ void __launch_bounds__(kAdj64Warps * 32) k_adj_grav_sym_f64(int n, int nt, const double4 *src,
+                                                                       const double4 *ab, double4 *xb, double eps2,
+                                                                       double G, const int *mass_mixed, int slices) {
+  grid_enter();
   __shared__ double red[2][kAdj64Warps][3][32];
-  if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
+  if (mass_mixed != nullptr && ldg(mass_mixed) == 0)
     adj_sym_f64_item<true>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, blockIdx.x % slices, slices);
   else
     adj_sym_f64_item<false>(blockIdx.x / slices, n, nt, src, ab, xb, eps2, G, red, blockIdx.x % slices, slices);
@@ -612,6 +616,7 @@ __global__ void __launch_bounds__(kAdj64Warps * 32) k_adj_grav_sym_f64(int n, in
 // density loop and skips the flat middle of ig).
 template <int S>
 __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
+  grid_enter();
   const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < a.n;
   double4 pi = make_double4(0, 0, 0, 1), vi = make_double4(0, 0, 0, 0), hi4 = make_double4(1, 0, 0, 0),
@@ -640,7 +645,7 @@ __global__ void __launch_bounds__(128) k_adj_hydro(AdjArgs a) {
   double xbx = 0, xby = 0, xbz = 0, vbx = 0, vby = 0, vbz = 0, ihb = 0;
   double prb_i = 0, cb_i = 0, bb_i = 0, omb_i = 0, psib_i = 0;
   for (int k = sub; k < cnt; k += S) {
-    const int j = __ldg(lst + k);
+    const int j = ldg(lst + k);
     if (j == s) continue;
     const double4 pj = ld4(a.src + j), vj = ld4(a.vpup + j), fj = ld4(a.aux + j);
     const double4 abj = ld4(a.ab + j);
@@ -753,6 +758,7 @@ __device__ __forceinline__ double pair_vs(const AdjArgs &a, int s, int j, double
 
 // one warp, its lanes over the list (one thread: 71 us)
 __global__ void k_adj_vsig(AdjArgs a) {
+  grid_enter();
   const double vsb = a.asc[2];
   const int s = (int)a.asc[3];
   if (vsb == 0 || s < 0 || s >= a.n) return;
@@ -796,6 +802,7 @@ __global__ void k_adj_vsig(AdjArgs a) {
 
 // -- 8. per particle: pr, c, b -> rho, P, div, curl, w; then the EOS ---------
 __global__ void k_adj_particle(AdjArgs a) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   const double4 h = a.hyd[i], d = a.dd[i], p = a.pos[i];
@@ -871,6 +878,7 @@ __global__ void k_adj_particle(AdjArgs a) {
 //   rho = R/h^3, om = O/(h^3 S), psi = Q/(h S), div = Dv/(rho h^5), curl = |Cv|/(rho h^5)
 template <int S>
 __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
+  grid_enter();
   const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < a.n;
   double4 pi = make_double4(0, 0, 0, 1), vi = make_double4(0, 0, 0, 0);
@@ -886,9 +894,9 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
   // forward sums: from the kept step when it recorded them, else summed again
   double R = 0, O = 0, Qs = 0, Sg = 0, Dv = 0, Cx = 0, Cy = 0, Cz = 0;
   for (int k = a.dsum ? cnt : sub; k < cnt; k += S) {
-    const int j = __ldg(lst + k);
+    const int j = ldg(lst + k);
     const double4 pj = ld4(a.pos + j), vj = ld4(a.vpup + j);
-    const double mj = __ldg(&a.vel[j].w);
+    const double mj = ldg(&a.vel[j].w);
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
     const double u = sqrt(dx * dx + dy * dy + dz * dz) * i2w;
@@ -953,7 +961,7 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
   // pairs
   double xbx = 0, xby = 0, xbz = 0, vbx = 0, vby = 0, vbz = 0;
   for (int k = sub; k < cnt; k += S) {
-    const int j = __ldg(lst + k);
+    const int j = ldg(lst + k);
     if (j == s) continue;
     const double4 pj = ld4(a.src + j), vj = ld4(a.vpup + j);
     const double mj = pj.w;
@@ -1001,6 +1009,7 @@ __global__ void __launch_bounds__(128) k_adj_density(AdjArgs a) {
 // The sum of F_w is the kept density loop's {S}, or is taken again.
 template <int S>
 __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
+  grid_enter();
   const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < a.n;
   double4 pi = make_double4(0, 0, 0, 1);
@@ -1019,7 +1028,7 @@ __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
     if (valid) Fw = a.dsum[s].x;
   } else {
     for (int k = sub; k < cnt; k += S) {
-      const double4 pj = ld4(a.src + __ldg(lst + k));
+      const double4 pj = ld4(a.src + ldg(lst + k));
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
       Fw -= k_digdh<double>(sqrt(dx * dx + dy * dy + dz * dz) * i2w);
     }
@@ -1032,7 +1041,7 @@ __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
   if (lam != 0) {
     const double f = -lam * i2w * i2w;  // -4 lambda / w^2
     for (int k = sub; k < cnt; k += S) {
-      const int j = __ldg(lst + k);
+      const int j = ldg(lst + k);
       if (j == s) continue;
       const double4 pj = ld4(a.src + j);
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
@@ -1052,6 +1061,7 @@ __global__ void __launch_bounds__(128) k_adj_hsolve(AdjArgs a) {
 
 // -- 11. predictor reverse + dtbar0 partials ---------------------------------
 __global__ void __launch_bounds__(kAT) k_adj_predict(AdjArgs a) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double s = 0;
   if (i < a.n) {
@@ -1080,6 +1090,7 @@ __global__ void __launch_bounds__(kAT) k_adj_predict(AdjArgs a) {
 }
 
 __global__ void __launch_bounds__(kFold) k_adj_predict_final(AdjArgs a, int nb) {
+  grid_enter();
   const double t = fold_sum(nb, a.part);
   if (threadIdx.x == 0) a.asc[1] += t;
 }
@@ -1101,12 +1112,12 @@ int launch_adjoint(AdjArgs a, const double4 *src, const int *mass_mixed, double 
   const bool small = n < kSmallSet;
   const int list_blocks = (int)(((long long)n * (small ? kSmall : kLarge) + 127) / 128);
   int launches = 0;
-  k_adj_init<<<nb, kAT, 0, st>>>(a); launches++;
-  k_adj_kick<<<nb, kAT, 0, st>>>(a); launches++;
+  launch(k_adj_init, nb, kAT, st, a); launches++;
+  launch(k_adj_kick, nb, kAT, st, a); launches++;
   AdjArgs b = a;
   b.part = a.part + nb;
-  k_adj_argmin<<<nb, kAT, 0, st>>>(b); launches++;
-  k_adj_timestep<<<1, kFold, 0, st>>>(a, nb, nb); launches++;
+  launch(k_adj_argmin, nb, kAT, st, b); launches++;
+  launch(k_adj_timestep, 1, kFold, st, a, nb, nb); launches++;
   {
     // diagonal tiles one-sided, then the
     // pairs above them once each (atomics on top)
@@ -1118,8 +1129,8 @@ int launch_adjoint(AdjArgs a, const double4 *src, const int *mass_mixed, double 
     // reverse sweep of 2,000 particles 1050 -> 133 us, 20,011 1358 -> 526; two
     // FP64 or three mixed symmetric blocks run on an SM
     const int blocks = (n + kGA - 1) / kGA, sb = grav_slices(blocks, tile ? tile : n, 148 * 4, kGA);
-    if (fp64) k_adj_grav_f64<<<blocks * sb, kGA, 0, st>>>(n, src, a.ab, a.xb, eps * eps, G, tile, sb);
-    else k_adj_grav_f32<<<blocks * sb, kGA, 0, st>>>(n, src, a.ab, a.xb, (float)(eps * eps), G, tile, sb);
+    if (fp64) launch(k_adj_grav_f64, blocks * sb, kGA, st, n, src, a.ab, a.xb, eps * eps, G, tile, sb);
+    else launch(k_adj_grav_f32, blocks * sb, kGA, st, n, src, a.ab, a.xb, (float)(eps * eps), G, tile, sb);
     launches++;
     if (nt >= 2) {
       const long long items = sym_items(nt), resident = 148 * (fp64 ? 2 : 3);
@@ -1127,22 +1138,22 @@ int launch_adjoint(AdjArgs a, const double4 *src, const int *mass_mixed, double 
       int si = grav_slices(items, per, resident * 16, 256);
       si *= grav_slices(items * si, per / si, resident * 2, 32);
       if (fp64)
-        k_adj_grav_sym_f64<<<(unsigned)(items * si), kAdj64Warps * 32, 0, st>>>(n, nt, src, a.ab, a.xb, eps * eps, G,
-                                                                                mass_mixed, si);
+        launch(k_adj_grav_sym_f64, (unsigned)(items * si), kAdj64Warps * 32, st, n, nt, src, a.ab, a.xb, eps * eps,
+               G, mass_mixed, si);
       else
-        k_adj_grav_sym_f32<<<(unsigned)(items * si), kAdjWarps * 32, 0, st>>>(n, nt, src, a.ab, a.xb,
-                                                                              (float)(eps * eps), G, mass_mixed, si);
+        launch(k_adj_grav_sym_f32, (unsigned)(items * si), kAdjWarps * 32, st, n, nt, src, a.ab, a.xb,
+               (float)(eps * eps), G, mass_mixed, si);
       launches++;
     }
   }
   launches += launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);  // the neighbours' factors
-  (small ? k_adj_hydro<kSmall> : k_adj_hydro<kLarge>)<<<list_blocks, 128, 0, st>>>(a); launches++;
-  k_adj_vsig<<<1, 32, 0, st>>>(a); launches++;
-  k_adj_particle<<<nb, kAT, 0, st>>>(a); launches++;
-  (small ? k_adj_density<kSmall> : k_adj_density<kLarge>)<<<list_blocks, 128, 0, st>>>(a); launches++;
-  (small ? k_adj_hsolve<kSmall> : k_adj_hsolve<kLarge>)<<<list_blocks, 128, 0, st>>>(a); launches++;
-  k_adj_predict<<<nb, kAT, 0, st>>>(a); launches++;
-  k_adj_predict_final<<<1, kFold, 0, st>>>(a, nb); launches++;
+  launch(small ? k_adj_hydro<kSmall> : k_adj_hydro<kLarge>, list_blocks, 128, st, a); launches++;
+  launch(k_adj_vsig, 1, 32, st, a); launches++;
+  launch(k_adj_particle, nb, kAT, st, a); launches++;
+  launch(small ? k_adj_density<kSmall> : k_adj_density<kLarge>, list_blocks, 128, st, a); launches++;
+  launch(small ? k_adj_hsolve<kSmall> : k_adj_hsolve<kLarge>, list_blocks, 128, st, a); launches++;
+  launch(k_adj_predict, nb, kAT, st, a); launches++;
+  launch(k_adj_predict_final, 1, kFold, st, a, nb); launches++;
   return launches;
 }
 

@@ -101,6 +101,37 @@ struct StepScalars {
   double v[4 + SPH_NSTATS];
 };
 
+// Programmatic dependent launch.  A step is about 30 kernels of which most
+// are short in a small set, and each used to start after the one before had
+// drained.  Launched with the attribute below, a kernel's blocks may be
+// placed while the last blocks of the one before still run, and wait in
+// grid_enter() until that one is complete and its writes are visible.
+// Every kernel launched so calls it before anything else, so a kernel's
+// completion implies that of all before it.  No load may move above it: the
+// kernels take their pointers without __restrict__, and read-only loads go
+// through ldg and ld4 below, which are volatile assembly like the wait itself.
+// Time per step, us, without / with: 2,049 particles 191 / 147, 16,384
+// 746 / 644; replayed from a graph 6,007 243 / 226.
+__device__ __forceinline__ void grid_enter() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// kernel<<<grid, block, 0, st>>>(args...), programmatic on a stream of its own
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = st != nullptr ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ double4 ld4(const double4 *p) {
@@ -108,7 +139,24 @@ __device__ __forceinline__ double4 ld4(const double4 *p) {
   // 32-byte-aligned record; against two 16-byte loads it halves the load
   // instructions of the list-driven gathers (N = 1M: hydro 1.89 -> 1.75 ms)
   double4 r;
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+
+// read-only loads (see grid_enter)
+__device__ __forceinline__ int ldg(const int *p) {
+  int r;
+  asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ double ldg(const double *p) {
+  double r;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(r) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float4 ldg(const float4 *p) {
+  float4 r;
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
   return r;
 }
 

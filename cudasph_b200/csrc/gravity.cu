@@ -101,9 +101,9 @@ __device__ __forceinline__ void store_sums(double4 *out, double x, double y, dou
 // tile > 0 the range is the tile of `tile` particles that holds the block
 // (the diagonal tiles of the symmetric form), else all n.
 template <int SOFT, int R>
-__global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *__restrict__ src,
-                                                        const double *__restrict__ h2src, double4 *__restrict__ out,
+__global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *src, const double *h2src, double4 *out,
                                                         double eps2, double G, int tile, int block0, int slices) {
+  grid_enter();
   __shared__ double4 sj[kGThreads];
   __shared__ double sh[SOFT == SPH_SOFT_SPLINE ? kGThreads : 1];
   const int t = threadIdx.x;
@@ -189,9 +189,9 @@ __device__ __forceinline__ void kahan_add(float &hi, float &lo, float v) {
 }
 
 template <int SOFT, int R>
-__global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *__restrict__ src,
-                                                        const double *__restrict__ h2src, double4 *__restrict__ out,
+__global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *src, const double *h2src, double4 *out,
                                                         float eps2, double G, int block0, int slices) {
+  grid_enter();
   __shared__ float4 sj[kGThreads];
   __shared__ float sh[SOFT == SPH_SOFT_SPLINE ? kGThreads : 1];
   const int t = threadIdx.x;
@@ -316,9 +316,9 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *__
 // tile > 0 the range is the tile of `tile` particles that holds the block
 // (the diagonal tiles of the symmetric form), else all n.
 template <int RP>  // i-particle pairs per thread
-__global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const double4 *__restrict__ src,
-                                                                  double4 *__restrict__ out, float eps2, double G,
-                                                                  int tile, int block0, int slices) {
+__global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const double4 *src, double4 *out, float eps2,
+                                                                  double G, int tile, int block0, int slices) {
+  grid_enter();
   __shared__ ulonglong2 sj[kGThreads][2];
   const int t = threadIdx.x;
   const int i0 = (blockIdx.x / slices + block0) * kGThreads * 2 * RP;
@@ -587,15 +587,16 @@ __device__ __forceinline__ void sym_plummer_item(long long item, int n, int nt, 
 
 // mass_mixed: device word, 0 when all masses are equal (nullptr: general form);
 // block b runs slice b % slices of work item item0 + b / slices
-__global__ void __launch_bounds__(kSymWarps * 32, 4) k_grav_sym_plummer(int n, int nt, const double4 *__restrict__ src,
-                                                                         double4 *__restrict__ out, float eps2,
-                                                                         double G, const int *__restrict__ mass_mixed,
-                                                                         long long item0, int slices) {
+__global__ void __launch_bounds__(kSymWarps * 32, 4) k_grav_sym_plummer(int n, int nt, const double4 *src,
+                                                                        double4 *out, float eps2, double G,
+                                                                        const int *mass_mixed, long long item0,
+                                                                        int slices) {
+  grid_enter();
   __shared__ float red[2][kSymWarps][4][32];
   __shared__ double iacc[2 * kSymRP * 4][kSymWarps * 32];  // [i-slot * 4 + component][thread]
   const long long item = item0 + blockIdx.x / slices;
   const unsigned slice = blockIdx.x % slices;
-  if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
+  if (mass_mixed != nullptr && ldg(mass_mixed) == 0)
     sym_plummer_item<true>(item, n, nt, src, out, eps2, G, red, iacc, slice, slices);
   else
     sym_plummer_item<false>(item, n, nt, src, out, eps2, G, red, iacc, slice, slices);
@@ -784,15 +785,15 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
 // block b runs slice b / 2 % slices of work item item0 + b / 2 / slices, on
 // one half of its i-tile (b & 1)
 template <int SOFT>
-__global__ void __launch_bounds__(kSym64Warps * 32) k_grav_sym_f64(int n, int nt, const double4 *__restrict__ src,
-                                                                  const double *__restrict__ h2src,
-                                                                  double4 *__restrict__ out, double eps2, double G,
-                                                                  const int *__restrict__ mass_mixed, long long item0,
-                                                                  int slices) {
+__global__ void __launch_bounds__(kSym64Warps * 32) k_grav_sym_f64(int n, int nt, const double4 *src,
+                                                                   const double *h2src, double4 *out, double eps2,
+                                                                   double G, const int *mass_mixed, long long item0,
+                                                                   int slices) {
+  grid_enter();
   __shared__ double red[2][kSym64Warps][4][32];
   const unsigned q = blockIdx.x >> 1;
   const long long item = item0 + q / slices;
-  if (mass_mixed != nullptr && __ldg(mass_mixed) == 0)
+  if (mass_mixed != nullptr && ldg(mass_mixed) == 0)
     sym_f64_item<true, SOFT>(item, n, nt, src, h2src, out, eps2, G, red, blockIdx.x & 1, q % slices, slices);
   else
     sym_f64_item<false, SOFT>(item, n, nt, src, h2src, out, eps2, G, red, blockIdx.x & 1, q % slices, slices);
@@ -877,32 +878,31 @@ int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out,
     // diagonal tiles one-sided (all pairs when there is a single tile), then the items above them
     const bool plummer = soft_mode == SPH_SOFT_PLUMMER;
     if (!blocks.empty()) {
-      (plummer ? k_grav_f64<SPH_SOFT_PLUMMER, R> : k_grav_f64<SPH_SOFT_SPLINE, R>)
-          <<<blocks.grid() * sb, kGThreads, 0, st>>>(n, src, h2src, out, eps2, G, g.tile, (int)blocks.lo, sb);
+      launch(plummer ? k_grav_f64<SPH_SOFT_PLUMMER, R> : k_grav_f64<SPH_SOFT_SPLINE, R>, blocks.grid() * sb,
+             kGThreads, st, n, src, h2src, out, eps2, G, g.tile, (int)blocks.lo, sb);
       launches++;
     }
     if (!items.empty()) {
-      (plummer ? k_grav_sym_f64<SPH_SOFT_PLUMMER> : k_grav_sym_f64<SPH_SOFT_SPLINE>)
-          <<<items.grid() * 2 * si, kSym64Warps * 32, 0, st>>>(n, nt, src, h2src, out, eps2, G, mass_mixed, items.lo,
-                                                               si);
+      launch(plummer ? k_grav_sym_f64<SPH_SOFT_PLUMMER> : k_grav_sym_f64<SPH_SOFT_SPLINE>, items.grid() * 2 * si,
+             kSym64Warps * 32, st, n, nt, src, h2src, out, eps2, G, mass_mixed, items.lo, si);
       launches++;
     }
   } else if (soft_mode == SPH_SOFT_PLUMMER) {
     constexpr int RP = 1;
     static_assert(kSymTile % (kGThreads * 2 * RP) == 0, "diagonal tiles must hold whole blocks");
     if (!blocks.empty()) {
-      k_grav_f32x2_plummer<RP><<<blocks.grid() * sb, kGThreads, 0, st>>>(n, src, out, (float)eps2, G, g.tile,
-                                                                        (int)blocks.lo, sb);
+      launch(k_grav_f32x2_plummer<RP>, blocks.grid() * sb, kGThreads, st, n, src, out, (float)eps2, G, g.tile,
+             (int)blocks.lo, sb);
       launches++;
     }
     if (!items.empty()) {
-      k_grav_sym_plummer<<<items.grid() * si, kSymWarps * 32, 0, st>>>(n, nt, src, out, (float)eps2, G, mass_mixed,
-                                                                       items.lo, si);
+      launch(k_grav_sym_plummer, items.grid() * si, kSymWarps * 32, st, n, nt, src, out, (float)eps2, G, mass_mixed,
+             items.lo, si);
       launches++;
     }
   } else if (!blocks.empty()) {
-    k_grav_f32<SPH_SOFT_SPLINE, 4><<<blocks.grid() * sb, kGThreads, 0, st>>>(n, src, h2src, out, (float)eps2, G,
-                                                                            (int)blocks.lo, sb);
+    launch(k_grav_f32<SPH_SOFT_SPLINE, 4>, blocks.grid() * sb, kGThreads, st, n, src, h2src, out, (float)eps2, G,
+           (int)blocks.lo, sb);
     launches++;
   }
   return launches;
@@ -912,8 +912,9 @@ int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out,
 // Also raises *mass_mixed (cleared before the launch) when some mass differs
 // from the first particle's: the symmetric kernels take their equal-mass form
 // when it stays 0.
-__global__ void k_pack_sources(int n, const double4 *__restrict__ pos, const double4 *__restrict__ vel,
-                               double4 *__restrict__ src, double *__restrict__ h2, int *__restrict__ mass_mixed) {
+__global__ void k_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2,
+                               int *mass_mixed) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool differs = false;
   if (i < n) {
@@ -921,7 +922,7 @@ __global__ void k_pack_sources(int n, const double4 *__restrict__ pos, const dou
     const double m = vel[i].w;
     src[i] = make_double4(p.x, p.y, p.z, m);
     h2[i] = p.w * p.w;
-    differs = m != __ldg(&vel[0].w);
+    differs = m != ldg(&vel[0].w);
   }
   if (__syncthreads_or(differs) && threadIdx.x == 0) atomicOr(mass_mixed, 1);
 }
@@ -929,11 +930,12 @@ __global__ void k_pack_sources(int n, const double4 *__restrict__ pos, const dou
 int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, int *mass_mixed,
                         cudaStream_t st) {
   cudaMemsetAsync(mass_mixed, 0, sizeof(int), st);
-  k_pack_sources<<<(n + 255) / 256, 256, 0, st>>>(n, pos, vel, src, h2, mass_mixed);
+  launch(k_pack_sources, (n + 255) / 256, 256, st, n, pos, vel, src, h2, mass_mixed);
   return 1;
 }
 
-__global__ void k_range_sq(int n, const double *__restrict__ r, double *__restrict__ h2) {
+__global__ void k_range_sq(int n, const double *r, double *h2) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) h2[i] = r ? r[i] * r[i] : 0.0;
 }
@@ -950,7 +952,7 @@ extern "C" int cudasph_gravity_direct(int n, const double *pos4, const double *r
   double *h2 = nullptr;
   if (soft_mode == SPH_SOFT_SPLINE) {
     SPH_CUDA_TRY(cudaMallocAsync((void **)&h2, sizeof(double) * n, st));
-    sph::k_range_sq<<<(n + 255) / 256, 256, 0, st>>>(n, range, h2);
+    sph::launch(sph::k_range_sq, (n + 255) / 256, 256, st, n, range, h2);
   }
   sph::launch_gravity(n, (const double4 *)pos4, h2, (double4 *)out4, soft_mode, eps, G, precision, nullptr, 0, 1, st);
   if (h2) SPH_CUDA_TRY(cudaFreeAsync(h2, st));

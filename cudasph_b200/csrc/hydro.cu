@@ -63,6 +63,7 @@ constexpr int kSubDensity = 2, kSubHydro = 4;
 
 template <int S>
 __global__ void __launch_bounds__(128) k_density(HydroArgs a) {
+  grid_enter();
   const int s = a.leaf0 * kLeaf + (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < min(a.leaf1 * kLeaf, a.n);
   double4 pi = make_double4(0, 0, 0, 0), vi = make_double4(0, 0, 0, 0);
@@ -78,10 +79,10 @@ __global__ void __launch_bounds__(128) k_density(HydroArgs a) {
   double dens = 0, om = 0, ps = 0, sdig = 0, div = 0, cx = 0, cy = 0, cz = 0;
   // the neighbours' records are gathered one pair ahead of their use and
   // the list entries two ahead, so the loads overlap the pair arithmetic
-  int jn = sub + S < cnt ? __ldg(lst + sub + S) : 0;
+  int jn = sub + S < cnt ? ldg(lst + sub + S) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn;
   if (sub < cnt) {
-    const int j0 = __ldg(lst + sub);
+    const int j0 = ldg(lst + sub);
     pn = ld4(a.pos + j0);
     vn = ld4(a.vel + j0);
   }
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(128) k_density(HydroArgs a) {
       if (k + S < cnt) {
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
-        if (k + 2 * S < cnt) jn = __ldg(lst + k + 2 * S);
+        if (k + 2 * S < cnt) jn = ldg(lst + k + 2 * S);
       }
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
       double r, ir;
@@ -182,7 +183,8 @@ __device__ __forceinline__ double pressure_of(double rho, double u, double mu, i
   return (pg + pr) / kPressureUnit;
 }
 
-__global__ void k_pressure(int n, double4 *__restrict__ hyd, int eos_mode, double gamma, unsigned *flags) {
+__global__ void k_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsigned *flags) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double4 h = hyd[i];
@@ -197,9 +199,9 @@ __global__ void k_pressure(int n, double4 *__restrict__ hyd, int eos_mode, doubl
 // the same operations the pair formula applies to them, and 1 / m, so the
 // pair loop gathers one record {c, P / rho^2, B, 1 / m} per neighbour instead
 // of hyd and dd and computes neither square root nor division per pair.
-__global__ void k_hydro_prep(int n, const double4 *__restrict__ pos, const double4 *__restrict__ vel,
-                             const double4 *__restrict__ hyd, const double4 *__restrict__ dd, double gamma,
-                             double4 *__restrict__ aux) {
+__global__ void k_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
+                             double gamma, double4 *aux) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double range = pos[i].w;
@@ -232,6 +234,7 @@ __device__ __forceinline__ void art_visc_pre(double ids, double drdv, const doub
 // 6, 1.89 ms with them at 4)
 template <int S>
 __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
+  grid_enter();
   const int s = a.leaf0 * kLeaf + (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
   const bool valid = s < min(a.leaf1 * kLeaf, a.n);
   double4 pi = make_double4(0, 0, 0, 0), vi = make_double4(0, 0, 0, 1), hi4 = make_double4(0, 0, 0, 0),
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
   double axi = 0, ayi = 0, azi = 0, udot = 0, vmax = 0;
   // the neighbours' records are gathered one pair ahead of their use and the
   // list entries two ahead (as in the density loop)
-  int jn = sub + S < cnt ? __ldg(lst + sub + S) : 0, jc = sub < cnt ? __ldg(lst + sub) : 0;
+  int jn = sub + S < cnt ? ldg(lst + sub + S) : 0, jc = sub < cnt ? ldg(lst + sub) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn, fn = pn;
   if (sub < cnt) {
     pn = ld4(a.pos + jc);
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
         fn = ld4(a.aux + jn);
-        if (k + 2 * S < cnt) jn = __ldg(lst + k + 2 * S);
+        if (k + 2 * S < cnt) jn = ldg(lst + k + 2 * S);
       }
       const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
       const double dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
@@ -317,18 +320,18 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
 int launch_density(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
   const int n = (a.leaf1 - a.leaf0) * kLeaf;
-  if (n < kSmallSet) k_density<kSubSmall><<<(n * kSubSmall + 127) / 128, 128, 0, st>>>(a);
-  else k_density<kSubDensity><<<(n * kSubDensity + 127) / 128, 128, 0, st>>>(a);
+  if (n < kSmallSet) launch(k_density<kSubSmall>, (n * kSubSmall + 127) / 128, 128, st, a);
+  else launch(k_density<kSubDensity>, (n * kSubDensity + 127) / 128, 128, st, a);
   return 1;
 }
 int launch_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsigned *flags, cudaStream_t st) {
-  k_pressure<<<(n + 255) / 256, 256, 0, st>>>(n, hyd, eos_mode, gamma, flags);
+  launch(k_pressure, (n + 255) / 256, 256, st, n, hyd, eos_mode, gamma, flags);
   return 1;
 }
 int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
                       double gamma, double4 *aux, cudaStream_t st) {
   if (n <= 0) return 0;
-  k_hydro_prep<<<(n + 255) / 256, 256, 0, st>>>(n, pos, vel, hyd, dd, gamma, aux);
+  launch(k_hydro_prep, (n + 255) / 256, 256, st, n, pos, vel, hyd, dd, gamma, aux);
   return 1;
 }
 
@@ -337,8 +340,8 @@ int launch_hydro(const HydroArgs &a, cudaStream_t st) {
   // every particle's factors: a shard's pairs reach outside its own leaves
   int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);
   const int n = (a.leaf1 - a.leaf0) * kLeaf;
-  if (n < kSmallSet) k_hydro<kSubSmall><<<(n * kSubSmall + 127) / 128, 128, 0, st>>>(a);
-  else k_hydro<kSubHydro><<<(n * kSubHydro + 127) / 128, 128, 0, st>>>(a);
+  if (n < kSmallSet) launch(k_hydro<kSubSmall>, (n * kSubSmall + 127) / 128, 128, st, a);
+  else launch(k_hydro<kSubHydro>, (n * kSubHydro + 127) / 128, 128, st, a);
   return launches + 1;
 }
 

@@ -45,6 +45,7 @@ __device__ __forceinline__ void split_ff(double v, float &hi, float &lo) {
 }
 
 __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
+  grid_enter();
   const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (leaf >= a.leaf1) return;
   const int lane = (int)lane_id();
@@ -63,10 +64,10 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
   float iw_hi = 0.f, iw_lo = 0.f;  // 2 / range as a float-float pair
   if (w > 0) split_ff(2.0 / w, iw_hi, iw_lo);
   KSum dens, om, ps, sdig, div, cx, cy, cz;
-  int jn = cnt > 1 ? __ldg(lst + 1) : 0;
+  int jn = cnt > 1 ? ldg(lst + 1) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn;
   if (cnt > 0) {
-    const int j0 = __ldg(lst);
+    const int j0 = ldg(lst);
     pn = ld4(a.pos + j0);
     vn = ld4(a.vel + j0);
   }
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
       if (k + 1 < cnt) {
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
-        if (k + 2 < cnt) jn = __ldg(lst + k + 2);
+        if (k + 2 < cnt) jn = ldg(lst + k + 2);
       }
       const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
       const float u = mul_ff(sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx))), iw_hi, iw_lo);
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
 // r_ij . v_ij in place of r_ij; the pair's force on j, m_i acc_ij (r_i - r_j),
 // is assembled in FP64 from the FP32 pair vectors dw r_ij, Pi dw r_ij, dig r_ij.
 __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
+  grid_enter();
   const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (leaf >= a.leaf1) return;
   const int lane = (int)lane_id();
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
   float vmax = 0.f;
   for (int k = 0; k < kmax; k++) {
     if (k < cnt) {
-      const int j = __ldg(lst + k);
+      const int j = ldg(lst + k);
       const double4 pj = ld4(a.pos + j), vj = ld4(a.vel + j), fj = ld4(a.aux + j);
       const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
       const float dvx = (float)(vi.x - vj.x), dvy = (float)(vi.y - vj.y), dvz = (float)(vi.z - vj.z);
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
 
 int launch_density_mixed(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
-  k_density_mixed<<<((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, 0, st>>>(a);
+  launch(k_density_mixed, ((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, st, a);
   return 1;
 }
 int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
@@ -221,7 +223,7 @@ int launch_hydro_mixed(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
   // every particle's factors {c, P / rho^2, B, 1 / m}: a shard's pairs reach outside its own leaves
   int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);
-  k_hydro_mixed<<<((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, 0, st>>>(a);
+  launch(k_hydro_mixed, ((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, st, a);
   return launches + 1;
 }
 

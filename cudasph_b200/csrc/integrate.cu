@@ -15,9 +15,9 @@ namespace sph {
 // scalars: v[0] = dt of the drift just taken, v[1] = current dt, v[2] = time
 constexpr int kS_DTOLD = 0, kS_DT = 1, kS_TIME = 2, kS_STATS = 4;
 
-__global__ void k_predict(int n, double4 *__restrict__ pos, double4 *__restrict__ vel, double4 *__restrict__ hyd,
-                          const double4 *__restrict__ dots, double4 *__restrict__ old,
-                          const double *__restrict__ sc) {
+__global__ void k_predict(int n, double4 *pos, double4 *vel, double4 *hyd, const double4 *dots, double4 *old,
+                          const double *sc) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double dt = sc[kS_DT], dth = 0.5 * dt;
@@ -46,14 +46,12 @@ enum {
 };
 constexpr int kFinThreads = 256;
 
-__global__ void __launch_bounds__(kFinThreads) k_finish_partial(int n, const double4 *__restrict__ pos,
-                                                                const double4 *__restrict__ vel,
-                                                                const double4 *__restrict__ hyd,
-                                                                double4 *__restrict__ dots,
-                                                                const double4 *__restrict__ grav,
-                                                                const double *__restrict__ vsig,
-                                                                const int *__restrict__ n_ngb, int add_gravity,
-                                                                double cn1, double cn2, double *__restrict__ part) {
+__global__ void __launch_bounds__(kFinThreads) k_finish_partial(int n, const double4 *pos, const double4 *vel,
+                                                                const double4 *hyd, double4 *dots,
+                                                                const double4 *grav, const double *vsig,
+                                                                const int *n_ngb, int add_gravity, double cn1,
+                                                                double cn2, double *part) {
+  grid_enter();
   double q[kQ_N];
 #pragma unroll
   for (int k = 0; k < kQ_NSUM; k++) q[k] = 0;
@@ -131,8 +129,9 @@ __global__ void __launch_bounds__(kFinThreads) k_finish_partial(int n, const dou
 // one warp per quantity: its lanes fold every 32nd partial in block order and
 // meet in a fixed shuffle tree (one thread per quantity walked up to 592
 // partials one after the other before: 220 us, now 6)
-__global__ void __launch_bounds__(kQ_N * 32) k_finish_final(int n, int nb, const double *__restrict__ part,
-                                                            double *__restrict__ sc, unsigned *flags) {
+__global__ void __launch_bounds__(kQ_N * 32) k_finish_final(int n, int nb, const double *part, double *sc,
+                                                            unsigned *flags) {
+  grid_enter();
   __shared__ double q[kQ_N];
   {
     const int k = threadIdx.x >> 5;
@@ -181,8 +180,8 @@ __global__ void __launch_bounds__(kQ_N * 32) k_finish_final(int n, int nb, const
 }
 
 // step.cpp:128-134: v = v_old + a (dt_new/2 + dt_old/2), u likewise
-__global__ void k_kick(int n, double4 *__restrict__ vel, double4 *__restrict__ hyd, const double4 *__restrict__ dots,
-                       const double4 *__restrict__ old, const double *__restrict__ sc) {
+__global__ void k_kick(int n, double4 *vel, double4 *hyd, const double4 *dots, const double4 *old, const double *sc) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double f = 0.5 * sc[kS_DT] + 0.5 * sc[kS_DTOLD];
@@ -196,7 +195,8 @@ __global__ void k_kick(int n, double4 *__restrict__ vel, double4 *__restrict__ h
 }
 
 // apply a permutation: dst[s] = src[order[s]] for every state array
-__global__ void k_permute(int n, const uint32_t *__restrict__ order, Fields src, Fields dst) {
+__global__ void k_permute(int n, const uint32_t *order, Fields src, Fields dst) {
+  grid_enter();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int o = (int)order[s];
@@ -211,14 +211,15 @@ __global__ void k_permute(int n, const uint32_t *__restrict__ order, Fields src,
 }
 
 // slot_of[id[s]] = s
-__global__ void k_invert(int n, const int *__restrict__ id, int *__restrict__ slot_of) {
+__global__ void k_invert(int n, const int *id, int *slot_of) {
+  grid_enter();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) slot_of[id[s]] = s;
 }
 
 int launch_predict(int n, double4 *pos, double4 *vel, double4 *hyd, const double4 *dots, double4 *old,
                    const double *sc, cudaStream_t st) {
-  k_predict<<<(n + 255) / 256, 256, 0, st>>>(n, pos, vel, hyd, dots, old, sc);
+  launch(k_predict, (n + 255) / 256, 256, st, n, pos, vel, hyd, dots, old, sc);
   return 1;
 }
 
@@ -234,14 +235,14 @@ int launch_finish(int n, const double4 *pos, const double4 *vel, const double4 *
                   const double4 *grav, const double *vsig, const int *n_ngb, int add_gravity, double cn1, double cn2,
                   double *part, double *sc, unsigned *flags, cudaStream_t st) {
   const int nb = finish_partial_blocks(n);
-  k_finish_partial<<<nb, kFinThreads, 0, st>>>(n, pos, vel, hyd, dots, grav, vsig, n_ngb, add_gravity, cn1, cn2, part);
-  k_finish_final<<<1, kQ_N * 32, 0, st>>>(n, nb, part, sc, flags);
+  launch(k_finish_partial, nb, kFinThreads, st, n, pos, vel, hyd, dots, grav, vsig, n_ngb, add_gravity, cn1, cn2, part);
+  launch(k_finish_final, 1, kQ_N * 32, st, n, nb, part, sc, flags);
   return 2;
 }
 
 int launch_kick(int n, double4 *vel, double4 *hyd, const double4 *dots, const double4 *old, const double *sc,
                 cudaStream_t st) {
-  k_kick<<<(n + 255) / 256, 256, 0, st>>>(n, vel, hyd, dots, old, sc);
+  launch(k_kick, (n + 255) / 256, 256, st, n, vel, hyd, dots, old, sc);
   return 1;
 }
 
@@ -250,9 +251,9 @@ int launch_kick(int n, double4 *vel, double4 *hyd, const double4 *dots, const do
 // pack: the shard's own slots [s0, s1) are copied in, every other slot is
 // zeroed, so the element-wise sum of the shards' buffers holds every
 // particle's values exactly once; unpack writes the summed buffer back.
-__global__ void k_shard_pack(int n, int s0, int s1, const double4 *__restrict__ pos, const double4 *__restrict__ hyd,
-                             const double4 *__restrict__ dd, const int *__restrict__ n_ngb,
-                             double4 *__restrict__ xbuf) {
+__global__ void k_shard_pack(int n, int s0, int s1, const double4 *pos, const double4 *hyd, const double4 *dd,
+                             const int *n_ngb, double4 *xbuf) {
+  grid_enter();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   double4 a = make_double4(0, 0, 0, 0), b = make_double4(0, 0, 0, 0);
@@ -265,8 +266,8 @@ __global__ void k_shard_pack(int n, int s0, int s1, const double4 *__restrict__ 
   xbuf[2 * s + 1] = b;
 }
 
-__global__ void k_shard_unpack(int n, const double4 *__restrict__ xbuf, double4 *__restrict__ pos,
-                               double4 *__restrict__ hyd, double4 *__restrict__ dd, int *__restrict__ n_ngb) {
+__global__ void k_shard_unpack(int n, const double4 *xbuf, double4 *pos, double4 *hyd, double4 *dd, int *n_ngb) {
+  grid_enter();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const double4 a = xbuf[2 * s], b = xbuf[2 * s + 1];
@@ -278,31 +279,31 @@ __global__ void k_shard_unpack(int n, const double4 *__restrict__ xbuf, double4 
 
 int launch_shard_pack(int n, int s0, int s1, const double4 *pos, const double4 *hyd, const double4 *dd,
                       const int *n_ngb, double4 *xbuf, cudaStream_t st) {
-  k_shard_pack<<<(n + 255) / 256, 256, 0, st>>>(n, s0, s1, pos, hyd, dd, n_ngb, xbuf);
+  launch(k_shard_pack, (n + 255) / 256, 256, st, n, s0, s1, pos, hyd, dd, n_ngb, xbuf);
   return 1;
 }
 
 int launch_shard_unpack(int n, const double4 *xbuf, double4 *pos, double4 *hyd, double4 *dd, int *n_ngb,
                         cudaStream_t st) {
-  k_shard_unpack<<<(n + 255) / 256, 256, 0, st>>>(n, xbuf, pos, hyd, dd, n_ngb);
+  launch(k_shard_unpack, (n + 255) / 256, 256, st, n, xbuf, pos, hyd, dd, n_ngb);
   return 1;
 }
 
 int launch_permute(int n, const uint32_t *order, const Fields &src, const Fields &dst, cudaStream_t st) {
-  k_permute<<<(n + 255) / 256, 256, 0, st>>>(n, order, src, dst);
+  launch(k_permute, (n + 255) / 256, 256, st, n, order, src, dst);
   return 1;
 }
 
 int launch_invert(int n, const int *id, int *slot_of, cudaStream_t st) {
-  k_invert<<<(n + 255) / 256, 256, 0, st>>>(n, id, slot_of);
+  launch(k_invert, (n + 255) / 256, 256, st, n, id, slot_of);
   return 1;
 }
 
 // field exchange between the caller's original order and tree order:
 // to_state: arr[s*stride + comp] = flat[id[s]]; else flat[id[s]] = arr[...].
 // stride < 0 selects an int array copied out as ints.
-__global__ void k_field_io(int n, double *__restrict__ arr, int stride, int comp, const int *__restrict__ id,
-                           double *__restrict__ flat, int to_state) {
+__global__ void k_field_io(int n, double *arr, int stride, int comp, const int *id, double *flat, int to_state) {
+  grid_enter();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int o = id[s];
@@ -314,19 +315,20 @@ __global__ void k_field_io(int n, double *__restrict__ arr, int stride, int comp
   else flat[o] = arr[(size_t)s * stride + comp];
 }
 
-__global__ void k_iota(int n, int *__restrict__ id) {
+__global__ void k_iota(int n, int *id) {
+  grid_enter();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) id[s] = s;
 }
 
 int launch_field_io(int n, double *arr, int stride, int comp, const int *id, double *flat, int to_state,
                     cudaStream_t st) {
-  k_field_io<<<(n + 255) / 256, 256, 0, st>>>(n, arr, stride, comp, id, flat, to_state);
+  launch(k_field_io, (n + 255) / 256, 256, st, n, arr, stride, comp, id, flat, to_state);
   return 1;
 }
 
 int launch_iota(int n, int *id, cudaStream_t st) {
-  k_iota<<<(n + 255) / 256, 256, 0, st>>>(n, id);
+  launch(k_iota, (n + 255) / 256, 256, st, n, id);
   return 1;
 }
 

@@ -138,7 +138,7 @@ struct Walk {
     bool hit = false;
     if (child < t.count[lev - 1]) {
       const long long at = t.base[lev - 1] + child;
-      hit = box_hit(q, __ldg(t.lo + at), __ldg(t.hi + at));
+      hit = box_hit(q, ldg(t.lo + at), ldg(t.hi + at));
     }
     return __ballot_sync(kFull, hit);
   }
@@ -252,7 +252,7 @@ struct Source {
         if (nlist >= 0) {
           bool hit = false;
           id = at + lane < nlist ? sm.list[at + lane] : 0;
-          if (at + lane < nlist) hit = box_hit(q, __ldg(t.lo + id), __ldg(t.hi + id));
+          if (at + lane < nlist) hit = box_hit(q, ldg(t.lo + id), ldg(t.hi + id));
           c = __ballot_sync(kFull, hit);
           at += 32;
           walk.more = at < nlist;
@@ -270,8 +270,8 @@ struct Source {
       if (c0 < take) j0 = sm.own.cell[(head + c0) % kQueue] * kCell + (lane & 7);
       if (c1 < take) j1 = sm.own.cell[(head + c1) % kQueue] * kCell + (lane & 7);
       float4 p0, p1;
-      if (j0 < t.n) p0 = __ldg(t.pf + j0);
-      if (j1 < t.n) p1 = __ldg(t.pf + j1);
+      if (j0 < t.n) p0 = ldg(t.pf + j0);
+      if (j1 < t.n) p1 = ldg(t.pf + j1);
       head += take;
       const bool in0 = j0 < t.n && dist2(p0.x - q.lo[0], p0.y - q.lo[1], p0.z - q.lo[2]) <= q.r2;
       const bool in1 = j1 < t.n && dist2(p1.x - q.lo[0], p1.y - q.lo[1], p1.z - q.lo[2]) <= q.r2;
@@ -533,7 +533,7 @@ __device__ __forceinline__ Rough rough_sums(const SolveArgs &a, Smem &sm, const 
       if (((c >> (4 * g)) & 15u) == 0u) continue;  // four cells: 32 consecutive particles
       const int j = (first + 4 * g) * kCell + lane;
       if (j >= a.t.n) continue;
-      const float4 o = __ldg(a.t.pf + j);
+      const float4 o = ldg(a.t.pf + j);
       const float u = sqrtf(dist2(o.x - q.lo[0], o.y - q.lo[1], o.z - q.lo[2])) * i2w;
       lf += k_ig<float>(u);
       lg -= k_digdh<float>(u);
@@ -692,7 +692,7 @@ struct Group {
       auto candidate = [&](int c) {
         const int k = r * 128 + c * 4 + (lane >> 3);
         const int j = k < nlist ? sm.list[k] * kCell + (lane & 7) : 0x7fffffff;
-        return j < a.t.n ? __ldg(a.t.pf + j) : make_float4(INFINITY, 0.f, 0.f, 0.f);
+        return j < a.t.n ? ldg(a.t.pf + j) : make_float4(INFINITY, 0.f, 0.f, 0.f);
       };
       for (int c = 0; c < chunks; c++) {
         const float4 o = candidate(c);
@@ -748,6 +748,7 @@ struct Group {
 // warps (steady solve of 2,000,003 particles 6.9 ms instead of 6.1).
 template <int G>
 __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(const __grid_constant__ SolveArgs a) {
+  grid_enter();
   __shared__ WarpSmem<G> smem[kNgbWarps];
   WarpSmem<G> &sm = smem[threadIdx.x >> 5];
   Group<G> g;
@@ -770,6 +771,7 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(cons
 // The rounds after it, until every target is done.
 template <int G>
 __global__ void __launch_bounds__(kNgbWarps * 32, kMoreBlocks) k_solve_more(const __grid_constant__ SolveArgs a) {
+  grid_enter();
   __shared__ WarpSmem<G> smem[kNgbWarps];
   WarpSmem<G> &sm = smem[threadIdx.x >> 5];
   const int warps = (int)(gridDim.x * blockDim.x) >> 5;
@@ -798,6 +800,7 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kMoreBlocks) k_solve_more(cons
 // ascending slot order, at ranges set from outside.
 template <int G>
 __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_find_ngb(const __grid_constant__ SolveArgs a) {
+  grid_enter();
   __shared__ WarpSmem<G> smem[kNgbWarps];
   WarpSmem<G> &sm = smem[threadIdx.x >> 5];
   Group<G> g;
@@ -822,12 +825,12 @@ template <int G>
 static void launch_group(const SolveArgs &a, bool solve, cudaStream_t st) {
   const int warps = (a.s1 - a.s0 + G - 1) / G, blocks = (warps + kNgbWarps - 1) / kNgbWarps;
   if (!solve) {
-    k_find_ngb<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
+    launch(k_find_ngb<G>, blocks, kNgbWarps * 32, st, a);
     return;
   }
   cudaMemsetAsync(a.queued, 0, sizeof(int), st);
-  k_solve_range<G><<<blocks, kNgbWarps * 32, 0, st>>>(a);
-  k_solve_more<G><<<blocks < 148 * kMoreBlocks ? blocks : 148 * kMoreBlocks, kNgbWarps * 32, 0, st>>>(a);
+  launch(k_solve_range<G>, blocks, kNgbWarps * 32, st, a);
+  launch(k_solve_more<G>, blocks < 148 * kMoreBlocks ? blocks : 148 * kMoreBlocks, kNgbWarps * 32, st, a);
 }
 
 // Four targets to a warp share the walk once that leaves enough warps: the

@@ -14,8 +14,9 @@
 
 namespace sph {
 
-__global__ void k_bbox_partial(int n, const double4 *__restrict__ pos, const double *__restrict__ x,
-                               const double *__restrict__ y, const double *__restrict__ z, double *__restrict__ part) {
+__global__ void k_bbox_partial(int n, const double4 *pos, const double *x, const double *y, const double *z,
+                               double *part) {
+  grid_enter();
   double lo[3] = {1e308, 1e308, 1e308}, hi[3] = {-1e308, -1e308, -1e308};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double c[3];
@@ -73,8 +74,8 @@ __device__ __forceinline__ void fold_box(int nb, const double *__restrict__ part
 }
 
 // box4 = {lo.x, lo.y, lo.z, scale}; scale = 2^21 / max extent (0 if degenerate)
-__global__ void __launch_bounds__(kBoxThreads) k_bbox_final(int nb, const double *__restrict__ part,
-                                                            double *__restrict__ box4) {
+__global__ void __launch_bounds__(kBoxThreads) k_bbox_final(int nb, const double *part, double *box4) {
+  grid_enter();
   double lo[3], hi[3];
   fold_box(nb, part, lo, hi);
   if (threadIdx.x != 0) return;
@@ -100,9 +101,9 @@ __device__ __forceinline__ uint32_t quant21(double c, double lo, double scale) {
   return v >= 2097151.0 ? 2097151u : (uint32_t)v;
 }
 
-__global__ void k_morton(int n, const double4 *__restrict__ pos, const double *__restrict__ x,
-                         const double *__restrict__ y, const double *__restrict__ z, const double *__restrict__ box4,
-                         uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+__global__ void k_morton(int n, const double4 *pos, const double *x, const double *y, const double *z,
+                         const double *box4, uint64_t *keys, uint32_t *vals) {
+  grid_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double c0, c1, c2;
@@ -221,9 +222,8 @@ __device__ __forceinline__ void rank_tile(RadixSmem<T> &sm, const uint64_t (&k)[
 
 // counts of the first digit, and the second table cleared
 template <int T>
-__global__ void __launch_bounds__(T) k_radix_count(int n, const uint64_t *__restrict__ keys,
-                                                               unsigned *__restrict__ table,
-                                                               unsigned *__restrict__ next) {
+__global__ void __launch_bounds__(T) k_radix_count(int n, const uint64_t *keys, unsigned *table, unsigned *next) {
+  grid_enter();
   __shared__ unsigned h[256];
   const int t = threadIdx.x;
   if (t < 256) h[t] = 0;
@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(T) k_radix_count(int n, const uint64_t *__rest
 
 // many tiles: each tile's counts replaced by those of the tiles before it,
 // and the digits' totals; 32 digits per block, 32 runs of tiles per digit
-__global__ void __launch_bounds__(1024) k_radix_prefix(int tiles, unsigned *__restrict__ table,
-                                                       unsigned *__restrict__ total) {
+__global__ void __launch_bounds__(1024) k_radix_prefix(int tiles, unsigned *table, unsigned *total) {
+  grid_enter();
   __shared__ unsigned run[32][33];
   const int d = threadIdx.x & 31, r = threadIdx.x >> 5, digit = blockIdx.x * 32 + d;
   const int b = (int)((long long)tiles * r / 32), e = (int)((long long)tiles * (r + 1) / 32);
@@ -264,14 +264,12 @@ __global__ void __launch_bounds__(1024) k_radix_prefix(int tiles, unsigned *__re
 // One pass.  total: null when the block adds the counts up itself.  next,
 // clear: null in the last pass.
 template <int T>
-__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_radix_pass(int n, int tiles, const uint64_t *__restrict__ kin,
-                                                              const uint32_t *__restrict__ vin,
-                                                              uint64_t *__restrict__ kout,
-                                                              uint32_t *__restrict__ vout, int shift,
-                                                              const unsigned *__restrict__ table,
-                                                              const unsigned *__restrict__ total,
-                                                              unsigned *__restrict__ next,
-                                                              unsigned *__restrict__ clear) {
+__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_radix_pass(int n, int tiles, const uint64_t *kin,
+                                                                    const uint32_t *vin, uint64_t *kout,
+                                                                    uint32_t *vout, int shift, const unsigned *table,
+                                                                    const unsigned *total, unsigned *next,
+                                                                    unsigned *clear) {
+  grid_enter();
   constexpr int kTile = T * kRadixItems;
   __shared__ RadixSmem<T> sm;
   const int t = threadIdx.x, w = t >> 5, l = t & 31, tile = blockIdx.x;
@@ -343,7 +341,8 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_radix_pass(int n, int t
 }
 
 // a single tile: all passes in one launch, in place
-__global__ void __launch_bounds__(512) k_radix_tile(int n, uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+__global__ void __launch_bounds__(512) k_radix_tile(int n, uint64_t *keys, uint32_t *vals) {
+  grid_enter();
   __shared__ RadixSmem<512> sm;
   const int t = threadIdx.x, w = t >> 5, l = t & 31;
   uint64_t k[kRadixItems];
@@ -404,18 +403,17 @@ static int radix_passes(int n, uint64_t *keys, uint32_t *vals, char *p, cudaStre
   unsigned *total = tiles > kDirectTiles ? (unsigned *)p : nullptr;
   uint64_t *ka = keys, *kb = k2;
   uint32_t *va = vals, *vb = v2;
-  k_radix_count<T><<<tiles, T, 0, st>>>(n, ka, table[0], table[1]);
+  launch(k_radix_count<T>, tiles, T, st, n, ka, table[0], table[1]);
   int launches = 1;
   for (int pass = 0; pass < 8; pass++) {
     unsigned *now = table[pass % 3];
     const bool last = pass == 7;
     if (total) {
-      k_radix_prefix<<<8, 1024, 0, st>>>(tiles, now, total);
+      launch(k_radix_prefix, 8, 1024, st, tiles, now, total);
       launches++;
     }
-    k_radix_pass<T><<<tiles, T, 0, st>>>(n, tiles, ka, va, kb, vb, pass * 8, now, total,
-                                         last ? nullptr : table[(pass + 1) % 3],
-                                         last ? nullptr : table[(pass + 2) % 3]);
+    launch(k_radix_pass<T>, tiles, T, st, n, tiles, ka, va, kb, vb, pass * 8, now, total,
+           last ? nullptr : table[(pass + 1) % 3], last ? nullptr : table[(pass + 2) % 3]);
     launches++;
     uint64_t *tk = ka; ka = kb; kb = tk;
     uint32_t *tv = va; va = vb; vb = tv;
@@ -432,7 +430,7 @@ static int radix_passes(int n, uint64_t *keys, uint32_t *vals, char *p, cudaStre
 int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStream_t st) {
   if (n <= 1) return 0;
   if (n <= kTileLarge) {
-    k_radix_tile<<<1, 512, 0, st>>>(n, keys, vals);
+    launch(k_radix_tile, 1, 512, st, n, keys, vals);
     return 1;
   }
   char *p = (char *)(((uintptr_t)scratch + 15) / 16 * 16);  // the tables are read 16 bytes at a time
@@ -446,9 +444,9 @@ int morton_keys(int n, const double4 *pos, const double *x, const double *y, con
   int nb = kBoxBlocks;
   if (nb * 256 > n) nb = (n + 255) / 256;
   if (nb < 1) nb = 1;
-  k_bbox_partial<<<nb, 256, 0, st>>>(n, pos, x, y, z, part);
-  k_bbox_final<<<1, kBoxThreads, 0, st>>>(nb, part, box4);
-  k_morton<<<(n + 255) / 256, 256, 0, st>>>(n, pos, x, y, z, box4, keys, vals);
+  launch(k_bbox_partial, nb, 256, st, n, pos, x, y, z, part);
+  launch(k_bbox_final, 1, kBoxThreads, st, nb, part, box4);
+  launch(k_morton, (n + 255) / 256, 256, st, n, pos, x, y, z, box4, keys, vals);
   return 3;
 }
 
@@ -571,8 +569,8 @@ __device__ __forceinline__ uint64_t ph_key(const uint16_t *tab, uint32_t x, uint
   return key;
 }
 
-__global__ void k_peano_int(int n, const int *__restrict__ x, const int *__restrict__ y, const int *__restrict__ z,
-                            int bits, uint64_t *__restrict__ keys) {
+__global__ void k_peano_int(int n, const int *x, const int *y, const int *z, int bits, uint64_t *keys) {
+  grid_enter();
   __shared__ uint16_t tab[kPhStates * 8];
   ph_load_table(tab);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -586,8 +584,8 @@ constexpr int kPhBits = 18;  // BITS_PER_DIMENSION, sort_bodies.cpp:3
 // float-rounded positions is the rounded double box): box4 = {lo.x, lo.y,
 // lo.z, domain_fac}, domain_fac = float(1.0 / size * 2^18) with size the
 // largest float extent; 0 for a degenerate box (all keys 0)
-__global__ void __launch_bounds__(kBoxThreads) k_peano_box_final(int nb, const double *__restrict__ part,
-                                                                 double *__restrict__ box4) {
+__global__ void __launch_bounds__(kBoxThreads) k_peano_box_final(int nb, const double *part, double *box4) {
+  grid_enter();
   double lo[3], hi[3];
   fold_box(nb, part, lo, hi);
   if (threadIdx.x != 0) return;
@@ -604,9 +602,9 @@ __global__ void __launch_bounds__(kBoxThreads) k_peano_box_final(int nb, const d
 
 // positions rounded to float (the reference's float4 state), offset and
 // scaled in float and truncated (sort_bodies.cpp:155-159), then keyed
-__global__ void k_peano_pos(int n, const double4 *__restrict__ pos, const double *__restrict__ x,
-                            const double *__restrict__ y, const double *__restrict__ z,
-                            const double *__restrict__ box4, uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+__global__ void k_peano_pos(int n, const double4 *pos, const double *x, const double *y, const double *z,
+                            const double *box4, uint64_t *keys, uint32_t *vals) {
+  grid_enter();
   __shared__ uint16_t tab[kPhStates * 8];
   ph_load_table(tab);
   const float lx = (float)box4[0], ly = (float)box4[1], lz = (float)box4[2], fac = (float)box4[3];
@@ -632,9 +630,9 @@ int peano_keys(int n, const double4 *pos, const double *x, const double *y, cons
   int nb = kBoxBlocks;
   if (nb * 256 > n) nb = (n + 255) / 256;
   if (nb < 1) nb = 1;
-  k_bbox_partial<<<nb, 256, 0, st>>>(n, pos, x, y, z, part);
-  k_peano_box_final<<<1, kBoxThreads, 0, st>>>(nb, part, box4);
-  k_peano_pos<<<(n + 255) / 256, 256, 0, st>>>(n, pos, x, y, z, box4, keys, vals);
+  launch(k_bbox_partial, nb, 256, st, n, pos, x, y, z, part);
+  launch(k_peano_box_final, 1, kBoxThreads, st, nb, part, box4);
+  launch(k_peano_pos, (n + 255) / 256, 256, st, n, pos, x, y, z, box4, keys, vals);
   return 3;
 }
 
@@ -778,7 +776,7 @@ extern "C" int cudasph_peano_hilbert_keys(int n, const int *x, const int *y, con
   if (!x || !y || !z || !keys) return SPH_ERR_ARG;
   int nb = (n + 255) / 256;
   if (nb > 148 * 8) nb = 148 * 8;
-  sph::k_peano_int<<<nb, 256, 0, (cudaStream_t)stream>>>(n, x, y, z, bits, keys);
+  sph::launch(sph::k_peano_int, nb, 256, (cudaStream_t)stream, n, x, y, z, bits, keys);
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
 }

@@ -17,10 +17,9 @@ namespace sph {
 // Boxes of the cells and of the level above them -- a block's 256 particles
 // are one node of level 1 -- and the positions rounded to float, for the
 // neighbour walk's first test.
-__global__ void __launch_bounds__(kCell * kFan) k_cell_boxes(int n, const double4 *__restrict__ pos,
-                                                             float4 *__restrict__ lo, float4 *__restrict__ hi,
-                                                             float4 *__restrict__ lo1, float4 *__restrict__ hi1,
-                                                             float4 *__restrict__ pf) {
+__global__ void __launch_bounds__(kCell * kFan) k_cell_boxes(int n, const double4 *pos, float4 *lo, float4 *hi,
+                                                             float4 *lo1, float4 *hi1, float4 *pf) {
+  grid_enter();
   __shared__ float4 slo[kFan], shi[kFan];
   const int s = blockIdx.x * (kCell * kFan) + threadIdx.x;
   double l0 = 1e308, l1 = 1e308, l2 = 1e308, h0 = -1e308, h1 = -1e308, h2 = -1e308;
@@ -64,8 +63,9 @@ __global__ void __launch_bounds__(kCell * kFan) k_cell_boxes(int n, const double
   }
 }
 
-__global__ void k_parent_boxes(int nchild, const float4 *__restrict__ clo, const float4 *__restrict__ chi,
-                               int nparent, float4 *__restrict__ plo, float4 *__restrict__ phi) {
+__global__ void k_parent_boxes(int nchild, const float4 *clo, const float4 *chi, int nparent, float4 *plo,
+                               float4 *phi) {
+  grid_enter();
   int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (node >= nparent) return;
   int c = node * kFan + (int)lane_id();
@@ -107,12 +107,12 @@ int build_tree(const TreeView &t, const double4 *pos, float4 *lo, float4 *hi, fl
                cudaStream_t st) {
   int launches = 1;
   const bool up = t.levels > 1;
-  k_cell_boxes<<<(t.n + kCell * kFan - 1) / (kCell * kFan), kCell * kFan, 0, st>>>(
-      t.n, pos, lo, hi, up ? lo + t.base[1] : nullptr, up ? hi + t.base[1] : nullptr, pf);
+  launch(k_cell_boxes, (t.n + kCell * kFan - 1) / (kCell * kFan), kCell * kFan, st, t.n, pos, lo, hi,
+         up ? lo + t.base[1] : nullptr, up ? hi + t.base[1] : nullptr, pf);
   for (int l = 2; l < t.levels; l++) {
     int np = t.count[l];
-    k_parent_boxes<<<(np * 32 + 255) / 256, 256, 0, st>>>(t.count[l - 1], lo + t.base[l - 1], hi + t.base[l - 1], np,
-                                                          lo + t.base[l], hi + t.base[l]);
+    launch(k_parent_boxes, (np * 32 + 255) / 256, 256, st, t.count[l - 1], lo + t.base[l - 1], hi + t.base[l - 1],
+           np, lo + t.base[l], hi + t.base[l]);
     launches++;
   }
   return launches;

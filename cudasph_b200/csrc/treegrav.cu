@@ -111,7 +111,8 @@ __device__ __forceinline__ int prefix(const uint64_t *__restrict__ k, int n, int
   return __clzll((long long)(a ^ b));
 }
 
-__global__ void k_radix_tree(int n, const uint64_t *__restrict__ keys, TgWork w) {
+__global__ void k_radix_tree(int n, const uint64_t *keys, TgWork w) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
   // direction of the node's range and its length by exponential + binary search
@@ -179,7 +180,8 @@ __device__ __forceinline__ void child_moments(int ref, const double4 *__restrict
   qb = make_double4(b0.x, b0.y, b1.x, b1.y);
 }
 
-__global__ void k_tree_moments(int n, const double4 *__restrict__ src, TgWork w) {
+__global__ void k_tree_moments(int n, const double4 *src, TgWork w) {
+  grid_enter();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   int node = w.lparent[p];
@@ -496,8 +498,8 @@ __device__ __forceinline__ void tree_group(const TreeGravArgs &a, TgSmem &sm, in
       float4 r0 = make_float4(0.f, 0.f, 0.f, -1.f), r1 = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live) {  // the child's record {cx, cy, cz, b}, {ref, first, count, -}
         const float4 *rp = reinterpret_cast<const float4 *>(a.w.rec + 2 * node + (int)(lane & 1u));
-        r0 = __ldg(rp);
-        r1 = __ldg(rp + 1);
+        r0 = ldg(rp);
+        r1 = ldg(rp + 1);
       }
       const int ref = __float_as_int(r1.x);
       bool accept = false, open = false;
@@ -578,6 +580,7 @@ __device__ __forceinline__ void tree_group(const TreeGravArgs &a, TgSmem &sm, in
 // one at a time lets a long group overlap the rest instead of ending the
 // launch alone on its SM.
 __global__ void __launch_bounds__(kTgWarps * 32, 5) k_tree_gravity(TreeGravArgs a) {
+  grid_enter();
   __shared__ TgSmem smem[kTgWarps];
   TgSmem &sm = smem[threadIdx.x >> 5];
   const unsigned groups = (unsigned)(a.leaf1 - a.leaf0);
@@ -601,8 +604,8 @@ int launch_tree_gravity(const TreeView &t, const uint64_t *keys, const double4 *
   const TgWork w = carve(ws, n);
   int launches = 0;
   if (n > 1) {
-    k_radix_tree<<<(n - 1 + 255) / 256, 256, 0, st>>>(n, keys, w);
-    k_tree_moments<<<(n + 255) / 256, 256, 0, st>>>(n, src, w);
+    launch(k_radix_tree, (n - 1 + 255) / 256, 256, st, n, keys, w);
+    launch(k_tree_moments, (n + 255) / 256, 256, st, n, src, w);
     launches += 2;
   }
   if (world > 1) cudaMemsetAsync(out, 0, sizeof(double4) * n, st);
@@ -637,7 +640,7 @@ int launch_tree_gravity(const TreeView &t, const uint64_t *keys, const double4 *
   }
   const int blocks = min((warps + kTgWarps - 1) / kTgWarps, sms * max(per_sm, 1));
   cudaMemsetAsync(w.next_group, 0, sizeof(unsigned), st);
-  k_tree_gravity<<<blocks, kTgWarps * 32, 0, st>>>(a);
+  launch(k_tree_gravity, blocks, kTgWarps * 32, st, a);
   return launches + 1;
 }
 
