@@ -43,8 +43,8 @@ int launch_shard_pack(int n, int s0, int s1, const double4 *pos, const double4 *
                       const int *n_ngb, double4 *xbuf, cudaStream_t st);
 int launch_shard_unpack(int n, const double4 *xbuf, double4 *pos, double4 *hyd, double4 *dd, int *n_ngb,
                         cudaStream_t st);
-int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, int *mass_mixed,
-                        cudaStream_t st);
+int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, cudaStream_t st);
+int launch_check_masses(int n, const double4 *vel, int *mass_mixed, cudaStream_t st);
 int launch_predict(int n, double4 *pos, double4 *vel, double4 *hyd, const double4 *dots, double4 *old,
                    const double *sc, cudaStream_t st);
 int finish_partial_doubles(int n);
@@ -100,7 +100,7 @@ struct sph_ctx {
   double4 *aux = nullptr;  // per-particle factors of the hydro pair loop (scratch)
   double4 *gsrc = nullptr;
   double *gh2 = nullptr;
-  int *mass_mixed = nullptr;  // 0 when all masses are equal (set with the gravity sources)
+  int *mass_mixed = nullptr;  // 0 when all masses are equal (kept up to date where masses are set)
   unsigned *flags = nullptr;
   double *sc = nullptr;  // StepScalars
   double *fin_part = nullptr;
@@ -384,6 +384,8 @@ extern "C" int cudasph_create(const sph_params *params, int n, int device, sph_c
   cudaMemsetAsync(c->nevals, 0, sizeof(int) * n, c->st);
   cudaMemsetAsync(c->old, 0, sizeof(double4) * n, c->st);
   cudaMemsetAsync(c->flags, 0, sizeof(unsigned), c->st);
+  cudaMemsetAsync(c->mass_mixed, 0, sizeof(int), c->st);  // all masses are zero
+  cudaMemsetAsync(c->solve_work, 0, 2 * sizeof(int), c->st);  // the solve's queue starts empty
   cudaMemsetAsync(c->sc, 0, sizeof(double) * (4 + SPH_NSTATS), c->st);
   launch_iota(n, c->f[0].id, c->st);
   e = cudaStreamSynchronize(c->st);
@@ -415,6 +417,8 @@ extern "C" int cudasph_get_params(const sph_ctx *c, sph_params *out) {
 
 extern "C" int cudasph_num_particles(const sph_ctx *c) { return c ? c->n : 0; }
 
+#define LAUNCHED(expr) (c->launches += (expr))
+
 // ------------------------------ state exchange ------------------------------
 static int copy_in(sph_ctx *c, const void *src, size_t bytes, int on_device, void *dst) {
   SPH_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->st));
@@ -442,6 +446,7 @@ static int put_field(sph_ctx *c, int field, const double *src, int on_device) {
   FieldRef r = field_ref(c, field);
   launch_field_io(c->n, r.base, r.stride, r.comp, c->f[c->cur].id, c->flat, 1, c->st);
   c->launches++;
+  if (field == SPH_M) LAUNCHED(launch_check_masses(c->n, c->f[c->cur].vel, c->mass_mixed, c->st));
   mark_changed(c, field);
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
@@ -573,7 +578,6 @@ extern "C" int cudasph_get_neighbours(sph_ctx *c, int *counts, int64_t *offsets,
 }
 
 // ------------------------------- the phases --------------------------------
-#define LAUNCHED(expr) (c->launches += (expr))
 
 extern "C" int cudasph_sort(sph_ctx *c) {
   if (!c) return SPH_ERR_ARG;
@@ -692,7 +696,6 @@ extern "C" int cudasph_hydro(sph_ctx *c) {
   SPH_CUDA_TRY(cudaSetDevice(c->device));
   PhaseScope ps(c, SPH_PH_HYDRO);
   Fields &F = c->f[c->cur];
-  SPH_CUDA_TRY(cudaMemsetAsync(F.dots, 0, sizeof(double4) * c->n, c->st));
   // a shard writes the signal speeds of its own particles only; zeros elsewhere make the sum over shards exact
   if (c->world > 1) SPH_CUDA_TRY(cudaMemsetAsync(F.vsig, 0, sizeof(double) * c->n, c->st));
   HydroArgs a = hydro_args(c);
@@ -723,14 +726,14 @@ extern "C" int cudasph_gravity(sph_ctx *c) {
   PhaseScope ps(c, SPH_PH_GRAVITY);
   Fields &F = c->f[c->cur];
   if (c->p.grav_mode == SPH_GRAV_TREE) {
-    LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, c->mass_mixed, c->st));
+    LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, c->st));
     // the radix tree is built from the sort's keys, which match the current order
     LAUNCHED(launch_tree_gravity(c->tree, c->keys, c->gsrc, c->tgws, F.grav, c->flags, c->p.eps, c->p.theta, c->p.G,
                                  c->rank, c->world, c->st));
     SPH_CUDA_TRY(cudaGetLastError());
     return SPH_OK;
   }
-  LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, c->mass_mixed, c->st));
+  LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, c->st));
   LAUNCHED(launch_gravity(c->n, c->gsrc, c->gh2, F.grav, c->p.soft_mode, c->p.eps, c->p.G, c->p.precision,
                           c->mass_mixed, c->rank, c->world, c->st));
   SPH_CUDA_TRY(cudaGetLastError());

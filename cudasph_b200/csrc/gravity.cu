@@ -909,28 +909,33 @@ int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out,
 }
 
 // pack the gravity sources {x, y, z, m} and range^2 from the state
-// Also raises *mass_mixed (cleared before the launch) when some mass differs
-// from the first particle's: the symmetric kernels take their equal-mass form
-// when it stays 0.
-__global__ void k_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2,
-                               int *mass_mixed) {
+__global__ void k_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2) {
   grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool differs = false;
-  if (i < n) {
-    const double4 p = pos[i];
-    const double m = vel[i].w;
-    src[i] = make_double4(p.x, p.y, p.z, m);
-    h2[i] = p.w * p.w;
-    differs = m != ldg(&vel[0].w);
-  }
+  if (i >= n) return;
+  const double4 p = pos[i];
+  src[i] = make_double4(p.x, p.y, p.z, vel[i].w);
+  h2[i] = p.w * p.w;
+}
+
+int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, cudaStream_t st) {
+  launch(k_pack_sources, (n + 255) / 256, 256, st, n, pos, vel, src, h2);
+  return 1;
+}
+
+// *mass_mixed = whether some mass differs from the first particle's: the
+// symmetric kernels take their equal-mass form when it stays 0.  Masses
+// change only when a caller sets them, so this runs then and not in the step.
+__global__ void k_check_masses(int n, const double4 *vel, int *mass_mixed) {
+  grid_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool differs = i < n && vel[i].w != vel[0].w;
   if (__syncthreads_or(differs) && threadIdx.x == 0) atomicOr(mass_mixed, 1);
 }
 
-int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, int *mass_mixed,
-                        cudaStream_t st) {
+int launch_check_masses(int n, const double4 *vel, int *mass_mixed, cudaStream_t st) {
   cudaMemsetAsync(mass_mixed, 0, sizeof(int), st);
-  launch(k_pack_sources, (n + 255) / 256, 256, st, n, pos, vel, src, h2, mass_mixed);
+  launch(k_check_masses, (n + 255) / 256, 256, st, n, vel, mass_mixed);
   return 1;
 }
 

@@ -199,8 +199,9 @@ __global__ void k_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsi
 // the same operations the pair formula applies to them, and 1 / m, so the
 // pair loop gathers one record {c, P / rho^2, B, 1 / m} per neighbour instead
 // of hyd and dd and computes neither square root nor division per pair.
+// dots (null: none): cleared for the loop's sums.
 __global__ void k_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
-                             double gamma, double4 *aux) {
+                             double gamma, double4 *aux, double4 *dots) {
   grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -209,6 +210,7 @@ __global__ void k_hydro_prep(int n, const double4 *pos, const double4 *vel, cons
   const double c = sqrt(gamma * h.y / h.x);
   const double b = fabs(d.x) / (fabs(d.x) + d.y + 0.0001 * c / (0.5 * range));
   aux[i] = make_double4(c, h.y / (h.x * h.x), b, 1.0 / vel[i].w);
+  if (dots) dots[i] = make_double4(0, 0, 0, 0);
 }
 
 // dev_art_visc.cu:8-32 on the per-particle factors of k_hydro_prep
@@ -228,7 +230,7 @@ __device__ __forceinline__ void art_visc_pre(double ids, double drdv, const doub
 }
 
 // hydro_dots (dev_hydro_dots.cu:25-113) plus the j-side of every pair.
-// dots must be zero on entry (xyz accumulate); dots.w (du/dt) is stored.
+// dots.xyz accumulate (cleared by k_hydro_prep); dots.w (du/dt) is stored.
 // 4 blocks per SM: the one-pair-ahead gathers need the registers (N = 1M:
 // 2.40 ms without them at 6 blocks per SM, 2.99 ms with them and spills at
 // 6, 1.89 ms with them at 4)
@@ -329,16 +331,16 @@ int launch_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsigned *f
   return 1;
 }
 int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
-                      double gamma, double4 *aux, cudaStream_t st) {
+                      double gamma, double4 *aux, double4 *dots, cudaStream_t st) {
   if (n <= 0) return 0;
-  launch(k_hydro_prep, (n + 255) / 256, 256, st, n, pos, vel, hyd, dd, gamma, aux);
+  launch(k_hydro_prep, (n + 255) / 256, 256, st, n, pos, vel, hyd, dd, gamma, aux, dots);
   return 1;
 }
 
 int launch_hydro(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
   // every particle's factors: a shard's pairs reach outside its own leaves
-  int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);
+  int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, a.dots, st);
   const int n = (a.leaf1 - a.leaf0) * kLeaf;
   if (n < kSmallSet) launch(k_hydro<kSubSmall>, (n * kSubSmall + 127) / 128, 128, st, a);
   else launch(k_hydro<kSubHydro>, (n * kSubHydro + 127) / 128, 128, st, a);

@@ -217,12 +217,12 @@ int launch_density_mixed(const HydroArgs &a, cudaStream_t st) {
   return 1;
 }
 int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
-                      double gamma, double4 *aux, cudaStream_t st);
+                      double gamma, double4 *aux, double4 *dots, cudaStream_t st);
 
 int launch_hydro_mixed(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
   // every particle's factors {c, P / rho^2, B, 1 / m}: a shard's pairs reach outside its own leaves
-  int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, st);
+  int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, a.dots, st);
   launch(k_hydro_mixed, ((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, st, a);
   return launches + 1;
 }

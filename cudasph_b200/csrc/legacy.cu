@@ -291,7 +291,6 @@ float host_sph_accelerations(int n_bodies, int ngb_tot, float av_alpha, float av
   }
   check_rc(cudasph_density(c), "dev_density_loop");
   check_rc(cudasph_pressure(c), "dev_compute_pressure");
-  check(cudaMemsetAsync(F.dots, 0, sizeof(double4) * n, st), "cudaMemset(bodies_dots)");
   HydroArgs a = ctx_hydro_args(c);
   a.ngb_acc = g_acc;
   a.jside = 0;  // the driver scatters the j-side itself (sph_accelerations.cpp:106-114)

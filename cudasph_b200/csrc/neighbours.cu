@@ -308,7 +308,8 @@ struct SolveArgs {
   int cap, stride;
   int s0, s1;   // slots processed by this launch
   // groups with targets left after the first round: {first slot, mask of the
-  // targets}, their number, and the targets' states by slot
+  // targets}, their number (queued[0]; zero between solves), and the targets'
+  // states by slot
   int2 *queue;
   int *queued;
   RangeIter *save;
@@ -775,7 +776,16 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kMoreBlocks) k_solve_more(cons
   __shared__ WarpSmem<G> smem[kNgbWarps];
   WarpSmem<G> &sm = smem[threadIdx.x >> 5];
   const int warps = (int)(gridDim.x * blockDim.x) >> 5;
-  const int queued = *a.queued;
+  // the queue's length; the last block to have read it empties the queue for
+  // the next solve
+  __shared__ int length;
+  if (threadIdx.x == 0) {
+    length = a.queued[0];
+    __threadfence();
+    if (atomicAdd(a.queued + 1, 1) == (int)gridDim.x - 1) a.queued[0] = a.queued[1] = 0;
+  }
+  __syncthreads();
+  const int queued = length;
   for (int q = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < queued; q += warps) {
     const int2 entry = a.queue[q];
     Group<G> g;
@@ -828,7 +838,6 @@ static void launch_group(const SolveArgs &a, bool solve, cudaStream_t st) {
     launch(k_find_ngb<G>, blocks, kNgbWarps * 32, st, a);
     return;
   }
-  cudaMemsetAsync(a.queued, 0, sizeof(int), st);
   launch(k_solve_range<G>, blocks, kNgbWarps * 32, st, a);
   launch(k_solve_more<G>, blocks < 148 * kMoreBlocks ? blocks : 148 * kMoreBlocks, kNgbWarps * 32, st, a);
 }
