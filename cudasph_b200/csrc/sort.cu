@@ -340,44 +340,72 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_radix_pass(int n, int t
   }
 }
 
-// a single tile: all passes in one launch, in place
-__global__ void __launch_bounds__(512) k_radix_tile(int n, uint64_t *keys, uint32_t *vals) {
+// Small sets: a key's place is the number of keys before it in the stable
+// order, counted directly.  n^2 comparisons are nothing to the whole GPU while
+// eight dependent passes cost some 30 us in one block and 75 in launches
+// (2,049 keys 34 -> 22 us, 6,007 75 -> 46; at 16,384 counting takes 83 us, the
+// passes 75: the comparisons run on the half-rate integer pipe).  Eight
+// lanes share R keys, each counting every eighth key of the tile in shared
+// memory.
+constexpr int kCountTile = 2048, kCountThreads = 256, kCountLanes = 8;
+template <int R>
+__global__ void __launch_bounds__(kCountThreads) k_count_sort(int n, const uint64_t *keys, const uint32_t *vals,
+                                                              uint64_t *kout, uint32_t *vout) {
   grid_enter();
-  __shared__ RadixSmem<512> sm;
-  const int t = threadIdx.x, w = t >> 5, l = t & 31;
-  uint64_t k[kRadixItems];
-  uint32_t v[kRadixItems];
+  __shared__ uint64_t tile[kCountTile];
+  const int t = threadIdx.x, q = t % kCountLanes;
+  const int first = blockIdx.x * (kCountThreads / kCountLanes * R), mine = first + t / kCountLanes * R;
+  uint64_t k[R];
+  unsigned before[R];
 #pragma unroll
-  for (int i = 0; i < kRadixItems; i++) {
-    const int at = w * (32 * kRadixItems) + i * 32 + l;
-    k[i] = at < n ? keys[at] : ~0ull;  // stable: these stay last among equals
-    v[i] = at < n ? vals[at] : 0u;
+  for (int r = 0; r < R; r++) {
+    k[r] = mine + r < n ? keys[mine + r] : 0ull;
+    before[r] = 0u;
   }
-#pragma unroll 1
-  for (int shift = 0; shift < 64; shift += 8) {
-    unsigned place[kRadixItems];
-    rank_tile(sm, k, shift, place);
+  for (int lo = 0; lo < n; lo += kCountTile) {
+    const int m = min(n - lo, kCountTile);
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kRadixItems; i++) sm.key[place[i]] = k[i];
+    for (int i = t; i < m; i += kCountThreads) tile[i] = keys[lo + i];
     __syncthreads();
+    if (lo + m <= first) {  // every key of the tile precedes the block's: equal ones count
+#pragma unroll 4
+      for (int i = q; i < m; i += kCountLanes) {
+        const uint64_t o = tile[i];
 #pragma unroll
-    for (int i = 0; i < kRadixItems; i++) k[i] = sm.key[w * (32 * kRadixItems) + i * 32 + l];
-    __syncthreads();
+        for (int r = 0; r < R; r++) before[r] += o <= k[r];
+      }
+    } else if (lo >= first + kCountThreads / kCountLanes * R) {
+#pragma unroll 4
+      for (int i = q; i < m; i += kCountLanes) {
+        const uint64_t o = tile[i];
 #pragma unroll
-    for (int i = 0; i < kRadixItems; i++) sm.val[place[i]] = v[i];
-    __syncthreads();
+        for (int r = 0; r < R; r++) before[r] += o < k[r];
+      }
+    } else {
+      for (int i = q; i < m; i += kCountLanes) {
+        const uint64_t o = tile[i];
 #pragma unroll
-    for (int i = 0; i < kRadixItems; i++) v[i] = sm.val[w * (32 * kRadixItems) + i * 32 + l];
-  }
-#pragma unroll
-  for (int i = 0; i < kRadixItems; i++) {
-    const int at = w * (32 * kRadixItems) + i * 32 + l;
-    if (at < n) {
-      keys[at] = k[i];
-      vals[at] = v[i];
+        for (int r = 0; r < R; r++) before[r] += o < k[r] || (o == k[r] && lo + i < mine + r);
+      }
     }
   }
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+#pragma unroll
+    for (int o = kCountLanes / 2; o > 0; o >>= 1) before[r] += __shfl_xor_sync(0xffffffffu, before[r], o);
+    if (q == 0 && mine + r < n) {
+      kout[before[r]] = k[r];
+      vout[before[r]] = vals[mine + r];
+    }
+  }
+}
+
+__global__ void k_sorted_back(int n, const uint64_t *kin, const uint32_t *vin, uint64_t *keys, uint32_t *vals) {
+  grid_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  keys[i] = kin[i];
+  vals[i] = vin[i];
 }
 
 constexpr size_t round256(size_t b) { return (b + 255) / 256 * 256; }
@@ -423,17 +451,23 @@ static int radix_passes(int n, uint64_t *keys, uint32_t *vals, char *p, cudaStre
 }
 
 // Stable sort of (keys, vals); result in keys/vals.  Returns launches.
-// Up to one large tile a single block does it all.  Small tiles while the
-// direct sum of the counts reaches (16,384 keys: small / large 73 / 101 us;
-// 262,144 104 / 116); then large ones, which halve the counts to add up
-// (1,048,576: 214 / 183).
+// Direct counting up to kCountMax keys, one key per lane group while that
+// leaves too few blocks.  Then the radix passes: small tiles while the direct
+// sum of the counts reaches (16,384 keys: small / large 73 / 101 us; 262,144
+// 104 / 116), and large ones, which halve the counts to add up (1,048,576:
+// 214 / 183).
+constexpr int kCountMax = 8192;
 int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStream_t st) {
   if (n <= 1) return 0;
-  if (n <= kTileLarge) {
-    launch(k_radix_tile, 1, 512, st, n, keys, vals);
-    return 1;
-  }
   char *p = (char *)(((uintptr_t)scratch + 15) / 16 * 16);  // the tables are read 16 bytes at a time
+  if (n <= kCountMax) {
+    uint64_t *k2 = (uint64_t *)p;
+    uint32_t *v2 = (uint32_t *)(p + round256((size_t)n * 8));
+    const int r = n <= 4096 ? 1 : 4, per = kCountThreads / kCountLanes * r;
+    launch(r == 1 ? k_count_sort<1> : k_count_sort<4>, (n + per - 1) / per, kCountThreads, st, n, keys, vals, k2, v2);
+    launch(k_sorted_back, (n + 255) / 256, 256, st, n, k2, v2, keys, vals);
+    return 2;
+  }
   return n <= kDirectTiles * kTileSmall ? radix_passes<256>(n, keys, vals, p, st)
                                         : radix_passes<512>(n, keys, vals, p, st);
 }

@@ -288,7 +288,7 @@ int cudasph_peano_keys(int n, const double *x, const double *y, const double *z,
  * footprint is fixed at start-up.  The caller passes only the keys and values
  * (device pointers, results in place, same stable order as
  * cudasph_radix_sort_u64); the scratch is a fixed array compiled into this
- * library, sized for at most CUDASPH_SORT_NOALLOC_MAX_KEYS keys (about 3.1 MB,
+ * library, sized for at most CUDASPH_SORT_NOALLOC_MAX_KEYS keys (about 3.5 MB,
  * held on every GPU that loads the library until the process exits).  Larger
  * n returns SPH_ERR_ARG with a message.  No cudaMalloc, cudaFree or other
  * allocating routine is called.  The first call on a device looks up the

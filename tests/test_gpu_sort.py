@@ -1,12 +1,13 @@
-"""The radix sort at the edges of its tiles and of its three forms (one block;
-small tiles; large tiles with the counts added up by the passes or by a launch
-of their own): keys and permutation equal to a stable CPU sort, bit for bit."""
+"""The radix sort at the edges of its tiles and of its three forms (direct
+counting; small tiles; large tiles with the counts added up by the passes or by
+a launch of their own): keys and permutation equal to a stable CPU sort, bit for bit."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 31, 255, 2047, 2048, 4095, 4096, 4097, 6144, 524287, 524288, 524289, 1048576, 1048577, 1300001]
+SIZES = [1, 2, 31, 255, 2047, 2048, 2049, 4095, 4096, 4097, 6144, 8191, 8192, 8193, 10241,
+         524287, 524288, 524289, 1048576, 1048577, 1300001]
 
 
 def _keys(n, kind):
