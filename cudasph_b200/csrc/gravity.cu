@@ -52,7 +52,26 @@ __device__ __forceinline__ float rsq<float>(float x) { return rsqrt_f32(x); }
 template <>
 __device__ __forceinline__ double rsq<double>(double x) { return rsqrt_f64(x); }
 
-// The near-field pair of the spline mode (r < max(range_i, range_j)),
+// One side of an FP64 pair inside its softening range, r2 < h2, inv = 1 / r (0
+// at r = 0): the factors of spline_poly over h^3 and over h.  All of 1/h, u and
+// 1/u come from reciprocal square roots; with sqrt and divisions the near pairs
+// cost several times the FP64 instructions (60,000 particles with 24
+// neighbours: diagonal tiles 622 -> 274 us, the rest 3,695 -> 3,143).
+__device__ __forceinline__ void spline_inside(double r2, double inv, double h2, double &g, double &p) {
+  const double ih = rsqrt_f64(h2), ih2 = ih * ih, u2 = r2 * ih2, u = r2 * inv * ih;
+  if (u < 0.5) {
+    g = fma(u2, fma(32.0, u, -38.4), 10.666666666667);
+    p = fma(u2, fma(u2, fma(6.4, u, -9.6), 5.333333333333), -2.8);
+  } else {
+    const double iu = inv * (h2 * ih);
+    g = fma(u, fma(u, fma(u, -10.666666666667, 38.4), -48.0), 21.333333333333) - 0.066666666667 * (iu * iu * iu);
+    p = fma(u2, fma(u, fma(u, fma(u, -2.133333333333, 9.6), -16.0), 10.666666666667), fma(0.066666666667, iu, -3.2));
+  }
+  g *= ih2 * ih;
+  p *= ih;
+}
+
+// The near-field pair of the mixed spline mode (r < max(range_i, range_j)),
 // bodyBodyInteraction's else-branch, sph_grav_kernel.cu:40-106.
 // dx = x_j - x_i; accumulates acceleration into a (a += contribution).
 template <class R>
@@ -81,6 +100,16 @@ __device__ __noinline__ void spline_near(R dx, R dy, R dz, R r2, R mj, R hi2, R 
   ax = fma(dx, g, ax);
   ay = fma(dy, g, ay);
   az = fma(dz, g, az);
+}
+
+// the same in FP64 without the mass: acceleration factor and potential at i
+__device__ __noinline__ double2 spline_at_i(double r2, double hi2, double hj2) {
+  const double inv = r2 > 0 ? rsqrt_f64(r2) : 0.0;
+  const double far = inv * inv * inv;
+  double gi = far, gj = far, pi = -inv, unused;
+  if (r2 < hi2) spline_inside(r2, inv, hi2, gi, pi);
+  if (r2 < hj2) spline_inside(r2, inv, hj2, gj, unused);
+  return make_double2(0.5 * (gi + gj), pi);
 }
 
 __device__ __forceinline__ void add_sums(double4 *out, double x, double y, double z, double w) {
@@ -165,7 +194,12 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *sr
               pot[r] -= s;
             }
           } else {
-            spline_near<double>(dx, dy, dz, r2, q.w, hi2[r], hj2, ax[r], ay[r], az[r], pot[r]);
+            const double2 v = spline_at_i(r2, hi2[r], hj2);
+            const double g = q.w * v.x;
+            ax[r] = fma(dx, g, ax[r]);
+            ay[r] = fma(dy, g, ay[r]);
+            az[r] = fma(dz, g, az[r]);
+            pot[r] = fma(q.w, v.y, pot[r]);
           }
         }
       }
@@ -621,7 +655,7 @@ constexpr int kSym64R = 8;
 static_assert(2 * kSym64Warps * 32 * kSym64R == kSymTile, "the FP64 form shares the tile layout");
 
 // Spline softening (SOFT), each pair once as well (one-sided before: 60,000
-// particles with 24 neighbours 21.2 -> 4.3 ms, 5,000 2.03 -> 0.28): a pair farther apart than both ranges is Newtonian,
+// particles with 24 neighbours 21.2 -> 3.4 ms, 5,000 2.03 -> 0.28): a pair farther apart than both ranges is Newtonian,
 // the rest -- about the neighbour count per particle -- follow the polynomials
 // of sph_grav_kernel.cu:40-106, whose acceleration factor is the same for both
 // sides and whose potential uses each side's own range.  "Far" is decided on
@@ -637,27 +671,13 @@ struct NearPair {
 
 __device__ __noinline__ NearPair spline_pair(double r2, double hi2, double hj2) {
   const double inv = r2 > 0 ? rsqrt_f64(r2) : 0.0;
-  const double far = 0.5 * inv * inv * inv;
+  const double far = inv * inv * inv;
+  double gi = far, gj = far;
   NearPair v;
-  v.g = far;
-  v.pi = -inv;
-  if (r2 < hi2) {
-    const double u2 = r2 / hi2, h = sqrt(hi2);
-    double ga;
-    spline_poly<double>(sqrt(u2), u2, ga, v.pi);
-    v.g = 0.5 * ga / (hi2 * h);
-    v.pi /= h;
-  }
-  double gj = far;
-  v.pj = -inv;
-  if (r2 < hj2) {
-    const double u2 = r2 / hj2, h = sqrt(hj2);
-    double ga;
-    spline_poly<double>(sqrt(u2), u2, ga, v.pj);
-    gj = 0.5 * ga / (hj2 * h);
-    v.pj /= h;
-  }
-  v.g += gj;
+  v.pi = v.pj = -inv;
+  if (r2 < hi2) spline_inside(r2, inv, hi2, gi, v.pi);
+  if (r2 < hj2) spline_inside(r2, inv, hj2, gj, v.pj);
+  v.g = 0.5 * (gi + gj);
   return v;
 }
 
