@@ -112,9 +112,14 @@ struct StepScalars {
 // through ldg and ld4 below, which are volatile assembly like the wait itself.
 // Time per step, us, without / with: 2,049 particles 191 / 147, 16,384
 // 746 / 644; replayed from a graph 6,007 243 / 226.
+// The next kernel is let in after the wait, not before it: before, a row of
+// short kernels came to sit on the SMs all at once, and the blocks of a kernel
+// of less than one wave among them (the direct sum) were packed into the SMs
+// that had room left (2,049 particles 127 -> 120 us a step, a 12,000-particle
+// rollout 9.90 -> 9.60 ms).
 __device__ __forceinline__ void grid_enter() {
-  asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // kernel<<<grid, block, 0, st>>>(args...), programmatic on a stream of its own
