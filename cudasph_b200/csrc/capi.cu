@@ -35,7 +35,7 @@ int launch_hydro(const HydroArgs &a, cudaStream_t st);
 int launch_density_mixed(const HydroArgs &a, cudaStream_t st);
 int launch_hydro_mixed(const HydroArgs &a, cudaStream_t st);
 int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out, int soft_mode, double eps, double G,
-                   int precision, const int *mass_mixed, int rank, int world, cudaStream_t st);
+                   int precision, const int *mass_mixed, int rank, int world, bool cleared, cudaStream_t st);
 int launch_tree_gravity(const TreeView &t, const uint64_t *keys, const double4 *src, void *ws, double4 *out,
                         unsigned *flags, double eps, double theta, double G, int rank, int world, cudaStream_t st);
 size_t tree_gravity_workspace_bytes(int n);
@@ -43,7 +43,8 @@ int launch_shard_pack(int n, int s0, int s1, const double4 *pos, const double4 *
                       const int *n_ngb, double4 *xbuf, cudaStream_t st);
 int launch_shard_unpack(int n, const double4 *xbuf, double4 *pos, double4 *hyd, double4 *dd, int *n_ngb,
                         cudaStream_t st);
-int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, cudaStream_t st);
+int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, double4 *clear,
+                        cudaStream_t st);
 int launch_check_masses(int n, const double4 *vel, int *mass_mixed, cudaStream_t st);
 int launch_predict(int n, double4 *pos, double4 *vel, double4 *hyd, const double4 *dots, double4 *old,
                    const double *sc, cudaStream_t st);
@@ -726,16 +727,16 @@ extern "C" int cudasph_gravity(sph_ctx *c) {
   PhaseScope ps(c, SPH_PH_GRAVITY);
   Fields &F = c->f[c->cur];
   if (c->p.grav_mode == SPH_GRAV_TREE) {
-    LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, c->st));
+    LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, nullptr, c->st));
     // the radix tree is built from the sort's keys, which match the current order
     LAUNCHED(launch_tree_gravity(c->tree, c->keys, c->gsrc, c->tgws, F.grav, c->flags, c->p.eps, c->p.theta, c->p.G,
                                  c->rank, c->world, c->st));
     SPH_CUDA_TRY(cudaGetLastError());
     return SPH_OK;
   }
-  LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, c->st));
+  LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, F.grav, c->st));
   LAUNCHED(launch_gravity(c->n, c->gsrc, c->gh2, F.grav, c->p.soft_mode, c->p.eps, c->p.G, c->p.precision,
-                          c->mass_mixed, c->rank, c->world, c->st));
+                          c->mass_mixed, c->rank, c->world, true, c->st));
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
 }

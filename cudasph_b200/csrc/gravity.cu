@@ -120,42 +120,50 @@ __device__ __forceinline__ void add_sums(double4 *out, double x, double y, doubl
   atomicAdd(o + 3, w);
 }
 
-__device__ __forceinline__ void store_sums(double4 *out, double x, double y, double z, double w, int slices) {
-  if (slices == 1) *out = make_double4(x, y, z, w);
-  else add_sums(out, x, y, z, w);
+__device__ __forceinline__ void store_sums(double4 *out, double x, double y, double z, double w, bool add) {
+  if (add) add_sums(out, x, y, z, w);
+  else *out = make_double4(x, y, z, w);
 }
 
 // -------------------------------- FP64 --------------------------------------
-// One-sided form: every i of the block against the sources [jlo, jhi); with
-// tile > 0 the range is the tile of `tile` particles that holds the block
-// (the diagonal tiles of the symmetric form), else all n.
-template <int SOFT, int R>
-__global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *src, const double *h2src, double4 *out,
-                                                        double eps2, double G, int tile, int block0, int slices) {
-  grid_enter();
-  __shared__ double4 sj[kGThreads];
-  __shared__ double sh[SOFT == SPH_SOFT_SPLINE ? kGThreads : 1];
+// One-sided form: the T * R particles of a block against the sources
+// [jlo, jhi); with tile > 0 the range is the tile of `tile` particles that
+// holds the block (the diagonal tiles of the symmetric form), else all n.
+// `bid`: block and slice, `shared`: the staged sources.  ADD: sums are added to
+// a cleared output, which others add to as well.
+template <int SOFT>
+struct Staged64 {
+  double4 j[kGThreads];
+  double h[SOFT == SPH_SOFT_SPLINE ? kGThreads : 1];
+};
+template <int SOFT, int T, int R, bool ADD>
+__device__ __forceinline__ void one_sided_f64(int n, const double4 *src, const double *h2src, double4 *out,
+                                              double eps2, double G, int tile, int block0, int slices, unsigned bid,
+                                              Staged64<SOFT> &shared) {
+  double4(&sj)[kGThreads] = shared.j;
+  double *sh = shared.h;
   const int t = threadIdx.x;
-  const int i0 = (blockIdx.x / slices + block0) * kGThreads * R;
+  const int i0 = (bid / slices + block0) * T * R;
   int jlo = tile > 0 ? (i0 / tile) * tile : 0;
   int jhi = tile > 0 ? min(jlo + tile, n) : n;
-  source_slice<32>(jlo, jhi, blockIdx.x % slices, slices);
+  source_slice<32>(jlo, jhi, bid % slices, slices);
   double xi[R], yi[R], zi[R], hi2[R], ax[R], ay[R], az[R], pot[R];
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const int i = min(i0 + r * kGThreads + t, n - 1);
+    const int i = min(i0 + r * T + t, n - 1);
     const double4 p = src[i];
     xi[r] = p.x; yi[r] = p.y; zi[r] = p.z;
     hi2[r] = (SOFT == SPH_SOFT_SPLINE) ? h2src[i] : 0.0;
     ax[r] = ay[r] = az[r] = pot[r] = 0.0;
   }
   for (int j0 = jlo; j0 < jhi; j0 += kGThreads) {
-    const int j = j0 + t;
     __syncthreads();
-    if (j < jhi) {
-      sj[t] = src[j];
-      if (SOFT == SPH_SOFT_SPLINE) sh[t] = h2src[j];
-    }
+#pragma unroll
+    for (int q = t; q < kGThreads; q += T)
+      if (j0 + q < jhi) {
+        sj[q] = src[j0 + q];
+        if (SOFT == SPH_SOFT_SPLINE) sh[q] = h2src[j0 + q];
+      }
     __syncthreads();
     const int m = min(kGThreads, jhi - j0);
     if (SOFT == SPH_SOFT_PLUMMER) {
@@ -207,9 +215,19 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *sr
   }
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const int i = i0 + r * kGThreads + t;
-    if (i < n) store_sums(out + i, G * ax[r], G * ay[r], G * az[r], G * pot[r], slices);
+    const int i = i0 + r * T + t;
+    if (i < n) store_sums(out + i, G * ax[r], G * ay[r], G * az[r], G * pot[r], ADD || slices > 1);
   }
+}
+
+// the one-sided form by itself: sets of one tile, and spline softening on
+// several ranks
+template <int SOFT, int R>
+__global__ void __launch_bounds__(kGThreads) k_grav_f64(int n, const double4 *src, const double *h2src, double4 *out,
+                                                        double eps2, double G, int tile, int block0, int slices) {
+  grid_enter();
+  __shared__ Staged64<SOFT> shared;
+  one_sided_f64<SOFT, kGThreads, R, false>(n, src, h2src, out, eps2, G, tile, block0, slices, blockIdx.x, shared);
 }
 
 // ----------------------------- mixed (FP32) ---------------------------------
@@ -331,7 +349,7 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *sr
     const int i = i0 + r * kGThreads + t;
     if (i < n)
       store_sums(out + i, G * ((double)ahi[r][0] + (double)alo[r][0]), G * ((double)ahi[r][1] + (double)alo[r][1]),
-                 G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]), slices);
+                 G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]), slices > 1);
   }
 }
 
@@ -346,26 +364,24 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *sr
 // have m = 0 at the anchor; eps > 0 keeps their r^2 > 0, so every tile is a
 // full tile.
 
-// One-sided form: every i of the block against the sources [jlo, jhi); with
-// tile > 0 the range is the tile of `tile` particles that holds the block
-// (the diagonal tiles of the symmetric form), else all n.
-template <int RP>  // i-particle pairs per thread
-__global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const double4 *src, double4 *out, float eps2,
-                                                                  double G, int tile, int block0, int slices) {
-  grid_enter();
-  __shared__ ulonglong2 sj[kGThreads][2];
+// One-sided form, as in FP64: T * 2 * RP particles of a block; the FP32 sums
+// run over kGThreads sources whatever T is.
+template <int T, int RP, bool ADD>  // RP: i-particle pairs per thread
+__device__ __forceinline__ void one_sided_f32x2(int n, const double4 *src, double4 *out, float eps2, double G,
+                                                int tile, int block0, int slices, unsigned bid,
+                                                ulonglong2 (&sj)[kGThreads][2]) {
   const int t = threadIdx.x;
-  const int i0 = (blockIdx.x / slices + block0) * kGThreads * 2 * RP;
+  const int i0 = (bid / slices + block0) * T * 2 * RP;
   int jlo = tile > 0 ? (i0 / tile) * tile : 0;
   int jhi = tile > 0 ? min(jlo + tile, n) : n;
-  source_slice<kGThreads>(jlo, jhi, blockIdx.x % slices, slices);
+  source_slice<kGThreads>(jlo, jhi, bid % slices, slices);
   const double4 anc = src[min(i0, n - 1)];
   f32x2 xi[RP], yi[RP], zi[RP];
   float ahi[2 * RP][4], alo[2 * RP][4];
 #pragma unroll
   for (int p = 0; p < RP; p++) {
-    const double4 a = src[min(i0 + (2 * p) * kGThreads + t, n - 1)];
-    const double4 b = src[min(i0 + (2 * p + 1) * kGThreads + t, n - 1)];
+    const double4 a = src[min(i0 + (2 * p) * T + t, n - 1)];
+    const double4 b = src[min(i0 + (2 * p + 1) * T + t, n - 1)];
     xi[p] = pk2((float)(a.x - anc.x), (float)(b.x - anc.x));
     yi[p] = pk2((float)(a.y - anc.y), (float)(b.y - anc.y));
     zi[p] = pk2((float)(a.z - anc.z), (float)(b.z - anc.z));
@@ -376,16 +392,18 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const d
     for (int c = 0; c < 4; c++) ahi[r][c] = alo[r][c] = 0.f;
   const f32x2 e2 = pk2(eps2, eps2);
   for (int j0 = jlo; j0 < jhi; j0 += kGThreads) {
-    const int j = j0 + t;
     __syncthreads();
-    if (j < jhi) {
-      const double4 q = src[j];
-      const float x = (float)(q.x - anc.x), y = (float)(q.y - anc.y), z = (float)(q.z - anc.z), m = (float)q.w;
-      sj[t][0] = make_ulonglong2(pk2(x, x), pk2(y, y));
-      sj[t][1] = make_ulonglong2(pk2(z, z), pk2(m, m));
-    } else {
-      sj[t][0] = make_ulonglong2(0ull, 0ull);
-      sj[t][1] = make_ulonglong2(0ull, 0ull);
+#pragma unroll
+    for (int q = t; q < kGThreads; q += T) {
+      if (j0 + q < jhi) {
+        const double4 v = src[j0 + q];
+        const float x = (float)(v.x - anc.x), y = (float)(v.y - anc.y), z = (float)(v.z - anc.z), m = (float)v.w;
+        sj[q][0] = make_ulonglong2(pk2(x, x), pk2(y, y));
+        sj[q][1] = make_ulonglong2(pk2(z, z), pk2(m, m));
+      } else {
+        sj[q][0] = make_ulonglong2(0ull, 0ull);
+        sj[q][1] = make_ulonglong2(0ull, 0ull);
+      }
     }
     __syncthreads();
     f32x2 px[RP], py[RP], pz[RP], pp[RP];
@@ -431,11 +449,19 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const d
   }
 #pragma unroll
   for (int r = 0; r < 2 * RP; r++) {
-    const int i = i0 + r * kGThreads + t;
+    const int i = i0 + r * T + t;
     if (i < n)
       store_sums(out + i, G * ((double)ahi[r][0] + (double)alo[r][0]), G * ((double)ahi[r][1] + (double)alo[r][1]),
-                 G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]), slices);
+                 G * ((double)ahi[r][2] + (double)alo[r][2]), G * ((double)ahi[r][3] + (double)alo[r][3]), ADD || slices > 1);
   }
+}
+
+template <int RP>
+__global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const double4 *src, double4 *out, float eps2,
+                                                                  double G, int tile, int block0, int slices) {
+  grid_enter();
+  __shared__ ulonglong2 sj[kGThreads][2];
+  one_sided_f32x2<kGThreads, RP, false>(n, src, out, eps2, G, tile, block0, slices, blockIdx.x, sj);
 }
 
 // ------------------ mixed (FP32), symmetric pair form -----------------------
@@ -451,7 +477,7 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const d
 // block owns one i-tile (kSymWarps warps, kSymRP packed i-pairs per lane) and
 // one work item = up to sym_chunk(nt) j-tiles strictly above its own, so the
 // upper triangle of tile pairs is covered once; the diagonal tiles run
-// through the one-sided kernel.  Inside a warp the j's travel: a batch of 32
+// through the one-sided form.  Inside a warp the j's travel: a batch of 32
 // sources, one per lane, rotates through the lanes by shuffles, each lane
 // meeting every source of the batch once; a source carries its own
 // accumulator with it, so after 32 steps lane l holds the batch-partial of
@@ -467,9 +493,8 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32x2_plummer(int n, const d
 // end of the item.  The FMA pipe is the limiter; moving work to the MUFU
 // pipe does not pay: s^-2 from a MUFU reciprocal instead of a multiply for
 // 2, 4 or 8 of the 8 i-pairs measured 308, 312 and 330 ms against 303.
-// The output therefore holds the diagonal-tile sums first (stored by the
-// one-sided kernel) and receives the off-diagonal sums by atomics, so the
-// order of the FP64 additions, not their values, varies between runs.
+// All sums meet by atomics in an output cleared beforehand, so the order of
+// the FP64 additions, not their values, varies between runs.
 //
 // Equal masses (UNI): when every particle has the same mass m (a flag the
 // source-packing kernel computes on the device every step), the mass factors
@@ -619,21 +644,43 @@ __device__ __forceinline__ void sym_plummer_item(long long item, int n, int nt, 
   }
 }
 
-// mass_mixed: device word, 0 when all masses are equal (nullptr: general form);
-// block b runs slice b % slices of work item item0 + b / slices
+// The whole direct sum of a launch: the one-sided blocks of the diagonal tiles
+// first (`diag` of them, from block0 on, each cut into dslices), then block b
+// runs slice b % slices of work item item0 + b / slices.  In a launch of their
+// own the diagonal blocks are one short, badly filled round for which the
+// symmetric blocks wait; gravity phase, us, in two launches / in one: FP64
+// 2,049 particles 27 / 21, 6,007 50 / 41, 16,384 236 / 225, spline 60,000
+// 3,408 / 3,372, mixed 65,536 1,316 / 1,305; from 130,000 on the same.
+// mass_mixed: device word, 0 when all masses are equal (nullptr: general form).
+struct DiagWork {
+  unsigned blocks;  // one-sided blocks x slices
+  int block0, slices;
+};
 __global__ void __launch_bounds__(kSymWarps * 32, 4) k_grav_sym_plummer(int n, int nt, const double4 *src,
                                                                         double4 *out, float eps2, double G,
                                                                         const int *mass_mixed, long long item0,
-                                                                        int slices) {
+                                                                        int slices, DiagWork diag) {
   grid_enter();
-  __shared__ float red[2][kSymWarps][4][32];
-  __shared__ double iacc[2 * kSymRP * 4][kSymWarps * 32];  // [i-slot * 4 + component][thread]
-  const long long item = item0 + blockIdx.x / slices;
-  const unsigned slice = blockIdx.x % slices;
+  __shared__ union Shared {
+    struct {
+      float red[2][kSymWarps][4][32];
+      double iacc[2 * kSymRP * 4][kSymWarps * 32];  // [i-slot * 4 + component][thread]
+    } sym;
+    ulonglong2 sj[kGThreads][2];
+    __device__ Shared() {}
+  } sm;
+  if (blockIdx.x < diag.blocks) {
+    one_sided_f32x2<kSymWarps * 32, 2, true>(n, src, out, eps2, G, kSymTile, diag.block0, diag.slices, blockIdx.x,
+                                             sm.sj);
+    return;
+  }
+  const unsigned q = blockIdx.x - diag.blocks;
+  const long long item = item0 + q / slices;
+  const unsigned slice = q % slices;
   if (mass_mixed != nullptr && ldg(mass_mixed) == 0)
-    sym_plummer_item<true>(item, n, nt, src, out, eps2, G, red, iacc, slice, slices);
+    sym_plummer_item<true>(item, n, nt, src, out, eps2, G, sm.sym.red, sm.sym.iacc, slice, slices);
   else
-    sym_plummer_item<false>(item, n, nt, src, out, eps2, G, red, iacc, slice, slices);
+    sym_plummer_item<false>(item, n, nt, src, out, eps2, G, sm.sym.red, sm.sym.iacc, slice, slices);
 }
 
 // ------------------- FP64, symmetric pair form ------------------------------
@@ -802,21 +849,30 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
   }
 }
 
-// block b runs slice b / 2 % slices of work item item0 + b / 2 / slices, on
-// one half of its i-tile (b & 1)
+// As k_grav_sym_plummer; symmetric block b runs slice b / 2 % slices of work
+// item item0 + b / 2 / slices, on one half of its i-tile (b & 1).
 template <int SOFT>
 __global__ void __launch_bounds__(kSym64Warps * 32) k_grav_sym_f64(int n, int nt, const double4 *src,
                                                                    const double *h2src, double4 *out, double eps2,
                                                                    double G, const int *mass_mixed, long long item0,
-                                                                   int slices) {
+                                                                   int slices, DiagWork diag) {
   grid_enter();
-  __shared__ double red[2][kSym64Warps][4][32];
-  const unsigned q = blockIdx.x >> 1;
+  __shared__ union Shared {
+    double red[2][kSym64Warps][4][32];
+    Staged64<SOFT> one;
+    __device__ Shared() {}
+  } sm;
+  if (blockIdx.x < diag.blocks) {
+    one_sided_f64<SOFT, kSym64Warps * 32, 4, true>(n, src, h2src, out, eps2, G, kSymTile, diag.block0, diag.slices,
+                                                   blockIdx.x, sm.one);
+    return;
+  }
+  const unsigned b = blockIdx.x - diag.blocks, q = b >> 1;
   const long long item = item0 + q / slices;
   if (mass_mixed != nullptr && ldg(mass_mixed) == 0)
-    sym_f64_item<true, SOFT>(item, n, nt, src, h2src, out, eps2, G, red, blockIdx.x & 1, q % slices, slices);
+    sym_f64_item<true, SOFT>(item, n, nt, src, h2src, out, eps2, G, sm.red, b & 1, q % slices, slices);
   else
-    sym_f64_item<false, SOFT>(item, n, nt, src, h2src, out, eps2, G, red, blockIdx.x & 1, q % slices, slices);
+    sym_f64_item<false, SOFT>(item, n, nt, src, h2src, out, eps2, G, sm.red, b & 1, q % slices, slices);
 }
 
 // blocks [lo, hi) of a one-sided or symmetric launch (nothing when empty)
@@ -864,11 +920,12 @@ static GravPlan grav_plan(int n, int soft_mode, int precision, int rank, int wor
 // src = {x, y, z, m} per particle; h2src = range^2 (spline mode only).
 // Shard `rank` of `world` (world > 1) computes its contiguous share of the
 // one-sided blocks (diagonal tiles, or all pairs for small n / spline
-// softening) and of the symmetric work items into `out`, which it zeroes
-// first: the element-wise sum of the shards' outputs is the whole sum.
-// FP64 spline softening on one rank takes the symmetric tiles as well.
+// softening) and of the symmetric work items into `out`: the element-wise sum
+// of the shards' outputs is the whole sum.  `cleared`: the caller has zeroed
+// `out` on the stream.  FP64 spline softening on one rank takes the symmetric
+// tiles as well.
 int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out, int soft_mode, double eps, double G,
-                   int precision, const int *mass_mixed, int rank, int world, cudaStream_t st) {
+                   int precision, const int *mass_mixed, int rank, int world, bool cleared, cudaStream_t st) {
   if (n <= 0) return 0;
   const double eps2 = eps * eps;
   GravPlan g = grav_plan(n, soft_mode, precision, rank, world);
@@ -878,68 +935,56 @@ int launch_gravity(int n, const double4 *src, const double *h2src, double4 *out,
     g.items = Span{0, sym_items(nt)};
   }
   const Span &blocks = g.blocks, &items = g.items;
+  const bool plummer = soft_mode == SPH_SOFT_PLUMMER, fp64 = precision == SPH_PREC_FP64;
   // one-sided blocks: four to an SM; symmetric blocks run four to an SM
   // (registers): sixteen rounds of them while a slice keeps 256 sources, two
   // rounds while it keeps 32
   const int sources = g.tile > 0 ? g.tile : n;
-  const int sb = blocks.empty() ? 1 : grav_slices(blocks.hi - blocks.lo, sources, 148 * 4,
-                                                  precision == SPH_PREC_FP64 ? 32 : kGThreads);
-  int si = 1;
+  const int sb = blocks.empty() ? 1 : grav_slices(blocks.hi - blocks.lo, sources, 148 * 4, fp64 ? 32 : kGThreads);
+  if (!cleared && (world > 1 || sb > 1 || !items.empty())) cudaMemsetAsync(out, 0, sizeof(double4) * n, st);
   if (!items.empty()) {
-    const long long per = (items.hi - items.lo) * (precision == SPH_PREC_FP64 ? 2 : 1);
-    si = grav_slices(per, g.chunk * kSymTile, 592 * 16, 256);
+    const long long per = (items.hi - items.lo) * (fp64 ? 2 : 1);
+    int si = grav_slices(per, g.chunk * kSymTile, 592 * 16, 256);
     si *= grav_slices(per * si, g.chunk * kSymTile / si, 592 * 2, 32);
+    const DiagWork diag{blocks.empty() ? 0u : blocks.grid() * sb, (int)blocks.lo, sb};
+    if (fp64)
+      launch(plummer ? k_grav_sym_f64<SPH_SOFT_PLUMMER> : k_grav_sym_f64<SPH_SOFT_SPLINE>,
+             diag.blocks + items.grid() * 2 * si, kSym64Warps * 32, st, n, nt, src, h2src, out, eps2, G, mass_mixed,
+             items.lo, si, diag);
+    else
+      launch(k_grav_sym_plummer, diag.blocks + items.grid() * si, kSymWarps * 32, st, n, nt, src, out, (float)eps2, G,
+             mass_mixed, items.lo, si, diag);
+    return 1;
   }
-  if (world > 1 || sb > 1) cudaMemsetAsync(out, 0, sizeof(double4) * n, st);
-  int launches = 0;
-  if (precision == SPH_PREC_FP64) {
-    constexpr int R = 2;
-    static_assert(kSymTile % (kGThreads * R) == 0, "diagonal tiles must hold whole blocks");
-    // diagonal tiles one-sided (all pairs when there is a single tile), then the items above them
-    const bool plummer = soft_mode == SPH_SOFT_PLUMMER;
-    if (!blocks.empty()) {
-      launch(plummer ? k_grav_f64<SPH_SOFT_PLUMMER, R> : k_grav_f64<SPH_SOFT_SPLINE, R>, blocks.grid() * sb,
-             kGThreads, st, n, src, h2src, out, eps2, G, g.tile, (int)blocks.lo, sb);
-      launches++;
-    }
-    if (!items.empty()) {
-      launch(plummer ? k_grav_sym_f64<SPH_SOFT_PLUMMER> : k_grav_sym_f64<SPH_SOFT_SPLINE>, items.grid() * 2 * si,
-             kSym64Warps * 32, st, n, nt, src, h2src, out, eps2, G, mass_mixed, items.lo, si);
-      launches++;
-    }
-  } else if (soft_mode == SPH_SOFT_PLUMMER) {
-    constexpr int RP = 1;
-    static_assert(kSymTile % (kGThreads * 2 * RP) == 0, "diagonal tiles must hold whole blocks");
-    if (!blocks.empty()) {
-      launch(k_grav_f32x2_plummer<RP>, blocks.grid() * sb, kGThreads, st, n, src, out, (float)eps2, G, g.tile,
-             (int)blocks.lo, sb);
-      launches++;
-    }
-    if (!items.empty()) {
-      launch(k_grav_sym_plummer, items.grid() * si, kSymWarps * 32, st, n, nt, src, out, (float)eps2, G, mass_mixed,
-             items.lo, si);
-      launches++;
-    }
-  } else if (!blocks.empty()) {
+  if (blocks.empty()) return 0;
+  if (fp64)
+    launch(plummer ? k_grav_f64<SPH_SOFT_PLUMMER, 2> : k_grav_f64<SPH_SOFT_SPLINE, 2>, blocks.grid() * sb, kGThreads,
+           st, n, src, h2src, out, eps2, G, g.tile, (int)blocks.lo, sb);
+  else if (plummer)
+    launch(k_grav_f32x2_plummer<1>, blocks.grid() * sb, kGThreads, st, n, src, out, (float)eps2, G, g.tile,
+           (int)blocks.lo, sb);
+  else
     launch(k_grav_f32<SPH_SOFT_SPLINE, 4>, blocks.grid() * sb, kGThreads, st, n, src, h2src, out, (float)eps2, G,
            (int)blocks.lo, sb);
-    launches++;
-  }
-  return launches;
+  return 1;
 }
 
-// pack the gravity sources {x, y, z, m} and range^2 from the state
-__global__ void k_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2) {
+// pack the gravity sources {x, y, z, m} and range^2 from the state; clear: the
+// direct sum's output, zeroed here (nullptr: none)
+__global__ void k_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2,
+                               double4 *clear) {
   grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double4 p = pos[i];
   src[i] = make_double4(p.x, p.y, p.z, vel[i].w);
   h2[i] = p.w * p.w;
+  if (clear) clear[i] = make_double4(0.0, 0.0, 0.0, 0.0);
 }
 
-int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, cudaStream_t st) {
-  launch(k_pack_sources, (n + 255) / 256, 256, st, n, pos, vel, src, h2);
+int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *src, double *h2, double4 *clear,
+                        cudaStream_t st) {
+  launch(k_pack_sources, (n + 255) / 256, 256, st, n, pos, vel, src, h2, clear);
   return 1;
 }
 
@@ -979,7 +1024,8 @@ extern "C" int cudasph_gravity_direct(int n, const double *pos4, const double *r
     SPH_CUDA_TRY(cudaMallocAsync((void **)&h2, sizeof(double) * n, st));
     sph::launch(sph::k_range_sq, (n + 255) / 256, 256, st, n, range, h2);
   }
-  sph::launch_gravity(n, (const double4 *)pos4, h2, (double4 *)out4, soft_mode, eps, G, precision, nullptr, 0, 1, st);
+  sph::launch_gravity(n, (const double4 *)pos4, h2, (double4 *)out4, soft_mode, eps, G, precision, nullptr, 0, 1,
+                      false, st);
   if (h2) SPH_CUDA_TRY(cudaFreeAsync(h2, st));
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
