@@ -16,11 +16,8 @@
 namespace sph {
 // kernels (launchers) from the other translation units
 size_t radix_scratch_bytes(int n);
-int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStream_t st);
-int morton_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
-                double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st);
-int peano_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
-               double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st);
+int sort_particles(int n, bool peano, const Fields &src, const Fields &dst, double *part, double *box4, uint64_t *keys,
+                   uint32_t *order, void *scratch, cudaStream_t st);
 int tree_layout(int n, TreeView *t);
 int build_tree(const TreeView &t, const double4 *pos, float4 *lo, float4 *hi, float4 *pf, cudaStream_t st);
 int launch_solve_range(const TreeView &t, double4 *pos, int *nevals, unsigned *flags, const sph_params &p,
@@ -54,7 +51,6 @@ int launch_finish(int n, const double4 *pos, const double4 *vel, const double4 *
                   double *part, double *sc, unsigned *flags, cudaStream_t st);
 int launch_kick(int n, double4 *vel, double4 *hyd, const double4 *dots, const double4 *old, const double *sc,
                 cudaStream_t st);
-int launch_permute(int n, const uint32_t *order, const Fields &src, const Fields &dst, cudaStream_t st);
 int launch_invert(int n, const int *id, int *slot_of, cudaStream_t st);
 int launch_field_io(int n, double *arr, int stride, int comp, const int *id, double *flat, int to_state,
                     cudaStream_t st);
@@ -587,12 +583,8 @@ extern "C" int cudasph_sort(sph_ctx *c) {
   const int n = c->n;
   Fields &S = c->f[c->cur];
   Fields &D = c->f[1 - c->cur];
-  if (c->p.key_mode == SPH_KEY_PEANO)
-    LAUNCHED(peano_keys(n, S.pos, nullptr, nullptr, nullptr, c->bbox_part, c->box4, c->keys, c->vals, c->st));
-  else
-    LAUNCHED(morton_keys(n, S.pos, nullptr, nullptr, nullptr, c->bbox_part, c->box4, c->keys, c->vals, c->st));
-  LAUNCHED(radix_sort_u64(n, c->keys, c->vals, c->sort_scratch, c->st));
-  LAUNCHED(launch_permute(n, c->vals, S, D, c->st));
+  LAUNCHED(sort_particles(n, c->p.key_mode == SPH_KEY_PEANO, S, D, c->bbox_part, c->box4, c->keys, c->vals,
+                          c->sort_scratch, c->st));
   c->cur = 1 - c->cur;
   c->need_sort = false;
   c->tree_ok = c->lists_ok = c->density_ok = false;

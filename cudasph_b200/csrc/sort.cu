@@ -74,16 +74,20 @@ __device__ __forceinline__ void fold_box(int nb, const double *__restrict__ part
 }
 
 // box4 = {lo.x, lo.y, lo.z, scale}; scale = 2^21 / max extent (0 if degenerate)
+__device__ __forceinline__ double4 morton_box(const double *lo, const double *hi) {
+  double size = hi[0] - lo[0];
+  if (hi[1] - lo[1] > size) size = hi[1] - lo[1];
+  if (hi[2] - lo[2] > size) size = hi[2] - lo[2];
+  return make_double4(lo[0], lo[1], lo[2], size > 0 ? __ddiv_rn(2097152.0, size) : 0.0);
+}
+
 __global__ void __launch_bounds__(kBoxThreads) k_bbox_final(int nb, const double *part, double *box4) {
   grid_enter();
   double lo[3], hi[3];
   fold_box(nb, part, lo, hi);
   if (threadIdx.x != 0) return;
-  double size = hi[0] - lo[0];
-  if (hi[1] - lo[1] > size) size = hi[1] - lo[1];
-  if (hi[2] - lo[2] > size) size = hi[2] - lo[2];
-  box4[0] = lo[0]; box4[1] = lo[1]; box4[2] = lo[2];
-  box4[3] = size > 0 ? __ddiv_rn(2097152.0, size) : 0.0;
+  const double4 b = morton_box(lo, hi);
+  box4[0] = b.x; box4[1] = b.y; box4[2] = b.z; box4[3] = b.w;
 }
 
 __device__ __forceinline__ uint64_t spread3(uint32_t v) {
@@ -101,10 +105,33 @@ __device__ __forceinline__ uint32_t quant21(double c, double lo, double scale) {
   return v >= 2097151.0 ? 2097151u : (uint32_t)v;
 }
 
-__global__ void k_morton(int n, const double4 *pos, const double *x, const double *y, const double *z,
-                         const double *box4, uint64_t *keys, uint32_t *vals) {
+// nb > 0: every warp folds the nb <= 32 block partials itself and block 0 keeps
+// the box, which spares small sets a launch of one block; else box4 is read.
+__global__ void k_morton(int n, const double4 *pos, const double *x, const double *y, const double *z, int nb,
+                         const double *part, double *box4, uint64_t *keys, uint32_t *vals) {
   grid_enter();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double4 box;
+  if (nb > 0) {
+    const int l = (int)lane_id();
+    double lo[3], hi[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      lo[d] = l < nb ? part[l * 6 + d] : 1e308;
+      hi[d] = l < nb ? part[l * 6 + 3 + d] : -1e308;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+    box = morton_box(lo, hi);
+    if (i == 0) { box4[0] = box.x; box4[1] = box.y; box4[2] = box.z; box4[3] = box.w; }
+  } else {
+    box = make_double4(box4[0], box4[1], box4[2], box4[3]);
+  }
   if (i >= n) return;
   double c0, c1, c2;
   if (pos) {
@@ -113,8 +140,7 @@ __global__ void k_morton(int n, const double4 *pos, const double *x, const doubl
   } else {
     c0 = x[i]; c1 = y[i]; c2 = z[i];
   }
-  double s = box4[3];
-  uint32_t qx = quant21(c0, box4[0], s), qy = quant21(c1, box4[1], s), qz = quant21(c2, box4[2], s);
+  const uint32_t qx = quant21(c0, box.x, box.w), qy = quant21(c1, box.y, box.w), qz = quant21(c2, box.z, box.w);
   keys[i] = (spread3(qx) << 2) | (spread3(qy) << 1) | spread3(qz);
   if (vals) vals[i] = (uint32_t)i;
 }
@@ -343,25 +369,26 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_radix_pass(int n, int t
 // Small sets: a key's place is the number of keys before it in the stable
 // order, counted directly.  n^2 comparisons are nothing to the whole GPU while
 // eight dependent passes cost some 30 us in one block and 75 in launches
-// (2,049 keys 34 -> 22 us, 6,007 75 -> 46; at 16,384 counting takes 83 us, the
-// passes 75: the comparisons run on the half-rate integer pipe).  Eight
-// lanes share R keys, each counting every eighth key of the tile in shared
-// memory.
-constexpr int kCountTile = 2048, kCountThreads = 256, kCountLanes = 8;
-template <int R>
+// (2,049 keys 34 -> 17 us, 6,007 75 -> 28; a step's sort of 10,000 particles
+// 75 -> 52 and of 12,000 77 -> 66, but of 16,384 76 -> 98: the comparisons run
+// on the half-rate integer pipe).  Sixteen lanes share a key, each counting
+// every sixteenth key of the tile in shared memory (eight: 6,007 particles
+// 32 -> 34 us, and fewer blocks than SMs below 4,700).  MOVE: the values are
+// the keys' indices, and eight of the lanes then move the particle's records
+// to its place (a step's sort, us, as six launches / as three: 2,049 particles
+// 26 / 20, 6,007 50 / 32).
+constexpr int kCountTile = 2048, kCountThreads = 256, kCountLanes = 16;
+template <bool MOVE>
 __global__ void __launch_bounds__(kCountThreads) k_count_sort(int n, const uint64_t *keys, const uint32_t *vals,
-                                                              uint64_t *kout, uint32_t *vout) {
+                                                              uint64_t *kout, uint32_t *vout, Fields src,
+                                                              Fields dst) {
   grid_enter();
   __shared__ uint64_t tile[kCountTile];
+  constexpr int per = kCountThreads / kCountLanes;
   const int t = threadIdx.x, q = t % kCountLanes;
-  const int first = blockIdx.x * (kCountThreads / kCountLanes * R), mine = first + t / kCountLanes * R;
-  uint64_t k[R];
-  unsigned before[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    k[r] = mine + r < n ? keys[mine + r] : 0ull;
-    before[r] = 0u;
-  }
+  const int first = blockIdx.x * per, mine = first + t / kCountLanes;
+  const uint64_t k = mine < n ? keys[mine] : 0ull;
+  unsigned s = 0u;  // keys before this one
   for (int lo = 0; lo < n; lo += kCountTile) {
     const int m = min(n - lo, kCountTile);
     __syncthreads();
@@ -369,34 +396,32 @@ __global__ void __launch_bounds__(kCountThreads) k_count_sort(int n, const uint6
     __syncthreads();
     if (lo + m <= first) {  // every key of the tile precedes the block's: equal ones count
 #pragma unroll 4
-      for (int i = q; i < m; i += kCountLanes) {
-        const uint64_t o = tile[i];
-#pragma unroll
-        for (int r = 0; r < R; r++) before[r] += o <= k[r];
-      }
-    } else if (lo >= first + kCountThreads / kCountLanes * R) {
+      for (int i = q; i < m; i += kCountLanes) s += tile[i] <= k;
+    } else if (lo >= first + per) {
 #pragma unroll 4
-      for (int i = q; i < m; i += kCountLanes) {
-        const uint64_t o = tile[i];
-#pragma unroll
-        for (int r = 0; r < R; r++) before[r] += o < k[r];
-      }
+      for (int i = q; i < m; i += kCountLanes) s += tile[i] < k;
     } else {
       for (int i = q; i < m; i += kCountLanes) {
         const uint64_t o = tile[i];
-#pragma unroll
-        for (int r = 0; r < R; r++) before[r] += o < k[r] || (o == k[r] && lo + i < mine + r);
+        s += o < k || (o == k && lo + i < mine);
       }
     }
   }
 #pragma unroll
-  for (int r = 0; r < R; r++) {
+  for (int o = kCountLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (mine >= n) return;
+  if (q == 0) {
+    kout[s] = k;
+    vout[s] = MOVE ? (uint32_t)mine : vals[mine];
+  }
+  if (MOVE) {
+    const double4 *from[6] = {src.pos, src.vel, src.hyd, src.dd, src.dots, src.grav};
+    double4 *to[6] = {dst.pos, dst.vel, dst.hyd, dst.dd, dst.dots, dst.grav};
 #pragma unroll
-    for (int o = kCountLanes / 2; o > 0; o >>= 1) before[r] += __shfl_xor_sync(0xffffffffu, before[r], o);
-    if (q == 0 && mine + r < n) {
-      kout[before[r]] = k[r];
-      vout[before[r]] = vals[mine + r];
-    }
+    for (int c = 0; c < 6; c++)
+      if (q == c) to[c][s] = from[c][mine];
+    if (q == 6) dst.vsig[s] = src.vsig[mine];
+    if (q == 7) dst.id[s] = src.id[mine];
   }
 }
 
@@ -407,6 +432,12 @@ __global__ void k_sorted_back(int n, const uint64_t *kin, const uint32_t *vin, u
   keys[i] = kin[i];
   vals[i] = vin[i];
 }
+
+int morton_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
+                double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st);
+int peano_keys(int n, const double4 *pos, const double *x, const double *y, const double *z, double *part,
+               double *box4, uint64_t *keys, uint32_t *vals, cudaStream_t st);
+int launch_permute(int n, const uint32_t *order, const Fields &src, const Fields &dst, cudaStream_t st);
 
 constexpr size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 
@@ -451,25 +482,49 @@ static int radix_passes(int n, uint64_t *keys, uint32_t *vals, char *p, cudaStre
 }
 
 // Stable sort of (keys, vals); result in keys/vals.  Returns launches.
-// Direct counting up to kCountMax keys, one key per lane group while that
-// leaves too few blocks.  Then the radix passes: small tiles while the direct
+// Direct counting up to kCountMax keys.  Then the radix passes: small tiles while the direct
 // sum of the counts reaches (16,384 keys: small / large 73 / 101 us; 262,144
 // 104 / 116), and large ones, which halve the counts to add up (1,048,576:
 // 214 / 183).
-constexpr int kCountMax = 8192;
+constexpr int kCountMax = 12288;
+static char *aligned_scratch(void *scratch) { return (char *)(((uintptr_t)scratch + 15) / 16 * 16); }
+
+template <bool MOVE>
+static void count_sort(int n, const uint64_t *keys, const uint32_t *vals, uint64_t *kout, uint32_t *vout,
+                       const Fields &src, const Fields &dst, cudaStream_t st) {
+  const int per = kCountThreads / kCountLanes;
+  launch(k_count_sort<MOVE>, (n + per - 1) / per, kCountThreads, st, n, keys, vals, kout, vout, src, dst);
+}
+
 int radix_sort_u64(int n, uint64_t *keys, uint32_t *vals, void *scratch, cudaStream_t st) {
   if (n <= 1) return 0;
-  char *p = (char *)(((uintptr_t)scratch + 15) / 16 * 16);  // the tables are read 16 bytes at a time
+  char *p = aligned_scratch(scratch);  // the tables are read 16 bytes at a time
   if (n <= kCountMax) {
     uint64_t *k2 = (uint64_t *)p;
     uint32_t *v2 = (uint32_t *)(p + round256((size_t)n * 8));
-    const int r = n <= 4096 ? 1 : 4, per = kCountThreads / kCountLanes * r;
-    launch(r == 1 ? k_count_sort<1> : k_count_sort<4>, (n + per - 1) / per, kCountThreads, st, n, keys, vals, k2, v2);
+    count_sort<false>(n, keys, vals, k2, v2, Fields{}, Fields{}, st);
     launch(k_sorted_back, (n + 255) / 256, 256, st, n, k2, v2, keys, vals);
     return 2;
   }
   return n <= kDirectTiles * kTileSmall ? radix_passes<256>(n, keys, vals, p, st)
                                         : radix_passes<512>(n, keys, vals, p, st);
+}
+
+// The step's sort of the particles themselves: keys of src.pos, sorted keys
+// and the permutation in keys / order, the records of src moved to dst.
+int sort_particles(int n, bool peano, const Fields &src, const Fields &dst, double *part, double *box4, uint64_t *keys,
+                   uint32_t *order, void *scratch, cudaStream_t st) {
+  const bool count = n <= kCountMax;
+  uint64_t *raw = count ? (uint64_t *)aligned_scratch(scratch) : keys;
+  uint32_t *vals = count ? nullptr : order;
+  int launches = peano ? peano_keys(n, src.pos, nullptr, nullptr, nullptr, part, box4, raw, vals, st)
+                       : morton_keys(n, src.pos, nullptr, nullptr, nullptr, part, box4, raw, vals, st);
+  if (count) {
+    count_sort<true>(n, raw, nullptr, keys, order, src, dst, st);
+    return launches + 1;
+  }
+  launches += radix_sort_u64(n, keys, order, scratch, st);
+  return launches + launch_permute(n, order, src, dst, st);
 }
 
 // bounding box + Morton keys of positions (double4 records or separate x/y/z)
@@ -479,9 +534,9 @@ int morton_keys(int n, const double4 *pos, const double *x, const double *y, con
   if (nb * 256 > n) nb = (n + 255) / 256;
   if (nb < 1) nb = 1;
   launch(k_bbox_partial, nb, 256, st, n, pos, x, y, z, part);
-  launch(k_bbox_final, 1, kBoxThreads, st, nb, part, box4);
-  launch(k_morton, (n + 255) / 256, 256, st, n, pos, x, y, z, box4, keys, vals);
-  return 3;
+  if (nb > 32) launch(k_bbox_final, 1, kBoxThreads, st, nb, part, box4);
+  launch(k_morton, (n + 255) / 256, 256, st, n, pos, x, y, z, nb > 32 ? 0 : nb, part, box4, keys, vals);
+  return nb > 32 ? 3 : 2;
 }
 
 // ---------------------------------------------------------------------------

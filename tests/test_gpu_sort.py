@@ -6,7 +6,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 31, 255, 2047, 2048, 2049, 4095, 4096, 4097, 6144, 8191, 8192, 8193, 10241,
+SIZES = [1, 2, 31, 255, 2047, 2048, 2049, 4095, 4096, 4097, 6144, 8191, 8192, 8193, 12287, 12288, 12289,
          524287, 524288, 524289, 1048576, 1048577, 1300001]
 
 
@@ -35,3 +35,25 @@ def test_radix_sort_is_the_stable_order(n, kind):
     check(lib().cudasph_radix_sort_u64(n, dk.data_ptr(), dv.data_ptr(), scratch.data_ptr(), s))
     assert np.array_equal(dk.cpu().numpy().view(np.uint64), k[order])
     assert np.array_equal(dv.cpu().numpy(), order)
+
+
+@pytest.mark.parametrize("key_mode", [0, 1])
+@pytest.mark.parametrize("n", [1, 33, 2049, 8193, 12288, 12289])
+def test_sort_moves_every_record(n, key_mode):
+    """A step's sort: the order is the stable sort of the oracle's keys (some
+    particles coincide), and every field still belongs to its particle."""
+    from cudasph_b200.simulation import FIELDS, Simulation, make_params
+    from oracle import oracle as O
+    rs = np.random.default_rng(n)
+    ic = {k: rs.normal(size=n) for k in FIELDS}
+    ic["m"] = np.full(n, 1.0 / n)
+    ic["range"] = rs.uniform(0.1, 0.2, n)
+    for k in ("x", "y", "z"):
+        ic[k][1::5] = ic[k][0::5][: ic[k][1::5].size]
+    sim = Simulation(ic, make_params(key_mode=key_mode))
+    sim.sort_bodies()
+    keys = (O.peano_keys if key_mode else O.morton_keys)(ic["x"], ic["y"], ic["z"])[0]
+    np.testing.assert_array_equal(sim.order(), np.argsort(keys, kind="stable"))
+    got = sim.get_state()
+    for k in FIELDS:
+        np.testing.assert_array_equal(got[k], ic[k], err_msg=k)
