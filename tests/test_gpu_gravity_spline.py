@@ -59,3 +59,23 @@ def test_spline_gravity_equal_mass_step(n):
     ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
     assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1025, 4096, 9001])
+def test_spline_gravity_separated_clumps(n):
+    """Tiles that hold no near pair beside tiles that do, and a few particles
+    whose range reaches across: the batches with and without the per-pair test."""
+    import torch
+    from cudasph_b200._capi import lib
+    rs = np.random.default_rng(n + 1)
+    p = np.concatenate([rs.normal(size=(n - n // 2, 3)) * 0.1, rs.normal(size=(n // 2, 3)) * 0.1 + 4.0])
+    m, r = rs.uniform(0.5, 1.5, n) / n, np.full(n, 0.02)
+    r[rs.integers(0, n, 5)] = 5.0
+    src = torch.from_numpy(np.column_stack([p, m]).copy()).cuda()
+    tr = torch.from_numpy(r.copy()).cuda()
+    out = torch.empty((n, 4), dtype=torch.float64, device="cuda")
+    assert lib().cudasph_gravity_direct(n, src.data_ptr(), tr.data_ptr(), out.data_ptr(), 0, 0.0, 1.0, 0,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+    got = out.cpu().numpy()
+    ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
