@@ -362,8 +362,10 @@ __device__ __forceinline__ void adj_sym_f32_item(long long item, int n, int nt, 
   int b, t_lo, t_hi;
   sym_item(item, nt, b, t_lo, t_hi);
   int j_lo = t_lo * kAdjTile, j_hi = min(t_hi * kAdjTile, n);
-  source_slice<32>(j_lo, j_hi, slice, slices);
-  if (j_lo >= j_hi) return;
+  if (slices > 1) {  // kept apart: the whole item's loop is scheduled better for it (N = 1M: 501 -> 489 ms)
+    source_slice<32>(j_lo, j_hi, slice, slices);
+    if (j_lo >= j_hi) return;
+  }
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nxt = (l + 1) & 31;
   const int i0 = b * kAdjTile;
   const double4 anc = src[i0];
