@@ -766,7 +766,7 @@ static int step_body(sph_ctx *c);
 
 // One step, replayed from a captured CUDA graph when the step is the steady
 // kind (sorted every step, no profiling events, no adjoint bookkeeping): the
-// ~45 launches of a step then cost one graph launch.  The first step of each
+// 20 to 35 launches of a step then cost one graph launch.  The first step of each
 // buffer parity runs under stream capture; the host bookkeeping it performs
 // (buffer flip, phase validity) is then repeated by hand on every replay.
 extern "C" int cudasph_step(sph_ctx *c) {

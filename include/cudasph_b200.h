@@ -170,7 +170,7 @@ int cudasph_step(sph_ctx *ctx);              /* the whole step */
  * re-sort when due (every sort_every steps, or after positions were set) */
 int cudasph_begin_step(sph_ctx *ctx);
 /* Replay steady steps (sorted every step, profiling and keep off) from a
- * captured CUDA graph: one graph launch per step instead of ~45 launches.
+ * captured CUDA graph: one graph launch per step instead of 20 to 35 launches.
  * Changing parameters drops the captured graphs. */
 int cudasph_set_graph(sph_ctx *ctx, int on);
 int cudasph_steps(sph_ctx *ctx, int k);      /* k whole steps */
