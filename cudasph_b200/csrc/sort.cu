@@ -1,13 +1,13 @@
-// sort.cu -- Morton keys and a stable LSD radix sort (the space-filling-curve
+// sort.cu -- Morton keys and a stable sort (the space-filling-curve
 // sort of sort_bodies.cpp:119-186, done on the device every step), and the
 // reference's Peano-Hilbert keys as an optional sort key.
 //
 // Keys: positions quantised to 21 bits per dimension in the bounding cube
 // (scale = 2^21 / max extent, like domain_fac of sort_bodies.cpp:135), bits
-// interleaved x-y-z from the top.  The sort is an 8-bit-digit LSD radix sort
-// (8 passes over 64-bit keys), one launch per pass, described below.  Ties
-// keep their input order, so with values = slot indices the permutation
-// equals a stable sort.
+// interleaved x-y-z from the top.  Up to 12,288 keys are placed by direct
+// counting, more by an 8-bit-digit LSD radix sort (8 passes over 64-bit keys,
+// one launch per pass); both are described below.  Ties keep their input
+// order, so with values = slot indices the permutation equals a stable sort.
 #include <cstdio>
 
 #include "common.cuh"
