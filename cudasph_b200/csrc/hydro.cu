@@ -338,9 +338,10 @@ int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const doubl
 }
 
 int launch_hydro(const HydroArgs &a, cudaStream_t st) {
-  if (a.leaf1 <= a.leaf0) return 0;
-  // every particle's factors: a shard's pairs reach outside its own leaves
+  // every particle's factors: a shard's pairs reach outside its own leaves, and
+  // a shard without leaves still clears the sums that the shards add up
   int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, a.dots, st);
+  if (a.leaf1 <= a.leaf0) return launches;
   const int n = (a.leaf1 - a.leaf0) * kLeaf;
   if (n < kSmallSet) launch(k_hydro<kSubSmall>, (n * kSubSmall + 127) / 128, 128, st, a);
   else launch(k_hydro<kSubHydro>, (n * kSubHydro + 127) / 128, 128, st, a);

@@ -220,9 +220,10 @@ int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const doubl
                       double gamma, double4 *aux, double4 *dots, cudaStream_t st);
 
 int launch_hydro_mixed(const HydroArgs &a, cudaStream_t st) {
-  if (a.leaf1 <= a.leaf0) return 0;
-  // every particle's factors {c, P / rho^2, B, 1 / m}: a shard's pairs reach outside its own leaves
+  // every particle's factors {c, P / rho^2, B, 1 / m}: a shard's pairs reach outside its own leaves, and
+  // a shard without leaves still clears the sums that the shards add up
   int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, a.dots, st);
+  if (a.leaf1 <= a.leaf0) return launches;
   launch(k_hydro_mixed, ((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, st, a);
   return launches + 1;
 }

@@ -91,6 +91,30 @@ def test_lockstep_shards_equal_unsharded_step(world, precision, soft, equal, gra
     ref.close()
 
 
+@pytest.mark.parametrize("n,world", [(100, 8), (33, 3)])
+@pytest.mark.parametrize("precision,mixed_sph,grav", [(0, 0, 0), (1, 3, 0), (1, 0, 1)])
+def test_shards_without_leaves_add_nothing(n, world, precision, mixed_sph, grav):
+    """More shards than leaves of 32 particles: a shard without leaves must
+    hand in zero accelerations, not those of the step before."""
+    from cudasph_b200.sharded import ShardedSimulation
+    from cudasph_b200.simulation import Simulation, make_params
+    ic = _ic(n=n)
+    par = dict(precision=precision, mixed_sph=mixed_sph, n_target=20.0, eos_mode=1, soft_mode=1, eps=0.01,
+               grav_mode=grav)
+    ref = Simulation(ic, make_params(**par))
+    shards = [ShardedSimulation(ic, make_params(**par), r, world) for r in range(world)]
+    for _ in range(3):
+        ref.step()
+        _lockstep(shards, 1)
+    assert any(a == b for a, b in (s.leaves() for s in shards))
+    for s in shards:
+        assert np.array_equal(s.n_ngb(), ref.n_ngb())
+        for k in FIELDS:
+            assert _rel(s.get(k), ref.get(k)) < 1e-9, k
+        s.close()
+    ref.close()
+
+
 def test_sharded_context_refuses_whole_step_and_adjoint():
     from cudasph_b200._capi import SphError
     from cudasph_b200.sharded import ShardedSimulation
