@@ -522,7 +522,7 @@ template <class Smem>
 __device__ __forceinline__ Rough rough_sums(const SolveArgs &a, Smem &sm, const double4 &p, double w) {
   const int lane = (int)lane_id();
   const Query q = make_ball(p.x, p.y, p.z, w * kWiden);
-  const float i2w = (float)(2.0 / w);
+  const float i2w = (float)(2.0 / w);  // a normal number, see clamped_for_sure
   Walk walk;
   walk.start(a.t, sm);
   double sf = 0, sg = 0, n = 0;
@@ -535,7 +535,9 @@ __device__ __forceinline__ Rough rough_sums(const SolveArgs &a, Smem &sm, const 
       const int j = (first + 4 * g) * kCell + lane;
       if (j >= a.t.n) continue;
       const float4 o = ldg(a.t.pf + j);
-      const float u = sqrtf(dist2(o.x - q.lo[0], o.y - q.lo[1], o.z - q.lo[2])) * i2w;
+      // scaled before it is squared: whatever the unit of length, what is too
+      // large for FP32 is then past u = 2 and what is too small is u = 0
+      const float u = sqrtf(dist2((o.x - q.lo[0]) * i2w, (o.y - q.lo[1]) * i2w, (o.z - q.lo[2]) * i2w));
       lf += k_ig<float>(u);
       lg -= k_digdh<float>(u);
     }
@@ -558,11 +560,12 @@ __device__ __forceinline__ Rough rough_sums(const SolveArgs &a, Smem &sm, const 
 // Whether those sums take the iteration the same way as the exact ones: in
 // the bracket phase a step clamped to f_scale w depends on the signs of f and
 // f' only, so it is certain when both, and |f / f'| > f_scale w, hold by more
-// than the sums' error.
+// than the sums' error.  A range near the ends of the FP32 exponents is left to
+// the exact sums.
 __device__ __forceinline__ bool clamped_for_sure(const RangeIter &it, const Rough &r, const SolveArgs &a) {
   const double f = fabs(r.sf - a.n_target), g = fabs(r.sg);
-  return (it.phase == kBr0 || it.phase == kBr1) && a.rel_err <= a.f_scale && f > r.err && g > r.err &&
-         f - r.err > a.f_scale * (g + r.err);
+  return (it.phase == kBr0 || it.phase == kBr1) && a.rel_err <= a.f_scale && it.w > 1e-30 && it.w < 1e30 &&
+         f > r.err && g > r.err && f - r.err > a.f_scale * (g + r.err);
 }
 
 // dev_solve_range (dev_solve_range.cu:137-189): per particle, bracket the

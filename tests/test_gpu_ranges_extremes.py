@@ -1,0 +1,37 @@
+"""The smoothing-length solve at the ends of what it accepts: units of length
+whose squares leave FP32, starting ranges of every size, parameters at the edge.
+
+Lengths multiplied by a power of two give the same solve bit for bit (every
+FP64 operation of it scales exactly), so the ranges must be equal after
+division and the evaluation counts and lists must be the same."""
+import numpy as np
+import pytest
+
+from cudasph_b200 import ics
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(ic, scale=1.0, wide=1.0, **kw):
+    from cudasph_b200.simulation import Simulation, make_params
+    ic = dict(ic)
+    for k in "xyz":
+        ic[k] = np.asarray(ic[k]) * scale
+    ic["range"] = np.asarray(ic["range"]) * (scale * wide)
+    with Simulation(ic, make_params(**dict(dict(n_target=50.0, eos_mode=0, soft_mode=1, eps=0.01), **kw))) as sim:
+        sim.sort_bodies()
+        order = sim.order()
+        sim.CUDA_solve_range()
+        cnt, _, lst = sim.neighbours()
+        return sim.get("range") / scale, sim.solve_evals(), cnt, lst, order
+
+
+@pytest.mark.parametrize("wide", [3.0, 6.0])
+@pytest.mark.parametrize("log2", [64, 66, 68, -66])
+def test_solve_from_wide_ranges_in_any_unit(log2, wide):
+    """ranges far too large, whose sums are first taken in FP32"""
+    ic = ics.polytrope(8200, n_ngb=50, seed=8200)
+    a, b = _solve(ic, 1.0, wide), _solve(ic, 2.0 ** log2, wide)
+    assert np.array_equal(a[0], b[0])
+    assert np.array_equal(a[1], b[1])
+    assert np.array_equal(a[2], b[2])
