@@ -692,11 +692,12 @@ struct Group {
 #pragma unroll
       for (int t = 0; t < G; t++) m[t] = 0u;
       const int chunks = min(32, (nlist - r * 128 + 3) >> 2);
-      // lane's candidate of chunk c; past the last: infinitely far from every target
+      // lane's candidate of chunk c; past the last: not a number, so that it is
+      // in no ball (a squared range may be infinite in FP32)
       auto candidate = [&](int c) {
         const int k = r * 128 + c * 4 + (lane >> 3);
         const int j = k < nlist ? sm.list[k] * kCell + (lane & 7) : 0x7fffffff;
-        return j < a.t.n ? ldg(a.t.pf + j) : make_float4(INFINITY, 0.f, 0.f, 0.f);
+        return j < a.t.n ? ldg(a.t.pf + j) : make_float4(NAN, 0.f, 0.f, 0.f);
       };
       for (int c = 0; c < chunks; c++) {
         const float4 o = candidate(c);

@@ -35,3 +35,18 @@ def test_solve_from_wide_ranges_in_any_unit(log2, wide):
     assert np.array_equal(a[0], b[0])
     assert np.array_equal(a[1], b[1])
     assert np.array_equal(a[2], b[2])
+
+
+def _cloud(n):
+    rs = np.random.default_rng(n)
+    x, y, z = rs.uniform(-1, 1, (3, n))
+    return {"x": x, "y": y, "z": z, "range": np.full(n, 0.4), "m": np.full(n, 1.0 / n), "u": np.ones(n),
+            "mu": np.full(n, 0.6)}
+
+
+@pytest.mark.parametrize("n", [1, 5, 100, 1001, 2045])
+def test_ranges_whose_square_is_infinite_in_fp32(n):
+    """sets that fit one list of cells, with a part-filled last cell and chunk"""
+    a, b = _solve(_cloud(n)), _solve(_cloud(n), 2.0 ** 70)
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
