@@ -139,6 +139,11 @@ inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, cudaStre
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
+// FP32 copies of coordinates for the tree and its queries.  Beyond 1e38 they
+// are moved to it: that only brings points closer, and no difference is
+// infinite or undefined.
+__device__ __forceinline__ float held_f32(float v) { return fminf(fmaxf(v, -1e38f), 1e38f); }
+
 __device__ __forceinline__ double4 ld4(const double4 *p) {
   // one 32-byte read-only load (sm_100's 256-bit vector load) of one
   // 32-byte-aligned record; against two 16-byte loads it halves the load

@@ -88,9 +88,9 @@ struct WarpSmem {
 // when lo = hi).  Centres are rounded to float and the squared radius widened
 // to cover every rounding of the float tests (the rounding of the centre and
 // of a candidate's or box's coordinates, the subtractions, squares and sums:
-// under 4e-7 (|x| + |y| + |z|) absolute and 1e-6 relative), so a j with
-// |x_j - x| < r, and a box that holds one, always passes.  Whatever else
-// passes is decided by the exact predicate.
+// under 4e-7 (|x| + |y| + |z|) absolute and 1e-6 relative, and 1e-44 where the
+// squares are denormal), so a j with |x_j - x| < r, and a box that holds one,
+// always passes.  Whatever else passes is decided by the exact predicate.
 struct Query {
   float lo[3], hi[3], r2;
 };
@@ -98,10 +98,10 @@ struct Query {
 __device__ __forceinline__ Query make_ball(double x, double y, double z, double r) {
   const double rr = r * (1.0 + 1e-6) + 4e-7 * (fabs(x) + fabs(y) + fabs(z));
   Query q;
-  q.lo[0] = q.hi[0] = (float)x;
-  q.lo[1] = q.hi[1] = (float)y;
-  q.lo[2] = q.hi[2] = (float)z;
-  q.r2 = __double2float_ru(rr * rr);
+  q.lo[0] = q.hi[0] = held_f32((float)x);
+  q.lo[1] = q.hi[1] = held_f32((float)y);
+  q.lo[2] = q.hi[2] = held_f32((float)z);
+  q.r2 = __double2float_ru(rr * rr + 1e-44);
   return q;
 }
 

@@ -26,11 +26,13 @@ __global__ void __launch_bounds__(kCell * kFan) k_cell_boxes(int n, const double
   if (s < n) {
     const double4 p = pos[s];
     l0 = h0 = p.x; l1 = h1 = p.y; l2 = h2 = p.z;
-    pf[s] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
+    pf[s] = make_float4(held_f32((float)p.x), held_f32((float)p.y), held_f32((float)p.z), 0.f);
   }
   // rounding is monotone: the rounded extrema are the extrema of the rounded
-  float4 l = make_float4(__double2float_rd(l0), __double2float_rd(l1), __double2float_rd(l2), 0.f);
-  float4 h = make_float4(__double2float_ru(h0), __double2float_ru(h1), __double2float_ru(h2), 0.f);
+  float4 l = make_float4(held_f32(__double2float_rd(l0)), held_f32(__double2float_rd(l1)),
+                         held_f32(__double2float_rd(l2)), 0.f);
+  float4 h = make_float4(held_f32(__double2float_ru(h0)), held_f32(__double2float_ru(h1)),
+                         held_f32(__double2float_ru(h2)), 0.f);
   auto merge = [&](int o) {
     l.x = fminf(l.x, __shfl_xor_sync(0xffffffffu, l.x, o));
     l.y = fminf(l.y, __shfl_xor_sync(0xffffffffu, l.y, o));

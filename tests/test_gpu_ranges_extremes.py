@@ -50,3 +50,14 @@ def test_ranges_whose_square_is_infinite_in_fp32(n):
     a, b = _solve(_cloud(n)), _solve(_cloud(n), 2.0 ** 70)
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("log2", [130, 128, -68, -72, -130])
+@pytest.mark.parametrize("n", [1001, 9000])
+def test_lengths_at_the_ends_of_fp32(n, log2):
+    """coordinates beyond FP32 and ranges whose squares are denormal in it"""
+    ic = _cloud(n)
+    ic["range"] = np.full(n, 0.4 * (1001 / n) ** (1 / 3))
+    a, b = _solve(ic), _solve(ic, 2.0 ** log2)
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
