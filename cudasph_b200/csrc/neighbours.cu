@@ -458,7 +458,9 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
   Eval e;
   e.count = 0;
   e.sliver = false;
-  const double iw = 1.0 / w;
+  // an infinite range, which a caller may start from, stands at the largest
+  // number: the quotients are 0 as they are for infinity
+  const double wd = fmin(w, 1.7976931348623157e308), iw = 1.0 / wd;
   double acc = 0, dmax = -1.0;
   int nb = 0, j;
   const Query q = make_ball(p.x, p.y, p.z, w * kWiden);
@@ -470,7 +472,7 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
       e.many = true;
       break;
     }
-    double d2 = 1e300;
+    double d2 = NAN;  // no candidate: inside no range, not even an infinite one
     if (j >= 0) {
       const double4 o = ld4(a.pos + j);
       d2 = ds2_exact(p.x - o.x, p.y - o.y, p.z - o.z);
@@ -486,7 +488,7 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
       e.sliver |= !hit && d2 < r2 * (1.0 + 0x1p-40);
       double tf = 0, tg = 0;
       if (hit) {
-        count_terms(div_by(2 * sqrt(d2), w, iw), tf, tg);
+        count_terms(div_by(2 * sqrt(d2), wd, iw), tf, tg);
         dmax = fmax(dmax, d2);
       }
       reinterpret_cast<double2 *>(sm.term)[lane] = make_double2(tf, -tg);

@@ -61,3 +61,18 @@ def test_lengths_at_the_ends_of_fp32(n, log2):
     a, b = _solve(ic), _solve(ic, 2.0 ** log2)
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [100, 3000])
+def test_infinite_starting_range(n):
+    """Every particle is inside and all weights are those of u = 0: the bracket
+    runs to its last iteration without a root and the range stays infinite."""
+    ic = _cloud(n)
+    ic["range"] = np.full(n, 0.4 * (1001 / n) ** (1 / 3))
+    a = _solve(ic)
+    ic["range"][5] = np.inf
+    b = _solve(ic)
+    assert b[0][5] == np.inf and b[2][5] == n and b[1][5] == 21
+    others = np.arange(n) != 5
+    for k in range(3):
+        assert np.array_equal(a[k][others], b[k][others])
