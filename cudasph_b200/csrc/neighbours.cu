@@ -463,7 +463,7 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
   const double wd = fmin(w, 1.7976931348623157e308), iw = 1.0 / wd;
   double acc = 0, dmax = -1.0;
   int nb = 0, j;
-  const Query q = make_ball(p.x, p.y, p.z, w * kWiden);
+  const Query q = make_ball(p.x, p.y, p.z, fabs(w) * kWiden);
   Source src;
   src.start(a.t, sm, nlist, total);
   e.many = false;
@@ -589,6 +589,10 @@ __device__ __forceinline__ bool clamped_for_sure(const RangeIter &it, const Roug
 // of 22 for 2,000,003 particles from estimated ranges).
 // One round for target t: evaluations as long as the group's candidates reach
 // (sm.bound, sm.w_list).  True when done.
+// A step of more than the range itself (f_scale > 1) goes through negative
+// ranges, whose square is what counts: they reach as far as their magnitude.
+// Every round evaluates each of its targets at least once, so the number of
+// iterations bounds the rounds.
 // FIRST: the round that is the last one for nearly every particle of a running
 // simulation; a range that is far too large is left to the next.
 template <bool FIRST, class Smem>
@@ -600,8 +604,8 @@ __device__ __forceinline__ bool solve_round(const SolveArgs &a, Smem &sm, int s,
   bool exact = false;
   while (it.phase != kDone) {
     const double w_eval = it.w;
-    if (w_eval > sm.bound) return false;
-    const Eval e = eval_range<true>(a, sm, s, p, w_eval, w_eval <= sm.w_list ? sm.nlist : -1, total, exact);
+    if (fabs(w_eval) > sm.bound) return false;
+    const Eval e = eval_range<true>(a, sm, s, p, w_eval, fabs(w_eval) <= sm.w_list ? sm.nlist : -1, total, exact);
     if (FIRST && e.many) return false;
     if (!FIRST && e.many) {
       Rough r = rough_sums(a, sm, p, w_eval);
@@ -631,7 +635,9 @@ __device__ __forceinline__ bool solve_round(const SolveArgs &a, Smem &sm, int s,
   }
   const double w = it.w;
   if (!listed)
-    count = eval_range<false>(a, sm, s, p, w, w <= sm.w_list ? sm.nlist : -1, w <= sm.bound ? total : -1, false).count;
+    count = eval_range<false>(a, sm, s, p, w, fabs(w) <= sm.w_list ? sm.nlist : -1, fabs(w) <= sm.bound ? total : -1,
+                              false).count;
+  if (!(w > 0)) count = 0;  // stored as no range
   if (lane_id() == 0) {
     if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
     a.pos[s].w = (w > 0) ? w : 0.0;
@@ -658,7 +664,7 @@ struct Group {
     // lanes whose target has no part in this repeat the first that has
     const int tt = (todo >> t0) & 1u ? t0 : __ffs(todo) - 1;
     double4 p = a.pos[first + tt];
-    if (SAVED) p.w = a.save[first + tt].w;
+    if (SAVED) p.w = fabs(a.save[first + tt].w);
     if (!(p.w > 0)) p.w = 0;
     Query mine = make_ball(p.x, p.y, p.z, p.w * slack * kWiden);
     Query q = mine;
@@ -722,7 +728,7 @@ struct Group {
     __syncwarp();  // the previous target's codes are read
     if (lane == 0) {
       sm.it = it;
-      sm.bound = it.w * slack;
+      sm.bound = fabs(it.w) * slack;
     }
     __syncwarp();
     if (nlist < 0) return -1;

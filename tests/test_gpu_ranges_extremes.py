@@ -76,3 +76,18 @@ def test_infinite_starting_range(n):
     others = np.arange(n) != 5
     for k in range(3):
         assert np.array_equal(a[k][others], b[k][others])
+
+
+@pytest.mark.parametrize("f_scale", [1.0, 1.5, 3.0])
+@pytest.mark.parametrize("wide", [0.3, 1.0, 5.0, 6.0])
+def test_steps_larger_than_the_range(f_scale, wide):
+    """Newton steps clamped to more than the range pass through negative ranges
+    (about a third of the particles at five times the range, where ig is flat)."""
+    from oracle import oracle as O
+    ic = _cloud(2000)
+    r, ev, cnt, _, order = _solve(ic, 1.0, wide, f_scale=f_scale)
+    assert np.all(cnt[r == 0] == 0)
+    x, y, z = (ic[k][order] for k in "xyz")
+    r_o, _, ev_o = O.solve_range(x, y, z, wide * ic["range"][order], O.make_params(n_target=50.0, f_scale=f_scale))
+    assert np.mean(r[order] == np.where(r_o > 0, r_o, 0.0)) >= 0.999  # a negative or undefined end is stored as 0
+    assert np.mean(ev[order] == ev_o) >= 0.999
