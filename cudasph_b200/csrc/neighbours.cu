@@ -64,6 +64,17 @@ struct RangeIter {
   int phase, iter, keep, nev;
 };
 
+// A query: everything within r of a point, or of the box [lo, hi] of several.
+// Both tests are in FP32 and let through whatever is within r; what else
+// passes is decided by the exact predicate.  Boxes are tested against r2: r
+// widened by 1e-6 for the subtractions, squares and sums; the centre's rounding
+// is in the boxes (tree.cu).  Particles are tested against c2, which also
+// covers the rounding of the centre's and the particle's coordinates (under
+// 4e-7 (|x| + |y| + |z|)).  1e-44 is for squares that are denormal.
+struct Query {
+  float lo[3], hi[3], r2, c2;
+};
+
 // shared memory of one warp
 template <int G>
 struct WarpSmem {
@@ -75,6 +86,7 @@ struct WarpSmem {
   int nlist;                          // cells in the list, -1: too many
   int list[kCells];                   // cells that may meet a ball of the group, ascending
   unsigned hits[G][kRounds][32];      // per target: candidates of each chunk of the list inside its ball
+  Query q;                            // the target's, when it walks by itself
   union {
     unsigned short code[kStage];      // the target's candidates from the list: 8 * list index + particle
     struct {
@@ -84,26 +96,23 @@ struct WarpSmem {
   };
 };
 
-// A query: everything within sqrt(r2) of the box [lo, hi] (a target's ball
-// when lo = hi).  Centres are rounded to float and the squared radius widened
-// to cover every rounding of the float tests (the rounding of the centre and
-// of a candidate's or box's coordinates, the subtractions, squares and sums:
-// under 4e-7 (|x| + |y| + |z|) absolute and 1e-6 relative, and 1e-44 where the
-// squares are denormal), so a j with |x_j - x| < r, and a box that holds one,
-// always passes.  Whatever else passes is decided by the exact predicate.
-struct Query {
-  float lo[3], hi[3], r2;
-};
-
 __device__ __forceinline__ Query make_ball(double x, double y, double z, double r) {
-  const double rr = r * (1.0 + 1e-6) + 4e-7 * (fabs(x) + fabs(y) + fabs(z));
+  const double rb = r * (1.0 + 1e-6), rc = rb + 4e-7 * (fabs(x) + fabs(y) + fabs(z));
   Query q;
   q.lo[0] = q.hi[0] = held_f32((float)x);
   q.lo[1] = q.hi[1] = held_f32((float)y);
   q.lo[2] = q.hi[2] = held_f32((float)z);
-  q.r2 = __double2float_ru(rr * rr + 1e-44);
+  q.r2 = __double2float_ru(rb * rb + 1e-44);
+  q.c2 = __double2float_ru(rc * rc + 1e-44);
   return q;
 }
+
+// Whether the rounding of the coordinates makes the particles' test useless
+// (ranges below about 2e-6 of the distance from the origin).  They are then
+// compared by differences taken in FP64 (100,000 particles of a star 1e5 and
+// 1e6 of its radii from the origin, steady solve, ms, with the rounded
+// coordinates / so: 3.41 / 0.42 and 50.0 / 0.69; at the origin 0.38).
+__device__ __forceinline__ bool far_out(const Query &q) { return q.c2 > 1.5f * q.r2; }
 
 __device__ __forceinline__ float dist2(float dx, float dy, float dz) { return fmaf(dz, dz, fmaf(dy, dy, dx * dx)); }
 
@@ -209,41 +218,49 @@ __device__ __forceinline__ int list_cells(const TreeView &t, Smem &sm, const Que
 }
 
 // Candidates of one target, ascending, up to 32 at a time (lane k holds
-// candidate k, -1 past the last): a superset of what its ball q holds.
-// Either the codes that the group's pass over its cell list left (total >=
-// 0), or a visit of the cells that meet the ball, taken from the group's list
-// (nlist >= 0, which must cover q) or from a walk of the tree: they queue up
+// candidate k, -1 past the last): a superset of what its ball holds.  Either
+// the `total` codes that the group's pass over its cell list left ...
+struct Coded {
+  int total, at;
+
+  template <class Smem>
+  __device__ __forceinline__ bool next(const TreeView &, Smem &sm, const double4 *, const double4 &, int &j) {
+    if (at >= total) return false;
+    const int k = at + (int)lane_id();
+    j = -1;
+    if (k < total) {
+      const int code = sm.code[k];
+      j = sm.list[code >> 3] * kCell + (code & 7);
+    }
+    at += 32;
+    return true;
+  }
+};
+
+// ... or a visit of the cells that meet the ball, taken from the group's list
+// (nlist >= 0, which must cover it) or from a walk of the tree: they queue up
 // until eight are at hand, then lanes 8c .. 8c + 7 load the particles of cell
 // c, four cells per load and two loads in flight.
-struct Source {
+struct Visited {
   Walk walk;
-  int nlist, total, at, staged;
+  int nlist, at, staged;
   unsigned head, tail;
 
   template <class Smem>
-  __device__ __forceinline__ void start(const TreeView &t, Smem &sm, int nlist_, int total_) {
+  __device__ __forceinline__ void start(const TreeView &t, Smem &sm, int nlist_, const double4 &p, double w) {
     nlist = nlist_;
-    total = total_;
     at = staged = 0;
     head = tail = 0;
-    if (total >= 0) return;
+    if (lane_id() == 0) sm.q = make_ball(p.x, p.y, p.z, fabs(w) * kWiden);
+    __syncwarp();
     if (nlist < 0) walk.start(t, sm);
     else walk.more = nlist > 0;
   }
   template <class Smem>
-  __device__ __forceinline__ bool next(const TreeView &t, Smem &sm, const Query &q, int &j) {
+  __device__ __forceinline__ bool next(const TreeView &t, Smem &sm, const double4 *pos, const double4 &p, int &j) {
     static_assert(kCell == 8, "four cells fill a warp");
     const int lane = (int)lane_id();
-    if (total >= 0) {
-      if (at >= total) return false;
-      j = -1;
-      if (at + lane < total) {
-        const int code = sm.code[at + lane];
-        j = sm.list[code >> 3] * kCell + (code & 7);
-      }
-      at += 32;
-      return true;
-    }
+    const Query &q = sm.q;
     const unsigned below = (1u << lane) - 1u;
     while (staged < 32 && (walk.more || tail != head)) {
       while (walk.more && tail - head < 8u) {
@@ -269,12 +286,23 @@ struct Source {
       int j0 = 0x7fffffff, j1 = 0x7fffffff;
       if (c0 < take) j0 = sm.own.cell[(head + c0) % kQueue] * kCell + (lane & 7);
       if (c1 < take) j1 = sm.own.cell[(head + c1) % kQueue] * kCell + (lane & 7);
-      float4 p0, p1;
-      if (j0 < t.n) p0 = ldg(t.pf + j0);
-      if (j1 < t.n) p1 = ldg(t.pf + j1);
       head += take;
-      const bool in0 = j0 < t.n && dist2(p0.x - q.lo[0], p0.y - q.lo[1], p0.z - q.lo[2]) <= q.r2;
-      const bool in1 = j1 < t.n && dist2(p1.x - q.lo[0], p1.y - q.lo[1], p1.z - q.lo[2]) <= q.r2;
+      bool in0, in1;
+      if (!far_out(q)) {
+        float4 p0, p1;
+        if (j0 < t.n) p0 = ldg(t.pf + j0);
+        if (j1 < t.n) p1 = ldg(t.pf + j1);
+        in0 = j0 < t.n && dist2(p0.x - q.lo[0], p0.y - q.lo[1], p0.z - q.lo[2]) <= q.c2;
+        in1 = j1 < t.n && dist2(p1.x - q.lo[0], p1.y - q.lo[1], p1.z - q.lo[2]) <= q.c2;
+      } else {
+        auto inside = [&](int k) {
+          if (k >= t.n) return false;
+          const double4 o = ld4(pos + k);
+          return ds2_exact(p.x - o.x, p.y - o.y, p.z - o.z) <= (double)q.r2;
+        };
+        in0 = inside(j0);
+        in1 = inside(j1);
+      }
       const unsigned m0 = __ballot_sync(kFull, in0), m1 = __ballot_sync(kFull, in1);
       if (in0) sm.own.stage[staged + __popc(m0 & below)] = j0;
       staged += __popc(m0);
@@ -447,10 +475,9 @@ struct Eval {
 // even and odd lanes add up the two sums' terms one by one.  Beyond a.ordered
 // batches (about twice the neighbours aimed at) it gives up, unless `exact`:
 // the range is far too large and rough_sums is the cheaper way to see that.
-// nlist, total: see Source.
-template <bool SUMS, class Smem>
-__device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, const double4 &p, double w, int nlist,
-                                           int total, bool exact) {
+template <bool SUMS, class Source, class Smem>
+__device__ __forceinline__ Eval eval_over(const SolveArgs &a, Smem &sm, int s, const double4 &p, double w, bool exact,
+                                          Source &src) {
   const int lane = (int)lane_id();
   const unsigned below = (1u << lane) - 1u;
   const double r2 = __dmul_rn(w, w);
@@ -463,11 +490,8 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
   const double wd = fmin(w, 1.7976931348623157e308), iw = 1.0 / wd;
   double acc = 0, dmax = -1.0;
   int nb = 0, j;
-  const Query q = make_ball(p.x, p.y, p.z, fabs(w) * kWiden);
-  Source src;
-  src.start(a.t, sm, nlist, total);
   e.many = false;
-  while (src.next(a.t, sm, q, j)) {
+  while (src.next(a.t, sm, a.pos, p, j)) {
     if (SUMS && nb == a.ordered && !exact) {
       e.many = true;
       break;
@@ -509,6 +533,25 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
     e.sliver = __any_sync(kFull, e.sliver);
   }
   return e;
+}
+
+// (the two sources' loops apart: in one, the registers of the visit cost the
+// steady solve 5 %)
+template <bool SUMS, class Smem>
+__device__ __forceinline__ Eval eval_visited(const SolveArgs &a, Smem &sm, int s, double w, int nlist, bool exact) {
+  const double4 p = ld4(a.pos + s);
+  Visited src;
+  src.start(a.t, sm, nlist, p, w);
+  return eval_over<SUMS>(a, sm, s, p, w, exact, src);
+}
+
+// total: the codes, or -1: none; nlist: see Visited
+template <bool SUMS, class Smem>
+__device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, const double4 &p, double w, int nlist,
+                                           int total, bool exact) {
+  if (total < 0) return eval_visited<SUMS>(a, sm, s, w, nlist, exact);
+  Coded src{total, 0};
+  return eval_over<SUMS>(a, sm, s, p, w, exact, src);
 }
 
 // The two sums of a range far too large, in FP32 over every particle of the
@@ -656,6 +699,45 @@ template <int G>
 struct Group {
   int first, count;
 
+  // which candidates of the list are inside the balls `mine` (lane t: target
+  // t's): sm.hits; load(j): candidate j's coordinates
+  template <class Load>
+  __device__ __forceinline__ void test_candidates(const SolveArgs &a, WarpSmem<G> &sm, const Query &mine, Load load) {
+    const int lane = (int)lane_id(), nlist = sm.nlist;
+    float tx[G], ty[G], tz[G], tr[G];
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      tx[t] = __shfl_sync(kFull, mine.lo[0], t);
+      ty[t] = __shfl_sync(kFull, mine.lo[1], t);
+      tz[t] = __shfl_sync(kFull, mine.lo[2], t);
+      tr[t] = __shfl_sync(kFull, mine.c2, t);
+    }
+    for (int r = 0; r < kRounds && r * 128 < nlist; r++) {
+      unsigned m[G];
+#pragma unroll
+      for (int t = 0; t < G; t++) m[t] = 0u;
+      const int chunks = min(32, (nlist - r * 128 + 3) >> 2);
+      // lane's candidate of chunk c; past the last: not a number, so that it is
+      // in no ball (a squared range may be infinite in FP32)
+      auto candidate = [&](int c) {
+        const int k = r * 128 + c * 4 + (lane >> 3);
+        const int j = k < nlist ? sm.list[k] * kCell + (lane & 7) : 0x7fffffff;
+        return j < a.t.n ? load(j) : make_float4(NAN, 0.f, 0.f, 0.f);
+      };
+      for (int c = 0; c < chunks; c++) {
+        const float4 o = candidate(c);
+#pragma unroll
+        for (int t = 0; t < G; t++) {
+          const unsigned b = __ballot_sync(kFull, dist2(o.x - tx[t], o.y - ty[t], o.z - tz[t]) <= tr[t]);
+          if (lane == c) m[t] = b;
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < G; t++) sm.hits[t][r][lane] = m[t];
+    }
+    __syncwarp();
+  }
+
   // for the targets of the mask `todo`, at their ranges or (SAVED) their
   // saved iterations'
   template <bool SAVED>
@@ -669,7 +751,7 @@ struct Group {
     Query mine = make_ball(p.x, p.y, p.z, p.w * slack * kWiden);
     Query q = mine;
     double w_list = p.w * slack;
-    if (tt != t0) mine.r2 = -1.f;
+    const bool far = __any_sync(kFull, p.w > 0 && far_out(mine));
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
 #pragma unroll
@@ -687,38 +769,19 @@ struct Group {
     }
     __syncwarp();
     if (nlist <= 0) return;
-    float tx[G], ty[G], tz[G], tr[G];
-#pragma unroll
-    for (int t = 0; t < G; t++) {
-      tx[t] = __shfl_sync(kFull, mine.lo[0], t);
-      ty[t] = __shfl_sync(kFull, mine.lo[1], t);
-      tz[t] = __shfl_sync(kFull, mine.lo[2], t);
-      tr[t] = __shfl_sync(kFull, mine.r2, t);
+    if (far) {
+      const double4 o = a.pos[first];
+      mine = make_ball(p.x - o.x, p.y - o.y, p.z - o.z, p.w * slack * kWiden);
+      if (tt != t0) mine.c2 = -1.f;
+      test_candidates(a, sm, mine, [&](int j) {
+        const double4 v = ld4(a.pos + j), o = ld4(a.pos + first);
+        return make_float4(held_f32((float)(v.x - o.x)), held_f32((float)(v.y - o.y)), held_f32((float)(v.z - o.z)),
+                           0.f);
+      });
+    } else {
+      if (tt != t0) mine.c2 = -1.f;
+      test_candidates(a, sm, mine, [&](int j) { return ldg(a.t.pf + j); });
     }
-    for (int r = 0; r < kRounds && r * 128 < nlist; r++) {
-      unsigned m[G];
-#pragma unroll
-      for (int t = 0; t < G; t++) m[t] = 0u;
-      const int chunks = min(32, (nlist - r * 128 + 3) >> 2);
-      // lane's candidate of chunk c; past the last: not a number, so that it is
-      // in no ball (a squared range may be infinite in FP32)
-      auto candidate = [&](int c) {
-        const int k = r * 128 + c * 4 + (lane >> 3);
-        const int j = k < nlist ? sm.list[k] * kCell + (lane & 7) : 0x7fffffff;
-        return j < a.t.n ? ldg(a.t.pf + j) : make_float4(NAN, 0.f, 0.f, 0.f);
-      };
-      for (int c = 0; c < chunks; c++) {
-        const float4 o = candidate(c);
-#pragma unroll
-        for (int t = 0; t < G; t++) {
-          const unsigned b = __ballot_sync(kFull, dist2(o.x - tx[t], o.y - ty[t], o.z - tz[t]) <= tr[t]);
-          if (lane == c) m[t] = b;
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < G; t++) sm.hits[t][r][lane] = m[t];
-    }
-    __syncwarp();
   }
   // target t, at iteration `it` (lane 0's): its candidates as codes; their
   // number, or -1 when they do not fit

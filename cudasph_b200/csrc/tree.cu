@@ -29,10 +29,12 @@ __global__ void __launch_bounds__(kCell * kFan) k_cell_boxes(int n, const double
     pf[s] = make_float4(held_f32((float)p.x), held_f32((float)p.y), held_f32((float)p.z), 0.f);
   }
   // rounding is monotone: the rounded extrema are the extrema of the rounded
-  float4 l = make_float4(held_f32(__double2float_rd(l0)), held_f32(__double2float_rd(l1)),
-                         held_f32(__double2float_rd(l2)), 0.f);
-  float4 h = make_float4(held_f32(__double2float_ru(h0)), held_f32(__double2float_ru(h1)),
-                         held_f32(__double2float_ru(h2)), 0.f);
+  // ... and they move out by 1.2e-7 of themselves, which covers the rounding of
+  // a query's centre as well (6e-8 of it: of the face and of the gap to it)
+  auto down = [](double v) { return held_f32(__double2float_rd(v - 1.2e-7 * fabs(v))); };
+  auto up = [](double v) { return held_f32(__double2float_ru(v + 1.2e-7 * fabs(v))); };
+  float4 l = make_float4(down(l0), down(l1), down(l2), 0.f);
+  float4 h = make_float4(up(h0), up(h1), up(h2), 0.f);
   auto merge = [&](int o) {
     l.x = fminf(l.x, __shfl_xor_sync(0xffffffffu, l.x, o));
     l.y = fminf(l.y, __shfl_xor_sync(0xffffffffu, l.y, o));

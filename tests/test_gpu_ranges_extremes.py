@@ -91,3 +91,33 @@ def test_steps_larger_than_the_range(f_scale, wide):
     r_o, _, ev_o = O.solve_range(x, y, z, wide * ic["range"][order], O.make_params(n_target=50.0, f_scale=f_scale))
     assert np.mean(r[order] == np.where(r_o > 0, r_o, 0.0)) >= 0.999  # a negative or undefined end is stored as 0
     assert np.mean(ev[order] == ev_o) >= 0.999
+
+
+@pytest.mark.parametrize("n", [8200, 90001])
+def test_solve_far_from_the_origin(n):
+    """At 1e6 the coordinates' FP32 copies say nothing about neighbours; the
+    solve is the oracle's there too, and takes about as long (a tenth of the
+    allowance is usual) as at the origin."""
+    from cudasph_b200.simulation import Simulation, make_params
+    from oracle import oracle as O
+    ms = []
+    for shift in (0.0, 1e6):
+        ic = ics.polytrope(n, n_ngb=50, seed=n)
+        ic["x"] = ic["x"] + shift
+        with Simulation(ic, make_params(n_target=50.0, eos_mode=0, soft_mode=1, eps=0.01)) as sim:
+            sim.sort_bodies()
+            order = sim.order()
+            sim.CUDA_solve_range()
+            r = sim.get("range")
+            sim.set_profiling(True)
+            t = []
+            for _ in range(5):
+                sim.reset_counters()
+                sim.CUDA_solve_range()
+                t.append(sim.phase_times()["solve_range"][0])
+            ms.append(min(t))
+        if n < 10000 or shift:
+            x, y, z = (np.asarray(ic[k])[order] for k in "xyz")
+            r_o, _, _ = O.solve_range(x, y, z, np.asarray(ic["range"])[order], O.make_params(n_target=50.0))
+            assert np.mean(r[order] == r_o) >= 0.999
+    assert ms[1] < 10 * ms[0]
