@@ -849,7 +849,10 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
           }
         }
         if (CHECK && __any_sync(0xffffffffu, near != 0u)) {
-          const int j = jb + ((l + s) & 31);  // the source at this lane now (near: a real one)
+          const int j = jb + ((l + s) & 31);  // the source at this lane now
+          // a range that is not a number or above 1.7e150 reaches the padding
+          // sources too: they have neither range nor force
+          if (j >= j_hi) near = 0u;
 #pragma unroll
           for (int r = 0; r < kSym64R; r++) {
             if ((near >> r) & 1u) {

@@ -79,3 +79,28 @@ def test_spline_gravity_separated_clumps(n):
     got = out.cpu().numpy()
     ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
     assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def _direct(p, m, r):
+    import torch
+    from cudasph_b200._capi import lib
+    n = m.size
+    src = torch.from_numpy(np.column_stack([p, m]).copy()).cuda()
+    tr = torch.from_numpy(np.asarray(r, np.float64).copy()).cuda()
+    out = torch.full((n, 4), np.nan, dtype=torch.float64, device="cuda")
+    assert lib().cudasph_gravity_direct(n, src.data_ptr(), tr.data_ptr(), out.data_ptr(), 0, 0.0, 1.0, 0,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("n", [1000, 1030, 2079, 5001])
+@pytest.mark.parametrize("odd", [np.nan, 2e150, -0.3])
+def test_spline_gravity_odd_ranges(n, odd):
+    """Ranges of single particles that are no number (the pair is Newtonian on
+    that side), beyond the place of the padding sources, and negative (the
+    square counts), where the last batch of sources is part-filled."""
+    p, m, r = _case(n, "near", equal=False)
+    r[[0, 3, n // 2, n - 1]] = odd
+    got = _direct(p, m, r)
+    ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
