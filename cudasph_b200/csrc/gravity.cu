@@ -60,7 +60,9 @@ __device__ __forceinline__ double rsq<double>(double x) { return rsqrt_f64(x); }
 // cost several times the FP64 instructions (60,000 particles with 24
 // neighbours: diagonal tiles 622 -> 274 us, the rest 3,695 -> 3,143).
 __device__ __forceinline__ void spline_inside(double r2, double inv, double h2, double &g, double &p) {
-  const double ih = rsqrt_f64(h2), ih2 = ih * ih, u2 = r2 * ih2, u = r2 * inv * ih;
+  // an infinite range, which a caller may give, stands at the largest number:
+  // no force and no potential, as divisions by it would give
+  const double ih = rsqrt_f64(fmin(h2, 1.7976931348623157e308)), ih2 = ih * ih, u2 = r2 * ih2, u = r2 * inv * ih;
   if (u < 0.5) {
     g = fma(u2, fma(32.0, u, -38.4), 10.666666666667);
     p = fma(u2, fma(u2, fma(6.4, u, -9.6), 5.333333333333), -2.8);

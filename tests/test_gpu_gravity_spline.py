@@ -104,3 +104,13 @@ def test_spline_gravity_odd_ranges(n, odd):
     got = _direct(p, m, r)
     ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
     assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("n", [1000, 1030, 5001])
+def test_spline_gravity_infinite_range(n):
+    """A pair inside an infinite range has no force and no potential from that side."""
+    p, m, r = _case(n, "near", equal=False)
+    r[[0, 3, n // 2, n - 1]] = np.inf
+    got = _direct(p, m, r)
+    ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
