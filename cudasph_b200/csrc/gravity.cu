@@ -54,8 +54,14 @@ __device__ __forceinline__ float rsq<float>(float x) { return rsqrt_f32(x); }
 template <>
 __device__ __forceinline__ double rsq<double>(double x) { return rsqrt_f64(x); }
 
-// One side of an FP64 pair inside its softening range, r2 < h2, inv = 1 / r (0
-// at r = 0): the factors of spline_poly over h^3 and over h.  All of 1/h, u and
+// 1 / r of an FP64 near pair; 0 at r = 0 and where the square of r is denormal
+// (r < 1.5e-154), which the seed of the reciprocal square root takes for 0
+__device__ __forceinline__ double near_inverse(double r2) {
+  return r2 >= 2.2250738585072014e-308 ? rsqrt_f64(r2) : 0.0;
+}
+
+// One side of an FP64 pair inside its softening range, r2 < h2, inv = 1 / r
+// (near_inverse): the factors of spline_poly over h^3 and over h.  All of 1/h, u and
 // 1/u come from reciprocal square roots; with sqrt and divisions the near pairs
 // cost several times the FP64 instructions (60,000 particles with 24
 // neighbours: diagonal tiles 622 -> 274 us, the rest 3,695 -> 3,143).
@@ -108,7 +114,7 @@ __device__ __noinline__ void spline_near(R dx, R dy, R dz, R r2, R mj, R hi2, R 
 
 // the same in FP64 without the mass: acceleration factor and potential at i
 __device__ __noinline__ double2 spline_at_i(double r2, double hi2, double hj2) {
-  const double inv = r2 > 0 ? rsqrt_f64(r2) : 0.0;
+  const double inv = near_inverse(r2);
   const double far = inv * inv * inv;
   double gi = far, gj = far, pi = -inv, unused;
   if (r2 < hi2) spline_inside(r2, inv, hi2, gi, pi);
@@ -722,7 +728,7 @@ struct NearPair {
 };
 
 __device__ __noinline__ NearPair spline_pair(double r2, double hi2, double hj2) {
-  const double inv = r2 > 0 ? rsqrt_f64(r2) : 0.0;
+  const double inv = near_inverse(r2);
   const double far = inv * inv * inv;
   double gi = far, gj = far;
   NearPair v;

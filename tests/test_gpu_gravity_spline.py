@@ -114,3 +114,14 @@ def test_spline_gravity_infinite_range(n):
     got = _direct(p, m, r)
     ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
     assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("n", [1000, 1030, 5001])
+def test_spline_gravity_separations_with_denormal_squares(n):
+    p, m, r = _case(n, "near", equal=False)
+    p[0] = 0.0
+    for k, d in ((1, [1e-160, 0, 0]), (n // 2, [0, 3e-158, -2e-159]), (n - 1, [-1e-154, 1e-155, 0])):
+        p[k] = d
+    got = _direct(p, m, r)
+    ref = np.stack(O.gravity(p[:, 0], p[:, 1], p[:, 2], m, r, O.make_params(soft_mode=0)), 1)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
