@@ -107,18 +107,36 @@ def _results(sim, *shapes):
     return [torch.empty(s, dtype=torch.float64, device=f"cuda:{sim.device}") for s in shapes]
 
 
+def _checked(n, x0, v0, u0, ic):
+    """The first three columns of x0 and v0, u0 as a vector, and the fields
+    taken from the initial conditions, each for the context's n particles (a
+    state of another size would be read past its end, or spread over all)."""
+    for name, t in (("x0", x0), ("v0", v0)):
+        if t.dim() < 2 or t.shape[1] < 3 or t[:, 0].numel() != n:
+            raise ValueError(f"rollout: {name} has shape {tuple(t.shape)}, ({n}, 3) is required")
+    if u0.numel() != n:
+        raise ValueError(f"rollout: u0 has {u0.numel()} values, {n} are required")
+    if "range" not in ic:
+        raise KeyError("range")
+    fields = {k: np.array(ic[k], np.float64).reshape(-1) for k in ("range", "ax", "ay", "az", "du") if k in ic}
+    for k, a in fields.items():
+        if a.size != n:
+            raise ValueError(f"rollout: {k} of the initial conditions has {a.size} values, {n} are required")
+    return x0[:, :3], v0[:, :3], u0.reshape(-1), fields
+
+
 class Rollout(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x0, v0, u0, rc: RolloutContext):
-        n = x0.shape[0]
+        n = rc.sim.n
+        x0, v0, u0, fields = _checked(n, x0, v0, u0, rc.ic)
         vK, rhoK = _results(rc.sim, (n, 3), (n,))
         with _OnStream(rc.sim) as on:
             rows = torch.zeros(len(STATE), n, dtype=torch.float64, device=on.device)
-            for k in ("range", "ax", "ay", "az", "du"):
-                if k in rc.ic:
-                    rows[ROW[k]].copy_(torch.from_numpy(np.array(rc.ic[k], np.float64)))
-            rows[ROW["x"]:ROW["z"] + 1] = on.take(x0).t()
-            rows[ROW["vx"]:ROW["vz"] + 1] = on.take(v0).t()
+            for k, a in fields.items():
+                rows[ROW[k]].copy_(torch.from_numpy(a))
+            rows[ROW["x"]:ROW["z"] + 1] = on.take(x0).transpose(0, 1).reshape(3, n)
+            rows[ROW["vx"]:ROW["vz"] + 1] = on.take(v0).transpose(0, 1).reshape(3, n)
             rows[ROW["u"]] = on.take(u0)
             rc._set((rows, float(rc.ic.get("time", 0.0)), float(rc.ic.get("dt", 0.0))))
             ckpt = {0: rc._get()}
