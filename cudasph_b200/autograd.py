@@ -83,6 +83,7 @@ class _OnStream:
     stream and stays inside (states) or is copied out."""
 
     def __init__(self, sim):
+        check(lib().cudasph_get_stream(sim._h, C.byref(C.c_void_p())), "rollout")  # a closed context has no stream
         self.stream = sim.torch_stream()
         self.device = torch.device("cuda", sim.device)
 

@@ -42,3 +42,19 @@ def test_rollout_is_the_same_from_every_device_and_stream():
     for where, side in (("cuda", False), ("cuda", True)):
         for a, b in zip(_grads(where, side), ref):
             assert (a - b).abs().max() <= 1e-11 * b.abs().max()
+
+
+def test_rollout_of_a_closed_context_is_refused():
+    from cudasph_b200._capi import SphError
+    from cudasph_b200.autograd import RolloutContext, rollout
+    from cudasph_b200.simulation import make_params
+    ic = ics.polytrope(700, n_ngb=40, seed=4)
+    rc = RolloutContext(ic, make_params(n_target=40.0, eos_mode=0, soft_mode=1, eps=0.02), steps=1)
+    x = torch.from_numpy(np.stack([ic[k] for k in "xyz"], 1)).requires_grad_(True)
+    v, u = torch.zeros(700, 3, dtype=torch.float64), torch.from_numpy(ic["u"])
+    vk, _ = rollout(x, v, u, rc)
+    rc.close()
+    with pytest.raises(SphError):
+        torch.autograd.grad(vk.sum(), x)
+    with pytest.raises(SphError):
+        rollout(x, v, u, rc)
