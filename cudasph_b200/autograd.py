@@ -17,11 +17,15 @@ its adjoint run in libcudasph_b200.so.
 Checkpoints, replayed states and the state adjoints stay on the device, in
 tensors of the context's own stream (exchanged through host arrays, 12 fields
 at a time, the transfers and their synchronisations were about 40 % of a
-rollout of 12,001 particles: 16.4 -> 9.9 ms).
+rollout of 12,001 particles: 16.4 -> 9.9 ms).  A state is 96 bytes per
+particle; a context holds as many on the device as fit in a quarter of the
+memory that was free when it was created, and the others on the host, so that
+the length of a rollout is not limited by the device's memory.
 """
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -34,25 +38,65 @@ ADJ = ("x", "y", "z", "vx", "vy", "vz", "u", "ax", "ay", "az", "du")
 ROW = {k: i for i, k in enumerate(STATE)}
 
 
-class RolloutContext:
-    """The simulation and the fixed part of the initial conditions."""
+class _Budget:
+    """Bytes of device memory that the states of a context may still take."""
 
-    def __init__(self, ic: dict, params, steps: int, every: int = 5, device: int = 0):
+    def __init__(self, left: int):
+        self.left = left
+        self.lock = threading.Lock()
+
+    def take(self, size: int) -> bool:
+        with self.lock:
+            fits = size <= self.left
+            if fits:
+                self.left -= size
+            return fits
+
+    def give(self, size: int):
+        with self.lock:
+            self.left += size
+
+
+class _State:
+    """A particle state: a (12, N) tensor of the rows STATE, on the device while
+    the budget lasts and else on the host, with time and dt."""
+
+    def __init__(self, rows, time: float, dt: float, budget: _Budget):
+        size = rows.numel() * rows.element_size()
+        self.held = size if budget.take(size) else 0
+        self.rows = rows if self.held else rows.cpu()
+        self.time, self.dt, self.budget = time, dt, budget
+
+    def __del__(self):
+        if getattr(self, "held", 0):
+            self.budget.give(self.held)
+
+
+class RolloutContext:
+    """The simulation and the fixed part of the initial conditions.
+    device_bytes: device memory for the states (default: a quarter of what is
+    free)."""
+
+    def __init__(self, ic: dict, params, steps: int, every: int = 5, device: int = 0, device_bytes: int | None = None):
         self.ic = ic
         self.params = params
         self.steps = int(steps)
         self.every = max(1, int(every))
         self.sim = Simulation(ic, params, device=device)
         self.sim.set_keep(True)
+        if device_bytes is None:
+            device_bytes = torch.cuda.mem_get_info(device)[0] // 4
+        self.budget = _Budget(device_bytes)
 
     def close(self):
         self.sim.close()
+        # torch keeps freed memory for the stream it was used on, which is gone
+        torch.cuda.empty_cache()
 
-    # A state is ((12, N) device tensor of the rows STATE, time, dt).  The
-    # library works on the context's stream; the callers below make that the
-    # current one, so every tensor here is allocated, written and freed on it.
-    def _set(self, state):
-        rows, time, dt = state
+    # The library works on the context's stream; the callers below make that
+    # the current one, so every tensor here is allocated, written and freed on it.
+    def _set(self, rows, time: float, dt: float):
+        rows = rows.to(f"cuda:{self.sim.device}")
         check(lib().cudasph_set_state(self.sim._h, _pointers(rows, STATE), 1), "set_state")
         self.sim.set_time(time, dt)
 
@@ -65,7 +109,7 @@ class RolloutContext:
         t, d = C.c_double(), C.c_double()
         rows = self._read(STATE)
         check(lib().cudasph_get_time(self.sim._h, C.byref(t), C.byref(d)), "get_time")
-        return rows, t.value, d.value
+        return _State(rows, t.value, d.value, self.budget)
 
 
 def _pointers(rows, names):
@@ -139,7 +183,7 @@ class Rollout(torch.autograd.Function):
             rows[ROW["x"]:ROW["z"] + 1] = on.take(x0).transpose(0, 1).reshape(3, n)
             rows[ROW["vx"]:ROW["vz"] + 1] = on.take(v0).transpose(0, 1).reshape(3, n)
             rows[ROW["u"]] = on.take(u0)
-            rc._set((rows, float(rc.ic.get("time", 0.0)), float(rc.ic.get("dt", 0.0))))
+            rc._set(rows, float(rc.ic.get("time", 0.0)), float(rc.ic.get("dt", 0.0)))
             ckpt = {0: rc._get()}
             for s in range(rc.steps):
                 rc.sim.step()
@@ -172,12 +216,13 @@ class Rollout(torch.autograd.Function):
                 s1 = starts[si + 1] if si + 1 < len(starts) else rc.steps
                 # pre-step states of the segment
                 pre = [ckpt[s0]]
-                rc._set(ckpt[s0])
+                rc._set(pre[0].rows, pre[0].time, pre[0].dt)
                 for s in range(s0, s1 - 1):
                     sim.step()
                     pre.append(rc._get())
                 for s in range(s1 - 1, s0 - 1, -1):
-                    rc._set(pre[s - s0])
+                    st = pre[s - s0]
+                    rc._set(st.rows, st.time, st.dt)
                     sim.step()  # replays step s with keep on
                     for i, k in enumerate(ADJ):
                         check(lib().cudasph_adjoint_set_field(h, ADJ_ID[k], adj[i].data_ptr(), 1), "adjoint_set")

@@ -58,3 +58,29 @@ def test_rollout_of_a_closed_context_is_refused():
         torch.autograd.grad(vk.sum(), x)
     with pytest.raises(SphError):
         rollout(x, v, u, rc)
+
+
+@pytest.mark.parametrize("states", [0, 2])
+def test_states_beyond_the_device_memory_are_held_on_the_host(states):
+    from cudasph_b200.autograd import RolloutContext, rollout
+    from cudasph_b200.simulation import make_params
+    ic = ics.polytrope(700, n_ngb=40, seed=4)
+    ic["dt"] = 1e-3
+    res = []
+    for limit in (None, states * 700 * 96):
+        rc = RolloutContext(ic, make_params(n_target=40.0, eos_mode=0, soft_mode=1, eps=0.02), steps=6, every=3,
+                            device_bytes=limit)
+        free = rc.budget.left
+        assert limit is not None or free > 1 << 30
+        x, v, u = (torch.from_numpy(a).requires_grad_(True) for a in (
+            np.stack([ic[k] for k in "xyz"], 1), 0.1 * np.stack([ic[k] for k in "yzx"], 1), ic["u"].copy()))
+        vk, rho = rollout(x, v, u, rc)
+        ckpt = vk.grad_fn.ckpt
+        assert [s.rows.is_cuda for s in ckpt.values()] == [limit is None or k < states for k in range(2)]
+        assert free - rc.budget.left == 700 * 96 * sum(s.rows.is_cuda for s in ckpt.values())
+        res.append([vk.detach(), rho.detach(), *torch.autograd.grad((vk * vk).sum() + rho[:50].mean(), (x, v, u))])
+        del vk, rho, ckpt
+        assert rc.budget.left == free
+        rc.close()
+    for a, b in zip(*res):
+        assert (a - b).abs().max() <= 1e-11 * b.abs().max()
