@@ -97,7 +97,8 @@ struct sph_ctx {
   double4 *aux = nullptr;  // per-particle factors of the hydro pair loop (scratch)
   double4 *gsrc = nullptr;
   double *gh2 = nullptr;
-  int *mass_mixed = nullptr;  // 0 when all masses are equal (kept up to date where masses are set)
+  int *mass_mixed = nullptr;  // 0 when all masses are equal, of the masses the sources were last packed with
+  bool masses_checked = true;  // whether that still holds for the masses of the state
   unsigned *flags = nullptr;
   double *sc = nullptr;  // StepScalars
   double *fin_part = nullptr;
@@ -443,7 +444,7 @@ static int put_field(sph_ctx *c, int field, const double *src, int on_device) {
   FieldRef r = field_ref(c, field);
   launch_field_io(c->n, r.base, r.stride, r.comp, c->f[c->cur].id, c->flat, 1, c->st);
   c->launches++;
-  if (field == SPH_M) LAUNCHED(launch_check_masses(c->n, c->f[c->cur].vel, c->mass_mixed, c->st));
+  if (field == SPH_M) c->masses_checked = false;
   mark_changed(c, field);
   SPH_CUDA_TRY(cudaGetLastError());
   return SPH_OK;
@@ -709,6 +710,15 @@ extern "C" int cudasph_sph_accelerations(sph_ctx *c) {
   return SPH_OK;
 }
 
+// Masses change only when a caller sets them, so the flag is made then, ahead
+// of the next sum (and outside a captured step); the reverse sweep of a step
+// taken before needs the old one.
+static void check_masses(sph_ctx *c) {
+  if (c->masses_checked) return;
+  LAUNCHED(launch_check_masses(c->n, c->f[c->cur].vel, c->mass_mixed, c->st));
+  c->masses_checked = true;
+}
+
 extern "C" int cudasph_gravity(sph_ctx *c) {
   if (!c) return SPH_ERR_ARG;
   if (c->p.grav_mode == SPH_GRAV_TREE && !c->tree_ok) {
@@ -726,6 +736,7 @@ extern "C" int cudasph_gravity(sph_ctx *c) {
     SPH_CUDA_TRY(cudaGetLastError());
     return SPH_OK;
   }
+  check_masses(c);
   LAUNCHED(launch_pack_sources(c->n, F.pos, F.vel, c->gsrc, c->gh2, F.grav, c->st));
   LAUNCHED(launch_gravity(c->n, c->gsrc, c->gh2, F.grav, c->p.soft_mode, c->p.eps, c->p.G, c->p.precision,
                           c->mass_mixed, c->rank, c->world, true, c->st));
@@ -779,6 +790,7 @@ extern "C" int cudasph_step(sph_ctx *c) {
   const bool graphable = c->use_graph && !c->need_sort && c->p.sort_every == 1 && !c->profiling && !c->keep;
   if (!graphable) return step_body(c);
   SPH_CUDA_TRY(cudaSetDevice(c->device));
+  check_masses(c);
   const int par = c->cur;
   if (c->gexec[par]) {
     SPH_CUDA_TRY(cudaGraphLaunch(c->gexec[par], c->st));

@@ -1056,8 +1056,8 @@ int launch_pack_sources(int n, const double4 *pos, const double4 *vel, double4 *
 }
 
 // *mass_mixed = whether some mass differs from the first particle's: the
-// symmetric kernels take their equal-mass form when it stays 0.  Masses
-// change only when a caller sets them, so this runs then and not in the step.
+// symmetric kernels take their equal-mass form when it stays 0.  Runs ahead of
+// the first sum after a caller has set masses, not in every step.
 __global__ void k_check_masses(int n, const double4 *vel, int *mass_mixed) {
   grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
