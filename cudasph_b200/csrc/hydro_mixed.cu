@@ -14,7 +14,7 @@
 // j-side pair force is assembled in FP64 from the FP32 pair vectors and the
 // owner's FP64 factors; outputs and atomics stay FP64.
 #include "common.cuh"
-#include "sph_math.cuh"
+#include "sphpair.cuh"
 
 namespace sph {
 
@@ -30,11 +30,18 @@ struct KSum {
   __device__ __forceinline__ double get() const { return (double)hi + (double)lo; }
 };
 
-__device__ __forceinline__ int leaf_max_count_m(int cnt) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, o));
-  return cnt;
-}
+// sum over the S lanes of a particle, in FP64
+template <int S>
+__device__ __forceinline__ double lanes_sum(const KSum &k) { return sub_sum<S>(k.get()); }
+
+// Lanes per particle, as in the FP64 loops: a list is a row of its own, and
+// one lane per particle reads 32 rows at a time (65,536 particles, hydro, us:
+// 217, and 164 when the lists of 32 particles were interleaved).  us, density
+// / hydro, with 16, 8, 4, 2 lanes and 1: 2,000 particles 12.6 / 18.9 (16), 16.8
+// / 23.2 (8), 67 / 101 (1); 16,384 with 8 / 4 / 2 / 1 lanes 31 / 50, 29 / 47,
+// 42 / 65, 71 / 109; 65,536 76 / 132, 76 / 127, 89 / 162, 92 / 217; 1,000,000
+// 1008 / 1827, 904 / 1661, 867 / 1728, 928 / 2115.
+constexpr int kSubSmall = 16, kSmallSet = 8192, kSub = 4;
 
 // x (hi + lo) for a float-float constant: the product to about 2^-46
 __device__ __forceinline__ float mul_ff(float x, float hi, float lo) { return fmaf(x, hi, x * lo); }
@@ -44,13 +51,11 @@ __device__ __forceinline__ void split_ff(double v, float &hi, float &lo) {
   lo = (float)(v - (double)hi);
 }
 
+template <int S>
 __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
   grid_enter();
-  const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (leaf >= a.leaf1) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
-  const bool valid = s < a.n;
+  const int s = a.leaf0 * kLeaf + (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
+  const bool valid = s < min(a.leaf1 * kLeaf, a.n);
   double4 pi = make_double4(0, 0, 0, 0), vi = make_double4(0, 0, 0, 0);
   int cnt = 0;
   if (valid) {
@@ -58,26 +63,25 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
     vi = a.vel[s];
     cnt = min(a.n_ngb[s], a.cap);
   }
-  const int kmax = leaf_max_count_m(cnt);
   const int *lst = a.list + (size_t)s * a.stride;
   const double w = pi.w;
   float iw_hi = 0.f, iw_lo = 0.f;  // 2 / range as a float-float pair
   if (w > 0) split_ff(2.0 / w, iw_hi, iw_lo);
   KSum dens, om, ps, sdig, div, cx, cy, cz;
-  int jn = cnt > 1 ? ldg(lst + 1) : 0;
+  int jn = sub + S < cnt ? ldg(lst + sub + S) : 0;
   double4 pn = make_double4(0, 0, 0, 0), vn = pn;
-  if (cnt > 0) {
-    const int j0 = ldg(lst);
+  if (sub < cnt) {
+    const int j0 = ldg(lst + sub);
     pn = ld4(a.pos + j0);
     vn = ld4(a.vel + j0);
   }
-  for (int k = 0; k < kmax; k++) {
-    if (k < cnt) {
+  for (int k = sub; k < cnt; k += S) {
+    {
       const double4 pj = pn, vj = vn;
-      if (k + 1 < cnt) {
+      if (k + S < cnt) {
         pn = ld4(a.pos + jn);
         vn = ld4(a.vel + jn);
-        if (k + 2 < cnt) jn = ldg(lst + k + 2);
+        if (k + 2 * S < cnt) jn = ldg(lst + k + 2 * S);
       }
       const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
       const float u = mul_ff(sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx))), iw_hi, iw_lo);
@@ -94,14 +98,16 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
       cz.add(wt * (dx * dvy - dy * dvx));
     }
   }
-  if (!valid) return;
-  if (a.dsum) a.dsum[s] = make_double4(sdig.get(), cx.get(), cy.get(), cz.get());
+  __syncwarp();
+  double de = lanes_sum<S>(dens), o = lanes_sum<S>(om), p = lanes_sum<S>(ps), dv = lanes_sum<S>(div);
+  const double sd = lanes_sum<S>(sdig), X = lanes_sum<S>(cx), Y = lanes_sum<S>(cy), Z = lanes_sum<S>(cz);
+  if (!valid || sub != 0) return;
+  if (a.dsum) a.dsum[s] = make_double4(sd, X, Y, Z);
   double4 d = make_double4(0, 0, 0, 0);
   double rho = 0;
   if (w > 0 && cnt > 0) {
     const double h = 0.5 * w;
     const double h3 = h * h * h, h5 = h3 * h * h;
-    double o = om.get(), p = ps.get(), sd = sdig.get(), de = dens.get();
     if (sd != 0) {
       o *= 1.0 / h3 / sd;
       p *= 1.0 / h / sd;
@@ -109,8 +115,7 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
       o = p = 0;
     }
     de *= 1.0 / h3;
-    const double dv = div.get() / de / h5;
-    const double X = cx.get(), Y = cy.get(), Z = cz.get();
+    dv = dv / de / h5;
     const double c = sqrt(X * X + Y * Y + Z * Z) / de / h5;
     rho = de;
     d = make_double4(dv, c, o, p);
@@ -127,13 +132,11 @@ __global__ void __launch_bounds__(128) k_density_mixed(HydroArgs a) {
 // du_i/dt = [A T1 + T2 / 2] / h^5 - A omega_i T3 / h^2 with the same sums of
 // r_ij . v_ij in place of r_ij; the pair's force on j, m_i acc_ij (r_i - r_j),
 // is assembled in FP64 from the FP32 pair vectors dw r_ij, Pi dw r_ij, dig r_ij.
+template <int S>
 __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
   grid_enter();
-  const int leaf = a.leaf0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (leaf >= a.leaf1) return;
-  const int lane = (int)lane_id();
-  const int s = leaf * kLeaf + lane;
-  const bool valid = s < a.n;
+  const int s = a.leaf0 * kLeaf + (int)((blockIdx.x * blockDim.x + threadIdx.x) / S), sub = (int)threadIdx.x % S;
+  const bool valid = s < min(a.leaf1 * kLeaf, a.n);
   double4 pi = make_double4(0, 0, 0, 0), vi = make_double4(0, 0, 0, 1), hi4 = make_double4(0, 0, 0, 0),
           di = make_double4(0, 0, 0, 0), fi = make_double4(0, 0, 0, 0);
   int cnt = 0;
@@ -145,7 +148,6 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
     fi = a.aux[s];
     cnt = min(a.n_ngb[s], a.cap);
   }
-  const int kmax = leaf_max_count_m(cnt);
   const int *lst = a.list + (size_t)s * a.stride;
   const double hh = 0.5 * pi.w;
   float ih_hi = 0.f, ih_lo = 0.f;  // 1 / h as a float-float pair
@@ -162,8 +164,8 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
   const float ci = (float)fi.x, pr_i = (float)fi.y, bal_i = (float)fi.z;
   KSum s1x, s1y, s1z, s2x, s2y, s2z, s3x, s3y, s3z, t1, t2, t3;
   float vmax = 0.f;
-  for (int k = 0; k < kmax; k++) {
-    if (k < cnt) {
+  for (int k = sub; k < cnt; k += S) {
+    {
       const int j = ldg(lst + k);
       const double4 pj = ld4(a.pos + j), vj = ld4(a.vel + j), fj = ld4(a.aux + j);
       const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
@@ -203,17 +205,25 @@ __global__ void __launch_bounds__(128) k_hydro_mixed(HydroArgs a) {
       }
     }
   }
-  if (!valid) return;
-  atomicAdd(&a.dots[s].x, -(prho2 * s1x.get() + 0.5 * s2x.get()) * ih5 + K * ih2 * s3x.get());
-  atomicAdd(&a.dots[s].y, -(prho2 * s1y.get() + 0.5 * s2y.get()) * ih5 + K * ih2 * s3y.get());
-  atomicAdd(&a.dots[s].z, -(prho2 * s1z.get() + 0.5 * s2z.get()) * ih5 + K * ih2 * s3z.get());
-  a.dots[s].w = (prho2 * t1.get() + 0.5 * t2.get()) * ih5 - prho2 * di.z * ih2 * t3.get();
-  a.vsig[s] = (double)vmax;
+  __syncwarp();
+  const double ax = -(prho2 * lanes_sum<S>(s1x) + 0.5 * lanes_sum<S>(s2x)) * ih5 + K * ih2 * lanes_sum<S>(s3x);
+  const double ay = -(prho2 * lanes_sum<S>(s1y) + 0.5 * lanes_sum<S>(s2y)) * ih5 + K * ih2 * lanes_sum<S>(s3y);
+  const double az = -(prho2 * lanes_sum<S>(s1z) + 0.5 * lanes_sum<S>(s2z)) * ih5 + K * ih2 * lanes_sum<S>(s3z);
+  const double du = (prho2 * lanes_sum<S>(t1) + 0.5 * lanes_sum<S>(t2)) * ih5 - prho2 * di.z * ih2 * lanes_sum<S>(t3);
+  const double vs = sub_max<S>((double)vmax);
+  if (!valid || sub != 0) return;
+  atomicAdd(&a.dots[s].x, ax);
+  atomicAdd(&a.dots[s].y, ay);
+  atomicAdd(&a.dots[s].z, az);
+  a.dots[s].w = du;
+  a.vsig[s] = vs;
 }
 
 int launch_density_mixed(const HydroArgs &a, cudaStream_t st) {
   if (a.leaf1 <= a.leaf0) return 0;
-  launch(k_density_mixed, ((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, st, a);
+  const int n = (a.leaf1 - a.leaf0) * kLeaf;
+  if (n < kSmallSet) launch(k_density_mixed<kSubSmall>, (n * kSubSmall + 127) / 128, 128, st, a);
+  else launch(k_density_mixed<kSub>, (n * kSub + 127) / 128, 128, st, a);
   return 1;
 }
 int launch_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
@@ -224,7 +234,9 @@ int launch_hydro_mixed(const HydroArgs &a, cudaStream_t st) {
   // a shard without leaves still clears the sums that the shards add up
   int launches = launch_hydro_prep(a.n, a.pos, a.vel, a.hyd, a.dd, a.gamma, a.aux, a.dots, st);
   if (a.leaf1 <= a.leaf0) return launches;
-  launch(k_hydro_mixed, ((a.leaf1 - a.leaf0) * 32 + 127) / 128, 128, st, a);
+  const int n = (a.leaf1 - a.leaf0) * kLeaf;
+  if (n < kSmallSet) launch(k_hydro_mixed<kSubSmall>, (n * kSubSmall + 127) / 128, 128, st, a);
+  else launch(k_hydro_mixed<kSub>, (n * kSub + 127) / 128, 128, st, a);
   return launches + 1;
 }
 
