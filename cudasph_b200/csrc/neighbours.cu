@@ -38,6 +38,14 @@
 
 namespace sph {
 
+// A particle's record for its position only: other warps of the solve store
+// the records' fourth entries meanwhile, which rules out read-only loads.
+__device__ __forceinline__ double4 ld4_xyz(const double4 *p) {
+  double4 r;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+  return r;
+}
+
 constexpr int kNgbWarps = 4;   // warps per block
 // queries reach a little past the range: the sliver test below needs it
 constexpr double kWiden = 1.0 + 1e-12;
@@ -297,7 +305,7 @@ struct Visited {
       } else {
         auto inside = [&](int k) {
           if (k >= t.n) return false;
-          const double4 o = ld4(pos + k);
+          const double4 o = ld4_xyz(pos + k);
           return ds2_exact(p.x - o.x, p.y - o.y, p.z - o.z) <= (double)q.r2;
         };
         in0 = inside(j0);
@@ -498,7 +506,7 @@ __device__ __forceinline__ Eval eval_over(const SolveArgs &a, Smem &sm, int s, c
     }
     double d2 = NAN;  // no candidate: inside no range, not even an infinite one
     if (j >= 0) {
-      const double4 o = ld4(a.pos + j);
+      const double4 o = ld4_xyz(a.pos + j);
       d2 = ds2_exact(p.x - o.x, p.y - o.y, p.z - o.z);
     }
     const bool hit = d2 < r2;
@@ -539,7 +547,7 @@ __device__ __forceinline__ Eval eval_over(const SolveArgs &a, Smem &sm, int s, c
 // steady solve 5 %)
 template <bool SUMS, class Smem>
 __device__ __forceinline__ Eval eval_visited(const SolveArgs &a, Smem &sm, int s, double w, int nlist, bool exact) {
-  const double4 p = ld4(a.pos + s);
+  const double4 p = ld4_xyz(a.pos + s);
   Visited src;
   src.start(a.t, sm, nlist, p, w);
   return eval_over<SUMS>(a, sm, s, p, w, exact, src);
@@ -774,7 +782,7 @@ struct Group {
       mine = make_ball(p.x - o.x, p.y - o.y, p.z - o.z, p.w * slack * kWiden);
       if (tt != t0) mine.c2 = -1.f;
       test_candidates(a, sm, mine, [&](int j) {
-        const double4 v = ld4(a.pos + j), o = ld4(a.pos + first);
+        const double4 v = ld4_xyz(a.pos + j), o = ld4_xyz(a.pos + first);
         return make_float4(held_f32((float)(v.x - o.x)), held_f32((float)(v.y - o.y)), held_f32((float)(v.z - o.z)),
                            0.f);
       });
