@@ -34,6 +34,7 @@
 // of their test, or the next records ahead of their evaluation, cost 5 - 9 %
 // (registers).
 #include "common.cuh"
+#include "divby.cuh"
 #include "sph_math.cuh"
 
 namespace sph {
@@ -427,17 +428,6 @@ __device__ __forceinline__ void solve_advance(RangeIter &it, double sf, double s
       it.phase = kDone;
     }
   }
-}
-
-
-// a / b rounded to nearest, y = 1 / b rounded to nearest: Markstein's method
-// (Computation of elementary functions on the IBM RISC System/6000, 1990).
-// The first correction brings q within an ulp, the second then rounds
-// correctly; b and the quotient are far from the ends of the exponent range.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  double q = __dmul_rn(a, y);
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
 // ig(u) and u d(ig)/du (k_ig and k_digdh of sph_math.cuh: the same operations
