@@ -122,19 +122,34 @@ __device__ __forceinline__ void grid_enter() {
   asm volatile("griddepcontrol.launch_dependents;");
 }
 
-// kernel<<<grid, block, 0, st>>>(args...), programmatic on a stream of its own
+// kernel<<<grid, block, 0, st>>>(args...), programmatic on a stream of its own,
+// in clusters of `cluster` blocks with `shared` bytes of dynamic shared memory
 template <class... P, class... A>
-inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline void launch_clusters(void (*kernel)(P...), unsigned grid, unsigned block, unsigned cluster, size_t shared,
+                            cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = {};
+  if (st != nullptr) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    if (cluster > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    cfg.numAttrs++;
+  }
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = shared;
   cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = st != nullptr ? 1 : 0;
+  cfg.attrs = attr;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+  launch_clusters(kernel, grid, block, 1, 0, st, args...);
 }
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
@@ -242,7 +257,8 @@ __host__ __device__ __forceinline__ long long sym_items(int nt) { return nt >= 2
 // a whole number of UNIT-source batches, the sources whose FP32 terms the
 // mixed kernels add up before they fold into FP64: the sums then do not
 // depend on the slices but by the order of the FP64 additions.  The parts
-// meet by atomics in an output cleared beforehand.
+// meet by atomics in an output cleared beforehand, or (direct sums of one
+// tile) are folded in order by a cluster.
 template <int UNIT>
 __device__ __forceinline__ void source_slice(int &lo, int &hi, unsigned q, int slices) {
   if (slices == 1) return;
@@ -262,9 +278,9 @@ __device__ __forceinline__ void source_slice(int &lo, int &hi, unsigned q, int s
 // 335, 65,536 1485 / 1331, 100,003 4303 / 2992, 262,144 19,980 / 19,360 (four
 // rounds instead of sixteen: 100,003 3193, 262,144 19,967).  From about
 // 400,000 particles on nothing is cut.
-inline int grav_slices(long long blocks, int sources, long long want, int least) {
+inline int grav_slices(long long blocks, int sources, long long want, int least, int most = 1 << 30) {
   int s = 1;
-  while (blocks * s < want && sources / (2 * s) >= least) s *= 2;
+  while (2 * s <= most && blocks * s < want && sources / (2 * s) >= least) s *= 2;
   return s;
 }
 

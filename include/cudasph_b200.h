@@ -318,7 +318,9 @@ int cudasph_gravity_plan(int n, int precision, int soft_mode, int rank, int worl
 int cudasph_gravity_item(int n, long long item, int *row, int *t_lo, int *t_hi);
 
 /* direct-N gravity of n sources on themselves: pos4 = {x,y,z,m}, range =
- * smoothing ranges (spline mode), out4 = {gx,gy,gz,phi}; double buffers. */
+ * smoothing ranges (spline mode), out4 = {gx,gy,gz,phi}; double buffers.
+ * Sets of up to 1,024 particles repeat bit for bit; in larger ones the parts
+ * of a sum may meet by FP64 atomics, and results repeat to their rounding. */
 int cudasph_gravity_direct(int n, const double *pos4, const double *range, double *out4, int soft_mode,
                            double eps, double G, int precision, void *stream);
 
