@@ -3,9 +3,11 @@
 // -> sph_accelerations.cpp:3-121 -> CUDA_calls.cpp / CUDA_gravity.cpp), but
 // every phase is a stream-ordered launch on device-resident FP64 state and
 // nothing is copied to the host inside a step.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -564,13 +566,21 @@ extern "C" int cudasph_get_neighbours(sph_ctx *c, int *counts, int64_t *offsets,
   offsets[0] = 0;
   for (int i = 0; i < n; i++) offsets[i + 1] = offsets[i] + counts[i];
   if (!list) return SPH_OK;
-  std::vector<int> lst((size_t)n * c->list_stride);
-  SPH_CUDA_TRY(cudaMemcpyAsync(lst.data(), c->list, sizeof(int) * lst.size(), cudaMemcpyDeviceToHost, c->st));
-  SPH_CUDA_TRY(cudaStreamSynchronize(c->st));
-  for (int s = 0; s < n; s++) {
-    const int m = cnt[s] < cap ? cnt[s] : cap;
-    int64_t o = offsets[ids[s]];
-    for (int k = 0; k < m; k++) list[o + k] = ids[lst[(size_t)s * c->list_stride + k]];
+  // by 4 MB of rows through one host buffer: new pages for all of them cost more
+  // than the copy (ms, at once / so: 3,000 particles 0.92 / 0.55, 30,000 9.6 /
+  // 5.4, 300,000 175 / 58)
+  const int chunk = std::min(n, std::max(1, (1 << 20) / c->list_stride));
+  const std::unique_ptr<int[]> rows(new int[(size_t)chunk * c->list_stride]);
+  for (int s0 = 0; s0 < n; s0 += chunk) {
+    const int s1 = std::min(n, s0 + chunk);
+    SPH_CUDA_TRY(cudaMemcpyAsync(rows.get(), c->list + (size_t)s0 * c->list_stride,
+                                 sizeof(int) * (size_t)c->list_stride * (s1 - s0), cudaMemcpyDeviceToHost, c->st));
+    SPH_CUDA_TRY(cudaStreamSynchronize(c->st));
+    for (int s = s0; s < s1; s++) {
+      const int *row = rows.get() + (size_t)(s - s0) * c->list_stride;
+      int *o = list + offsets[ids[s]];
+      for (int k = 0; k < std::min(cnt[s], cap); k++) o[k] = ids[row[k]];
+    }
   }
   return SPH_OK;
 }
