@@ -58,8 +58,9 @@ __device__ __forceinline__ double rsq<double>(double x) { return rsqrt_f64(x); }
 
 // 1 / r of an FP64 near pair; 0 at r = 0 and where the square of r is denormal
 // (r < 1.5e-154), which the seed of the reciprocal square root takes for 0
+// (told by the exponent, off the FP64 pipe)
 __device__ __forceinline__ double near_inverse(double r2) {
-  return r2 >= 2.2250738585072014e-308 ? rsqrt_f64(r2) : 0.0;
+  return (unsigned)__double2hiint(r2) - 0x00100000u < 0x7fe00000u ? rsqrt_f64(r2) : 0.0;
 }
 
 // One side of an FP64 pair inside its softening range, r2 < h2, inv = 1 / r
@@ -68,9 +69,7 @@ __device__ __forceinline__ double near_inverse(double r2) {
 // cost several times the FP64 instructions (60,000 particles with 24
 // neighbours: diagonal tiles 622 -> 274 us, the rest 3,695 -> 3,143).
 __device__ __forceinline__ void spline_inside(double r2, double inv, double h2, double &g, double &p) {
-  // an infinite range, which a caller may give, stands at the largest number:
-  // no force and no potential, as divisions by it would give
-  const double ih = rsqrt_f64(fmin(h2, 1.7976931348623157e308)), ih2 = ih * ih, u2 = r2 * ih2, u = r2 * inv * ih;
+  const double ih = rsqrt_f64(h2), ih2 = ih * ih, u2 = r2 * ih2, u = r2 * inv * ih;
   if (u < 0.5) {
     g = fma(u2, fma(32.0, u, -38.4), 10.666666666667);
     p = fma(u2, fma(u2, fma(6.4, u, -9.6), 5.333333333333), -2.8);
@@ -897,10 +896,8 @@ __device__ __forceinline__ void sym_f64_item(long long item, int n, int nt, cons
           }
         }
         if (CHECK && __any_sync(0xffffffffu, near != 0u)) {
-          const int j = jb + ((l + s) & 31);  // the source at this lane now
-          // a range that is not a number or above 1.7e150 reaches the padding
-          // sources too: they have neither range nor force
-          if (j >= j_hi) near = 0u;
+          // the source at this lane now (near: a real one, softening_range)
+          const int j = jb + ((l + s) & 31);
 #pragma unroll
           for (int r = 0; r < kSym64R; r++) {
             if ((near >> r) & 1u) {
@@ -1100,7 +1097,7 @@ __global__ void k_pack_sources(int n, const double4 *pos, const double4 *vel, do
   if (i >= n) return;
   const double4 p = pos[i];
   src[i] = make_double4(p.x, p.y, p.z, vel[i].w);
-  h2[i] = p.w * p.w;
+  h2[i] = softening_range(p.w * p.w);
   if (clear) clear[i] = make_double4(0.0, 0.0, 0.0, 0.0);
 }
 
@@ -1129,7 +1126,7 @@ int launch_check_masses(int n, const double4 *vel, int *mass_mixed, cudaStream_t
 __global__ void k_range_sq(int n, const double *r, double *h2) {
   grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) h2[i] = r ? r[i] * r[i] : 0.0;
+  if (i < n) h2[i] = r ? softening_range(r[i] * r[i]) : 0.0;
 }
 
 }  // namespace sph

@@ -134,7 +134,7 @@ __global__ void k_grav_in(int n, const float4 *__restrict__ pos, const float4 *_
   if (i >= n) return;
   const float4 p = pos[i], v = vel[i];
   src[i] = make_double4(p.x, p.y, p.z, p.w);
-  h2[i] = v.w;
+  h2[i] = softening_range(v.w);
 }
 
 __global__ void k_grav_out(int n, const double4 *__restrict__ g, float4 *__restrict__ acc) {
