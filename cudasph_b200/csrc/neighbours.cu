@@ -1,15 +1,16 @@
 // neighbours.cu -- smoothing-length solve (dev_solve_range.cu:17-189) and
 // neighbour search (dev_find_ngb.cu:13-87) on the Morton tree.
 //
-// One warp owns one target particle at a time.  It walks the tree for that
-// particle alone: at every internal node each lane tests one child box
-// against the target's ball, a ballot keeps the children hit, and the leaves
-// come out in ascending index order.  In a visited leaf lane k tests
-// candidate k in FP32 (a conservative test on float copies of the positions)
-// and the survivors are staged, in order, in the warp's shared memory; every
-// 32 staged candidates go through the exact FP64 predicate ds2 < range^2 at
-// once, one per lane, and the hits are appended to the particle's list row
-// in ascending slot order and evaluated one per lane.
+// One warp owns one target particle, or four neighbouring ones in large sets.
+// It walks the tree once for the box of them: at every internal node each lane
+// tests one child box, a ballot keeps the children hit, and the cells of 8
+// particles come out in ascending index order.  The listed cells' particles are
+// tested against every target's ball in FP32 (a conservative test on float
+// copies of the positions).  Then, target by target, 32 survivors at a time go
+// through the exact FP64 predicate ds2 < range^2, one per lane, and the hits
+// are appended to the particle's list row in ascending slot order and evaluated
+// one per lane.  A target that is not covered by its group's list walks by
+// itself.
 //
 // This translation unit is compiled without FMA contraction: the h solve and
 // the predicate then perform the same IEEE operations, in the same order
@@ -24,13 +25,13 @@
 // 266, 262,144 (an oscillating star, 1.4 evaluations per particle) 1833 /
 // 1151, 1,048,576 4283 / 3769; from estimated ranges (3.7 evaluations, some
 // ranges holding half the star) 130,001 particles 69,300 / 3,760, 1,000,000
-// 61,000 / 13,200.  A uniform steady set with 1.00 evaluations per particle
-// is the one that loses: 2,000,003 particles 5485 / 6111 (from estimates
-// 21,300 / 22,200).  The kernel is bound by instruction issue (73 % of the
+// 61,000 / 13,200; a uniform steady set with 1.00 evaluations per particle,
+// 2,000,003 particles, 6095 / 5860 (6605 before a group's targets were stepped
+// together).  The kernel is bound by instruction issue (73 % of the
 // cycles at 262,144, about 2,700 instructions per particle; FP64 pipe 24 %,
 // XU 18 %), so what helps is fewer instructions: cells of 8 particles instead
 // of leaves of 32 with walks shared by a group (5,400 -> 3,100), the group's
-// candidate pass (2,600), and occupancy.  Loading the next candidates ahead
+// candidate pass (2,600), the steps of four targets at once, and occupancy.  Loading the next candidates ahead
 // of their test, or the next records ahead of their evaluation, cost 5 - 9 %
 // (registers).
 #include "common.cuh"
@@ -84,9 +85,27 @@ struct Query {
   float lo[3], hi[3], r2, c2;
 };
 
+// one evaluation of a range
+struct Eval {
+  double sf, sg;   // smooth count and its derivative sum
+  double dmax;     // largest d2 inside the range
+  int count;       // particles inside the range
+  bool sliver;     // some candidate in [w^2, w^2 (1 + 2^-40))
+  bool many;       // given up: more than a.ordered batches
+};
+
+// the first evaluations of a group's targets (none are kept of a single one:
+// 32 bytes more per warp, and the compiler spills three times as much)
+template <int G>
+struct FirstEvals {
+  Eval first[G];
+};
+template <>
+struct FirstEvals<1> {};
+
 // shared memory of one warp
 template <int G>
-struct WarpSmem {
+struct WarpSmem : FirstEvals<G> {
   alignas(16) double term[64];        // a batch's terms of the two sums, interleaved
   unsigned mask[kMaxLevels];          // the walk: per level the children still to visit ...
   int node[kMaxLevels];               // ... of this node
@@ -457,15 +476,6 @@ __device__ __forceinline__ void count_terms(double u, double &ig, double &digdh)
   }
 }
 
-// one evaluation of a range
-struct Eval {
-  double sf, sg;   // smooth count and its derivative sum
-  double dmax;     // largest d2 inside the range
-  int count;       // particles inside the range
-  bool sliver;     // some candidate in [w^2, w^2 (1 + 2^-40))
-  bool many;       // given up: more than a.ordered batches
-};
-
 // One walk at range w: writes the list row and, when `sums`, evaluates
 // f = sum ig and its derivative over it (dev_solve_range.cu:55-87).
 // The sums run in list order -- ascending index, the order of the CPU loop --
@@ -550,6 +560,22 @@ __device__ __forceinline__ Eval eval_range(const SolveArgs &a, Smem &sm, int s, 
   if (total < 0) return eval_visited<SUMS>(a, sm, s, w, nlist, exact);
   Coded src{total, 0};
   return eval_over<SUMS>(a, sm, s, p, w, exact, src);
+}
+
+// Whether the row written at w_eval is the list of the range w as well.
+__device__ __forceinline__ bool same_list(const Eval &e, double w_eval, double w) {
+  const double w2 = __dmul_rn(w, w);
+  return w == w_eval || (w < w_eval && e.dmax < w2) ||
+         (w > w_eval && !e.sliver && w2 < __dmul_rn(w_eval, w_eval) * (1.0 + 0x1p-40));
+}
+
+// A particle's results, by one lane.
+__device__ __forceinline__ void store_result(const SolveArgs &a, int s, double w, int count, int nev) {
+  if (!(w > 0)) count = 0;  // stored as no range
+  if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
+  a.pos[s].w = (w > 0) ? w : 0.0;
+  a.n_ngb[s] = count;
+  if (a.nevals) a.nevals[s] = nev;
 }
 
 // The two sums of a range far too large, in FP32 over every particle of the
@@ -669,22 +695,14 @@ __device__ __forceinline__ bool solve_round(const SolveArgs &a, Smem &sm, int s,
     __syncwarp();
     if (lane_id() == 0) solve_advance(it, e.sf, e.sg, a);
     __syncwarp();
-    const double w = it.w, wf2 = __dmul_rn(w, w);
-    listed = w == w_eval || (w < w_eval && e.dmax < wf2) ||
-             (w > w_eval && !e.sliver && wf2 < __dmul_rn(w_eval, w_eval) * (1.0 + 0x1p-40));
+    listed = same_list(e, w_eval, it.w);
     if (sm.nlist < 0 && it.phase != kDone) return false;  // a smaller range may find a list
   }
   const double w = it.w;
   if (!listed)
     count = eval_range<false>(a, sm, s, p, w, fabs(w) <= sm.w_list ? sm.nlist : -1, fabs(w) <= sm.bound ? total : -1,
                               false).count;
-  if (!(w > 0)) count = 0;  // stored as no range
-  if (lane_id() == 0) {
-    if (count > a.cap) raise_flag(a.flags, SPH_FLAG_NGB_OVERFLOW);
-    a.pos[s].w = (w > 0) ? w : 0.0;
-    a.n_ngb[s] = count;
-    if (a.nevals) a.nevals[s] = it.nev;
-  }
+  if (lane_id() == 0) store_result(a, s, w, count, it.nev);
   return true;
 }
 
@@ -781,17 +799,11 @@ struct Group {
       test_candidates(a, sm, mine, [&](int j) { return ldg(a.t.pf + j); });
     }
   }
-  // target t, at iteration `it` (lane 0's): its candidates as codes; their
-  // number, or -1 when they do not fit
-  __device__ __forceinline__ int stage(WarpSmem<G> &sm, int t, const RangeIter &it, double slack) {
+  // target t's candidates as codes; their number, or -1 when they do not fit
+  __device__ __forceinline__ int stage(WarpSmem<G> &sm, int t) {
     const int lane = (int)lane_id(), nlist = sm.nlist;
     int total = 0;
     __syncwarp();  // the previous target's codes are read
-    if (lane == 0) {
-      sm.it = it;
-      sm.bound = fabs(it.w) * slack;
-    }
-    __syncwarp();
     if (nlist < 0) return -1;
     for (int r = 0; r < kRounds && r * 128 < nlist; r++) {
       unsigned m = sm.hits[t][r][lane];
@@ -816,7 +828,11 @@ struct Group {
   }
 };
 
-// The first round.  A group with a target left goes on a queue for
+// The first round.  Several targets are evaluated one after the other and then
+// stepped at once, a lane each (one by one: 2,000,003 particles, steady, 6.6 ms
+// instead of 5.9, 1,048,576 3.87 / 3.62; a single target gains nothing and
+// loses registers, 2,049 particles 25.5 / 29 us); those that want more go
+// through the round's other evaluations.  A group with a target left goes on a queue for
 // k_solve_more, its targets' states by their slots: in one kernel the later
 // rounds' code would cost the first one registers and with them resident
 // warps (steady solve of 2,000,003 particles 6.9 ms instead of 6.1).
@@ -831,12 +847,53 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(cons
   if (g.count <= 0) return;
   g.template open<false>(a, sm, (1u << g.count) - 1u, kSlack);
   unsigned todo = 0u;
-  for (int t = 0; t < g.count; t++) {
-    const int s = g.first + t;
-    const int total = g.stage(sm, t, start_iter(a.pos[s].w), kSlack);
-    if (!solve_round<true>(a, sm, s, total)) {
-      todo |= 1u << t;
+  if constexpr (G == 1) {
+    const int s = g.first;
+    const RangeIter it = start_iter(a.pos[s].w);
+    if (lane_id() == 0) {
+      sm.it = it;
+      sm.bound = fabs(it.w) * kSlack;
+    }
+    if (!solve_round<true>(a, sm, s, g.stage(sm, 0))) {
+      todo = 1u;
       if (lane_id() == 0) a.save[s] = sm.it;
+    }
+  } else {
+    for (int t = 0; t < g.count; t++) {
+      const int s = g.first + t;
+      const double4 p = a.pos[s];
+      if (!(p.w > 0)) continue;
+      const Eval e = eval_range<true>(a, sm, s, p, p.w, sm.nlist, g.stage(sm, t), false);
+      if (lane_id() == 0) sm.first[t] = e;
+    }
+    __syncwarp();
+    const int lane = (int)lane_id(), mine = g.first + lane;
+    RangeIter it;
+    double w0 = 0;
+    bool more = false;
+    if (lane < g.count) {  // lane t steps target t
+      w0 = a.pos[mine].w;
+      const Eval e = sm.first[lane % G];
+      it = start_iter(w0);
+      if (w0 > 0 && !e.many) solve_advance(it, e.sf, e.sg, a);
+      more = it.phase != kDone || (w0 > 0 && !same_list(e, w0, it.w));
+      if (!more) store_result(a, mine, it.w, w0 > 0 ? e.count : 0, it.nev);
+    }
+    for (unsigned left = __ballot_sync(kFull, more); left != 0u; left &= left - 1u) {
+      const int t = __ffs(left) - 1, s = g.first + t;
+      __syncwarp();
+      if (lane == t) {
+        sm.it = it;
+        sm.bound = w0 * kSlack;
+      }
+      __syncwarp();
+      // whether its next evaluation, or its list, can be had in this round
+      const bool here =
+          sm.it.phase == kDone || (!sm.first[t].many && sm.nlist >= 0 && fabs(sm.it.w) <= sm.bound);
+      if (!here || !solve_round<true>(a, sm, s, g.stage(sm, t))) {
+        todo |= 1u << t;
+        if (lane == 0) a.save[s] = sm.it;
+      }
     }
   }
   if (todo != 0u && lane_id() == 0) a.queue[atomicAdd(a.queued, 1)] = make_int2(g.first, (int)todo);
@@ -870,7 +927,12 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kMoreBlocks) k_solve_more(cons
       for (unsigned m = todo; m != 0u; m &= m - 1u) {
         const int t = __ffs(m) - 1;
         const int s = g.first + t;
-        const int total = g.stage(sm, t, a.save[s], kSlackMore);
+        __syncwarp();
+        if (lane_id() == 0) {
+          sm.it = a.save[s];
+          sm.bound = fabs(sm.it.w) * kSlackMore;
+        }
+        const int total = g.stage(sm, t);
         if (solve_round<false>(a, sm, s, total)) todo &= ~(1u << t);
         else if (lane_id() == 0) a.save[s] = sm.it;
       }
@@ -894,7 +956,7 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_find_ngb(const _
   for (int t = 0; t < g.count; t++) {
     const int s = g.first + t;
     const double4 p = a.pos[s];
-    const int total = g.stage(sm, t, start_iter(p.w), 1.0);
+    const int total = g.stage(sm, t);
     int count = 0;
     if (p.w > 0) count = eval_range<false>(a, sm, s, p, p.w, sm.nlist, total, false).count;
     if (lane_id() == 0) {
