@@ -37,24 +37,17 @@ constexpr int kGThreads = 128;
 
 
 // reference spline softening polynomials, sph_grav_kernel.cu:53-61
-template <class R>
-__device__ __forceinline__ void spline_poly(R u, R u2, R &gacc, R &gpot) {
-  const R u3 = u2 * u;
-  if (u < (R)0.5) {
-    gacc = (R)10.666666666667 + u2 * ((R)32.0 * u - (R)38.4);
-    gpot = (R)(-2.8) + u2 * ((R)5.333333333333 + u2 * ((R)6.4 * u - (R)9.6));
+__device__ __forceinline__ void spline_poly(float u, float u2, float &gacc, float &gpot) {
+  const float u3 = u2 * u;
+  if (u < 0.5f) {
+    gacc = 10.666666666667f + u2 * (32.0f * u - 38.4f);
+    gpot = -2.8f + u2 * (5.333333333333f + u2 * (6.4f * u - 9.6f));
   } else {
-    gacc = (R)21.333333333333 - (R)48.0 * u + (R)38.4 * u2 - (R)10.666666666667 * u3 - (R)0.066666666667 / u3;
-    gpot = (R)(-3.2) + (R)0.066666666667 / u + u2 * ((R)10.666666666667 + u * ((R)(-16.0) + u * ((R)9.6 - (R)2.133333333333 * u)));
+    gacc = 21.333333333333f - 48.0f * u + 38.4f * u2 - 10.666666666667f * u3 - 0.066666666667f / u3;
+    gpot = -3.2f + 0.066666666667f / u +
+           u2 * (10.666666666667f + u * (-16.0f + u * (9.6f - 2.133333333333f * u)));
   }
 }
-
-template <class R>
-__device__ __forceinline__ R rsq(R x);
-template <>
-__device__ __forceinline__ float rsq<float>(float x) { return rsqrt_f32(x); }
-template <>
-__device__ __forceinline__ double rsq<double>(double x) { return rsqrt_f64(x); }
 
 // 1 / r of an FP64 near pair; 0 at r = 0 and where the square of r is denormal
 // (r < 1.5e-154), which the seed of the reciprocal square root takes for 0
@@ -85,26 +78,26 @@ __device__ __forceinline__ void spline_inside(double r2, double inv, double h2, 
 // The near-field pair of the mixed spline mode (r < max(range_i, range_j)),
 // bodyBodyInteraction's else-branch, sph_grav_kernel.cu:40-106.
 // dx = x_j - x_i; accumulates acceleration into a (a += contribution).
-template <class R>
-__device__ __noinline__ void spline_near(R dx, R dy, R dz, R r2, R mj, R hi2, R hj2, R &ax, R &ay, R &az, R &pot) {
-  R inv = r2 > 0 ? rsq<R>(r2) : (R)0;
-  R s3h = (R)0.5 * mj * inv * inv * inv;
-  R g;
+__device__ __noinline__ void spline_near(float dx, float dy, float dz, float r2, float mj, float hi2, float hj2,
+                                         float &ax, float &ay, float &az, float &pot) {
+  const float inv = r2 > 0 ? rsqrt_f32(r2) : 0.f;
+  const float s3h = 0.5f * mj * inv * inv * inv;
+  float g;
   if (r2 < hi2) {
-    const R u2 = r2 / hi2, h = sqrt(hi2), u = sqrt(u2);
-    R ga, gp;
-    spline_poly<R>(u, u2, ga, gp);
-    g = (R)0.5 * mj * ga / (hi2 * h);
+    const float u2 = r2 / hi2, h = sqrt(hi2), u = sqrt(u2);
+    float ga, gp;
+    spline_poly(u, u2, ga, gp);
+    g = 0.5f * mj * ga / (hi2 * h);
     pot += mj * gp / h;
   } else {
     g = s3h;
     pot -= mj * inv;
   }
   if (r2 < hj2) {
-    const R u2 = r2 / hj2, h = sqrt(hj2), u = sqrt(u2);
-    R ga, gp;
-    spline_poly<R>(u, u2, ga, gp);
-    g += (R)0.5 * mj * ga / (hj2 * h);
+    const float u2 = r2 / hj2, h = sqrt(hj2), u = sqrt(u2);
+    float ga, gp;
+    spline_poly(u, u2, ga, gp);
+    g += 0.5f * mj * ga / (hj2 * h);
   } else {
     g += s3h;
   }
@@ -369,7 +362,7 @@ __global__ void __launch_bounds__(kGThreads) k_grav_f32(int n, const double4 *sr
               pp[r] -= s;
             }
           } else {
-            spline_near<float>(dx, dy, dz, r2, q.w, hi2[r], hj2, px[r], py[r], pz[r], pp[r]);
+            spline_near(dx, dy, dz, r2, q.w, hi2[r], hj2, px[r], py[r], pz[r], pp[r]);
           }
         }
       }
@@ -546,8 +539,8 @@ __global__ void __launch_bounds__(kGThreads, 7)
 // All sums meet by atomics in an output cleared beforehand, so the order of
 // the FP64 additions, not their values, varies between runs.
 //
-// Equal masses (UNI): when every particle has the same mass m (a flag the
-// source-packing kernel computes on the device every step), the mass factors
+// Equal masses (UNI): when every particle has the same mass m (a device word
+// made by k_check_masses after masses were set), the mass factors
 // out of both sums -- a_i = m sum_j d / s^3, a_j = -m sum_i d / s^3,
 // phi = -m sum 1/s -- and is applied once per batch partial (FP64) instead
 // of per pair: 16 packed instructions per two pairs instead of 18, the same
@@ -1012,7 +1005,9 @@ static GravPlan grav_plan(int n, int soft_mode, int precision, int rank, int wor
   GravPlan g;
   g.nt = (n + kSymTile - 1) / kSymTile;
   g.chunk = g.nt >= 2 ? sym_chunk(g.nt) : 1;
-  const bool sym = soft_mode == SPH_SOFT_PLUMMER;  // the spline kernels are one-sided over all pairs
+  // spline softening is one-sided over all pairs here; launch_gravity puts the
+  // symmetric items in its place for a single FP64 rank
+  const bool sym = soft_mode == SPH_SOFT_PLUMMER;
   // FP64: R = 2 particles per thread; mixed Plummer: one packed i-pair per
   // thread (measured fastest at N = 1M: 68 registers, more resident warps to
   // cover the MUFU latency); mixed spline: R = 4
@@ -1029,7 +1024,9 @@ static GravPlan grav_plan(int n, int soft_mode, int precision, int rank, int wor
 // softening) and of the symmetric work items into `out`: the element-wise sum
 // of the shards' outputs is the whole sum.  `cleared`: the caller has zeroed
 // `out` on the stream.  FP64 spline softening on one rank takes the symmetric
-// tiles as well.
+// tiles as well; the shares of several ranks (cudasph_gravity_plan) are still
+// one-sided (60,000 particles, 24 neighbours: a half 3.8 ms, a quarter 2.0, the
+// whole on one rank 3.1).
 // Slices whose sums meet in a cluster: all that sets of one tile are cut into
 // but those of 1,024 particles, 32 by their size (FP64, us, by atomics / folded:
 // 100 particles 11.6 / 9.1, 1,000 11.6 / 11.4, 1,024 10.4 / 11.4, spline 1,000

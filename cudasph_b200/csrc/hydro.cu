@@ -198,7 +198,8 @@ __global__ void k_pressure(int n, double4 *hyd, int eos_mode, double gamma, unsi
 // |div| / (|div| + |curl| + 1e-4 c / h) -- computed once per particle with
 // the same operations the pair formula applies to them, and 1 / m, so the
 // pair loop gathers one record {c, P / rho^2, B, 1 / m} per neighbour instead
-// of hyd and dd and computes neither square root nor division per pair.
+// of hyd and dd, with no square root and one division per pair in compression
+// (by c_i + c_j, art_visc_pre).
 // dots (null: none): cleared for the loop's sums.
 __global__ void k_hydro_prep(int n, const double4 *pos, const double4 *vel, const double4 *hyd, const double4 *dd,
                              double gamma, double4 *aux, double4 *dots) {
@@ -255,8 +256,8 @@ __global__ void __launch_bounds__(128, 4) k_hydro(HydroArgs a) {
   const double prho2 = (hi4.x > 0) ? hi4.y / (hi4.x * hi4.x) : 0;
   const double h2 = hh * hh, h5 = h2 * h2 * hh;
   const double psi_i = a.use_psi ? di.w : 0;
-  // per-particle reciprocals and factors: the pair loop divides only by the
-  // neighbour's mass (and, in compression, by ds and c_i + c_j)
+  // per-particle reciprocals and factors: the pair loop divides only in
+  // compression, by c_i + c_j
   const double ihh = 1.0 / hh, ih5 = 1.0 / h5;
   const double gi = (prho2 * di.z + 0.5 * psi_i) / h2;  // grad-h term of the force
   const double ei = prho2 * di.z / h2;                   // grad-h term of du/dt

@@ -160,8 +160,8 @@ __global__ void k_morton(int n, const double4 *pos, const double *x, const doubl
 //
 // Before, a pass was a histogram, a scan in one block and a scatter with four
 // block barriers per 256 keys: 25 - 45 us a pass at every size.  Whole
-// sort, us, before / now: 2,049 keys 134 / 34, 16,384 184 / 73, 262,144 207 /
-// 104, 1,048,576 353 / 183, 2,000,003 656 / 340.
+// sort, us, before / now: 16,384 keys 184 / 73, 262,144 207 / 104, 1,048,576
+// 353 / 183, 2,000,003 656 / 340.
 // ---------------------------------------------------------------------------
 constexpr int kRadixItems = 8;  // keys per thread
 constexpr int kTileSmall = 256 * kRadixItems, kTileLarge = 512 * kRadixItems;
