@@ -26,6 +26,7 @@ from __future__ import annotations
 
 import ctypes as C
 import threading
+from collections import deque
 
 import numpy as np
 import torch
@@ -41,20 +42,32 @@ ROW = {k: i for i, k in enumerate(STATE)}
 class _Budget:
     """Bytes of device memory that the states of a context may still take."""
 
-    def __init__(self, left: int):
-        self.left = left
-        self.lock = threading.Lock()
+    def __init__(self, size: int):
+        self._left = size
+        self._given = deque()
+        self._lock = threading.Lock()
+
+    def _gather(self):
+        while self._given:
+            self._left += self._given.popleft()
 
     def take(self, size: int) -> bool:
-        with self.lock:
-            fits = size <= self.left
+        with self._lock:
+            self._gather()
+            fits = size <= self._left
             if fits:
-                self.left -= size
+                self._left -= size
             return fits
 
     def give(self, size: int):
-        with self.lock:
-            self.left += size
+        # without the lock: the garbage collector may free a state inside take()
+        self._given.append(size)
+
+    @property
+    def left(self) -> int:
+        with self._lock:
+            self._gather()
+            return self._left
 
 
 class _State:

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from cudasph_b200.autograd import _checked
+from cudasph_b200.autograd import _Budget, _checked, _State
 
 N = 7
 
@@ -38,3 +38,16 @@ def test_accepted_forms():
     assert _checked(N, **_inputs(v0=torch.zeros(N, 3, 1)))[1].shape == (N, 3, 1)
     assert x.shape == v.shape == (N, 3) and x[1, 0] == 4 and u.shape == (N,) and u[3] == 3
     assert set(f) == {"range"} and f["range"].shape == (N,)
+
+
+def test_budget_of_the_states():
+    b = _Budget(200)
+    rows = torch.zeros(2, 10, dtype=torch.float64)  # 160 bytes
+    first = _State(rows, 0.0, 0.0, b)
+    second = _State(rows, 0.0, 0.0, b)
+    assert first.held == 160 and second.held == 0 and b.left == 40
+    del second
+    assert b.left == 40
+    with b._lock:  # freed by the garbage collector while a state is being made
+        del first
+    assert b.left == 200 and b.take(200) and not b.take(1)
