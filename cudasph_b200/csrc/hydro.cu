@@ -57,7 +57,11 @@ __device__ __forceinline__ DensityKernels density_kernels(double u, double iu) {
 // bound by the FP64 pipe (density) and by L1 and the atomics (hydro), where
 // the shuffles at the end count (1,048,576 particles, density / hydro, ms, 2,
 // 4, 8, 16 lanes and one: 0.74 / 1.70, 0.77 / 1.61, 0.86 / 1.79, 1.08 / 2.22,
-// 0.84 / 1.78).
+// 0.84 / 1.78).  Between (us, 2, 4, 8, 16 lanes): density of 8,192 particles 27,
+// 19, 17, 17, of 16,384 30, 23, 24, 25, of 65,536 67, 61, 64, 74, of 262,144
+// 202, 205, 228, 285; hydro 40, 28, 28, 30, then 46, 43, 43, 48, 132, 119, 122,
+// 142, and 439, 418, 455, 556: the line lies where 16 lanes are no longer the
+// best for hydro; density loses up to 8 us just above it.
 constexpr int kSubSmall = 16, kSmallSet = 8192;
 constexpr int kSubDensity = 2, kSubHydro = 4;
 
