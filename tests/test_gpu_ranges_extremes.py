@@ -121,3 +121,35 @@ def test_solve_far_from_the_origin(n):
             r_o, _, _ = O.solve_range(x, y, z, np.asarray(ic["range"])[order], O.make_params(n_target=50.0))
             assert np.mean(r[order] == r_o) >= 0.999
     assert ms[1] < 10 * ms[0]
+
+
+@pytest.mark.parametrize("wide,rel_err", [(1.0, 1e-3), (1.02, 1e-3), (0.9, 1e-10)])
+def test_groups_of_four_solve_as_single_targets(wide, rel_err):
+    """Four targets to a warp and one (a shard of half the set takes the latter)
+    give the same ranges, counts and evaluations, also with targets of no range,
+    of ranges that are not a number, infinite, tiny and huge among the four."""
+    from cudasph_b200.sharded import ShardedSimulation
+    from cudasph_b200.simulation import Simulation, make_params
+    n = 90_003
+    ic = ics.polytrope(n, n_ngb=50, seed=5)
+    rs = np.random.default_rng(5)
+    r = np.asarray(ic["range"]) * wide
+    for value in (0.0, np.nan, -0.1, np.inf, 1e-12, 3.0):
+        r[rs.integers(0, n, 5 if value in (np.inf, 3.0) else 500)] = value
+    ic["range"] = r
+    par = make_params(n_target=50.0, eos_mode=0, soft_mode=1, eps=0.01, rel_err=rel_err)
+    with Simulation(ic, par) as sim:
+        sim.sort_bodies()
+        sim.CUDA_solve_range()
+        order, want = sim.order(), (sim.get("range"), sim.n_ngb(), sim.solve_evals())
+        status = sim.device_status()
+    for rank in range(2):
+        with ShardedSimulation(ic, par, rank, 2) as half:
+            half.sort_bodies()
+            half.CUDA_solve_range()
+            assert np.array_equal(half.order(), order)
+            lo, hi = half.leaves()
+            own = order[lo * 32:min(hi * 32, n)]
+            for a, b in zip((half.get("range"), half.n_ngb(), half.solve_evals()), want):
+                assert np.array_equal(a[own], b[own])
+            assert half.device_status() & ~status == 0
