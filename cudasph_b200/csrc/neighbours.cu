@@ -31,9 +31,9 @@
 // cycles at 262,144, about 2,700 instructions per particle; FP64 pipe 24 %,
 // XU 18 %), so what helps is fewer instructions: cells of 8 particles instead
 // of leaves of 32 with walks shared by a group (5,400 -> 3,100), the group's
-// candidate pass (2,600), the steps of four targets at once, and occupancy.  Loading the next candidates ahead
-// of their test, or the next records ahead of their evaluation, cost 5 - 9 %
-// (registers).
+// candidate pass (2,600), the steps of four targets at once, one copy of the
+// evaluation, and occupancy.  Loading the next candidates ahead of their test,
+// or the next records ahead of their evaluation, cost 5 - 9 % (registers).
 #include "common.cuh"
 #include "divby.cuh"
 #include "sph_math.cuh"
@@ -94,18 +94,19 @@ struct Eval {
   bool many;       // given up: more than a.ordered batches
 };
 
-// the first evaluations of a group's targets (none are kept of a single one:
-// 32 bytes more per warp, and the compiler spills three times as much)
+// the iterations of a group's targets and their evaluations (not for a single
+// target: its kernel is shorter without, and spills less)
 template <int G>
-struct FirstEvals {
-  Eval first[G];
+struct GroupState {
+  RangeIter its[G];
+  Eval evals[G];
 };
 template <>
-struct FirstEvals<1> {};
+struct GroupState<1> {};
 
 // shared memory of one warp
 template <int G>
-struct WarpSmem : FirstEvals<G> {
+struct WarpSmem : GroupState<G> {
   alignas(16) double term[64];        // a batch's terms of the two sums, interleaved
   unsigned mask[kMaxLevels];          // the walk: per level the children still to visit ...
   int node[kMaxLevels];               // ... of this node
@@ -139,7 +140,7 @@ __device__ __forceinline__ Query make_ball(double x, double y, double z, double 
 // (ranges below about 2e-6 of the distance from the origin).  They are then
 // compared by differences taken in FP64 (100,000 particles of a star 1e5 and
 // 1e6 of its radii from the origin, steady solve, ms, with the rounded
-// coordinates / so: 3.41 / 0.42 and 50.0 / 0.69; at the origin 0.38).
+// coordinates / so: 3.41 / 0.36 and 50.0 / 0.57; at the origin 0.33).
 __device__ __forceinline__ bool far_out(const Query &q) { return q.c2 > 1.5f * q.r2; }
 
 __device__ __forceinline__ float dist2(float dx, float dy, float dz) { return fmaf(dz, dz, fmaf(dy, dy, dx * dx)); }
@@ -493,9 +494,7 @@ __device__ __forceinline__ Eval eval_over(const SolveArgs &a, Smem &sm, int s, c
   Eval e;
   e.count = 0;
   e.sliver = false;
-  // an infinite range, which a caller may start from, stands at the largest
-  // number: the quotients are 0 as they are for infinity
-  const double wd = fmin(w, 1.7976931348623157e308), iw = 1.0 / wd;
+  const double iw = 1.0 / w;
   double acc = 0, dmax = -1.0;
   int nb = 0, j;
   e.many = false;
@@ -520,7 +519,7 @@ __device__ __forceinline__ Eval eval_over(const SolveArgs &a, Smem &sm, int s, c
       e.sliver |= !hit && d2 < r2 * (1.0 + 0x1p-40);
       double tf = 0, tg = 0;
       if (hit) {
-        count_terms(div_by(2 * sqrt(d2), wd, iw), tf, tg);
+        count_terms(div_by(2 * sqrt(d2), w, iw), tf, tg);
         dmax = fmax(dmax, d2);
       }
       reinterpret_cast<double2 *>(sm.term)[lane] = make_double2(tf, -tg);
@@ -672,7 +671,12 @@ __device__ __forceinline__ bool solve_round(const SolveArgs &a, Smem &sm, int s,
   while (it.phase != kDone) {
     const double w_eval = it.w;
     if (fabs(w_eval) > sm.bound) return false;
-    const Eval e = eval_range<true>(a, sm, s, p, w_eval, fabs(w_eval) <= sm.w_list ? sm.nlist : -1, total, exact);
+    // an infinite range, which a caller may start from: all weights are those of u = 0
+    const bool infinite = isinf(w_eval);
+    if (FIRST && infinite) return false;
+    Eval e = {0.0, 0.0, -1.0, 0, false, false};
+    if (FIRST || !infinite)
+      e = eval_range<true>(a, sm, s, p, w_eval, fabs(w_eval) <= sm.w_list ? sm.nlist : -1, total, exact);
     if (FIRST && e.many) return false;
     if (!FIRST && e.many) {
       Rough r = rough_sums(a, sm, p, w_eval);
@@ -695,7 +699,7 @@ __device__ __forceinline__ bool solve_round(const SolveArgs &a, Smem &sm, int s,
     __syncwarp();
     if (lane_id() == 0) solve_advance(it, e.sf, e.sg, a);
     __syncwarp();
-    listed = same_list(e, w_eval, it.w);
+    listed = (FIRST || !infinite) && same_list(e, w_eval, it.w);
     if (sm.nlist < 0 && it.phase != kDone) return false;  // a smaller range may find a list
   }
   const double w = it.w;
@@ -778,14 +782,16 @@ struct Group {
       q.r2 = fmaxf(q.r2, __shfl_xor_sync(kFull, q.r2, o));
       w_list = fmax(w_list, __shfl_xor_sync(kFull, w_list, o));
     }
-    const int nlist = list_cells(a.t, sm, q);
+    // (far out, the later rounds' targets walk by themselves: a second pass over
+    // the candidates made their kernel's code so long that every set paid 5 %)
+    const int nlist = SAVED && far ? -1 : list_cells(a.t, sm, q);
     if (lane == 0) {
       sm.w_list = w_list;
       sm.nlist = nlist;
     }
     __syncwarp();
     if (nlist <= 0) return;
-    if (far) {
+    if (!SAVED && far) {
       const double4 o = a.pos[first];
       mine = make_ball(p.x - o.x, p.y - o.y, p.z - o.z, p.w * slack * kWiden);
       if (tt != t0) mine.c2 = -1.f;
@@ -828,11 +834,15 @@ struct Group {
   }
 };
 
-// The first round.  Several targets are evaluated one after the other and then
-// stepped at once, a lane each (one by one: 2,000,003 particles, steady, 6.6 ms
-// instead of 5.9, 1,048,576 3.87 / 3.62; a single target gains nothing and
-// loses registers, 2,049 particles 25.5 / 29 us); those that want more go
-// through the round's other evaluations.  A group with a target left goes on a queue for
+// The first round.  A group's targets are evaluated one after the other and
+// then take their steps of the iteration at once, a lane each (a step is some
+// 250 scalar instructions with divisions); those that want another evaluation
+// and stay within the candidates are evaluated again, with the same code: with a
+// second copy of it in the kernel the instruction cache was missed.  Solve, us,
+// step by step / at once: 2,000,003 particles, steady, 6600 / 5860, 1,048,576
+// 3900 / 3490, 262,144 with 1.2 evaluations each 1040 / 925, 211,797 with 1.3
+// 962 / 877.  A single target gains nothing and loses registers (2,049 particles
+// 25.5 / 29).  A group with a target left goes on a queue for
 // k_solve_more, its targets' states by their slots: in one kernel the later
 // rounds' code would cost the first one registers and with them resident
 // warps (steady solve of 2,000,003 particles 6.9 ms instead of 6.1).
@@ -859,41 +869,44 @@ __global__ void __launch_bounds__(kNgbWarps * 32, kNgbBlocks) k_solve_range(cons
       if (lane_id() == 0) a.save[s] = sm.it;
     }
   } else {
-    for (int t = 0; t < g.count; t++) {
-      const int s = g.first + t;
-      const double4 p = a.pos[s];
-      if (!(p.w > 0)) continue;
-      const Eval e = eval_range<true>(a, sm, s, p, p.w, sm.nlist, g.stage(sm, t), false);
-      if (lane_id() == 0) sm.first[t] = e;
-    }
-    __syncwarp();
+    // evaluations one after the other, then the steps at once, lane t target t's
     const int lane = (int)lane_id(), mine = g.first + lane;
-    RangeIter it;
-    double w0 = 0;
     bool more = false;
-    if (lane < g.count) {  // lane t steps target t
-      w0 = a.pos[mine].w;
-      const Eval e = sm.first[lane % G];
-      it = start_iter(w0);
-      if (w0 > 0 && !e.many) solve_advance(it, e.sf, e.sg, a);
-      more = it.phase != kDone || (w0 > 0 && !same_list(e, w0, it.w));
-      if (!more) store_result(a, mine, it.w, w0 > 0 ? e.count : 0, it.nev);
+    if (lane < g.count) {
+      const RangeIter it = start_iter(a.pos[mine].w);
+      sm.its[lane] = it;
+      more = it.phase != kDone;
+      if (!more) store_result(a, mine, 0.0, 0, 0);
     }
-    for (unsigned left = __ballot_sync(kFull, more); left != 0u; left &= left - 1u) {
-      const int t = __ffs(left) - 1, s = g.first + t;
-      __syncwarp();
-      if (lane == t) {
-        sm.it = it;
-        sm.bound = w0 * kSlack;
+    for (unsigned left = __ballot_sync(kFull, more); left != 0u; left = __ballot_sync(kFull, more)) {
+      for (unsigned m = left; m != 0u; m &= m - 1u) {
+        const int t = __ffs(m) - 1, s = g.first + t;
+        const double4 p = a.pos[s];
+        const int total = g.stage(sm, t);
+        const double w = sm.its[t].w;
+        Eval e = {0.0, 0.0, -1.0, 0, false, true};  // infinite: left to the later rounds
+        if (!isinf(w)) e = eval_range<true>(a, sm, s, p, w, sm.nlist, total, false);
+        if (lane == 0) sm.evals[t] = e;
       }
       __syncwarp();
-      // whether its next evaluation, or its list, can be had in this round
-      const bool here =
-          sm.it.phase == kDone || (!sm.first[t].many && sm.nlist >= 0 && fabs(sm.it.w) <= sm.bound);
-      if (!here || !solve_round<true>(a, sm, s, g.stage(sm, t))) {
-        todo |= 1u << t;
-        if (lane == 0) a.save[s] = sm.it;
+      bool later = false;
+      if (more) {
+        const Eval e = sm.evals[lane % G];
+        RangeIter it = sm.its[lane % G];
+        const double w = it.w;
+        if (!e.many) solve_advance(it, e.sf, e.sg, a);
+        if (it.phase == kDone && same_list(e, w, it.w)) {
+          store_result(a, mine, it.w, e.count, it.nev);
+          more = false;
+        } else {
+          // whether its next evaluation can be had in this round
+          later = it.phase == kDone || e.many || sm.nlist < 0 || fabs(it.w) > a.pos[mine].w * kSlack;
+          if (later) a.save[mine] = it;
+          else sm.its[lane % G] = it;
+          more = !later;
+        }
       }
+      todo |= __ballot_sync(kFull, later);
     }
   }
   if (todo != 0u && lane_id() == 0) a.queue[atomicAdd(a.queued, 1)] = make_int2(g.first, (int)todo);
